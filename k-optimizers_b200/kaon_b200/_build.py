@@ -3,7 +3,8 @@
     python -m kaon_b200._build [--force] [-v]     (from the directory that holds the package)
 
 Every .cu file is compiled to an object of its own (in parallel, only when it or a header changed) and
-the objects are linked into the shared library.
+the objects are linked into the shared library.  host_ext.cpp becomes the CPython module _kaon_host (the
+per-tensor host work of a step), against the installed torch's headers.
 -fmad=false: the kernels spell out every fused multiply-add the reference's torch ops perform and
 must not get any other.  The library has no torch dependency: it is loaded with ctypes.
 """
@@ -13,12 +14,15 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(PKG), "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(PKG, "libkaon_b200.so")
+HOST_SRC = os.path.join(CSRC, "host_ext.cpp")
+HOST_LIB = os.path.join(PKG, "_kaon_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-fmad=false",
@@ -41,10 +45,26 @@ def _obj(src: str) -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or _host_stale():
         return True
     t = os.path.getmtime(LIB)
     return any(os.path.getmtime(d) > t for d in sources() + headers())
+
+
+def _host_stale() -> bool:
+    return not os.path.exists(HOST_LIB) or os.path.getmtime(HOST_LIB) < os.path.getmtime(HOST_SRC)
+
+
+def _build_host(env: dict) -> None:
+    """The host module: torch's headers for the layout of a tensor object, its libraries for the symbols
+    (they are loaded by ``import torch`` before the module is)."""
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    subprocess.check_call(
+        ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+         *[f"-I{p}" for p in include_paths()], f"-I{sysconfig.get_paths()['include']}", HOST_SRC, "-o", HOST_LIB,
+         f"-L{libs}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", f"-Wl,-rpath,{libs}"], env=env)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -70,7 +90,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return obj
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        host = pool.submit(_build_host, env) if force or _host_stale() else None
         objs = list(pool.map(compile_one, sources()))
+        if host is not None:
+            host.result()
     subprocess.check_call([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "--shared", "-o", LIB, *objs],
                           env=env)
     return LIB

@@ -104,12 +104,32 @@ class GroupPlan:
                 if t is not None:
                     setattr(d, field, t.data_ptr())
                     self._keep.append(t)
+        self.states = states
         self.handle = C.c_void_p()
         with torch.cuda.device(self.device):
             L.check(lib.kaon_plan_create(C.byref(self.handle), optimizer_kind, _PARAM_DT[p0.dtype], mk,
                                          descs, self.n))
-        self._grad_ptrs: list[int] | None = None
-        self._grad_arr = (C.c_void_p * self.n)()
+        # where the weights were when the plan was built, and where the gradients were when their column was
+        # last uploaded (0: none, as in a fresh plan)
+        self._param_arr = (C.c_int64 * self.n)(*self.param_ptrs)
+        self.grad_arr = (C.c_int64 * self.n)()
+        self._param_addr, self.grad_addr = C.addressof(self._param_arr), C.addressof(self.grad_arr)
+
+    def refresh(self, stream: int) -> bool | None:
+        """The native form of ``set_grads`` for a step like the last one: True / False as there, None when
+        anything but the gradients' addresses changed (``set_grads`` then raises or its caller rebuilds)."""
+        mask = L.host().scan(self.params, self.states, self._param_addr, self.grad_addr)
+        if mask & L.SCAN_UNUSUAL:
+            return None
+        if mask & L.SCAN_CHANGED:
+            self._upload(stream)
+        return bool(mask & L.SCAN_ANY)
+
+    def _upload(self, stream: int) -> None:
+        rc = L.lib().kaon_plan_set_grads(self.handle, self.grad_arr, self.n, C.c_void_p(stream))
+        if rc:
+            C.memset(self.grad_addr, 0xFF, C.sizeof(self.grad_arr))   # what the device holds is not this
+            L.check(rc)
 
     def set_grads(self, stream: int) -> bool:
         """Refresh the gradient-pointer column; returns False when nothing has a gradient."""
@@ -125,12 +145,11 @@ class GroupPlan:
             if g.dtype != dt or not g.is_contiguous():
                 raise NotImplementedError("kaon_b200: gradients must be contiguous and of the parameter's dtype")
             ptrs.append(g.data_ptr())
-        if ptrs != self._grad_ptrs:
-            arr = self._grad_arr
+        arr = self.grad_arr
+        if ptrs != list(arr):
             for i, v in enumerate(ptrs):
                 arr[i] = v
-            L.check(L.lib().kaon_plan_set_grads(self.handle, arr, self.n, C.c_void_p(stream)))
-            self._grad_ptrs = ptrs
+            self._upload(stream)
         return any(ptrs)
 
     def params_moved(self) -> bool:
@@ -189,6 +208,7 @@ class FusedStepMixin:
         self._plans: dict[tuple, GroupPlan] = {}
         self._plan_members: dict[tuple, tuple[int, ...]] = {}
         self._group_buckets: dict[int, tuple] = {}   # per group: (params list, its length, momentum dtype, buckets)
+        self._steady: dict[int, tuple] = {}          # per group: what its next step is checked against, and its plans
         self._t = 0                 # completed steps; the SR stream uses the 1-based index
         self.sr_seed: int | None = None  # None -> torch.initial_seed() at the first step
         self._mirrors: tuple[int, int, list[int]] | None = None
@@ -214,6 +234,7 @@ class FusedStepMixin:
         self._plans.clear()
         self._plan_members.clear()
         self._group_buckets.clear()
+        self._steady.clear()
 
     def _seed(self) -> int:
         if self.sr_seed is None:
@@ -233,8 +254,42 @@ class FusedStepMixin:
     def _momentum_dtype(self, group: dict[str, Any]) -> str | None:
         return group["momentum_dtype"]
 
-    def _group_plans(self, gi: int, group: dict[str, Any], state_of) -> list[GroupPlan]:
+    def _plans_to_step(self, gi: int, group: dict[str, Any]) -> list[tuple[GroupPlan, int]]:
+        """(plan, stream) of every plan of the group with a gradient to step, its gradient column refreshed.
+
+        A group that looks as it did at its last step (same list, state, momentum dtype; no gradient on a tensor
+        that has no state yet) needs one native pass per plan; everything else takes ``_group_plans``."""
+        params, md = group["params"], self._momentum_dtype(group)
+        steady = self._steady.get(gi)
+        if (steady is not None and steady[0] is params and steady[1] == len(params) and steady[2] == md
+                and steady[3] is self.state and steady[4] == len(self.state)
+                and (not steady[5] or L.host().grads_present(steady[5]) == 0)):
+            out = []
+            for pl in steady[6]:
+                stream = L.raw_stream(pl.device.index)
+                some = pl.refresh(stream)
+                if some is None:
+                    break
+                if some:
+                    out.append((pl, stream))
+            else:
+                return out
+        self._steady.pop(gi, None)
+        out = []
+        plans = self._group_plans(gi, group)
+        for pl in plans:
+            with torch.cuda.device(pl.device):
+                stream = L.raw_stream(pl.device.index)
+                if pl.set_grads(stream):
+                    out.append((pl, stream))
+        if plans:
+            rest = [p for p in params if p not in self.state or not self.state[p]]
+            self._steady[gi] = (params, len(params), md, self.state, len(self.state), rest, plans)
+        return out
+
+    def _group_plans(self, gi: int, group: dict[str, Any]) -> list[GroupPlan]:
         """Plans covering every parameter of the group that has a gradient now or had one before."""
+        state_of = lambda p: self.state[p]  # noqa: E731
         params = group["params"]
         fresh = active = False
         for p in params:
@@ -287,17 +342,14 @@ class FusedStepMixin:
             plans.append(pl)
         return plans
 
-    def _run_groups(self, state_of=None) -> None:
-        state_of = state_of or (lambda p: self.state[p])
+    def _run_groups(self) -> None:
         self._t += 1
         for gi, group in enumerate(self.param_groups):
             if self.before_group is not None:
                 self.before_group(gi)
-            for pl in self._group_plans(gi, group, state_of):
-                with torch.cuda.device(pl.device):
-                    stream = torch.cuda.current_stream(pl.device).cuda_stream
-                    if pl.set_grads(stream):
-                        self._launch(pl, group, self._t, stream)
+            for pl, stream in self._plans_to_step(gi, group):
+                with L.on_device(pl.device):
+                    self._launch(pl, group, self._t, stream)
             if self.after_group is not None:
                 self.after_group(gi)
 

@@ -4,8 +4,11 @@ There is no CPU fallback: if the library is missing or a call fails, this raises
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
+
+import torch
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libkaon_b200.so")
@@ -100,6 +103,37 @@ def lib() -> C.CDLL:
         if _lib.kaon_abi_version() != 2:
             raise KaonError("libkaon_b200.so ABI version mismatch")
     return _lib
+
+
+# what the host module's scan() reports (host_ext.cpp)
+SCAN_ANY, SCAN_CHANGED, SCAN_UNUSUAL = 1, 2, 4
+_host = None
+
+
+def host():
+    """The native per-tensor host work (csrc/host_ext.cpp); fail loudly if it has not been built."""
+    global _host
+    if _host is None:
+        try:
+            from . import _kaon_host
+        except ImportError as e:
+            raise KaonError(f"the host module _kaon_host cannot be loaded ({e}): build it with "
+                            "`python -m kaon_b200._build`") from e
+        _host = _kaon_host
+    return _host
+
+
+def raw_stream(index: int) -> int:
+    """The current stream of a device as the driver's handle."""
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)``, at no cost when the device is the current one."""
+    return _NO_GUARD if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def check(rc: int) -> None:

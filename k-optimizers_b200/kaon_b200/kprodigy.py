@@ -226,11 +226,8 @@ class KProdigy(FusedStepMixin, Optimizer):
             if factored and wd != 0 and not group["decouple"]:
                 raise NotImplementedError("kaon_b200.KProdigy: coupled weight decay (decouple=False) folds the weights "
                                           "into the gradient the factored statistics see; that combination is not built")
-            for pl in self._group_plans(gindex[id(group)], group, lambda p: self.state[p]):
-                with torch.cuda.device(pl.device):
-                    stream = torch.cuda.current_stream(pl.device).cuda_stream
-                    if not pl.set_grads(stream):
-                        continue
+            for pl, stream in self._plans_to_step(gindex[id(group)], group):
+                with L.on_device(pl.device):
                     seen = True
                     hp = L.KProdigyPass1(
                         beta1=beta1, beta2=beta2, beta3=beta3, d=d, alpha_s=alpha_s,
@@ -242,12 +239,14 @@ class KProdigy(FusedStepMixin, Optimizer):
                     launched.append((pl, group, stream))
                     if do_d:
                         # the reference's fp32 left fold over the tensors (src/kaon/kprodigy.py:451-455, 580-588)
-                        sums = np.ctypeslib.as_array(pl.sums)
-                        for i, p in enumerate(pl.params):
-                            if p.grad is None:
-                                continue
-                            delta_numerator = np.float32(delta_numerator + np.float32(sums[2 * i] * const))
-                            d_denom = np.float32(d_denom + sums[2 * i + 1])
+                        # (np.add.accumulate adds element after element in fp32; a tensor without a gradient adds nothing)
+                        sums = np.ctypeslib.as_array(pl.sums).reshape(-1, 2)
+                        has = np.ctypeslib.as_array(pl.grad_arr) != 0
+                        if not has.all():
+                            sums = sums[has]
+                        if len(sums):
+                            delta_numerator = np.add.accumulate(np.concatenate(([delta_numerator], sums[:, 0] * const)), dtype=np.float32)[-1]
+                            d_denom = np.add.accumulate(np.concatenate(([d_denom], sums[:, 1])), dtype=np.float32)[-1]
         if self._shard_group is not None and should_update_d and lr > 0.0:
             import torch.distributed as dist
             dev = self.param_groups[0]["params"][0].device
@@ -271,10 +270,8 @@ class KProdigy(FusedStepMixin, Optimizer):
                     group["d_hat"] = d_hat
         # pass 2 keeps the dlr of the top of the step and takes d as just updated, like the reference
         for pl, group, stream in launched:
-            with torch.cuda.device(pl.device):
-                for p in pl.params:
-                    if p.grad is not None:
-                        self.state[p]["step"] += 1
+            with L.on_device(pl.device):
+                L.host().bump(pl.states, "step", pl.grad_addr)
                 wd = group["weight_decay"]
                 hp2 = L.KProdigyPass2(
                     d=d, dlr=dlr, eps=group["eps"],

@@ -145,7 +145,7 @@ class Nekaon(AutoLRMixin, Optimizer):
 
     def _all_momentum_tensors_have_grads(self) -> bool:
         for group in self.param_groups:
-            if not self._has_momentum(group):
+            if not self._has_momentum(group) or L.host().grads_present(group["params"]) == 2:
                 continue
             for p in group["params"]:
                 if p.grad is None and self.inner.state.get(p):
