@@ -1,0 +1,519 @@
+// COUNT and APPLY of the Adakaon family's factored tensors as launches of their own (rows a multiple of eight
+// elements; 4-bit blocks of 128).
+//
+// COUNT: the update chain and the momentum EMA, the kept count of the cautious mask and the row maxima int8 momentum
+// is scaled by.  APPLY: the chain again, momentum encoded and stored, weights written; the Nekaon removal of the
+// previous climb and the new climb ride on the same read and write of each weight (with weight decay the mask looks
+// at the weights after the removal, so then COUNT takes the climb out and APPLY finds the weights without it).
+//
+// Bound by instruction issue, so the work is arranged for few instructions: a WARP claims a unit of 512..8192
+// consecutive elements and streams it, eight elements a lane and trip, with nothing shared between warps: no staging, no
+// barrier.  What is per row is one 16-byte table entry (left by FINAL), what is per column two vector loads that hit
+// L1; rows and columns advance by an addition, without a division.  Arithmetic is on packed pairs in the
+// reference's order of roundings; the mask is one saturating FMA an element; codes are rounded from the correctly
+// rounded quotient m' / scale (reciprocal and residual), so no vector needs a second look.
+#include <algorithm>
+#include <type_traits>
+#include <vector>
+
+#include "adakaon_dev.h"
+#include "kaon_host.h"
+#include "kaon_ops.cuh"
+#include "kaon_packed.cuh"
+
+namespace kaon {
+
+constexpr int SWT = 256;   // threads per CTA
+
+// The cautious mask of one element as a factor: x > 0 as 1.0f / 0.0f by one saturating FMA, (big, add) = (2^127, 0);
+// mask off: 1.0f always, (0, 1).  A NaN gives 0.  A product below 2^-127 (subnormal) would come out in between; it
+// does not occur where both factors are normal gradients and updates.
+__device__ __forceinline__ float mask1(float x, float big, float add) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(big), "f"(add));
+  return r;
+}
+
+__device__ __forceinline__ void philox8(const AdaDev& hp, uint32_t tensor, uint64_t q, uint32_t tag, uint32_t out[4]) {
+  uint32_t c0 = (uint32_t)q, c1 = tensor, c2 = hp.step, c3 = tag | ((uint32_t)(q >> 32) << 8);
+#pragma unroll
+  for (int r = 0; r < KAON_PHILOX_ROUNDS; ++r) {
+    const unsigned long long p0 = (unsigned long long)0xD2511F53u * c0;
+    const unsigned long long p1 = (unsigned long long)0xCD9E8D57u * c2;
+    const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ hp.rk0[r];
+    const uint32_t n2 = (uint32_t)(p0 >> 32) ^ c3 ^ hp.rk1[r];
+    c1 = (uint32_t)p1;
+    c3 = (uint32_t)p0;
+    c0 = n0;
+    c2 = n2;
+  }
+  out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
+}
+
+// Eight weights on their way through a step: bf16 stays packed between the writes (four registers, not eight).
+template <typename PT>
+struct W8;
+
+template <>
+struct W8<__nv_bfloat16> {
+  uint32_t w[4];
+  __device__ __forceinline__ void load(const void* p) {
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
+    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
+  }
+  __device__ __forceinline__ f32x2 pair(int j) const { return pack2(bf16lo(w[j]), bf16hi(w[j])); }
+  // stochastic rounding of w + D: 16 noise bits (the halves of nz[j], added by one dot-product instruction each) below
+  // the kept mantissa
+  __device__ __forceinline__ void add_sr(const f32x2 D[4], const uint32_t nz[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const f32x2 r = add2(pair(j), D[j]);
+      w[j] = prmt(__dp2a_lo(nz[j], 0x00000001u, __float_as_uint(r.x)), __dp2a_lo(nz[j], 0x00000100u, __float_as_uint(r.y)), 0x7632u);
+    }
+  }
+  __device__ __forceinline__ void set(int j, f32x2 v) { w[j] = prmt(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632u); }
+  __device__ __forceinline__ void store(void* p, const Peers* pr) const {
+    const uint4 q = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(p) = q;
+    mirror16(pr, p, q);
+  }
+};
+
+template <>
+struct W8<float> {
+  f32x2 v[4];
+  __device__ __forceinline__ void load(const void* p) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = pack2(a.x, a.y); v[1] = pack2(a.z, a.w); v[2] = pack2(b.x, b.y); v[3] = pack2(b.z, b.w);
+  }
+  __device__ __forceinline__ f32x2 pair(int j) const { return v[j]; }
+  __device__ __forceinline__ void set(int j, f32x2 x) { v[j] = x; }
+  __device__ __forceinline__ void store(void* p, const Peers* pr) const {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      unsigned char* a = reinterpret_cast<unsigned char*>(p) + 16 * h;
+      const uint4 q = make_uint4(__float_as_uint(v[2 * h].x), __float_as_uint(v[2 * h].y),
+                                 __float_as_uint(v[2 * h + 1].x), __float_as_uint(v[2 * h + 1].y));
+      *reinterpret_cast<uint4*>(a) = q;
+      mirror16(pr, a, q);
+    }
+  }
+};
+
+// x less a row mean (bits as the row table holds them; 0 without centralization), rounded to x's dtype
+template <typename T>
+__device__ __forceinline__ void center(const W8<T>& x, float mu, f32x2 out[4]) {
+  if constexpr (Elems<T>::IS_BF16) {
+    const uint32_t m2 = __float_as_uint(mu);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w = sub_bf16x2(x.w[j], m2);
+      out[j] = pack2(bf16lo(w), bf16hi(w));
+    }
+  } else {
+    const f32x2 M = pack2(mu, mu);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[j] = sub2(x.pair(j), M);
+  }
+}
+
+// The stored momentum of eight elements as it lies in memory.
+template <int MK> struct MRaw { };
+template <> struct MRaw<KAON_M_4BIT> { uint32_t w; float sc; };
+template <> struct MRaw<KAON_M_INT8> { uint2 w; };
+template <> struct MRaw<KAON_M_BF16> { W8<__nv_bfloat16> w; };
+template <> struct MRaw<KAON_M_F32> { W8<float> w; };
+
+// MUON (AdaMuon's factored tensors): the signal is the orthogonalised matrix (bf16, `pv.signal`), the chain carries no
+// momentum, and the mask compares with the raw gradient.  MS: the build with the Nekaon climb.
+template <typename PT, int MKP, bool MUON, bool MS, bool APPLY>
+__global__ void __launch_bounds__(SWT, 4) ada_sweep_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+  using E = Elems<PT>;
+  using ST = typename std::conditional<MUON, __nv_bfloat16, PT>::type;
+  using S = Elems<ST>;
+  constexpr int MK = MUON ? KAON_M_NONE : MKP;
+  constexpr bool CODED = MK == KAON_M_INT8 || MK == KAON_M_4BIT;
+  constexpr int MBITS = MK == KAON_M_4BIT ? 4 : MK == KAON_M_INT8 ? 8 : MK == KAON_M_BF16 ? 16 : MK == KAON_M_F32 ? 32 : 0;
+  if (on_reserved_sm(pv.sm_reserve)) return;
+  const int lane = threadIdx.x & 31;
+  // with weight decay the mask looks at the weights after the removal: COUNT writes them, APPLY finds them
+  const bool count_p = hp.has_wd && hp.cautious;
+  const bool rem_here = MS && hp.remove && (APPLY ? !count_p : count_p);
+  const bool need_p = APPLY || count_p;
+  auto claim = [&]() -> int {
+    int i = 0;
+    if (lane == 0) {
+      const unsigned st = *reinterpret_cast<volatile unsigned*>(pv.status);
+      i = st ? 0x7fffffff : (int)atomicAdd(pv.task_counter, 1u);
+    }
+    return i;   // lane 0's: broadcast where it is used, so that the atomic is in flight meanwhile
+  };
+  int cur = __shfl_sync(0xffffffffu, claim(), 0);
+  while (cur < pv.n_tasks) {
+    const int next = claim();
+    const Task t = pv.tasks[cur];
+    const unsigned char* gbase = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
+    if (gbase != nullptr) {
+      const DevTensor& d = pv.tensors[t.tensor];
+      const long long e0 = t.e0;
+      const int nvec = t.n >> 3;
+      const int nv = d.cols >> 3;                       // vectors per row
+      const unsigned char* sig = MUON ? reinterpret_cast<const unsigned char*>(pv.signal[t.tensor]) : gbase;
+      const unsigned char* sp = sig + (e0 + lane * 8) * S::BYTES;
+      const unsigned char* rawp = gbase + (e0 + lane * 8) * E::BYTES;
+      unsigned char* pp = reinterpret_cast<unsigned char*>(d.p) + (e0 + lane * 8) * E::BYTES;
+      unsigned char* mp = MBITS ? reinterpret_cast<unsigned char*>(d.m) + (e0 + lane * 8) * MBITS / 8 : nullptr;
+      float* msc = d.m_scale + (MK == KAON_M_4BIT ? (e0 >> 7) + (lane >> 4) : 0);
+      const float4 scal = __ldcg(reinterpret_cast<const float4*>(pv.aux + aux_scal(d)));
+      const float div = scal.y, rcp_div = scal.w;       // the clip divisor
+      const bool clipped = div != 1.0f;
+      float nrcp_denom = -1.0f;                         // minus the reciprocal of the kept share
+      if (APPLY && hp.cautious)
+        nrcp_denom = -__fdiv_rn(1.0f, fmaxf(__fdiv_rn((float)__ldcg(pv.kept + t.tensor), (float)d.numel), 1e-8f));
+      const float4* rowtab = reinterpret_cast<const float4*>(pv.aux + aux_rowtab(d));
+      const float* cfac = pv.aux + aux_cfac(d);
+      unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
+      uint64_t q = (uint64_t)(e0 >> 3) + (unsigned)lane;
+      // row and vector-in-row of this lane; a trip advances by 32 vectors
+      int row = t.row0, cv = (t.pad >> 3) + lane;
+      if (cv >= nv) { const int k = cv / nv; row += k; cv -= k * nv; }
+      const int adv_r = 32 / nv, adv_c = 32 - adv_r * nv;
+      f32x2 kept2 = pack2(0.0f, 0.0f);
+
+      W8<ST> gq;
+      W8<PT> P;
+      MRaw<MK> mq;
+      auto load = [&]() {
+        gq.load(sp);
+        if constexpr (MK == KAON_M_4BIT) { mq.w = *reinterpret_cast<const uint32_t*>(mp); mq.sc = *msc; }
+        else if constexpr (MK == KAON_M_INT8) mq.w = *reinterpret_cast<const uint2*>(mp);
+        else if constexpr (MK != KAON_M_NONE) mq.w.load(mp);
+        if (need_p) P.load(pp);
+      };
+      // a climb of eight elements (reference src/kaon/msam.py:222-230); `wild`: a momentum that decodes to NaN or
+      // infinity (a corrupt scale) keeps the reference's nan_to_num
+      auto climb8 = [&](const f32x2 M[4], float alpha, float bound, bool wild, f32x2 D[4]) {
+        const f32x2 A = pack2(alpha, alpha);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          f32x2 e = mul2(M[j], A);
+          if (wild) { if (e.x != e.x) e.x = 0.0f; if (e.y != e.y) e.y = 0.0f; }
+          D[j] = pack2(fminf(fmaxf(e.x, -bound), bound), fminf(fmaxf(e.y, -bound), bound));
+        }
+      };
+      auto add_noisy = [&](const f32x2 D[4], uint32_t tag) {
+        if constexpr (E::IS_BF16) {
+          uint32_t nz[4];
+          philox8(hp, d.tensor_id, q, tag, nz);
+          P.add_sr(D, nz);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) P.v[j] = add2(P.v[j], D[j]);
+        }
+      };
+      auto amax8 = [](const f32x2 M[4]) {
+        float a = max3f(fabsf(M[0].x), fabsf(M[0].y), fabsf(M[1].x));
+        a = max3f(a, fabsf(M[1].y), fabsf(M[2].x));
+        a = max3f(a, fabsf(M[2].y), fabsf(M[3].x));
+        return fmaxf(a, fabsf(M[3].y));
+      };
+      // the vector whose words are in gq, mq, P; `act`: this lane has one
+      auto trip = [&](const bool act) {
+        const float4 f = __ldcg(rowtab + row);   // {mean, r_i, int8: scale of the stored codes, -}
+        f32x2 CF[4], G[4], MO[4];
+        {
+          const float4 a = __ldg(reinterpret_cast<const float4*>(cfac) + 2 * cv), b = __ldg(reinterpret_cast<const float4*>(cfac) + 2 * cv + 1);
+          CF[0] = pack2(a.x, a.y); CF[1] = pack2(a.z, a.w); CF[2] = pack2(b.x, b.y); CF[3] = pack2(b.z, b.w);
+        }
+        center<ST>(gq, MUON ? 0.0f : f.x, G);
+        // ---- stored momentum ----
+        float sc_old = 1.0f;
+        if constexpr (MK == KAON_M_4BIT) {
+          sc_old = mq.sc;
+          const uint32_t wl = mq.w & 0x0F0F0F0Fu, wh = (mq.w >> 4) & 0x0F0F0F0Fu;
+          const f32x2 BIAS = pack2(-8388616.0f, -8388616.0f), SC = pack2(sc_old, sc_old);   // -(2^23 + 8)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            MO[j] = mul2(add2(pack2(__uint_as_float(prmt(wl, 0x4B000000u, 0x7540u | (uint32_t)j)),
+                                    __uint_as_float(prmt(wh, 0x4B000000u, 0x7540u | (uint32_t)j))), BIAS), SC);
+        } else if constexpr (MK == KAON_M_INT8) {
+          sc_old = f.z;
+          const uint32_t x0 = mq.w.x ^ 0x80808080u, x1 = mq.w.y ^ 0x80808080u;  // code + 128 in every byte
+          const f32x2 BIAS = pack2(-8388736.0f, -8388736.0f), SC = pack2(sc_old, sc_old);   // -(2^23 + 128)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t x = j < 2 ? x0 : x1;
+            const uint32_t b = (uint32_t)(2 * (j & 1));
+            MO[j] = mul2(add2(pack2(__uint_as_float(prmt(x, 0x4B000000u, 0x7540u | b)),
+                                    __uint_as_float(prmt(x, 0x4B000000u, 0x7540u | (b + 1u)))), BIAS), SC);
+          }
+        } else if constexpr (MK != KAON_M_NONE) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) MO[j] = mq.w.pair(j);
+        }
+        if (MS && rem_here) {   // take the previous climb out (the mirrors get the step's last write only)
+          f32x2 D[4];
+          climb8(MO, hp.a_remove, hp.b_remove, CODED ? !(fabsf(sc_old) <= 3.0e38f) : true, D);
+          add_noisy(D, KAON_TAG_REMOVE);
+          if (!APPLY && act) P.store(pp, nullptr);
+        }
+        // ---- u = ((g r) c) / div * scale (reference src/kaon/adakaon.py:885-888), m' = lerp(m, u) ----
+        f32x2 MN[4], F[4];
+        const f32x2 RF = pack2(f.y, f.y);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) MN[j] = mul2(mul2(G[j], RF), CF[j]);
+        if (clipped) {
+          const f32x2 DIVN = pack2(-div, -div), RCPD = pack2(rcp_div, rcp_div);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const f32x2 qq = mul2(MN[j], RCPD);
+            MN[j] = fma2(fma2(qq, DIVN, MN[j]), RCPD, qq);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          MN[j] = mul2(MN[j], pack2(hp.upd_scale, hp.upd_scale));
+          if constexpr (MK == KAON_M_BF16) {
+            const uint32_t ub = pack_bf16_rn(MN[j].x, MN[j].y);
+            MN[j] = pack2(bf16lo(ub), bf16hi(ub));
+          }
+        }
+        if constexpr (MK != KAON_M_NONE) {
+          if (hp.small_w1) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) MN[j] = fma2(pack2(hp.w1, hp.w1), sub2(MN[j], MO[j]), MO[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) MN[j] = fma2(pack2(hp.w1m1, hp.w1m1), sub2(MN[j], MO[j]), MN[j]);
+          }
+        }
+        if constexpr (MK == KAON_M_BF16) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t mb = pack_bf16_rn(MN[j].x, MN[j].y);
+            MN[j] = pack2(bf16lo(mb), bf16hi(mb));
+          }
+        }
+        // ---- delta = m' + (lr wd) p; the mask; APPLY: the update, negated: -(delta if kept else 0) / (kept / numel) ----
+#pragma unroll
+        for (int j = 0; j < 4; ++j) F[j] = MN[j];
+        if (hp.has_wd && need_p) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) F[j] = fma2(P.pair(j), pack2(hp.lrwd, hp.lrwd), F[j]);
+        }
+        if constexpr (MUON) {
+          W8<PT> rq;
+          rq.load(act ? rawp : gbase);
+          center<PT>(rq, f.x, G);
+        }
+        f32x2 K[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 X = mul2(F[j], G[j]);
+          K[j] = pack2(mask1(X.x, hp.mask_big, hp.mask_add), mask1(X.y, hp.mask_big, hp.mask_add));
+        }
+        if constexpr (!APPLY) {
+          const f32x2 k2 = add2(add2(K[0], K[1]), add2(K[2], K[3]));
+          if (act) kept2 = add2(kept2, k2);
+          if constexpr (MK == KAON_M_INT8) {
+            unsigned bits = act ? __float_as_uint(amax8(MN)) : 0u;
+            const int row_l0 = __shfl_sync(0xffffffffu, row, 0);
+            if (__all_sync(0xffffffffu, !act || row == row_l0)) {
+              bits = __reduce_max_sync(0xffffffffu, bits);
+              if (lane == 0) atomicMax(rowmax + row_l0, bits);
+            } else if (act) {
+              atomicMax(rowmax + row, bits);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) F[j] = mul2(mul2(F[j], K[j]), pack2(nrcp_denom, nrcp_denom));
+          // ---- store the new momentum; MO <- the momentum as stored ----
+          float sc = 1.0f;
+          if constexpr (CODED) {
+            if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(act ? amax8(MN) : 0.0f, lane), 1e-12f));
+            else sc = div127_exact(fmaxf(__uint_as_float(__ldcg(rowmax + row)), 1e-12f));
+            float inv;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
+            // R = rint(m'/sc) + magic, from the correctly rounded quotient; T = -rint(m'/sc)
+            constexpr float MAGIC = MK == KAON_M_4BIT ? 12582920.0f : 12582912.0f;   // 1.5 * 2^23 (+ 8)
+            const f32x2 INV = pack2(inv, inv), MG = pack2(MAGIC, MAGIC), NSC = pack2(-sc, -sc);
+            f32x2 T[4], R[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const f32x2 qq = mul2(MN[j], INV);
+              R[j] = add2(fma2(fma2(qq, NSC, MN[j]), INV, qq), MG);
+            }
+            if constexpr (MK == KAON_M_4BIT) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) T[j] = sub2(MG, R[j]);
+              // sum_k (8 - t_k) 16^k = 0x8888 - (t0 + 16 t1 + 256 t2 + 4096 t3), exact in fp32; adding 2^23 leaves it
+              // in the low 16 mantissa bits
+              const f32x2 K256 = pack2(256.0f, 256.0f);
+              const f32x2 Xl = fma2(T[1], K256, T[0]), Yl = fma2(T[3], K256, T[2]);
+              const float lo4 = __fsub_rn(8423560.0f, __fmaf_rn(Xl.y, 16.0f, Xl.x));
+              const float hi4 = __fsub_rn(8423560.0f, __fmaf_rn(Yl.y, 16.0f, Yl.x));
+              if (act) {
+                stg_u32(mp, prmt(__float_as_uint(lo4), __float_as_uint(hi4), 0x5410u));
+                if ((lane & 15) == 0) stg_f32(msc, sc);
+              }
+            } else {
+              if (MS && hp.climb) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) T[j] = sub2(MG, R[j]);
+              }
+              if (act) {  // the low byte of every R is the code in two's complement
+                const uint32_t w0 = prmt(prmt(__float_as_uint(R[0].x), __float_as_uint(R[0].y), 0x0040u),
+                                         prmt(__float_as_uint(R[1].x), __float_as_uint(R[1].y), 0x0040u), 0x5410u);
+                const uint32_t w1 = prmt(prmt(__float_as_uint(R[2].x), __float_as_uint(R[2].y), 0x0040u),
+                                         prmt(__float_as_uint(R[3].x), __float_as_uint(R[3].y), 0x0040u), 0x5410u);
+                *reinterpret_cast<uint2*>(mp) = make_uint2(w0, w1);
+                if (cv == 0) msc[row] = sc;
+              }
+            }
+            if (MS && hp.climb) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) MO[j] = mul2(T[j], NSC);
+            }
+          } else if constexpr (MK != KAON_M_NONE) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { MO[j] = MN[j]; mq.w.set(j, MN[j]); }
+            if (act) mq.w.store(mp, nullptr);
+          }
+          // ---- weights: p <- round(p - update), then the climb from the momentum as stored ----
+          if constexpr (E::IS_BF16) {
+            if (hp.sr) {
+              add_noisy(F, KAON_TAG_UPDATE);
+            } else if (hp.kahan) {
+              unsigned char* she = reinterpret_cast<unsigned char*>(d.shift) + q * 16;
+              W8<PT> SH;
+              if (act) SH.load(she); else SH.load(d.shift);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                f32x2 p = P.pair(j), sv = SH.pair(j);
+                kahan_step(p.x, sv.x, -F[j].x);
+                kahan_step(p.y, sv.y, -F[j].y);
+                P.set(j, p);
+                SH.set(j, sv);
+              }
+              if (act) SH.store(she, nullptr);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint32_t fb = pack_bf16_rn(F[j].x, F[j].y);
+                const f32x2 s = add2(P.pair(j), pack2(bf16lo(fb), bf16hi(fb)));
+                P.w[j] = pack_bf16_rn(s.x, s.y);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) P.v[j] = add2(P.v[j], F[j]);
+          }
+          if (MS && hp.climb) {
+            f32x2 D[4];
+            climb8(MO, hp.a_climb, hp.b_climb, CODED ? !(sc <= 3.0e38f) : true, D);
+            add_noisy(D, KAON_TAG_CLIMB);
+          }
+          if (act) P.store(pp, &pv.peers);
+        }
+      };
+      auto advance = [&]() {
+        sp += 256 * S::BYTES;
+        rawp += 256 * E::BYTES;
+        pp += 256 * E::BYTES;
+        if constexpr (MBITS > 0) mp += 32 * MBITS;
+        if constexpr (MK == KAON_M_4BIT) msc += 2;
+        q += 32;
+        row += adv_r;
+        cv += adv_c;
+        if (cv >= nv) { cv -= nv; ++row; }
+      };
+      const int full = nvec >> 5;
+      for (int k = 0; k < full; ++k) {
+        load();
+        trip(true);
+        advance();
+      }
+      if (nvec & 31) {   // a tensor's last vectors
+        const bool act = lane < (nvec & 31);
+        if (act) load();
+        else {   // (in bounds, and of no consequence)
+          row = t.row0; cv = 0;
+          sp = sig; pp = reinterpret_cast<unsigned char*>(d.p);
+          if constexpr (MBITS > 0) mp = reinterpret_cast<unsigned char*>(d.m);
+          if constexpr (MK == KAON_M_4BIT) msc = d.m_scale;
+          load();
+        }
+        trip(act);
+      }
+      if constexpr (!APPLY) {
+        const unsigned kept = __reduce_add_sync(0xffffffffu, (unsigned)(kept2.x + kept2.y + 0.5f));
+        if (lane == 0 && kept) atomicAdd(pv.kept + t.tensor, kept);
+      }
+    }
+    cur = __shfl_sync(0xffffffffu, next, 0);
+  }
+}
+
+// ----------------------------------------------------------------------------- host
+
+typedef void (*SweepKernel)(PlanView, AdaDev);
+
+template <typename PT, bool MS, bool APPLY>
+static SweepKernel pick_sweep_pt(int mk) {
+  switch (mk) {
+    case KAON_M_F32: return ada_sweep_kernel<PT, KAON_M_F32, false, MS, APPLY>;
+    case KAON_M_BF16: return ada_sweep_kernel<PT, KAON_M_BF16, false, MS, APPLY>;
+    case KAON_M_INT8: return ada_sweep_kernel<PT, KAON_M_INT8, false, MS, APPLY>;
+    case KAON_M_4BIT: return ada_sweep_kernel<PT, KAON_M_4BIT, false, MS, APPLY>;
+    case KAON_M_NONE: return ada_sweep_kernel<PT, KAON_M_NONE, false, false, APPLY>;
+    default: return nullptr;
+  }
+}
+template <bool APPLY>
+static SweepKernel pick_sweep(int pdt, int mk, bool muon, bool ms) {
+  const bool bf = pdt == KAON_DT_BF16;
+  if (muon) return bf ? ada_sweep_kernel<__nv_bfloat16, KAON_M_NONE, true, false, APPLY> : ada_sweep_kernel<float, KAON_M_NONE, true, false, APPLY>;
+  if (ms) return bf ? pick_sweep_pt<__nv_bfloat16, true, APPLY>(mk) : pick_sweep_pt<float, true, APPLY>(mk);
+  return bf ? pick_sweep_pt<__nv_bfloat16, false, APPLY>(mk) : pick_sweep_pt<float, false, APPLY>(mk);
+}
+
+// The units of the tensors marked in `elig`: as large as leaves each warp of the machine a dozen (a warp's time per
+// unit is then small beside the launch's), at most 8192 elements, where the fetches at a unit's head cost little.
+void sweep_units(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out) {
+  long long total = 0;
+  for (int i = 0; i < pl->n_tensors; ++i) if (elig[i]) total += pl->h_tensors[i].numel;
+  long long u = 8192;
+  while (u > 512 && total / u < 12ll * pl->sm_count * 32) u /= 2;
+  for (int i = 0; i < pl->n_tensors; ++i) {
+    if (!elig[i]) continue;
+    const DevTensor& t = pl->h_tensors[i];
+    for (long long e = 0; e < t.numel; e += u)
+      out.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(u, t.numel - e), (int)(e / t.cols), 0, (int)(e % t.cols)});
+  }
+}
+
+// The COUNT (where something is counted) and APPLY launches over the plan's units; `base` carries the plan's
+// pointers (and AdaMuon's signal column).
+int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s) {
+  const bool muon = pl->optimizer == KAON_OPT_ADAMUON;
+  const bool ms = hp.remove || hp.climb;
+  PlanView va = base;
+  va.tasks = pl->d_tasks_apply2;
+  va.n_tasks = pl->n_tasks_apply2;
+  const int want = (pl->n_tasks_apply2 + SWT / 32 - 1) / (SWT / 32), most = pl->sm_count * 4;
+  const int grid = base.sm_reserve ? most : std::max(1, std::min(want, most));
+  if (hp.cautious || hp.int8) {
+    va.task_counter = base.counters2 + 1;
+    pick_sweep<false>(pl->param_dtype, pl->momentum_kind, muon, ms)<<<grid, SWT, 0, s>>>(va, hp);
+    KAON_CUDA(cudaGetLastError());
+    pl->launches += 1;
+  }
+  va.task_counter = base.counters2 + 2;
+  pick_sweep<true>(pl->param_dtype, pl->momentum_kind, muon, ms)<<<grid, SWT, 0, s>>>(va, hp);
+  KAON_CUDA(cudaGetLastError());
+  pl->launches += 1;
+  return KAON_OK;
+}
+
+}  // namespace kaon

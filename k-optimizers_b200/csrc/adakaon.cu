@@ -17,10 +17,9 @@
 // Each of STATS / COUNT / APPLY exists twice.  The staged form above (ada_stats, ada_rows) handles any
 // shape.  The streaming form (ada_stats_stream, ada_stream) needs rows that are a multiple of 8
 // elements and reads gradient, momentum and weights straight from global memory, with what is per row
-// or per column fetched from the scratch in L2; it has no barrier in its loops.  When every factored
-// tensor of a plan streams, COUNT and APPLY leave this kernel altogether and run as launches of
-// adakaon_apply_kernel (256-thread CTAs, four per SM, one bulk-copied flat item each), ordered by the
-// stream instead of by completion counters.
+// or per column fetched from the scratch in L2; it has no barrier in its loops.  COUNT and APPLY of the tensors
+// that stream leave this kernel and run as launches of their own (ada_sweep.cu), ordered by the stream instead of
+// by completion counters.
 #include <map>
 #include <vector>
 #include <mutex>
@@ -897,6 +896,7 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
       scal[0] = rowmean;
       scal[1] = fmaxf(__fdiv_rn(rms, hp.clip), 1.0f);
       scal[2] = rms;
+      scal[3] = __fdiv_rn(1.0f, scal[1]);
       sm.part_s[0] = rowmean;
     }
   }
@@ -904,7 +904,13 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
   if (last) {  // the whole CTA: r_i of every row, then release COUNT / APPLY
     const float rowmean = sm.part_s[0];
     float* rfac = pv.aux + aux_rfac(d);
-    for (int r = tid; r < d.rows; r += AT) rfac[r] = rsqrt_torch(__fdiv_rn(__ldcg(d.stat_a + r), rowmean));
+    float4* rowtab = reinterpret_cast<float4*>(pv.aux + aux_rowtab(d));
+    for (int r = tid; r < d.rows; r += AT) {
+      const float rf = rsqrt_torch(__fdiv_rn(__ldcg(d.stat_a + r), rowmean));
+      rfac[r] = rf;
+      const float mu = hp.gc ? __ldcg(pv.aux + aux_mean(d) + r) : 0.0f;
+      rowtab[r] = make_float4(pv.param_bf16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, rf, hp.int8 ? d.m_scale[r] : 1.0f, 0.0f);
+    }
     if (hp.int8) {  // int8 momentum: COUNT starts from zeroed row maxima; APPLY decodes with the old scales
       unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
       float* oldsc = pv.aux + aux_oldsc(d);
@@ -1901,620 +1907,6 @@ __global__ void __launch_bounds__(256) msam_axpy_kernel(PlanView pv, float alpha
   }
 }
 
-// ----------------------------------------------------------------------------- APPLY as its own kernel
-
-// When every factored tensor of the plan takes the streaming form, the APPLY stage leaves the
-// persistent kernel above and runs as a second launch built like the Lion kernel: 256-thread CTAs,
-// several per SM, each bringing one flat item of at most APPLY_CAP elements (gradient, weights,
-// momentum bytes) into shared memory with bulk copies while the other CTAs of the SM compute.  Stream
-// order replaces the completion counters: every COUNT item has finished when this kernel starts.
-// Items are flat runs (no row structure: what is per row or per column comes from the scratch in L2),
-// so the int8 row scales of the previous step are read from the copy COUNT set aside.
-constexpr int APPLY_CAP = 8192;
-constexpr int APPLY_THREADS = 256;
-
-// APPLY = false is the COUNT stage in the same form (kept count, int8 row maxima; no stores but those).
-// MUON (AdaMuon): the chain runs on the orthogonalised momentum (bf16, `pv.signal`) with no momentum of
-// its own, the cautious mask compares with the raw gradient, which is staged where the momentum bytes
-// go otherwise.
-template <typename PT, int MKP, bool APPLY, bool MUON>
-__global__ void __launch_bounds__(APPLY_THREADS, 4) adakaon_apply_kernel(PlanView pv, AdaDev hp) {
-  using E = Elems<PT>;
-  using S = Elems<typename std::conditional<MUON, __nv_bfloat16, PT>::type>;
-  constexpr int MK = MUON ? KAON_M_NONE : MKP;
-  constexpr int GB = 8 * E::BYTES;
-  constexpr int SB = 8 * S::BYTES;
-  constexpr int MB = MUON ? GB : MK == KAON_M_4BIT ? 4 : MK == KAON_M_INT8 ? 8 : MK == KAON_M_BF16 ? 16 : MK == KAON_M_F32 ? 32 : 0;
-  extern __shared__ __align__(128) unsigned char dyn[];
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ int next_s[2];
-  __shared__ unsigned red_s[APPLY_THREADS / 32];
-  const bool need_p = APPLY || hp.has_wd;
-  unsigned char* g_s = dyn;
-  unsigned char* p_s = dyn + (size_t)APPLY_CAP * E::BYTES;
-  unsigned char* m_s = dyn + (size_t)2 * APPLY_CAP * E::BYTES;
-  const int tid = threadIdx.x;
-  if (on_reserved_sm(pv.sm_reserve)) return;
-  auto claim_next = [&](int slot) {
-    if (tid == 0) {
-      const unsigned st = *reinterpret_cast<volatile unsigned*>(pv.status);
-      next_s[slot] = st ? 0x7fffffff : (int)atomicAdd(pv.task_counter, 1u);
-    }
-  };
-  if (tid == 0) mbar_init(&bar, 1);
-  claim_next(0);
-  __syncthreads();
-  unsigned parity = 0u;
-  int slot = 0;
-  int cur = next_s[0];
-  SrStream s_upd{Philox{hp.k0, hp.k1}, hp.step, KAON_TAG_UPDATE};
-  SrStream s_rem{Philox{hp.k0, hp.k1}, hp.step, KAON_TAG_REMOVE};
-  SrStream s_clb{Philox{hp.k0, hp.k1}, hp.step, KAON_TAG_CLIMB};
-  const bool sr = hp.sr != 0;
-  const bool gc = hp.gc != 0 && !MUON;
-  // AdaMuon with gradient centralization: the statistics run on the orthogonalised matrix, which is not
-  // centralised; the cautious mask compares with the CENTRALISED raw gradient (row means in the scratch)
-  const bool gcr = hp.gc != 0 && MUON;
-  while (cur < pv.n_tasks) {
-    claim_next(slot ^ 1);
-    const Task t = pv.tasks[cur];
-    const DevTensor d = pv.tensors[t.tensor];
-    const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
-    bool ok = g != nullptr;
-    const int n = t.n;
-    if (ok) {
-      const unsigned char* gsrc = MUON ? reinterpret_cast<const unsigned char*>(pv.signal[t.tensor]) + t.e0 * S::BYTES
-                                       : g + t.e0 * E::BYTES;
-      const unsigned char* msrc = MUON ? g + t.e0 * E::BYTES : m_ptr<MK>(d, t.e0);
-      const unsigned mbytes = MUON ? (unsigned)n * E::BYTES : m_bytes<MK>(n);
-      const unsigned char* psrc = reinterpret_cast<const unsigned char*>(d.p) + t.e0 * E::BYTES;
-      const unsigned ghead = stage_tail(g_s, gsrc, (unsigned)n * S::BYTES, tid);
-      const unsigned phead = need_p ? stage_tail(p_s, psrc, (unsigned)n * E::BYTES, tid) : 0u;
-      unsigned mhead = 0u;
-      if constexpr (MB > 0) mhead = stage_tail(m_s, msrc, mbytes, tid);
-      if (ghead + phead + mhead) {
-        if (tid == 0) {
-          fence_async_smem();
-          mbar_expect_tx(&bar, ghead + phead + mhead);
-          if (ghead) bulk_g2s(g_s, gsrc, ghead, &bar);
-          if (phead) bulk_g2s(p_s, psrc, phead, &bar);
-          if constexpr (MB > 0) { if (mhead) bulk_g2s(m_s, msrc, mhead, &bar); }
-        }
-        ok = mbar_wait(&bar, parity, pv.status, 15001u);
-        parity ^= 1u;
-      }
-    }
-    ok = __syncthreads_and(ok) != 0;
-    unsigned kept_local = 0;
-    if (ok) {
-      const int C = d.cols;
-      const long long row0 = t.e0 / C;
-      const int col0 = (int)(t.e0 - row0 * C);
-      const float* scal = pv.aux + aux_scal(d);
-      Chain ch;
-      ch.div = __ldcg(scal + 1);
-      ch.use_div = ch.div != 1.0f;
-      ch.rcp_div = __fdiv_rn(1.0f, ch.div);
-      float denom = 1.0f, rcp_denom = 1.0f;
-      if (APPLY && hp.cautious) {
-        const unsigned kept_t = __ldcg(pv.kept + t.tensor);
-        denom = fmaxf(__fdiv_rn((float)kept_t, (float)d.numel), 1e-8f);
-        rcp_denom = __fdiv_rn(1.0f, denom);
-      }
-      const float* cfac = pv.aux + aux_cfac(d);
-      const float* mean = pv.aux + aux_mean(d);
-      unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
-      const float* oldsc = pv.aux + aux_oldsc(d);
-      const float* rfac = pv.aux + aux_rfac(d);
-      unsigned char* pbase = reinterpret_cast<unsigned char*>(d.p) + t.e0 * E::BYTES;
-      const int nvec = n >> 3;
-      const int nvec_pad = (nvec + 31) & ~31;
-      // ---- fast path: bf16 weights, int8 / 4-bit momentum (or AdaMuon's chain, which carries none and takes
-      //      the orthogonalised matrix as its signal), stochastic-rounding write (or the COUNT stage), no Kahan buffer.  Same arithmetic as the general loop below, element for element, on packed
-      //      pairs (f32x2), with the cautious mask and the quantised codes gathered by byte permutes and
-      //      one exactness check per vector; the rare vectors that fail a check are redone the plain way. ----
-      constexpr bool FASTABLE = E::IS_BF16 && (MUON || MK == KAON_M_INT8 || MK == KAON_M_4BIT);
-      bool fast = false;
-      if constexpr (FASTABLE) fast = !hp.kahan && (!APPLY || sr);
-      if constexpr (FASTABLE) if (fast) {
-        const f32x2 DIVN = pack2(-ch.div, -ch.div), RCPD = pack2(ch.rcp_div, ch.rcp_div);
-        const f32x2 SCALE = pack2(hp.upd_scale, hp.upd_scale);
-        const f32x2 W1 = pack2(hp.w1, hp.w1), W1M1 = pack2(hp.w1m1, hp.w1m1);
-        const f32x2 LRWD = pack2(hp.lrwd, hp.lrwd);
-        const f32x2 DENN = pack2(-denom, -denom), RCPN = pack2(rcp_denom, rcp_denom);
-        const uint32_t* gsm = reinterpret_cast<const uint32_t*>(g_s);
-        const uint32_t* psm = reinterpret_cast<const uint32_t*>(p_s);
-        const long long blk0 = t.e0 >> 7;
-        const uint64_t q0 = (uint64_t)(t.e0 >> 3);
-        auto clamp2 = [](f32x2 e, float b) { return pack2(fminf(fmaxf(e.x, -b), b), fminf(fmaxf(e.y, -b), b)); };
-        // one stochastic-rounding write of eight weights held as four pairs: P <- trunc16(bits(P + D) + noise)
-        auto sr_write = [&](f32x2 P[4], const f32x2 D[4], const SrStream& stream, uint64_t q) {
-          uint32_t nz[4];
-          stream.draw8(d.tensor_id, q, nz);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const f32x2 r = add2(P[j], D[j]);
-            P[j] = pack2(__uint_as_float((__float_as_uint(r.x) + (nz[j] & 0xffffu)) & 0xFFFF0000u),
-                         __uint_as_float((__float_as_uint(r.y) + (nz[j] >> 16)) & 0xFFFF0000u));
-          }
-        };
-        auto trip = [&](const int v, auto guard_tag, auto small_tag) {
-          constexpr bool GUARD = decltype(guard_tag)::value;
-          constexpr bool SMALL_W1 = decltype(small_tag)::value;
-          const bool act = !GUARD || v < nvec;
-          const int vv = act ? v : 0;
-          const unsigned i = (unsigned)col0 + (unsigned)vv * 8u;
-          const int r = row_of(i, d);
-          const int row = (int)row0 + r;
-          const int col = (int)i - r * C;
-          const float rf = __ldcg(rfac + row);
-          const float4 c0v = __ldcg(reinterpret_cast<const float4*>(cfac + col));
-          const float4 c1v = __ldcg(reinterpret_cast<const float4*>(cfac + col + 4));
-          const uint4 gq = *reinterpret_cast<const uint4*>(gsm + (size_t)vv * 4);
-          uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
-          if (gc) {
-            const float mu = __ldcg(mean + row);
-            const uint32_t mu2 = pack_bf16_rn(mu, mu);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) gw[j] = sub_bf16x2(gw[j], mu2);
-          }
-          uint32_t mu2r = 0u;   // AdaMuon: the centralization mean of the raw gradient's row, two bf16 copies
-          if (MUON && gcr) {
-            const float mur = __ldcg(mean + row);
-            mu2r = pack_bf16_rn(mur, mur);
-          }
-          f32x2 P[4];
-          if (need_p) {
-            const uint4 pq = *reinterpret_cast<const uint4*>(psm + (size_t)vv * 4);
-            P[0] = pack2(bf16lo(pq.x), bf16hi(pq.x)); P[1] = pack2(bf16lo(pq.y), bf16hi(pq.y));
-            P[2] = pack2(bf16lo(pq.z), bf16hi(pq.z)); P[3] = pack2(bf16lo(pq.w), bf16hi(pq.w));
-          } else {
-            P[0] = P[1] = P[2] = P[3] = pack2(0.0f, 0.0f);
-          }
-          // ---- old momentum ----
-          f32x2 MO[4];
-          float sc_old;
-          if constexpr (MK == KAON_M_4BIT) {
-            sc_old = d.m_scale[blk0 + (vv >> 4)];
-            const uint32_t w = reinterpret_cast<const uint32_t*>(m_s)[vv];
-            const uint32_t wl = w & 0x0F0F0F0Fu, wh = (w >> 4) & 0x0F0F0F0Fu;
-            const f32x2 BIAS = pack2(-8388616.0f, -8388616.0f), SC = pack2(sc_old, sc_old);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              MO[j] = mul2(add2(pack2(__uint_as_float(prmt(wl, 0x4B000000u, 0x7540u | (uint32_t)j)),
-                                      __uint_as_float(prmt(wh, 0x4B000000u, 0x7540u | (uint32_t)j))), BIAS), SC);
-          } else if constexpr (MK == KAON_M_NONE) {
-            sc_old = 1.0f;
-            MO[0] = MO[1] = MO[2] = MO[3] = pack2(0.0f, 0.0f);
-          } else {
-            sc_old = APPLY ? __ldcg(oldsc + row) : d.m_scale[row];
-            const uint2 w = reinterpret_cast<const uint2*>(m_s)[vv];
-            const uint32_t x0 = w.x ^ 0x80808080u, x1 = w.y ^ 0x80808080u;  // code + 128 in every byte
-            const f32x2 BIAS = pack2(-8388736.0f, -8388736.0f), SC = pack2(sc_old, sc_old);  // -(2^23 + 128)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint32_t x = j < 2 ? x0 : x1;
-              const uint32_t b = (uint32_t)(2 * (j & 1));
-              MO[j] = mul2(add2(pack2(__uint_as_float(prmt(x, 0x4B000000u, 0x7540u | b)),
-                                      __uint_as_float(prmt(x, 0x4B000000u, 0x7540u | (b + 1u)))), BIAS), SC);
-            }
-          }
-          const uint64_t q = q0 + (uint64_t)vv;
-          // a momentum that decodes to NaN or infinity (a corrupt scale) keeps the reference's nan_to_num
-          const bool wild = !(fabsf(sc_old) <= 3.0e38f);
-          if (hp.remove && need_p) {
-            const f32x2 AR = pack2(hp.a_remove, hp.a_remove);
-            f32x2 Dr[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              f32x2 e = mul2(MO[j], AR);
-              if (wild) { if (e.x != e.x) e.x = 0.0f; if (e.y != e.y) e.y = 0.0f; }
-              Dr[j] = clamp2(e, hp.b_remove);
-            }
-            sr_write(P, Dr, s_rem, q);
-          }
-          // ---- update chain: u = ((g r) c) / divisor * scale; m' = lerp(m, u); delta = m' + (lr wd) p ----
-          // (a divisor of 1 and a zero weight decay go through the same operations: x/1 and fma(p, 0, m')
-          //  give x and m' back; a delta of -0 that becomes +0 is masked out or subtracted either way)
-          const f32x2 RF = pack2(rf, rf);
-          const f32x2 CF[4] = {pack2(c0v.x, c0v.y), pack2(c0v.z, c0v.w), pack2(c1v.x, c1v.y), pack2(c1v.z, c1v.w)};
-          f32x2 MN[4], DV[4];
-          float a[8];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const f32x2 G = pack2(bf16lo(gw[j]), bf16hi(gw[j]));
-            f32x2 U = mul2(mul2(G, RF), CF[j]);
-            const f32x2 qq = mul2(U, RCPD);
-            U = mul2(fma2(fma2(qq, DIVN, U), RCPD, qq), SCALE);
-            if constexpr (MK == KAON_M_NONE) {
-              MN[j] = U;  // no momentum of its own: delta = u
-            } else {
-              const f32x2 diff = sub2(U, MO[j]);
-              MN[j] = SMALL_W1 ? fma2(W1, diff, MO[j]) : fma2(W1M1, diff, U);
-            }
-            DV[j] = fma2(P[j], LRWD, MN[j]);
-            if constexpr (MUON) {  // the mask compares with the raw gradient, staged where the momentum goes otherwise
-              uint32_t rw = reinterpret_cast<const uint32_t*>(m_s)[(size_t)vv * 4 + j];
-              if (gcr) rw = sub_bf16x2(rw, mu2r);
-              unpack2(mul2(DV[j], pack2(bf16lo(rw), bf16hi(rw))), a[2 * j], a[2 * j + 1]);
-            } else {
-              unpack2(mul2(DV[j], G), a[2 * j], a[2 * j + 1]);
-            }
-          }
-          // ---- cautious mask: kept <=> delta * g > 0 (sign bits; a zero or underflowing product is rare
-          //      and decided by the comparison itself) ----
-          float amin = min3f(fabsf(a[0]), fabsf(a[1]), fabsf(a[2]));
-          amin = min3f(amin, fabsf(a[3]), fabsf(a[4]));
-          amin = min3f(amin, fabsf(a[5]), fabsf(a[6]));
-          amin = fminf(amin, fabsf(a[7]));
-          float amax = max3f(fabsf(MN[0].x), fabsf(MN[0].y), fabsf(MN[1].x));
-          amax = max3f(amax, fabsf(MN[1].y), fabsf(MN[2].x));
-          amax = max3f(amax, fabsf(MN[2].y), fabsf(MN[3].x));
-          amax = fmaxf(amax, fabsf(MN[3].y));
-          if constexpr (!APPLY) {
-            unsigned kept = 0;
-            if (amin > 0.0f) {
-              const uint32_t am_lo = prmt(prmt(__float_as_uint(a[0]), __float_as_uint(a[1]), 0x00FBu),
-                                          prmt(__float_as_uint(a[2]), __float_as_uint(a[3]), 0x00FBu), 0x5410u);
-              const uint32_t am_hi = prmt(prmt(__float_as_uint(a[4]), __float_as_uint(a[5]), 0x00FBu),
-                                          prmt(__float_as_uint(a[6]), __float_as_uint(a[7]), 0x00FBu), 0x5410u);
-              kept = 8u - (unsigned)__popc(am_lo & 0x01010101u) - (unsigned)__popc(am_hi & 0x01010101u);
-            } else {
-#pragma unroll
-              for (int k = 0; k < 8; ++k) kept += a[k] > 0.0f ? 1u : 0u;
-            }
-            if (act) kept_local += kept;
-            if constexpr (MK == KAON_M_INT8) {
-              unsigned bits = act ? __float_as_uint(amax) : 0u;
-              const int row_l0 = __shfl_sync(0xffffffffu, row, 0);
-              if (__all_sync(0xffffffffu, !act || row == row_l0)) {
-                bits = __reduce_max_sync(0xffffffffu, bits);
-                if ((tid & 31) == 0 && bits) atomicMax(rowmax + row_l0, bits);
-              } else if (act) {
-                atomicMax(rowmax + row, bits);
-              }
-            }
-            return;
-          } else {
-            // ---- the update: delta, or under the cautious mask (delta if kept else 0) / denom ----
-            f32x2 F[4];
-            if (hp.cautious) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const f32x2 qq = mul2(DV[j], RCPN);
-                const f32x2 f = fma2(fma2(qq, DENN, DV[j]), RCPN, qq);
-                // masked out where the product delta * g is negative (its sign bit spread over the word)
-                F[j] = pack2(__uint_as_float(__float_as_uint(f.x) & ~(uint32_t)((int)__float_as_uint(a[2 * j]) >> 31)),
-                             __uint_as_float(__float_as_uint(f.y) & ~(uint32_t)((int)__float_as_uint(a[2 * j + 1]) >> 31)));
-              }
-              if (!(amin > 0.0f)) {  // some product is zero: those elements are masked out as well
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  if (!(a[2 * j] > 0.0f)) F[j].x = 0.0f;
-                  if (!(a[2 * j + 1] > 0.0f)) F[j].y = 0.0f;
-                }
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) F[j] = DV[j];
-            }
-            // ---- quantise and store the new momentum; MD = the momentum as stored, decoded ----
-            f32x2 MD[4];
-            float sc = 1.0f;
-            if constexpr (MK == KAON_M_NONE) {
-              MD[0] = MD[1] = MD[2] = MD[3] = pack2(0.0f, 0.0f);
-            } else {
-            if constexpr (MK == KAON_M_4BIT) {
-              const float am = fmaxf(half_warp_max(act ? amax : 0.0f, tid), 1e-12f);
-              __syncwarp();  // every lane of the block has read the old scale before it is replaced
-              sc = div7_exact(am);
-            } else {
-              sc = div127_exact(fmaxf(__uint_as_float(__ldcg(rowmax + row)), 1e-12f));
-            }
-            float inv;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
-            const f32x2 INV = pack2(inv, inv), NSC = pack2(-sc, -sc);
-            // r = rint(n*inv) (+8) + magic in one rounding; T = -rint(n*inv); e = n*inv - rint(n*inv) exactly
-            constexpr float MAGIC = MK == KAON_M_4BIT ? 12582920.0f : 12582912.0f;
-            const f32x2 MG = pack2(MAGIC, MAGIC);
-            f32x2 T[4], R[4];
-            float e8[8];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              R[j] = fma2(MN[j], INV, MG);
-              T[j] = sub2(MG, R[j]);
-              unpack2(fma2(MN[j], INV, T[j]), e8[2 * j], e8[2 * j + 1]);
-              MD[j] = mul2(T[j], NSC);
-            }
-            float worst = max3f(fabsf(e8[0]), fabsf(e8[1]), fabsf(e8[2]));
-            worst = max3f(worst, fabsf(e8[3]), fabsf(e8[4]));
-            worst = max3f(worst, fabsf(e8[5]), fabsf(e8[6]));
-            worst = fmaxf(worst, fabsf(e8[7]));
-            uint32_t w0, w1 = 0u;
-            if constexpr (MK == KAON_M_4BIT) {
-              const f32x2 K256 = pack2(256.0f, 256.0f);
-              const f32x2 X = fma2(T[1], K256, T[0]), Y = fma2(T[3], K256, T[2]);
-              const float lo4 = __fsub_rn(8423560.0f, __fmaf_rn(X.y, 16.0f, X.x));
-              const float hi4 = __fsub_rn(8423560.0f, __fmaf_rn(Y.y, 16.0f, Y.x));
-              w0 = prmt(__float_as_uint(lo4), __float_as_uint(hi4), 0x5410u);
-            } else {  // the low byte of every r is the code in two's complement
-              w0 = prmt(prmt(__float_as_uint(R[0].x), __float_as_uint(R[0].y), 0x0040u),
-                        prmt(__float_as_uint(R[1].x), __float_as_uint(R[1].y), 0x0040u), 0x5410u);
-              w1 = prmt(prmt(__float_as_uint(R[2].x), __float_as_uint(R[2].y), 0x0040u),
-                        prmt(__float_as_uint(R[3].x), __float_as_uint(R[3].y), 0x0040u), 0x5410u);
-            }
-            // Rare: a product n*inv too close to a rounding boundary to trust the reciprocal (it is good to
-            // 2^-22: |n*inv - n/sc| < 127 * 2^-22 = 3e-5, 7 * 2^-22 for 4 bits), or a scale that is not
-            // finite: the codes of this vector again, by the true division.
-            if (worst > 0.5f - (MK == KAON_M_4BIT ? 1e-5f : 1e-4f) || !(sc <= 3.0e38f)) {
-              const float inv2 = __fdividef(1.0f, sc);
-              float n8[8], md8[8];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) unpack2(MN[j], n8[2 * j], n8[2 * j + 1]);
-              w0 = 0u; w1 = 0u;
-#pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                if constexpr (MK == KAON_M_4BIT) {
-                  const int qi = min(max((int)quant_round(n8[k], sc, inv2, 1e-4f), -7), 7);
-                  md8[k] = __fmul_rn((float)qi, sc);
-                  w0 |= (uint32_t)(qi + 8) << (4 * k);
-                } else {
-                  const int qi = min(max((int)quant_round(n8[k], sc, inv2, 1e-3f), -127), 127);
-                  md8[k] = __fmul_rn((float)qi, sc);
-                  const uint32_t byte = (uint32_t)(qi & 0xFF);
-                  if (k < 4) w0 |= byte << (8 * k); else w1 |= byte << (8 * (k - 4));
-                }
-              }
-#pragma unroll
-              for (int j = 0; j < 4; ++j) MD[j] = pack2(md8[2 * j], md8[2 * j + 1]);
-            }
-            if (act) {
-              if constexpr (MK == KAON_M_4BIT) {
-                stg_u32(reinterpret_cast<unsigned char*>(d.m) + (t.e0 >> 1) + (size_t)v * 4, w0);
-                if ((v & 15) == 0) stg_f32(d.m_scale + blk0 + (v >> 4), sc);
-              } else {
-                *reinterpret_cast<uint2*>(reinterpret_cast<unsigned char*>(d.m) + t.e0 + (size_t)v * 8) = make_uint2(w0, w1);
-                if (col == 0) d.m_scale[row] = sc;
-              }
-            }
-            }  // MK != NONE
-            // ---- weights: p <- SR(p - update), then the Nekaon climb from the momentum as stored ----
-#pragma unroll
-            for (int j = 0; j < 4; ++j) F[j] = pack2(-F[j].x, -F[j].y);
-            sr_write(P, F, s_upd, q);
-            if (hp.climb && MK != KAON_M_NONE) {
-              const f32x2 AC = pack2(hp.a_climb, hp.a_climb);
-              const bool wild2 = !(sc <= 3.0e38f);
-              f32x2 Dc[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                f32x2 e = mul2(MD[j], AC);
-                if (wild2) { if (e.x != e.x) e.x = 0.0f; if (e.y != e.y) e.y = 0.0f; }
-                Dc[j] = clamp2(e, hp.b_climb);
-              }
-              sr_write(P, Dc, s_clb, q);
-            }
-            if (act) {
-              const uint4 out = make_uint4(prmt(__float_as_uint(P[0].x), __float_as_uint(P[0].y), 0x7632u),
-                                           prmt(__float_as_uint(P[1].x), __float_as_uint(P[1].y), 0x7632u),
-                                           prmt(__float_as_uint(P[2].x), __float_as_uint(P[2].y), 0x7632u),
-                                           prmt(__float_as_uint(P[3].x), __float_as_uint(P[3].y), 0x7632u));
-              *reinterpret_cast<uint4*>(pbase + (size_t)v * 16) = out;
-              mirror16(&pv.peers, pbase + (size_t)v * 16, out);
-            }
-          }
-        };
-        const int nfull = nvec & ~31;
-        if (hp.small_w1) {
-          for (int v = tid; v < nfull; v += APPLY_THREADS) trip(v, std::false_type{}, std::true_type{});
-          if (nfull != nvec && tid < 32) trip(nfull + tid, std::true_type{}, std::true_type{});
-        } else {
-          for (int v = tid; v < nfull; v += APPLY_THREADS) trip(v, std::false_type{}, std::false_type{});
-          if (nfull != nvec && tid < 32) trip(nfull + tid, std::true_type{}, std::false_type{});
-        }
-      }
-      if (!fast)
-      for (int v = tid; v < nvec_pad; v += APPLY_THREADS) {
-        const bool act = v < nvec;
-        const int vv = act ? v : 0;
-        const unsigned i = (unsigned)col0 + (unsigned)vv * 8u;  // < APPLY_CAP + cols: row_of is exact
-        const int r = row_of(i, d);
-        const int row = (int)row0 + r;
-        const int col = (int)i - r * C;
-        float gv[8], mo[8], mn[8], pc[8], dl[8];
-        const float mu = (gc || gcr) ? __ldcg(mean + row) : 0.0f;
-        const float rf = __ldcg(rfac + row);
-        const float4 c0v = __ldcg(reinterpret_cast<const float4*>(cfac + col));
-        const float4 c1v = __ldcg(reinterpret_cast<const float4*>(cfac + col + 4));
-        const float cf[8] = {c0v.x, c0v.y, c0v.z, c0v.w, c1v.x, c1v.y, c1v.z, c1v.w};
-        S::load8(g_s + (size_t)vv * SB, gv);
-        float raw[8];
-        if (MUON) E::load8(m_s + (size_t)vv * GB, raw);
-        if (MUON && gcr) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) raw[k] = centered<PT>(raw[k], mu, true);
-        }
-        if (need_p) E::load8(p_s + (size_t)vv * GB, pc);
-        else {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) pc[k] = 0.0f;
-        }
-        if constexpr (MK == KAON_M_4BIT) {
-          decode8<MK>(m_s, vv, 8, d.m_scale[(t.e0 >> 7) + (vv >> 4)], mo);
-        } else if constexpr (MK == KAON_M_INT8) {
-          decode8<MK>(m_s, vv, 8, APPLY ? __ldcg(oldsc + row) : d.m_scale[row], mo);
-        } else if constexpr (MK == KAON_M_NONE) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) mo[k] = 0.0f;
-        } else {
-          decode8<MK>(m_s, vv, 8, 1.0f, mo);
-        }
-        if (hp.remove && need_p) {
-          uint32_t nz[4] = {0u, 0u, 0u, 0u};
-          if (E::IS_BF16) s_rem.draw8(d.tensor_id, (uint64_t)((t.e0 >> 3) + vv), nz);
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            pc[k] = write_step<PT>(pc[k], climb_e(mo[k], hp.a_remove, hp.b_remove), 1.0f, E::IS_BF16, noise_lane(nz, k));
-        }
-        if (gc) {
-#pragma unroll
-          for (int k = 0; k < 8; k += 2) {
-            const float x0 = __fsub_rn(gv[k], mu), x1 = __fsub_rn(gv[k + 1], mu);
-            if (E::IS_BF16) {
-              const uint32_t pk = pack_bf16_rn(x0, x1);
-              gv[k] = bf16lo(pk); gv[k + 1] = bf16hi(pk);
-            } else {
-              gv[k] = x0; gv[k + 1] = x1;
-            }
-          }
-        }
-        unsigned kept = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float u = update_of(gv[k], rf, cf[k], ch, hp.upd_scale);
-          mn[k] = ema_of<MK>(mo[k], u, hp);
-          const float dv = hp.has_wd ? __fmaf_rn(pc[k], hp.lrwd, mn[k]) : mn[k];
-          dl[k] = dv;
-          if (__fmul_rn(dv, MUON ? raw[k] : gv[k]) > 0.0f) kept |= 1u << k;
-        }
-        if constexpr (!APPLY) {
-          if (act) kept_local += __popc(kept);
-          if constexpr (MK == KAON_M_INT8) {
-            float a = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) a = fmaxf(a, fabsf(mn[k]));
-            unsigned bits = act ? __float_as_uint(a) : 0u;
-            const int row_l0 = __shfl_sync(0xffffffffu, row, 0);
-            if (__all_sync(0xffffffffu, !act || row == row_l0)) {
-              bits = __reduce_max_sync(0xffffffffu, bits);
-              if ((tid & 31) == 0 && bits) atomicMax(rowmax + row_l0, bits);
-            } else if (act) {
-              atomicMax(rowmax + row, bits);
-            }
-          }
-          continue;
-        }
-        float md[8];  // the momentum as stored (decoded), for the Nekaon climb
-        if constexpr (MK == KAON_M_4BIT) {
-          float a = 0.0f;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) a = fmaxf(a, act ? fabsf(mn[k]) : 0.0f);
-          a = fmaxf(group_max(a, 16), 1e-12f);
-          __syncwarp();  // every lane of the block has read the old scale before it is replaced
-          const float sc = __fdiv_rn(a, 7.0f);
-          const float inv = __fdividef(1.0f, sc);
-          uint32_t word = 0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float q = quant_round(mn[k], sc, inv, 1e-4f);
-            const int qi = min(max((int)q, -7), 7);
-            md[k] = __fmul_rn((float)qi, sc);
-            word |= (uint32_t)(qi + 8) << (4 * k);
-          }
-          if (act) {
-            *reinterpret_cast<uint32_t*>((unsigned char*)d.m + (t.e0 >> 1) + (size_t)v * 4) = word;
-            if ((v & 15) == 0) d.m_scale[(t.e0 >> 7) + (v >> 4)] = sc;
-          }
-        } else if constexpr (MK == KAON_M_INT8) {
-          const float sc = __fdiv_rn(fmaxf(__uint_as_float(__ldcg(rowmax + row)), 1e-12f), 127.0f);
-          const float inv = __fdividef(1.0f, sc);
-          uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int qi = min(max((int)quant_round(mn[k], sc, inv, 1e-3f), -127), 127);
-            md[k] = __fmul_rn((float)qi, sc);
-            const uint32_t byte = (uint32_t)(qi & 0xFF);
-            if (k < 4) w0 |= byte << (8 * k); else w1 |= byte << (8 * (k - 4));
-          }
-          if (act) {
-            *reinterpret_cast<uint2*>((unsigned char*)d.m + t.e0 + (size_t)v * 8) = make_uint2(w0, w1);
-            if (col == 0) d.m_scale[row] = sc;
-          }
-        } else if constexpr (MK == KAON_M_BF16 || MK == KAON_M_F32) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) md[k] = mn[k];
-          if (act) {
-            if constexpr (MK == KAON_M_BF16) store8<__nv_bfloat16>((unsigned char*)d.m + t.e0 * 2 + (size_t)v * 16, 8, mn, nullptr);
-            else store8<float>((unsigned char*)d.m + t.e0 * 4 + (size_t)v * 32, 8, mn, nullptr);
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) md[k] = 0.0f;
-        }
-        if (act) {
-          if (E::IS_BF16 && hp.kahan) {
-            unsigned char* she = reinterpret_cast<unsigned char*>(d.shift) + (size_t)t.e0 * 2 + (size_t)v * 16;
-            float sh[8];
-            load8_guard<__nv_bfloat16>(she, 8, sh);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              float f = dl[k];
-              if (hp.cautious) f = ((kept >> k) & 1u) ? div_shared(f, denom, rcp_denom) : 0.0f;
-              kahan_step(pc[k], sh[k], f);
-            }
-            store8<__nv_bfloat16>(she, 8, sh, nullptr);
-          } else {
-            uint32_t nz[4] = {0u, 0u, 0u, 0u};
-            if (sr) s_upd.draw8(d.tensor_id, (uint64_t)((t.e0 >> 3) + v), nz);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              float f = dl[k];
-              if (hp.cautious) f = ((kept >> k) & 1u) ? div_shared(f, denom, rcp_denom) : 0.0f;
-              pc[k] = write_step<PT>(pc[k], f, -1.0f, sr, noise_lane(nz, k));
-            }
-          }
-          if (hp.climb && MK != KAON_M_NONE) {
-            uint32_t nc[4] = {0u, 0u, 0u, 0u};
-            if (E::IS_BF16) s_clb.draw8(d.tensor_id, (uint64_t)((t.e0 >> 3) + v), nc);
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              pc[k] = write_step<PT>(pc[k], climb_e(md[k], hp.a_climb, hp.b_climb), 1.0f, E::IS_BF16, noise_lane(nc, k));
-          }
-          store8<PT>(pbase + (size_t)v * 8 * E::BYTES, 8, pc, &pv.peers);
-        }
-      }
-    }
-    if constexpr (!APPLY) {  // the item's kept count
-      for (int o = 16; o > 0; o >>= 1) kept_local += __shfl_xor_sync(0xffffffffu, kept_local, o);
-      if ((tid & 31) == 0) red_s[tid >> 5] = kept_local;
-    }
-    __syncthreads();
-    if constexpr (!APPLY) {
-      if (tid == 0 && ok) {
-        unsigned tot = 0;
-        for (int w = 0; w < APPLY_THREADS / 32; ++w) tot += red_s[w];
-        if (tot) atomicAdd(pv.kept + t.tensor, tot);
-      }
-    }
-    slot ^= 1;
-    cur = next_s[slot];
-  }
-}
-
-typedef void (*ApplyKernel)(PlanView, AdaDev);
-
-template <typename PT, bool APPLY>
-static ApplyKernel pick_apply_pt(int mk) {
-  switch (mk) {
-    case KAON_M_F32: return adakaon_apply_kernel<PT, KAON_M_F32, APPLY, false>;
-    case KAON_M_BF16: return adakaon_apply_kernel<PT, KAON_M_BF16, APPLY, false>;
-    case KAON_M_INT8: return adakaon_apply_kernel<PT, KAON_M_INT8, APPLY, false>;
-    case KAON_M_4BIT: return adakaon_apply_kernel<PT, KAON_M_4BIT, APPLY, false>;
-    case KAON_M_NONE: return adakaon_apply_kernel<PT, KAON_M_NONE, APPLY, false>;
-    default: return nullptr;
-  }
-}
-
-static ApplyKernel pick_apply(int pdt, int mk, bool apply, bool muon) {
-  if (muon) {
-    if (pdt == KAON_DT_BF16) return apply ? adakaon_apply_kernel<__nv_bfloat16, KAON_M_NONE, true, true>
-                                          : adakaon_apply_kernel<__nv_bfloat16, KAON_M_NONE, false, true>;
-    return apply ? adakaon_apply_kernel<float, KAON_M_NONE, true, true> : adakaon_apply_kernel<float, KAON_M_NONE, false, true>;
-  }
-  if (apply) return pdt == KAON_DT_BF16 ? pick_apply_pt<__nv_bfloat16, true>(mk) : pick_apply_pt<float, true>(mk);
-  return pdt == KAON_DT_BF16 ? pick_apply_pt<__nv_bfloat16, false>(mk) : pick_apply_pt<float, false>(mk);
-}
-
 typedef void (*AxpyKernel)(PlanView, float, float, SrStream);
 
 template <typename PT, bool MUON>
@@ -2591,8 +1983,8 @@ int configure_launch_adakaon(kaon_plan* pl, const cudaDeviceProp& prop, int max_
 }
 
 // One-time set-up of the launches beside the persistent kernel.  Per factored tensor: its COUNT and
-// APPLY items go to the flat COUNT / APPLY launches when its rows stream (a multiple of 8 elements; 16
-// with int8 momentum; 4-bit block 128), and its STATS items to the STATS launch when they qualify
+// APPLY items go to the COUNT / APPLY launches (ada_sweep.cu) when its rows stream (a multiple of 8 elements; 4-bit
+// block 128), and its STATS items to the STATS launch when they qualify
 // (stats_item_ok, bf16 gradients or AdaMuon's bf16 signal).  Everything else - FINAL, the 1-D tensors,
 // the stages of tensors that do not qualify - stays in the persistent kernel, whose two lists (with
 // COUNT items for the cautious mask, without them otherwise) are the plan's lists minus what left.
@@ -2603,31 +1995,16 @@ int ensure_apply2(kaon_plan* pl) {
   const int mk = muon ? KAON_M_NONE : pl->momentum_kind;
   std::vector<Task> items;
   std::vector<char> elig((size_t)pl->n_tensors, 0);
+  bool any = false;
   for (int i = 0; i < pl->n_tensors; ++i) {
     const DevTensor& t = pl->h_tensors[i];
-    if (t.rows <= 0 || t.numel == 0) continue;
-    if ((t.cols & 7) != 0) continue;
+    if (t.rows <= 0 || t.numel == 0 || (t.cols & 7) != 0) continue;
     if (mk == KAON_M_4BIT && t.block != 128u) continue;
-    if (mk == KAON_M_INT8 && (t.cols & 15) != 0) continue;
     elig[i] = 1;
-    for (long long e = 0; e < t.numel; e += APPLY_CAP)
-      items.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(APPLY_CAP, t.numel - e), 0, 0, 0});
+    any = true;
   }
-  if (items.empty()) return KAON_OK;
-  ApplyKernel k = pick_apply(pl->param_dtype, mk, true, muon);
-  ApplyKernel kc = pick_apply(pl->param_dtype, mk, false, muon);
-  if (!k || !kc) return KAON_OK;
-  const size_t esz = pl->param_dtype == KAON_DT_BF16 ? 2 : 4;
-  const size_t mb = muon ? APPLY_CAP * esz
-                         : mk == KAON_M_4BIT ? APPLY_CAP / 2 : mk == KAON_M_INT8 ? APPLY_CAP : mk == KAON_M_BF16 ? APPLY_CAP * 2
-                         : mk == KAON_M_F32 ? APPLY_CAP * 4 : 0;
-  pl->apply_smem = 2 * (size_t)APPLY_CAP * esz + mb;
-  KAON_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl->apply_smem));
-  KAON_CUDA(cudaFuncSetAttribute((const void*)kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl->apply_smem));
-  int per_sm = 0;
-  KAON_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, APPLY_THREADS, pl->apply_smem));
-  if (per_sm < 1) return KAON_OK;
-  pl->apply_grid = pl->sm_count * per_sm;
+  if (!any) return KAON_OK;
+  sweep_units(pl, elig, items);
   // the persistent kernel's lists and the STATS launch's
   const bool stats_dtype = muon || pl->param_dtype == KAON_DT_BF16;
   std::vector<Task> stats;
@@ -2667,8 +2044,6 @@ int ensure_apply2(kaon_plan* pl) {
   return KAON_OK;
 }
 
-// The COUNT (cautious mask on) and APPLY launches over the plan's flat items; `base` carries the
-// plan's pointers (and AdaMuon's signal column).
 // STATS as a launch of its own over the plan's qualifying STATS items (the persistent kernel's lists
 // do not hold them); KAON_OK also when there are none.
 int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s) {
@@ -2682,10 +2057,6 @@ bool stats_item_ok(const kaon_plan* pl, const Task& t) {
 }
 
 int launch_stats_tasks(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* tasks, int n, cudaStream_t s) {
-  if (pl->d_counter2 == nullptr) {
-    KAON_CUDA(cudaMalloc((void**)&pl->d_counter2, 256));
-    pl->device_bytes += 256;
-  }
   if (pl->stats_grid == 0) {
     int per_sm = 0;
     KAON_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)ada_stats_kernel, STT, 0));
@@ -2694,33 +2065,8 @@ int launch_stats_tasks(kaon_plan* pl, const PlanView& base, const AdaDev& hp, co
   PlanView vs = base;
   vs.tasks = tasks;
   vs.n_tasks = n;
-  vs.task_counter = pl->d_counter2;
-  KAON_CUDA(cudaMemsetAsync(pl->d_counter2, 0, sizeof(unsigned), s));
+  vs.task_counter = base.counters2;
   ada_stats_kernel<<<pl->stats_grid, STT, 0, s>>>(vs, hp);
-  KAON_CUDA(cudaGetLastError());
-  pl->launches += 1;
-  return KAON_OK;
-}
-
-int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s) {
-  if (pl->d_counter2 == nullptr) {
-    KAON_CUDA(cudaMalloc((void**)&pl->d_counter2, 256));
-    pl->device_bytes += 256;
-  }
-  const bool muon = pl->optimizer == KAON_OPT_ADAMUON;
-  const int mk = muon ? KAON_M_NONE : pl->momentum_kind;
-  PlanView va = base;
-  va.tasks = pl->d_tasks_apply2;
-  va.n_tasks = pl->n_tasks_apply2;
-  va.task_counter = pl->d_counter2;
-  if (hp.cautious) {
-    KAON_CUDA(cudaMemsetAsync(pl->d_counter2, 0, sizeof(unsigned), s));
-    pick_apply(pl->param_dtype, mk, false, muon)<<<pl->apply_grid, APPLY_THREADS, pl->apply_smem, s>>>(va, hp);
-    KAON_CUDA(cudaGetLastError());
-    pl->launches += 1;
-  }
-  KAON_CUDA(cudaMemsetAsync(pl->d_counter2, 0, sizeof(unsigned), s));
-  pick_apply(pl->param_dtype, mk, true, muon)<<<pl->apply_grid, APPLY_THREADS, pl->apply_smem, s>>>(va, hp);
   KAON_CUDA(cudaGetLastError());
   pl->launches += 1;
   return KAON_OK;
@@ -2758,12 +2104,13 @@ extern "C" int kaon_adakaon_step(kaon_plan* pl, const kaon_adakaon_hparams* h, u
   hp.a_remove = (float)h->msam_alpha_remove; hp.b_remove = (float)h->msam_bound_remove;
   hp.a_climb = (float)h->msam_alpha_climb; hp.b_climb = (float)h->msam_bound_climb;
   hp.step = step; hp.k0 = (uint32_t)seed; hp.k1 = (uint32_t)(seed >> 32);
+  ada_finish(hp);
   cudaStream_t s = (cudaStream_t)stream;
   PlanView v = pl->view;
   if (int rc = ensure_apply2(pl)) return rc;
-  // two launches when the plan is eligible (int8 momentum also needs the COUNT stage's row maxima)
-  const bool two = pl->apply2 == 1 && (pl->momentum_kind != KAON_M_INT8 || hp.cautious);
-  if (pl->has_long_rows && !(two && pl->long_rows_ok))
+  // COUNT and APPLY as launches of their own when the plan is eligible (int8 momentum always takes COUNT's row maxima)
+  const bool two = pl->apply2 == 1;
+  if (pl->has_long_rows && !(two && pl->long_rows_ok && (pl->momentum_kind != KAON_M_INT8 || hp.cautious)))
     return fail(KAON_E_UNSUPPORTED,
                 "a tensor's rows exceed a work item of %d elements: such rows are stepped by the streaming launches "
                 "only (bf16 weights, a row length that is a multiple of 8 (16 with int8 momentum), 4-bit block 128, "

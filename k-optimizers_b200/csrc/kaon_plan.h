@@ -55,7 +55,7 @@ struct DevTensor {
   int n_count;          // COUNT items
   long long aux_off;    // float index of this tensor's scratch in `aux`:
                         //   colpart[n_stats][2][cols] | cfac[cols] | rowpart[n_stats] (double) |
-                        //   tpart[n_strips] (double) | scal[4] = {rowmean, divisor, rms, -} | rowmax[rows] | mean[rows]
+                        //   tpart[n_strips] (double) | scal[4] = {rowmean, divisor, rms, 1 / divisor} | rowmax[rows] | mean[rows]
   void* shift;          // Kahan compensation buffer (bf16 [numel]) or null
 };
 
@@ -67,7 +67,7 @@ __host__ __device__ inline int blk_lanes(const DevTensor& d) { return d.bshift >
 __host__ __device__ inline long long aux_cfac(const DevTensor& d) { return d.aux_off + 2ll * d.n_stats * d.cols; }
 __host__ __device__ inline long long aux_rowpart(const DevTensor& d) { return (aux_cfac(d) + d.cols + 1) / 2 * 2; }
 __host__ __device__ inline long long aux_tpart(const DevTensor& d) { return aux_rowpart(d) + 2ll * d.n_stats; }
-__host__ __device__ inline long long aux_scal(const DevTensor& d) { return aux_tpart(d) + 2ll * d.n_strips; }
+__host__ __device__ inline long long aux_scal(const DevTensor& d) { return (aux_tpart(d) + 2ll * d.n_strips + 3) / 4 * 4; }
 // int8 momentum: bits of each row's absmax of the new momentum, left by COUNT for APPLY
 __host__ __device__ inline long long aux_rowmax(const DevTensor& d) { return aux_scal(d) + 4; }
 // centralization mean of every row, left by STATS for COUNT / APPLY
@@ -79,7 +79,9 @@ __host__ __device__ inline long long aux_rfac(const DevTensor& d) { return aux_o
 // scratch of a 1-D tensor stepped from global memory: 8 floats | n floats (padded) | one word per 4-bit block (>= 32 elements)
 __host__ __device__ inline long long flat_long_pad(long long n) { return (n + 63) / 64 * 64; }
 __host__ __device__ inline long long flat_long_size(long long n) { return 8 + flat_long_pad(n) + ((n + 31) / 32 + 1 + 63) / 64 * 64; }
-__host__ __device__ inline long long aux_size(const DevTensor& d) { return aux_rfac(d) + d.rows - d.aux_off; }
+// {mean (bf16 weights: two bf16 copies), r_i, int8: old scale, -} of every row, for COUNT / APPLY (16-byte aligned)
+__host__ __device__ inline long long aux_rowtab(const DevTensor& d) { return (aux_rfac(d) + d.rows + 3) / 4 * 4; }
+__host__ __device__ inline long long aux_size(const DevTensor& d) { return aux_rowtab(d) + 4ll * d.rows - d.aux_off; }
 
 struct Task {
   int tensor;
@@ -111,11 +113,13 @@ struct PlanView {
   unsigned* done;          // Lion: [n_tensors] MAIN items finished.  Adakaon: [4][n_tensors] =
                            //   STATS items done | FINAL strips arrived | FINAL complete | COUNT items done
   unsigned* kept;          // [n_tensors] cautious kept count
+  unsigned* counters2;     // [4] claim counters of the Adakaon launches beside the persistent kernel: STATS, COUNT, APPLY, -
   float* aux;              // Adakaon scratch (see DevTensor::aux_off)
   const void* const* signal;  // AdaMuon: per-tensor orthogonalised momentum (bf16); null otherwise
   unsigned* status;        // 0 = ok; else the code of the first bounded wait that ran out
   unsigned char* codes;    // 2 bits per element
   Peers peers;             // n == 0: no mirrors
+  int param_bf16;          // weights are bf16 (else fp32)
   unsigned spin_limit;     // polls a completion-counter wait makes before it gives up (0: the default)
   unsigned sm_reserve;     // multiprocessors (the highest ids) whose CTAs leave at once, so that a collective's
                            // CTAs find them empty beside the persistent step (0: none)
@@ -165,9 +169,6 @@ struct kaon_plan {
   // STATS as a launch of its own: the STATS items that qualify
   kaon::Task* d_tasks_stats = nullptr;
   int n_tasks_stats = 0, stats_grid = 0;
-  unsigned* d_counter2 = nullptr;            // claim counter of the COUNT / APPLY launches
-  int apply_grid = 0;
-  size_t apply_smem = 0;
   unsigned* d_counters = nullptr;  // task_counter, status, done[n], kept[n] (contiguous; memset per step)
   size_t counters_bytes = 0;
   int64_t device_bytes = 0;

@@ -309,7 +309,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   size_t o_t = 0, o_g = o_t + up(sizeof(DevTensor) * n), o_f = o_g + up(sizeof(void*) * n);
   size_t o_m = o_f + up(sizeof(Task) * full_list.size()), o_a = o_m + up(sizeof(Task) * main_list.size());
   size_t o_c = o_a + up(sizeof(Task) * axpy_list.size());
-  pl->counters_bytes = sizeof(unsigned) * (size_t)(2 + 5 * n);
+  pl->counters_bytes = sizeof(unsigned) * (size_t)(2 + 5 * n + 4);
   size_t tot = o_c + up(pl->counters_bytes);
   ce = cudaMalloc(&pl->d_block, tot);
   if (ce != cudaSuccess) { delete pl; return cuda_fail(ce, "cudaMalloc(plan tables)"); }
@@ -350,10 +350,12 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   v.tensors = (const DevTensor*)(base + o_t);
   v.grads = (const void* const*)(base + o_g);
   v.n_tensors = n;
+  v.param_bf16 = param_dtype == KAON_DT_BF16;
   v.status = pl->d_counters;            // sticky: not cleared per step
   v.task_counter = pl->d_counters + 1;  // cleared per step from here on
   v.done = pl->d_counters + 2;
   v.kept = pl->d_counters + 2 + 4 * n;
+  v.counters2 = pl->d_counters + 2 + 5 * n;
   v.codes = pl->d_codes;
   v.aux = pl->d_aux;
   *out = pl;
@@ -385,7 +387,6 @@ int kaon_plan_destroy(kaon_plan* pl) {
   cudaFree(pl->d_tasks_na[0]);
   cudaFree(pl->d_tasks_na[1]);
   cudaFree(pl->d_tasks_stats);
-  cudaFree(pl->d_counter2);
   cudaFree((void*)pl->d_signal);
   if (pl->muon_lanes_ready) {
     for (int l = 0; l < 4; ++l) {
