@@ -14,12 +14,10 @@
 // 1-D tensor: FLAT, the whole tensor in one work item.
 // Every cross-item sum is taken in a fixed order: results do not depend on scheduling.
 //
-// Each of STATS / COUNT / APPLY exists twice.  The staged form above (ada_stats, ada_rows) handles any
-// shape.  The streaming form (ada_stats_stream, ada_stream) needs rows that are a multiple of 8
-// elements and reads gradient, momentum and weights straight from global memory, with what is per row
-// or per column fetched from the scratch in L2; it has no barrier in its loops.  COUNT and APPLY of the tensors
-// that stream leave this kernel and run as launches of their own (ada_sweep.cu), ordered by the stream instead of
-// by completion counters.
+// This kernel's stages handle any shape.  Tensors whose rows are a multiple of 8 elements (4-bit blocks of 128)
+// leave it: COUNT and APPLY run as launches of their own (ada_sweep.cu), STATS of bf16 rows of at least 256
+// elements too (ada_stats_kernel below; other such rows stream through ada_stats_stream here), and tensors of at most
+// ADA_SMALL_MAX elements are stepped whole by one CTA each (ada_small_kernel).
 #include <map>
 #include <vector>
 #include <mutex>
@@ -71,6 +69,14 @@ __device__ __forceinline__ float div_shared(float x, float d, float rcp) {
   float q0 = __fmul_rn(x, rcp);
   float r = __fmaf_rn(-q0, d, x);
   return __fmaf_rn(r, rcp, q0);
+}
+
+// a warp's sum of fp32 values, taken in double: a row statistic one ulp off moves codes of the row
+__device__ __forceinline__ float warp_sum_d(float v) {
+  double t = (double)v;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return (float)t;
 }
 
 // Nekaon perturbation of one element (reference src/kaon/msam.py:222-230)
@@ -192,7 +198,7 @@ __device__ __forceinline__ float row_mean(const unsigned char* rowp, int C, int 
   } else {
     for (int i = lane; i < C; i += 32) s += E::load1(rowp, i);
   }
-  s = warp_sum(s);
+  s = warp_sum_d(s);
   float mean = __fdiv_rn(s, (float)C);
   return E::IS_BF16 ? round_bf16(mean) : mean;
 }
@@ -220,7 +226,7 @@ __device__ __forceinline__ float row_part(const unsigned char* rowp, int C, int 
   } else {
     for (int i = part * 32 + lane; i < C; i += G * 32) s += term(E::load1(rowp, i));
   }
-  return warp_sum(s);
+  return warp_sum_d(s);
 }
 
 template <typename PT>
@@ -343,7 +349,7 @@ __device__ void ada_stats(const PlanView& pv, const AdaDev& hp, const Task& t, S
           s += sq;
         }
       }
-      s = warp_sum(s);
+      s = warp_sum_d(s);
       if (lane == 0) {
         const int row = t.row0 + c0 + r;
         const float mean = __fdiv_rn(s, (float)C);
@@ -471,7 +477,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
             a0 = add2(a0, add2(pairs(q0.x), pairs(q0.y)));
             a1v = add2(a1v, add2(pairs(q0.z), pairs(q0.w)));
           }
-          const float s = warp_sum((a0.x + a0.y) + (a1v.x + a1v.y));
+          const float s = warp_sum_d((a0.x + a0.y) + (a1v.x + a1v.y));
           mu = round_bf16(__fdiv_rn(s, (float)C));
         }
         const uint32_t mu2 = pack_bf16_rn(mu, mu);
@@ -495,7 +501,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
           b0 = add2(b0, add2(sq2(q0.x), sq2(q0.y)));
           b1 = add2(b1, add2(sq2(q0.z), sq2(q0.w)));
         }
-        s2 = warp_sum((b0.x + b0.y) + (b1.x + b1.y));
+        s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y));
       } else {
         if (gc) {
           float s = 0.0f;
@@ -504,7 +510,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
             E::load8(rowp + (size_t)v * 8 * E::BYTES, x);
             s += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
           }
-          s = warp_sum(s);
+          s = warp_sum_d(s);
           mu = __fdiv_rn(s, (float)C);
         }
         for (int v = lane; v < nv; v += 32) {
@@ -519,7 +525,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
           }
           s2 += ((sq[0] + sq[1]) + (sq[2] + sq[3])) + ((sq[4] + sq[5]) + (sq[6] + sq[7]));
         }
-        s2 = warp_sum(s2);
+        s2 = warp_sum_d(s2);
       }
       if (lane == 0) {
         const float mean = __fdiv_rn(s2, (float)C);
@@ -690,7 +696,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
             a0 = add2(a0, add2(pairs(q0.x), pairs(q0.y)));
             a1 = add2(a1, add2(pairs(q0.z), pairs(q0.w)));
           }
-          mu = round_bf16(__fdiv_rn(warp_sum((a0.x + a0.y) + (a1.x + a1.y)), (float)C));
+          mu = round_bf16(__fdiv_rn(warp_sum_d((a0.x + a0.y) + (a1.x + a1.y)), (float)C));
         }
         const uint32_t mu2 = pack_bf16_rn(mu, mu);
         auto sq2 = [&](uint32_t w) {
@@ -712,7 +718,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
           b0 = add2(b0, add2(sq2(q0.x), sq2(q0.y)));
           b1 = add2(b1, add2(sq2(q0.z), sq2(q0.w)));
         }
-        const float s2 = warp_sum((b0.x + b0.y) + (b1.x + b1.y));
+        const float s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y));
         if (lane == 0) {
           const float rn = lerp_torch(old, __fdiv_rn(s2, (float)C), hp.w2, hp.w2m1, hp.small_w2 != 0);
           d.stat_a[row] = rn;
@@ -850,7 +856,7 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
   float* cfac = pv.aux + aux_cfac(d);
   double tl = 0.0;
   for (int j = tid; j < nc; j += AT) {
-    float s1 = 0.0f, s2 = 0.0f;
+    double s1 = 0.0, s2 = 0.0;
     int s = 0;
     for (; s + 8 <= d.n_stats; s += 8) {  // eight slots' loads in flight; the sums keep the slot order
       float x1[8], x2[8];
@@ -860,17 +866,17 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
         x2[u] = __ldcg(part + 2ll * (s + u) * C + C + j0 + j);
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) { s1 += x1[u]; s2 += x2[u]; }
+      for (int u = 0; u < 8; ++u) { s1 += (double)x1[u]; s2 += (double)x2[u]; }
     }
     for (; s < d.n_stats; ++s) {
-      s1 += __ldcg(part + 2ll * s * C + j0 + j);
-      s2 += __ldcg(part + 2ll * s * C + C + j0 + j);
+      s1 += (double)__ldcg(part + 2ll * s * C + j0 + j);
+      s2 += (double)__ldcg(part + 2ll * s * C + C + j0 + j);
     }
-    const float mean = __fdiv_rn(s1, (float)d.rows);
+    const float mean = __fdiv_rn((float)s1, (float)d.rows);
     const float cn = lerp_torch(d.stat_b[j0 + j], mean, hp.w2, hp.w2m1, hp.small_w2 != 0);
     d.stat_b[j0 + j] = cn;
     cfac[j0 + j] = rsqrt_torch(cn);
-    tl += (double)s2 / (double)cn;
+    tl += s2 / (double)cn;
   }
   const double tot = block_sum_d(tl, sm.red, tid);
   double* tpart = reinterpret_cast<double*>(pv.aux + aux_tpart(d));
@@ -1362,260 +1368,6 @@ __device__ void ada_rows(const PlanView& pv, const AdaDev& hp, const Task& t, St
 
 // ----------------------------------------------------------------------------- COUNT / APPLY, streaming
 
-// The same two work items for the common case - rows a multiple of 8 elements, gradient as the signal -
-// without shared-memory staging and without a barrier in the loop: every thread streams its vectors
-// straight from global memory (gradient, momentum, weights) and fetches what is per row or per column
-// (centralization mean, row statistic, column factor, int8 scales) from L2, where the earlier stages
-// left it.  Rows of an item belong to this CTA alone, so the int8 row maxima are reduced with
-// atomicMax on the tensor's scratch (COUNT) and the old row scales are set aside once per item (APPLY).
-// Results are bit-identical to ada_rows: same arithmetic, same noise indices.
-template <typename PT, int MKP, bool APPLY, bool MUON>
-__device__ void ada_stream(const PlanView& pv, const AdaDev& hp, const Task& t, const AdaSmem& sm, int tid) {
-  using E = Elems<PT>;
-  using S = Elems<typename std::conditional<MUON, __nv_bfloat16, PT>::type>;  // the signal's element type
-  constexpr int MK = MUON ? KAON_M_NONE : MKP;
-  const DevTensor d = pv.tensors[t.tensor];
-  const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
-  if (g == nullptr) {
-    if (!APPLY) {
-      __syncthreads();
-      if (tid == 0) signal_counter(pv.done + 3 * pv.n_tensors + t.tensor, 1u);
-    }
-    return;
-  }
-  bool ok = true;
-  if (tid == 0) {
-    ok = wait_counter(pv.done + 2 * pv.n_tensors + t.tensor, 1u, pv.status, 12001u);
-    if (ok && APPLY && hp.cautious)
-      ok = wait_counter(pv.done + 3 * pv.n_tensors + t.tensor, (unsigned)d.n_count, pv.status, 13001u);
-  }
-  ok = __syncthreads_and(ok) != 0;
-  const int C = d.cols;
-  const int nrows = t.n / C;
-  const bool gc = hp.gc != 0 && !MUON;
-  // AdaMuon with gradient centralization: the statistics run on the orthogonalised matrix, which is not
-  // centralised; the cautious mask compares with the CENTRALISED raw gradient (row means in the scratch)
-  const bool gcr = hp.gc != 0 && MUON;
-  // AdaMuon: the chain runs on the orthogonalised momentum, the cautious mask on the raw gradient
-  const unsigned char* sig = MUON ? reinterpret_cast<const unsigned char*>(pv.signal[t.tensor]) : g;
-  const float* scal = pv.aux + aux_scal(d);
-  const float rowmean = __ldcg(scal + 0);
-  Chain ch;
-  ch.div = __ldcg(scal + 1);
-  ch.use_div = ch.div != 1.0f;
-  ch.rcp_div = __fdiv_rn(1.0f, ch.div);
-  float denom = 1.0f, rcp_denom = 1.0f;
-  if (APPLY && hp.cautious) {
-    const unsigned kept = __ldcg(pv.kept + t.tensor);
-    denom = fmaxf(__fdiv_rn((float)kept, (float)d.numel), 1e-8f);
-    rcp_denom = __fdiv_rn(1.0f, denom);
-  }
-  const float* cfac = pv.aux + aux_cfac(d);
-  const float* mean = pv.aux + aux_mean(d);
-  unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
-  float* oldsc = pv.aux + aux_oldsc(d);
-  const float* rfac = pv.aux + aux_rfac(d);
-  SrStream s_upd{Philox{hp.k0, hp.k1}, hp.step, KAON_TAG_UPDATE};
-  SrStream s_rem{Philox{hp.k0, hp.k1}, hp.step, KAON_TAG_REMOVE};
-  SrStream s_clb{Philox{hp.k0, hp.k1}, hp.step, KAON_TAG_CLIMB};
-  const bool sr = hp.sr != 0;
-  const bool need_p = APPLY || hp.has_wd;
-  const int lane = tid & 31;
-  unsigned kept_local = 0;
-
-  for (int c0 = 0; ok && c0 < nrows; c0 += d.chunk_rows) {
-    const int nrc = min(d.chunk_rows, nrows - c0);
-    const int nvec = (nrc * C) >> 3;
-    const int nvec_pad = (nvec + 31) & ~31;
-    const long long e0 = t.e0 + (long long)c0 * C;
-    const unsigned char* gbase = sig + e0 * S::BYTES;
-    const unsigned char* rawbase = g + e0 * E::BYTES;
-    const unsigned char* mbase = m_ptr<MK>(d, e0);
-    unsigned char* pbase = reinterpret_cast<unsigned char*>(d.p) + e0 * E::BYTES;
-    for (int v = tid; v < nvec_pad; v += AT) {
-      const bool act = v < nvec;
-      const int vv = act ? v : 0;
-      const int r = row_of((unsigned)vv * 8u, d);
-      const int row = t.row0 + c0 + r;
-      const int col = vv * 8 - r * C;
-      float gv[8], mo[8], mn[8], pc[8], dl[8];
-      // ---- loads ----
-      S::load8(gbase + (size_t)vv * 8 * S::BYTES, gv);
-      float raw[8];
-      if (MUON) E::load8(rawbase + (size_t)vv * 8 * E::BYTES, raw);
-      if (need_p) E::load8(pbase + (size_t)vv * 8 * E::BYTES, pc);
-      else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) pc[k] = 0.0f;
-      }
-      const float mu = (gc || gcr) ? __ldcg(mean + row) : 0.0f;
-      if (MUON && gcr) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) raw[k] = centered<PT>(raw[k], mu, true);
-      }
-      const float rf = __ldcg(rfac + row);
-      const float4 c0v = __ldcg(reinterpret_cast<const float4*>(cfac + col));
-      const float4 c1v = __ldcg(reinterpret_cast<const float4*>(cfac + col + 4));
-      const float cf[8] = {c0v.x, c0v.y, c0v.z, c0v.w, c1v.x, c1v.y, c1v.z, c1v.w};
-      if constexpr (MK == KAON_M_4BIT) {
-        const float sc_old = d.m_scale[d.block == 128u ? ((e0 >> 7) + (vv >> 4)) : 0];
-        decode8<MK>(mbase, vv, 8, sc_old, mo);
-      } else if constexpr (MK == KAON_M_INT8) {
-        const float sc_old = APPLY ? __ldcg(oldsc + row) : d.m_scale[row];
-        decode8<MK>(mbase, vv, 8, sc_old, mo);
-      } else if constexpr (MK == KAON_M_NONE) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) mo[k] = 0.0f;
-      } else {
-        decode8<MK>(mbase, vv, 8, 1.0f, mo);
-      }
-      // ---- the chain ----
-      if (hp.remove && need_p) {
-        uint32_t nz[4] = {0u, 0u, 0u, 0u};
-        if (E::IS_BF16) s_rem.draw8(d.tensor_id, (uint64_t)((e0 >> 3) + vv), nz);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          pc[k] = write_step<PT>(pc[k], climb_e(mo[k], hp.a_remove, hp.b_remove), 1.0f, E::IS_BF16, noise_lane(nz, k));
-      }
-      if (gc) {
-#pragma unroll
-        for (int k = 0; k < 8; k += 2) {
-          const float x0 = __fsub_rn(gv[k], mu), x1 = __fsub_rn(gv[k + 1], mu);
-          if (E::IS_BF16) {
-            const uint32_t pk = pack_bf16_rn(x0, x1);
-            gv[k] = bf16lo(pk); gv[k + 1] = bf16hi(pk);
-          } else {
-            gv[k] = x0; gv[k + 1] = x1;
-          }
-        }
-      }
-      unsigned kept = 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float u = update_of(gv[k], rf, cf[k], ch, hp.upd_scale);
-        mn[k] = ema_of<MK>(mo[k], u, hp);
-        const float dv = hp.has_wd ? __fmaf_rn(pc[k], hp.lrwd, mn[k]) : mn[k];
-        dl[k] = dv;
-        if (__fmul_rn(dv, MUON ? raw[k] : gv[k]) > 0.0f) kept |= 1u << k;
-      }
-      if constexpr (!APPLY) {
-        if (act) kept_local += __popc(kept);
-        if constexpr (MK == KAON_M_INT8) {
-          float a = 0.0f;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) a = fmaxf(a, fabsf(mn[k]));
-          unsigned bits = act ? __float_as_uint(a) : 0u;
-          const int row_l0 = __shfl_sync(0xffffffffu, row, 0);
-          if (__all_sync(0xffffffffu, !act || row == row_l0)) {
-            bits = __reduce_max_sync(0xffffffffu, bits);
-            if (lane == 0 && bits) atomicMax(rowmax + row_l0, bits);
-          } else if (act) {
-            atomicMax(rowmax + row, bits);
-          }
-        }
-      } else {
-        float md[8];  // the momentum as stored (decoded), for the Nekaon climb
-        if constexpr (MK == KAON_M_4BIT) {
-          float a = 0.0f;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) a = fmaxf(a, act ? fabsf(mn[k]) : 0.0f);
-          a = fmaxf(group_max(a, 16), 1e-12f);
-          __syncwarp();  // every lane of the block has read the old scale before it is replaced
-          const float sc = __fdiv_rn(a, 7.0f);
-          const float inv = __fdividef(1.0f, sc);
-          uint32_t word = 0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float q = quant_round(mn[k], sc, inv, 1e-4f);
-            const int qi = min(max((int)q, -7), 7);
-            md[k] = __fmul_rn((float)qi, sc);
-            word |= (uint32_t)(qi + 8) << (4 * k);
-          }
-          if (act) {
-            *reinterpret_cast<uint32_t*>((unsigned char*)d.m + (e0 >> 1) + (size_t)v * 4) = word;
-            if ((v & 15) == 0) d.m_scale[(d.block == 128u) ? ((e0 >> 7) + (v >> 4)) : 0] = sc;
-          }
-        } else if constexpr (MK == KAON_M_INT8) {
-          const float sc = __fdiv_rn(fmaxf(__uint_as_float(__ldcg(rowmax + row)), 1e-12f), 127.0f);
-          const float inv = __fdividef(1.0f, sc);
-          uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int qi = min(max((int)quant_round(mn[k], sc, inv, 1e-3f), -127), 127);
-            md[k] = __fmul_rn((float)qi, sc);
-            const uint32_t byte = (uint32_t)(qi & 0xFF);
-            if (k < 4) w0 |= byte << (8 * k); else w1 |= byte << (8 * (k - 4));
-          }
-          if (act) {
-            *reinterpret_cast<uint2*>((unsigned char*)d.m + e0 + (size_t)v * 8) = make_uint2(w0, w1);
-            if (col == 0) d.m_scale[row] = sc;
-          }
-        } else if constexpr (MK == KAON_M_BF16 || MK == KAON_M_F32) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) md[k] = mn[k];
-          if (act) {
-            if constexpr (MK == KAON_M_BF16) store8<__nv_bfloat16>((unsigned char*)d.m + e0 * 2 + (size_t)v * 16, 8, mn, nullptr);
-            else store8<float>((unsigned char*)d.m + e0 * 4 + (size_t)v * 32, 8, mn, nullptr);
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) md[k] = 0.0f;
-        }
-        if (act) {
-          if (E::IS_BF16 && hp.kahan) {
-            unsigned char* she = reinterpret_cast<unsigned char*>(d.shift) + (size_t)e0 * 2 + (size_t)v * 16;
-            float sh[8];
-            load8_guard<__nv_bfloat16>(she, 8, sh);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              float f = dl[k];
-              if (hp.cautious) f = ((kept >> k) & 1u) ? div_shared(f, denom, rcp_denom) : 0.0f;
-              kahan_step(pc[k], sh[k], f);
-            }
-            store8<__nv_bfloat16>(she, 8, sh, nullptr);
-          } else {
-            uint32_t nz[4] = {0u, 0u, 0u, 0u};
-            if (sr) s_upd.draw8(d.tensor_id, (uint64_t)((e0 >> 3) + v), nz);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              float f = dl[k];
-              if (hp.cautious) f = ((kept >> k) & 1u) ? div_shared(f, denom, rcp_denom) : 0.0f;
-              pc[k] = write_step<PT>(pc[k], f, -1.0f, sr, noise_lane(nz, k));
-            }
-          }
-          if (hp.climb && MK != KAON_M_NONE) {
-            uint32_t nc[4] = {0u, 0u, 0u, 0u};
-            if (E::IS_BF16) s_clb.draw8(d.tensor_id, (uint64_t)((e0 >> 3) + v), nc);
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              pc[k] = write_step<PT>(pc[k], climb_e(md[k], hp.a_climb, hp.b_climb), 1.0f, E::IS_BF16, noise_lane(nc, k));
-          }
-          store8<PT>(pbase + (size_t)v * 8 * E::BYTES, 8, pc, &pv.peers);
-        }
-      }
-    }
-  }
-  if constexpr (!APPLY) {
-    const unsigned tot = block_sum_u(kept_local, sm.red, tid);
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-      if (ok) atomicAdd(pv.kept + t.tensor, tot);
-      signal_counter(pv.done + 3 * pv.n_tensors + t.tensor, 1u);
-    }
-  }
-}
-
-// Whether the streaming form handles this tensor and these settings (otherwise: ada_rows).
-template <int MK>
-__device__ __forceinline__ bool stream_ok(const DevTensor& d, const AdaDev& hp, const void* g, const void* sig) {
-  if ((d.cols & 7) != 0) return false;
-  if ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(sig)) & 15) return false;  // 16-byte vector loads
-  if (MK == KAON_M_4BIT && d.block != 128u) return false;
-  if (MK == KAON_M_INT8 && !hp.cautious) return false;  // no COUNT item to find the row maxima
-  return true;
-}
-
 // ----------------------------------------------------------------------------- FLAT (1-D tensors)
 
 // reference src/kaon/adakaon.py:908-966: full second moment v, no factoring, no centralization.
@@ -1843,14 +1595,10 @@ __global__ void __launch_bounds__(AT, 1) adakaon_kernel(PlanView pv, AdaDev hp, 
       }
       case PH_ADA_FINAL: ada_final(pv, hp, t, sm_stats, tid); break;
       case PH_ADA_COUNT:
-        if (stream_ok<MUON ? KAON_M_NONE : MK>(pv.tensors[t.tensor], hp, pv.grads[t.tensor], MUON && pv.grads[t.tensor] ? pv.signal[t.tensor] : nullptr))
-          ada_stream<PT, MK, false, MUON>(pv, hp, t, sm_rows, tid);
-        else ada_rows<PT, MK, false, MUON>(pv, hp, t, st, sm_rows, tid);
+        ada_rows<PT, MK, false, MUON>(pv, hp, t, st, sm_rows, tid);
         break;
       case PH_ADA_APPLY:
-        if (stream_ok<MUON ? KAON_M_NONE : MK>(pv.tensors[t.tensor], hp, pv.grads[t.tensor], MUON && pv.grads[t.tensor] ? pv.signal[t.tensor] : nullptr))
-          ada_stream<PT, MK, true, MUON>(pv, hp, t, sm_rows, tid);
-        else ada_rows<PT, MK, true, MUON>(pv, hp, t, st, sm_rows, tid);
+        ada_rows<PT, MK, true, MUON>(pv, hp, t, st, sm_rows, tid);
         break;
       case PH_ADA_FLAT: ada_flat<PT, MK>(pv, hp, t, st, sm_rows, tid); break;
       default: break;
@@ -1909,6 +1657,8 @@ __global__ void __launch_bounds__(256) msam_axpy_kernel(PlanView pv, float alpha
 
 typedef void (*AxpyKernel)(PlanView, float, float, SrStream);
 
+typedef void (*AdaKernel)(PlanView, AdaDev, int);
+
 template <typename PT, bool MUON>
 static AdaKernel pick_ada_pt(int mk) {
   switch (mk) {
@@ -1920,7 +1670,7 @@ static AdaKernel pick_ada_pt(int mk) {
     default: return nullptr;
   }
 }
-AdaKernel pick_ada(int pdt, int mk, bool muon) {
+static AdaKernel pick_ada(int pdt, int mk, bool muon) {
   if (muon) return pdt == KAON_DT_BF16 ? pick_ada_pt<__nv_bfloat16, true>(mk) : pick_ada_pt<float, true>(mk);
   return pdt == KAON_DT_BF16 ? pick_ada_pt<__nv_bfloat16, false>(mk) : pick_ada_pt<float, false>(mk);
 }
@@ -1937,7 +1687,7 @@ static AxpyKernel pick_axpy_pt(int mk) {
 }
 
 // bytes reserved after the gradient stage for the momentum bytes (AdaMuon: the raw gradient) of a chunk
-size_t x_offset_rows(const kaon_plan* pl) {
+static size_t x_offset_rows(const kaon_plan* pl) {
   size_t b = momentum_bytes_per_cap(pl->momentum_kind);
   if (pl->optimizer == KAON_OPT_ADAMUON) b = std::max<size_t>(b, (size_t)CAP * (pl->param_dtype == KAON_DT_BF16 ? 2 : 4));
   return (b + 127) / 128 * 128;
@@ -1995,11 +1745,18 @@ int ensure_apply2(kaon_plan* pl) {
   const int mk = muon ? KAON_M_NONE : pl->momentum_kind;
   std::vector<Task> items;
   std::vector<char> elig((size_t)pl->n_tensors, 0);
+  std::vector<char> small((size_t)pl->n_tensors, 0);
+  {
+    std::vector<Task> h((size_t)pl->n_tasks_small);
+    if (!h.empty()) KAON_CUDA(cudaMemcpy(h.data(), pl->d_tasks_small, sizeof(Task) * h.size(), cudaMemcpyDeviceToHost));
+    for (const Task& t : h) small[t.tensor] = 1;
+  }
   bool any = false;
   for (int i = 0; i < pl->n_tensors; ++i) {
     const DevTensor& t = pl->h_tensors[i];
     if (t.rows <= 0 || t.numel == 0 || (t.cols & 7) != 0) continue;
     if (mk == KAON_M_4BIT && t.block != 128u) continue;
+    if (small[i]) continue;
     elig[i] = 1;
     any = true;
   }
@@ -2044,6 +1801,18 @@ int ensure_apply2(kaon_plan* pl) {
   return KAON_OK;
 }
 
+// The persistent kernel over the list in `v` (nothing where it is empty; no more CTAs than items).
+int launch_persistent(kaon_plan* pl, const PlanView& v, const AdaDev& hp, cudaStream_t s) {
+  if (v.n_tasks == 0) return KAON_OK;
+  AdaKernel k = pick_ada(pl->param_dtype, pl->momentum_kind, pl->optimizer == KAON_OPT_ADAMUON);
+  if (!k) return fail(KAON_E_INVALID, "no Adakaon kernel for this dtype combination");
+  const int grid = v.sm_reserve ? pl->grid : std::min(pl->grid, v.n_tasks);
+  k<<<grid, AT, pl->smem_bytes, s>>>(v, hp, (int)x_offset_rows(pl) | (pl->double_buffer ? 1 : 0));
+  KAON_CUDA(cudaGetLastError());
+  pl->launches += 1;
+  return KAON_OK;
+}
+
 // STATS as a launch of its own over the plan's qualifying STATS items (the persistent kernel's lists
 // do not hold them); KAON_OK also when there are none.
 int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s) {
@@ -2066,7 +1835,8 @@ int launch_stats_tasks(kaon_plan* pl, const PlanView& base, const AdaDev& hp, co
   vs.tasks = tasks;
   vs.n_tasks = n;
   vs.task_counter = base.counters2;
-  ada_stats_kernel<<<pl->stats_grid, STT, 0, s>>>(vs, hp);
+  if (n == 0) return KAON_OK;
+  ada_stats_kernel<<<base.sm_reserve ? pl->stats_grid : std::min(pl->stats_grid, n), STT, 0, s>>>(vs, hp);
   KAON_CUDA(cudaGetLastError());
   pl->launches += 1;
   return KAON_OK;
@@ -2123,10 +1893,8 @@ extern "C" int kaon_adakaon_step(kaon_plan* pl, const kaon_adakaon_hparams* h, u
   KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
   if (two)
     if (int rc = launch_stats(pl, pl->view, hp, s)) return rc;
-  AdaKernel k = pick_ada(pl->param_dtype, pl->momentum_kind, false);
-  k<<<pl->grid, AT, pl->smem_bytes, s>>>(v, hp, (int)x_offset_rows(pl) | (pl->double_buffer ? 1 : 0));
-  KAON_CUDA(cudaGetLastError());
-  pl->launches += 1;
+  if (int rc = launch_persistent(pl, v, hp, s)) return rc;
+  if (int rc = launch_small(pl, pl->view, hp, s)) return rc;
   if (two) {
     if (int rc = launch_count_apply(pl, pl->view, hp, s)) return rc;
   }

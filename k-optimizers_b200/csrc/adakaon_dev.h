@@ -17,22 +17,23 @@ struct AdaDev {
   float a_remove, b_remove, a_climb, b_climb;
   uint32_t step, k0, k1;
   uint32_t rk0[KAON_PHILOX_ROUNDS], rk1[KAON_PHILOX_ROUNDS];  // Philox round keys (k + r * Weyl), from the host
+  int stats_only;        // second moment only (AdaPNM, KProdigy)
   float mask_big, mask_add;   // the cautious mask as one saturating FMA (mask1 in ada_sweep.cu)
 };
 
 // round keys and mask constants from k0, k1 and cautious
 inline void ada_finish(AdaDev& hp) {
   for (int r = 0; r < KAON_PHILOX_ROUNDS; ++r) { hp.rk0[r] = hp.k0 + 0x9E3779B9u * (uint32_t)r; hp.rk1[r] = hp.k1 + 0xBB67AE85u * (uint32_t)r; }
+  if (!hp.has_eps) hp.eps1 = 0.0f;
   hp.mask_big = hp.cautious ? 0x1p127f : 0.0f;
   hp.mask_add = hp.cautious ? 0.0f : 1.0f;
 }
 
-typedef void (*AdaKernel)(PlanView, AdaDev, int);
-AdaKernel pick_ada(int param_dtype, int momentum_kind, bool muon);
-size_t x_offset_rows(const kaon_plan* pl);
+int launch_persistent(kaon_plan* pl, const PlanView& v, const AdaDev& hp, cudaStream_t s);
 // COUNT and APPLY as launches of their own (ada_sweep.cu), for the factored tensors whose rows stream
 void sweep_units(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out);
 int ensure_apply2(kaon_plan* pl);
+int launch_small(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
 int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
 int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
 // the STATS launch over a caller's list of STATS items (all of which pass stats_item_ok); KAON_OK or an error

@@ -646,17 +646,15 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
     AdaDev ad{};
     ad.w2 = (float)(1.0 - b2); ad.w2m1 = ad.w2 - 1.0f; ad.small_w2 = ad.w2 < 0.5f;
     ad.w1 = 1.0f; ad.eps1 = (float)h->eps; ad.has_eps = h->eps > 0.0; ad.clip = 1.0f;
-    ad.gc = hp.gc; ad.step = step; ad.k0 = hp.k0; ad.k1 = hp.k1;
+    ad.gc = hp.gc; ad.step = step; ad.k0 = hp.k0; ad.k1 = hp.k1; ad.stats_only = 1;
+    ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
     if (ph->d_stats != nullptr)
       if (int rc = launch_stats_tasks(pl, pl->view, ad, ph->d_stats, ph->n_stats, s)) return rc;
     v.tasks = ph->d_final; v.n_tasks = ph->n_final;
-    // the variant the plan's launch configuration was made for (STATS and FINAL do not depend on the momentum kind)
-    AdaKernel k = pick_ada(pl->param_dtype, pl->momentum_kind, false);
-    k<<<pl->grid, ADA_THREADS, pl->smem_bytes, s>>>(v, ad, (int)x_offset_rows(pl) | (pl->double_buffer ? 1 : 0));
-    KAON_CUDA(cudaGetLastError());
-    pl->launches += 1;
+    if (int rc = launch_persistent(pl, v, ad, s)) return rc;
+    if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
     // 2-4. the two sweeps over the flat items
     const int grid = std::min(x.n_items, pl->sm_count * 8);
     if (mk == KAON_M_INT8) {

@@ -28,7 +28,8 @@ enum : int { PH_LION_MAIN = 0, PH_LION_APPLY = 1, PH_AXPY = 2,
               PH_ADA_STATS = 10, PH_ADA_FINAL = 11, PH_ADA_COUNT = 12, PH_ADA_APPLY = 13, PH_ADA_FLAT = 14 };
 
 constexpr int ADA_THREADS = 512;
-constexpr int FINAL_STRIP = 2048;  // columns per FINAL item
+constexpr int FINAL_STRIP = 512;   // columns per FINAL item: one per thread
+constexpr int ADA_SMALL_MAX = 16384;  // elements of a factored tensor that one CTA steps on its own
 
 // One tensor as the kernels see it (device copy of kaon_tensor_desc plus planner-derived fields).
 struct DevTensor {
@@ -166,6 +167,8 @@ struct kaon_plan {
   kaon::Task* d_tasks_na[2] = {nullptr, nullptr};
   int n_tasks_na[2] = {0, 0};
   bool long_rows_ok = false;                 // every tensor whose rows exceed a work item left the persistent kernel
+  kaon::Task* d_tasks_small = nullptr;       // factored tensors one CTA steps on its own
+  int n_tasks_small = 0, small_max = 0;      // and the elements of the largest
   // STATS as a launch of its own: the STATS items that qualify
   kaon::Task* d_tasks_stats = nullptr;
   int n_tasks_stats = 0, stats_grid = 0;

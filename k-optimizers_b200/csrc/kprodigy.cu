@@ -536,16 +536,15 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
     AdaDev ad{};
     ad.w2 = (float)(1.0 - h->beta2); ad.w2m1 = ad.w2 - 1.0f; ad.small_w2 = ad.w2 < 0.5f;
     ad.w1 = 1.0f; ad.eps1 = (float)h->eps_factored; ad.has_eps = h->eps_factored > 0.0; ad.clip = 1.0f;
-    ad.gc = hp.gc;
+    ad.gc = hp.gc; ad.stats_only = 1;
+    ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
     if (kh->d_stats != nullptr)
       if (int rc = launch_stats_tasks(pl, pl->view, ad, kh->d_stats, kh->n_stats, s)) return rc;
     v.tasks = kh->d_final; v.n_tasks = kh->n_final;
-    AdaKernel k = pick_ada(pl->param_dtype, pl->momentum_kind, false);
-    k<<<pl->grid, ADA_THREADS, pl->smem_bytes, s>>>(v, ad, (int)x_offset_rows(pl) | (pl->double_buffer ? 1 : 0));
-    KAON_CUDA(cudaGetLastError());
-    pl->launches += 1;
+    if (int rc = launch_persistent(pl, v, ad, s)) return rc;
+    if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
   } else if (hp.gc && x.n_fact > 0) {
     if (pl->param_dtype == KAON_DT_BF16) kp_rowmean_kernel<__nv_bfloat16><<<pl->sm_count * 8, KP_THREADS, 0, s>>>(pl->view, x);
     else kp_rowmean_kernel<float><<<pl->sm_count * 8, KP_THREADS, 0, s>>>(pl->view, x);

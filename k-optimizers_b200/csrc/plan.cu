@@ -213,6 +213,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
 
   // Per-tensor stages.  Lion: MAIN, APPLY.  Adakaon (factored): STATS, FINAL, COUNT, APPLY; (1-D): FLAT.
   std::vector<std::vector<std::vector<Task>>> stages(n);
+  std::vector<Task> small_list;
   long long aux_floats = 0;
   int max_cols = 1;
   if (optimizer == KAON_OPT_LION) {
@@ -245,9 +246,21 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
         max_cols = std::max<int>(max_cols, (int)C);
         t.chunk_rows = (int)(per[i][0].n / C);
       }
-      // rows per run: column partials (8 B per column per run) stay under ~10 % of the run's gradient
-      // bytes, and a run is at least ~128 K elements
-      long long run_rows = std::max<long long>(40, (131072 + C - 1) / C);
+      if (t.numel <= ADA_SMALL_MAX && (C & 7) == 0 && !long_rows[i] && (momentum_kind != KAON_M_4BIT || t.bshift == 7)) {
+        // one CTA steps the whole tensor (ada_small_kernel)
+        small_list.push_back(Task{i, 0, 0, (int)t.numel, 0, 0, 0});
+        pl->small_max = std::max(pl->small_max, (int)t.numel);
+        t.n_stats = 1; t.n_strips = 1; t.n_count = 1;
+        t.aux_off = aux_floats;
+        aux_floats += (aux_size(t) + 63) / 64 * 64;
+        continue;
+      }
+      // rows per run: about a 32nd of the tensor between 8 K elements and 128 K, and 8 (a big tensor: 20) rows (column
+      // partials, 8 B per column and run, are then at most ~10 % of the gradient's bytes, and a tensor alone in its
+      // list still fills a part of the machine).  The tensor alone decides, not the list: its sums must not depend on
+      // how a list is split.
+      const long long run_elems = std::max<long long>(8192, std::min<long long>(131072, t.numel / 32));
+      long long run_rows = std::max<long long>(t.numel >= (1ll << 22) ? 20 : 8, (run_elems + C - 1) / C);
       run_rows = (run_rows + t.chunk_rows - 1) / t.chunk_rows * t.chunk_rows;
       stages[i].resize(4);
       int slot = 0;
@@ -304,11 +317,11 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
     if (tens[i].m)
       for (const Task& t : per[i]) { Task a = t; a.phase = PH_AXPY; axpy_list.push_back(a); }
 
-  // One device allocation: tensors | grads | tasks(full) | tasks(main) | tasks(axpy) | counters.
+  // One device allocation: tensors | grads | tasks(full) | tasks(main) | tasks(axpy) | tasks(small) | counters.
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   size_t o_t = 0, o_g = o_t + up(sizeof(DevTensor) * n), o_f = o_g + up(sizeof(void*) * n);
   size_t o_m = o_f + up(sizeof(Task) * full_list.size()), o_a = o_m + up(sizeof(Task) * main_list.size());
-  size_t o_c = o_a + up(sizeof(Task) * axpy_list.size());
+  size_t o_s = o_a + up(sizeof(Task) * axpy_list.size()), o_c = o_s + up(sizeof(Task) * small_list.size());
   pl->counters_bytes = sizeof(unsigned) * (size_t)(2 + 5 * n + 4);
   size_t tot = o_c + up(pl->counters_bytes);
   ce = cudaMalloc(&pl->d_block, tot);
@@ -338,6 +351,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   cudaMemcpy(base + o_g, grads.data(), sizeof(void*) * n, cudaMemcpyHostToDevice);
   cudaMemcpy(base + o_f, full_list.data(), sizeof(Task) * full_list.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(base + o_m, main_list.data(), sizeof(Task) * main_list.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(base + o_s, small_list.data(), sizeof(Task) * small_list.size(), cudaMemcpyHostToDevice);
   ce = cudaMemcpy(base + o_a, axpy_list.data(), sizeof(Task) * axpy_list.size(), cudaMemcpyHostToDevice);
   if (ce != cudaSuccess) { kaon_plan_destroy(pl); return cuda_fail(ce, "cudaMemcpy(plan tables)"); }
   pl->h_tensors = tens;
@@ -345,6 +359,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   pl->d_tasks_full = (Task*)(base + o_f); pl->n_tasks_full = (int)full_list.size();
   pl->d_tasks_main = (Task*)(base + o_m); pl->n_tasks_main = (int)main_list.size();
   pl->d_tasks_axpy = (Task*)(base + o_a); pl->n_tasks_axpy = (int)axpy_list.size();
+  pl->d_tasks_small = (Task*)(base + o_s); pl->n_tasks_small = (int)small_list.size();
   pl->d_counters = (unsigned*)(base + o_c);
   PlanView& v = pl->view;
   v.tensors = (const DevTensor*)(base + o_t);
