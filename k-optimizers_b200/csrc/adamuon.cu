@@ -7,31 +7,38 @@
 // the signal, no further momentum, scale 0.2*lr, and the cautious mask taken against the raw gradient.
 // 1-D tensors run the FLAT work item (Adam-style, momentum of the update) inside step (3)'s kernel.
 #include <algorithm>
+#include <cstring>
+#include <vector>
 
 #include "adakaon_dev.h"
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
+#include "kaon_packed.cuh"
+#include "ns_batch.h"
 
 namespace kaon {
 
-int ns_run(const __nv_bfloat16* x_in, long long R, long long C, int steps, __nv_bfloat16* out, void* ws,
-           unsigned* status, cudaStream_t stream, long long* launches);
-size_t ns_workspace_bytes(long long R, long long C);
-
 constexpr int ET = 256;
 
-// Row-chunk items [t0, t1) of ONE tensor: gradient and momentum straight from global memory.
+struct EmaOut { __nv_bfloat16* x; long long ld; };   // a tensor's matrix for Newton-Schulz and its row stride
+
+// The general form, a CTA per item (a run of whole rows): any row length, block size, centralization.  Gradient and
+// momentum straight from global memory; the item's sum of squares of what Newton-Schulz will read goes along.
 template <typename PT, int MK>
-__global__ void __launch_bounds__(ET) muon_ema_kernel(PlanView pv, const Task* tasks, int t0, int t1,
+__global__ void __launch_bounds__(ET) muon_ema_kernel(PlanView pv, const Task* tasks, int n_tasks,
                                                       float w1, float w1m1, int small_w1, int gc,
-                                                      __nv_bfloat16* x_out) {
+                                                      const EmaOut* outs, double* part) {
   using E = Elems<PT>;
   __shared__ unsigned rowmax_s[MAX_TASK_ROWS];
   __shared__ float scale_s[MAX_TASK_ROWS];
   __shared__ float mean_s[MAX_TASK_ROWS];  // centralization mean of each row of the item
+  __shared__ double red_s[ET / 32];
   const int tid = threadIdx.x;
-  for (int ti = t0 + blockIdx.x; ti < t1; ti += gridDim.x) {
+  for (int ti = blockIdx.x; ti < n_tasks; ti += gridDim.x) {
     const Task t = tasks[ti];
+    if (pv.grads[t.tensor] == nullptr) continue;
+    const EmaOut xo_t = outs[t.tensor];
+    double ss = 0.0;
     const DevTensor d = pv.tensors[t.tensor];
     const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]) + t.e0 * E::BYTES;
     const int n = t.n, C = d.cols;
@@ -166,20 +173,179 @@ __global__ void __launch_bounds__(ET) muon_ema_kernel(PlanView pv, const Task* t
       }
       // the matrix Newton-Schulz reads: bf16 of the fp32 pre-requant momentum
       if (cnt > 0) {
-        __nv_bfloat16* xo = x_out + t.e0 + (size_t)v * 8;
-        if (cnt == 8 && (reinterpret_cast<uintptr_t>(xo) & 15) == 0) {
-          *reinterpret_cast<uint4*>(xo) = make_uint4(pack_bf16_rn(mn[0], mn[1]), pack_bf16_rn(mn[2], mn[3]),
-                                                    pack_bf16_rn(mn[4], mn[5]), pack_bf16_rn(mn[6], mn[7]));
+        if (cnt == 8 && row_uniform) {   // (its rows are then not padded)
+          *reinterpret_cast<uint4*>(xo_t.x + t.e0 + (size_t)v * 8) =
+              make_uint4(pack_bf16_rn(mn[0], mn[1]), pack_bf16_rn(mn[2], mn[3]), pack_bf16_rn(mn[4], mn[5]), pack_bf16_rn(mn[6], mn[7]));
         } else {
-          for (int k = 0; k < cnt; ++k) xo[k] = __float2bfloat16_rn(mn[k]);
+          for (int k = 0; k < cnt; ++k) {
+            const int r = row_of((unsigned)(v * 8 + k), d);
+            xo_t.x[(t.row0 + r) * xo_t.ld + (v * 8 + k - r * C)] = __float2bfloat16_rn(mn[k]);
+          }
+        }
+        for (int k = 0; k < cnt; ++k) {
+          const float x = round_bf16(mn[k]);
+          ss += (double)x * (double)x;
         }
       }
+    }
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((tid & 31) == 0) red_s[tid >> 5] = ss;
+    __syncthreads();
+    if (tid == 0) {
+      double tot = 0.0;
+      for (int w = 0; w < ET / 32; ++w) tot += red_s[w];
+      part[t.slot] = tot;
     }
     __syncthreads();
   }
 }
 
-typedef void (*EmaKernel)(PlanView, const Task*, int, int, float, float, int, int, __nv_bfloat16*);
+// The common case (rows a multiple of eight elements, 4-bit blocks of 128, no centralization), a warp per unit: runs of
+// whole rows with int8 momentum (a row's maximum comes before its codes: two passes over the row, the second from
+// L1), flat runs otherwise.  No barriers; packed pairs; the unit's sum of squares of what Newton-Schulz will read goes
+// along.  (A CTA per 16 K-element item with scalar arithmetic and a separate norm pass: 2.4 + 1.2 ms on 453 M elements.)
+template <typename PT, int MK>
+__global__ void __launch_bounds__(ET, 4) muon_ema_fast_kernel(const __grid_constant__ PlanView pv, const Task* tasks, int n_tasks,
+                                                              float w1, float w1m1, int small_w1, const EmaOut* outs, double* part) {
+  using E = Elems<PT>;
+  const int lane = threadIdx.x & 31;
+  const int nw = gridDim.x * (ET / 32);
+  for (int i = __shfl_sync(0xffffffffu, (int)(blockIdx.x * (ET / 32) + (threadIdx.x >> 5)), 0); i < n_tasks; i += nw) {
+    const Task t = tasks[i];
+    const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
+    if (g == nullptr) continue;
+    const DevTensor& d = pv.tensors[t.tensor];
+    __nv_bfloat16* x_out = outs[t.tensor].x;
+    unsigned char* m = reinterpret_cast<unsigned char*>(d.m);
+    const int nv = MK == KAON_M_INT8 ? d.cols >> 3 : t.n >> 3;   // vectors of a row (or of the flat run)
+    const int rows = MK == KAON_M_INT8 ? t.n / d.cols : 1;
+    double ss = 0.0;
+    for (int r = 0; r < rows; ++r) {
+      const long long e0 = t.e0 + (long long)r * (MK == KAON_M_INT8 ? d.cols : 0);
+      const float row_sc = MK == KAON_M_INT8 ? d.m_scale[t.row0 + r] : 1.0f;
+      // the new momentum of vector v
+      auto fresh = [&](int v, f32x2 MN[4]) {
+        const long long e = e0 + v * 8ll;
+        float gx[8], mo[8];
+        E::load8(g + e * E::BYTES, gx);
+        if constexpr (MK == KAON_M_4BIT) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(m + (e >> 1));
+          const uint32_t wl = w & 0x0F0F0F0Fu, wh = (w >> 4) & 0x0F0F0F0Fu;
+          const float sc = d.m_scale[e >> 7];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const f32x2 x = mul2(add2(pack2(__uint_as_float(prmt(wl, 0x4B000000u, 0x7540u | (uint32_t)j)),
+                                            __uint_as_float(prmt(wh, 0x4B000000u, 0x7540u | (uint32_t)j))),
+                                      pack2(-8388616.0f, -8388616.0f)), pack2(sc, sc));
+            mo[2 * j] = x.x; mo[2 * j + 1] = x.y;
+          }
+        } else if constexpr (MK == KAON_M_INT8) {
+          const uint2 w = *reinterpret_cast<const uint2*>(m + e);
+          const uint32_t x0 = w.x ^ 0x80808080u, x1 = w.y ^ 0x80808080u;  // code + 128 in every byte
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t x = j < 2 ? x0 : x1, b = (uint32_t)(2 * (j & 1));
+            const f32x2 y = mul2(add2(pack2(__uint_as_float(prmt(x, 0x4B000000u, 0x7540u | b)),
+                                            __uint_as_float(prmt(x, 0x4B000000u, 0x7540u | (b + 1u)))),
+                                      pack2(-8388736.0f, -8388736.0f)), pack2(row_sc, row_sc));
+            mo[2 * j] = y.x; mo[2 * j + 1] = y.y;
+          }
+        } else if constexpr (MK == KAON_M_BF16) {
+          Elems<__nv_bfloat16>::load8(m + e * 2, mo);
+        } else if constexpr (MK == KAON_M_F32) {
+          Elems<float>::load8(m + e * 4, mo);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          f32x2 G = pack2(gx[2 * j], gx[2 * j + 1]);
+          if constexpr (MK == KAON_M_NONE) {
+            MN[j] = G;
+          } else {
+            const f32x2 M = pack2(mo[2 * j], mo[2 * j + 1]);
+            if constexpr (MK == KAON_M_BF16) G = pack2(round_bf16(G.x), round_bf16(G.y));
+            MN[j] = small_w1 ? fma2(pack2(w1, w1), sub2(G, M), M) : fma2(pack2(w1m1, w1m1), sub2(G, M), G);
+            if constexpr (MK == KAON_M_BF16) MN[j] = pack2(round_bf16(MN[j].x), round_bf16(MN[j].y));
+          }
+        }
+      };
+      auto amax8 = [](const f32x2 M[4]) {
+        float a = max3f(fabsf(M[0].x), fabsf(M[0].y), fabsf(M[1].x));
+        a = max3f(a, fabsf(M[1].y), fabsf(M[2].x));
+        a = max3f(a, fabsf(M[2].y), fabsf(M[3].x));
+        return fmaxf(a, fabsf(M[3].y));
+      };
+      float sc = 1.0f;
+      if constexpr (MK == KAON_M_INT8) {
+        float amax = 0.0f;
+#pragma unroll 2
+        for (int v = lane; v < nv; v += 32) {
+          f32x2 MN[4];
+          fresh(v, MN);
+          amax = fmaxf(amax, amax8(MN));
+        }
+        __syncwarp();
+        amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+        sc = div127_exact(fmaxf(amax, 1e-12f));
+      }
+      for (int v0 = 0; v0 < nv; v0 += 32) {
+        const int v = v0 + lane;
+        const bool act = v < nv;
+        f32x2 MN[4];
+        fresh(act ? v : 0, MN);
+        const long long e = e0 + v * 8ll;
+        if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(act ? amax8(MN) : 0.0f, lane), 1e-12f));
+        if (!act) continue;
+        if constexpr (MK == KAON_M_4BIT || MK == KAON_M_INT8) {
+          // rint(m'/sc) + magic, from the correctly rounded quotient
+          float inv;
+          asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
+          constexpr float MAGIC = MK == KAON_M_4BIT ? 12582920.0f : 12582912.0f;
+          uint32_t R[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const f32x2 INV = pack2(inv, inv), qq = mul2(MN[j], INV);
+            const f32x2 x = add2(fma2(fma2(qq, pack2(-sc, -sc), MN[j]), INV, qq), pack2(MAGIC, MAGIC));
+            R[2 * j] = __float_as_uint(x.x); R[2 * j + 1] = __float_as_uint(x.y);
+          }
+          if constexpr (MK == KAON_M_4BIT) {
+            uint32_t w = 0u;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w |= (R[k] & 0xFu) << (4 * k);
+            *reinterpret_cast<uint32_t*>(m + (e >> 1)) = w;
+            if ((lane & 15) == 0) d.m_scale[e >> 7] = sc;
+          } else {
+            *reinterpret_cast<uint2*>(m + e) = make_uint2(prmt(prmt(R[0], R[1], 0x0040u), prmt(R[2], R[3], 0x0040u), 0x5410u),
+                                                          prmt(prmt(R[4], R[5], 0x0040u), prmt(R[6], R[7], 0x0040u), 0x5410u));
+            if (v == 0) d.m_scale[t.row0 + r] = sc;
+          }
+        }
+        const uint4 x = make_uint4(pack_bf16_rn(MN[0].x, MN[0].y), pack_bf16_rn(MN[1].x, MN[1].y),
+                                   pack_bf16_rn(MN[2].x, MN[2].y), pack_bf16_rn(MN[3].x, MN[3].y));
+        *reinterpret_cast<uint4*>(x_out + e) = x;   // bf16 of the momentum before requantisation
+        if constexpr (MK == KAON_M_BF16) *reinterpret_cast<uint4*>(m + e * 2) = x;
+        if constexpr (MK == KAON_M_F32) {
+          float4* md = reinterpret_cast<float4*>(m + e * 4);
+          md[0] = make_float4(MN[0].x, MN[0].y, MN[1].x, MN[1].y);
+          md[1] = make_float4(MN[2].x, MN[2].y, MN[3].x, MN[3].y);
+        }
+        const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+        f32x2 q = pack2(0.0f, 0.0f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 y = pack2(bf16lo(xw[j]), bf16hi(xw[j]));
+          q = fma2(y, y, q);
+        }
+        ss += (double)(q.x + q.y);
+      }
+      __syncwarp();
+    }
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) part[t.slot] = ss;
+  }
+}
+
+typedef void (*EmaKernel)(PlanView, const Task*, int, float, float, int, int, const EmaOut*, double*);
+typedef void (*EmaFastKernel)(PlanView, const Task*, int, float, float, int, const EmaOut*, double*);
 
 template <typename PT>
 static EmaKernel pick_ema_pt(int mk) {
@@ -192,38 +358,170 @@ static EmaKernel pick_ema_pt(int mk) {
     default: return nullptr;
   }
 }
+template <typename PT>
+static EmaFastKernel pick_ema_fast_pt(int mk) {
+  switch (mk) {
+    case KAON_M_F32: return muon_ema_fast_kernel<PT, KAON_M_F32>;
+    case KAON_M_BF16: return muon_ema_fast_kernel<PT, KAON_M_BF16>;
+    case KAON_M_INT8: return muon_ema_fast_kernel<PT, KAON_M_INT8>;
+    case KAON_M_4BIT: return muon_ema_fast_kernel<PT, KAON_M_4BIT>;
+    case KAON_M_NONE: return muon_ema_fast_kernel<PT, KAON_M_NONE>;
+    default: return nullptr;
+  }
+}
 
 static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Matrices are independent of each other until the second-moment stage, so their EMA pre-pass and
-// Newton-Schulz chains run round robin on NS_LANES internal streams, each with a staging matrix and a
-// Newton-Schulz scratch of its own: when the last tiles of one matrix's GEMM leave most SMs idle, the next
-// matrix's kernels start on them.
-constexpr int NS_LANES = 3;
+// Matrices are independent of each other until the second-moment stage: they run in batches, every matrix of a batch
+// at the same stage of its chain in one launch (EMA, norms, three products per iteration).  A batch holds what NS_BATCH
+// bytes of scratch allow (a list of small matrices is one batch; a width-3072 DiT block is one).  Batches alternate
+// between NS_LANES internal streams with a scratch each, so that one's last tiles and pre-pass share the machine with
+// the other's products.
+constexpr int NS_LANES = 2;
+constexpr size_t NS_BATCH = (size_t)768 << 20;
 
 struct MuonLayout {
-  std::vector<size_t> o_off;  // per tensor: byte offset of O in the workspace (factored tensors)
-  size_t x0_off = 0, ns_off = 0, lane_stride = 0, total = 0;  // lane l: x0_off + l * lane_stride, ns_off + l * lane_stride
+  std::vector<size_t> o_off;     // per tensor: byte offset of O in the workspace (factored tensors)
+  std::vector<int> batch;        // per tensor: its batch, or -1
+  std::vector<size_t> s_off;     // per tensor: offset of its scratch inside its lane's
+  int n_batches = 0;
+  size_t scratch_off = 0, lane_stride = 0, total = 0;
 };
 
 static MuonLayout muon_layout(const kaon_plan* pl) {
   MuonLayout L;
   L.o_off.assign(pl->n_tensors, 0);
-  size_t cur = 0, max_x = 0, max_ns = 0;
+  L.s_off.assign(pl->n_tensors, 0);
+  L.batch.assign(pl->n_tensors, -1);
+  size_t cur = 0, used = 0;
   for (int i = 0; i < pl->n_tensors; ++i) {
     const DevTensor& t = pl->h_tensors[i];
     if (t.rows <= 0 || t.numel == 0) continue;
     L.o_off[i] = cur;
     cur += up256((size_t)t.numel * 2);
-    max_x = std::max(max_x, up256((size_t)t.numel * 2));
-    max_ns = std::max(max_ns, up256(ns_workspace_bytes(t.rows, t.cols)));
+    const size_t need = up256(ns_scratch_bytes(t.rows, t.cols));
+    if (L.n_batches == 0 || used + need > NS_BATCH) { ++L.n_batches; used = 0; }
+    L.batch[i] = L.n_batches - 1;
+    L.s_off[i] = used;
+    used += need;
+    L.lane_stride = std::max(L.lane_stride, used);
   }
-  L.x0_off = cur;
-  L.ns_off = cur + max_x;
-  L.lane_stride = max_x + max_ns;
-  cur += (size_t)NS_LANES * L.lane_stride;
-  L.total = cur + 256;
+  L.scratch_off = cur;
+  L.total = cur + (size_t)std::min(NS_LANES, std::max(L.n_batches, 1)) * L.lane_stride + 256;
   return L;
+}
+
+// What a plan keeps between steps: the batches' launch tables, rebuilt when the workspace, the number of iterations or
+// the set of matrices with a gradient changes.
+struct MuonHost {
+  MuonLayout layout;
+  struct Batch {
+    NsBatch ns;
+    size_t ns_off = 0;                    // its tables in `block`
+    int fast0 = 0, n_fast = 0;            // EMA units, general items of the tensors without units, items of all
+    int rest0 = 0, n_rest = 0;
+    int all0 = 0, n_all = 0;
+    int scale_f0 = 0, scale_a0 = 0, n_mats = 0;
+  };
+  std::vector<Batch> batches;
+  std::vector<char> key;                  // which tensors have a gradient
+  const void* base = nullptr;
+  int steps = 0;
+  unsigned char* block = nullptr;
+  size_t block_bytes = 0, off_fast = 0, off_rest = 0, off_all = 0, off_outs = 0, off_scale = 0, off_part = 0;
+};
+
+void muon_free(kaon_plan* pl) {
+  MuonHost* h = reinterpret_cast<MuonHost*>(pl->muon);
+  if (!h) return;
+  cudaFree(h->block);
+  delete h;
+  pl->muon = nullptr;
+}
+
+static int muon_build(kaon_plan* pl, MuonHost& h, unsigned char* ws, int steps, const std::vector<char>& key, cudaStream_t s) {
+  const int n = pl->n_tensors;
+  const MuonLayout& L = h.layout;
+  std::vector<Task> fast, rest, all;
+  std::vector<EmaOut> outs(n, EmaOut{nullptr, 0});
+  std::vector<NsScale> scales;
+  h.batches.assign(L.n_batches, MuonHost::Batch());
+  int slots = 0;
+  size_t tab = 0;
+  for (int b = 0; b < L.n_batches; ++b) {
+    MuonHost::Batch& B = h.batches[b];
+    B.fast0 = (int)fast.size(); B.rest0 = (int)rest.size(); B.all0 = (int)all.size();
+    std::vector<NsMat> mats;
+    std::vector<NsScale> sf, sa;
+    for (int i = 0; i < n; ++i) {
+      if (L.batch[i] != b || !key[i]) continue;
+      const DevTensor& t = pl->h_tensors[i];
+      NsMat m{};
+      m.R = t.rows; m.C = t.cols;
+      ns_scratch_layout(m, ws + L.scratch_off + (size_t)(b % NS_LANES) * L.lane_stride + L.s_off[i]);
+      m.out = reinterpret_cast<__nv_bfloat16*>(ws + L.o_off[i]);
+      mats.push_back(m);
+      outs[i] = EmaOut{m.x0, m.ld};
+      // general items: runs of whole rows
+      const int a0 = slots;
+      const size_t first = all.size();
+      for (long long r = 0; r < t.rows; r += t.chunk_rows) {
+        const long long nr = std::min<long long>(t.chunk_rows, t.rows - r);
+        all.push_back(Task{i, 0, r * t.cols, (int)(nr * t.cols), (int)r, slots++, 0});
+      }
+      sa.push_back(NsScale{a0, slots, m.scal});
+      const bool units = (t.cols & 7) == 0 && (pl->momentum_kind != KAON_M_4BIT || t.bshift == 7);
+      if (!units) {
+        rest.insert(rest.end(), all.begin() + (long)first, all.end());
+        sf.push_back(sa.back());
+        continue;
+      }
+      // a warp's units: about 4096 elements, of whole rows with int8 momentum
+      const int f0 = slots;
+      const long long len = pl->momentum_kind == KAON_M_INT8 ? std::max<long long>(1, 4096 / t.cols) * t.cols : 4096;
+      for (long long e = 0; e < t.numel; e += len)
+        fast.push_back(Task{i, 0, e, (int)std::min<long long>(len, t.numel - e), (int)(e / t.cols), slots++, 0});
+      sf.push_back(NsScale{f0, slots, m.scal});
+    }
+    B.n_fast = (int)fast.size() - B.fast0; B.n_rest = (int)rest.size() - B.rest0; B.n_all = (int)all.size() - B.all0;
+    B.n_mats = (int)mats.size();
+    B.scale_f0 = (int)scales.size(); scales.insert(scales.end(), sf.begin(), sf.end());
+    B.scale_a0 = (int)scales.size(); scales.insert(scales.end(), sa.begin(), sa.end());
+    if (int rc = ns_batch_build(mats, steps, B.ns)) return rc;
+    B.ns_off = tab;
+    tab += up256(B.ns.bytes);
+  }
+  size_t o = tab;
+  auto take = [&](size_t bytes) { const size_t at = o; o += up256(std::max<size_t>(bytes, 1)); return at; };
+  h.off_fast = take(sizeof(Task) * fast.size());
+  h.off_rest = take(sizeof(Task) * rest.size());
+  h.off_all = take(sizeof(Task) * all.size());
+  h.off_outs = take(sizeof(EmaOut) * outs.size());
+  h.off_scale = take(sizeof(NsScale) * scales.size());
+  const size_t uploaded = o;
+  h.off_part = take(sizeof(double) * (size_t)slots);
+  if (o > h.block_bytes) {
+    if (h.block) { KAON_CUDA(cudaStreamSynchronize(s)); cudaFree(h.block); h.block = nullptr; }
+    KAON_CUDA(cudaMalloc((void**)&h.block, o));
+    pl->device_bytes += (int64_t)(o - h.block_bytes);
+    h.block_bytes = o;
+  }
+  std::vector<unsigned char> img(uploaded, 0);
+  for (const MuonHost::Batch& B : h.batches)
+    if (B.ns.bytes) std::memcpy(img.data() + B.ns_off, B.ns.host.data(), B.ns.bytes);
+  auto put = [&](size_t at, const void* src, size_t bytes) { if (bytes) std::memcpy(img.data() + at, src, bytes); };
+  put(h.off_fast, fast.data(), sizeof(Task) * fast.size());
+  put(h.off_rest, rest.data(), sizeof(Task) * rest.size());
+  put(h.off_all, all.data(), sizeof(Task) * all.size());
+  put(h.off_outs, outs.data(), sizeof(EmaOut) * outs.size());
+  put(h.off_scale, scales.data(), sizeof(NsScale) * scales.size());
+  // pageable source: staged before the call returns, ordered on the step's stream after the steps before it
+  KAON_CUDA(cudaMemcpyAsync(h.block, img.data(), uploaded, cudaMemcpyHostToDevice, s));
+  for (MuonHost::Batch& B : h.batches) { B.ns.host.clear(); B.ns.host.shrink_to_fit(); }
+  h.key = key;
+  h.base = ws;
+  h.steps = steps;
+  return KAON_OK;
 }
 
 }  // namespace kaon
@@ -252,31 +550,29 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
   if (h->ns_steps < 1) return fail(KAON_E_INVALID, "ns_steps must be >= 1");
   const bool has_m = pl->momentum_kind != KAON_M_NONE;
   if (has_m != (h->beta1 > 0.0)) return fail(KAON_E_INVALID, "beta1 %g does not match the plan's momentum kind", h->beta1);
-  const MuonLayout L = muon_layout(pl);
+  if (!pl->muon) {
+    MuonHost* fresh = new MuonHost();
+    fresh->layout = muon_layout(pl);
+    pl->muon = fresh;
+  }
+  MuonHost& H = *reinterpret_cast<MuonHost*>(pl->muon);
+  const MuonLayout& L = H.layout;
   if (!workspace || ((uintptr_t)workspace & 255) || workspace_bytes < (int64_t)L.total)
     return fail(KAON_E_INVALID, "kaon_adamuon_step: workspace missing, misaligned or smaller than %zu bytes", L.total);
   cudaStream_t s = (cudaStream_t)stream;
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
   const int n = pl->n_tensors;
 
-  // one-time: row-chunk work list of the factored tensors; per-workspace: the O pointers
-  if (!pl->d_tasks_ema) {
-    std::vector<Task> list;
-    pl->ema_begin.assign(n + 1, 0);
-    for (int i = 0; i < n; ++i) {
-      pl->ema_begin[i] = (int)list.size();
-      const DevTensor& t = pl->h_tensors[i];
-      if (t.rows <= 0 || t.numel == 0) continue;
-      for (long long r = 0; r < t.rows; r += t.chunk_rows) {
-        const long long nr = std::min<long long>(t.chunk_rows, t.rows - r);
-        list.push_back(Task{i, 0, r * t.cols, (int)(nr * t.cols), (int)r, 0, 0});
-      }
-    }
-    pl->ema_begin[n] = (int)list.size();
-    KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_ema, sizeof(Task) * std::max<size_t>(list.size(), 1)));
-    KAON_CUDA(cudaMemcpy(pl->d_tasks_ema, list.data(), sizeof(Task) * list.size(), cudaMemcpyHostToDevice));
+  // one-time: the O column; per workspace, iteration count and set of gradients: the batches' tables
+  if (!pl->d_signal) {
     KAON_CUDA(cudaMalloc((void**)&pl->d_signal, sizeof(void*) * (size_t)n));
-    pl->device_bytes += (int64_t)(sizeof(Task) * list.size() + sizeof(void*) * n);
+    pl->device_bytes += (int64_t)(sizeof(void*) * n);
+  }
+  {
+    std::vector<char> key(n, 0);
+    for (int i = 0; i < n; ++i) key[i] = L.batch[i] >= 0 && pl->h_grads[i] != nullptr;
+    if (H.base != workspace || H.steps != h->ns_steps || H.key != key)
+      if (int rc = muon_build(pl, H, ws, h->ns_steps, key, s)) { H.base = nullptr; return rc; }
   }
   if (pl->signal_base != workspace) {
     std::vector<const void*> sig(n, nullptr);
@@ -287,16 +583,18 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
   }
 
   const float w1 = (float)(1.0 - h->beta1);
-  EmaKernel ek = pl->param_dtype == KAON_DT_BF16 ? pick_ema_pt<__nv_bfloat16>(pl->momentum_kind)
-                                                 : pick_ema_pt<float>(pl->momentum_kind);
-  if (!ek) return fail(KAON_E_INVALID, "no AdaMuon EMA kernel for this dtype combination");
+  const bool bf = pl->param_dtype == KAON_DT_BF16;
+  EmaKernel ek = bf ? pick_ema_pt<__nv_bfloat16>(pl->momentum_kind) : pick_ema_pt<float>(pl->momentum_kind);
+  EmaFastKernel ef = bf ? pick_ema_fast_pt<__nv_bfloat16>(pl->momentum_kind) : pick_ema_fast_pt<float>(pl->momentum_kind);
+  if (!ek || !ef) return fail(KAON_E_INVALID, "no AdaMuon EMA kernel for this dtype combination");
   PlanView v = pl->view;
   v.signal = pl->d_signal;
   KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
 
-  // (1) + (2): per factored tensor with a gradient: EMA pre-pass, then Newton-Schulz into its O slot,
-  // round robin over the lanes (forked from the caller's stream, joined before stage 3)
-  if (!pl->muon_lanes_ready) {
+  // (1) + (2): batch by batch, EMA pre-pass and Newton-Schulz into the O slots, on the caller's stream or (more than
+  // one batch) alternating over the lanes, forked from it and joined before stage 3
+  const bool lanes = H.batches.size() > 1;
+  if (lanes && !pl->muon_lanes_ready) {
     for (int l = 0; l < NS_LANES; ++l) {
       KAON_CUDA(cudaStreamCreateWithFlags(&pl->muon_stream[l], cudaStreamNonBlocking));
       KAON_CUDA(cudaEventCreateWithFlags(&pl->muon_join[l], cudaEventDisableTiming));
@@ -304,29 +602,39 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
     KAON_CUDA(cudaEventCreateWithFlags(&pl->muon_fork, cudaEventDisableTiming));
     pl->muon_lanes_ready = true;
   }
-  KAON_CUDA(cudaEventRecord(pl->muon_fork, s));
-  for (int l = 0; l < NS_LANES; ++l) KAON_CUDA(cudaStreamWaitEvent(pl->muon_stream[l], pl->muon_fork, 0));
-  int turn = 0;
-  for (int i = 0; i < n; ++i) {
-    const DevTensor& t = pl->h_tensors[i];
-    if (t.rows <= 0 || t.numel == 0 || pl->h_grads[i] == nullptr) continue;
-    const int lane = turn++ % NS_LANES;
-    cudaStream_t sl = pl->muon_stream[lane];
-    __nv_bfloat16* x0 = reinterpret_cast<__nv_bfloat16*>(ws + L.x0_off + (size_t)lane * L.lane_stride);
-    const int t0 = pl->ema_begin[i], t1 = pl->ema_begin[i + 1];
-    const int grid = std::min(t1 - t0, pl->sm_count * 8);
-    ek<<<grid, ET, 0, sl>>>(v, pl->d_tasks_ema, t0, t1, w1, w1 - 1.0f, w1 < 0.5f, h->gradient_centralization != 0, x0);
-    KAON_CUDA(cudaGetLastError());
-    pl->launches += 1;
-    long long nl = 0;
-    int rc = ns_run(x0, t.rows, t.cols, h->ns_steps, reinterpret_cast<__nv_bfloat16*>(ws + L.o_off[i]),
-                    ws + L.ns_off + (size_t)lane * L.lane_stride, v.status, sl, &nl);
-    pl->launches += nl;
-    if (rc) return rc;
+  if (lanes) {
+    KAON_CUDA(cudaEventRecord(pl->muon_fork, s));
+    for (int l = 0; l < NS_LANES; ++l) KAON_CUDA(cudaStreamWaitEvent(pl->muon_stream[l], pl->muon_fork, 0));
   }
-  for (int l = 0; l < NS_LANES; ++l) {
-    KAON_CUDA(cudaEventRecord(pl->muon_join[l], pl->muon_stream[l]));
-    KAON_CUDA(cudaStreamWaitEvent(s, pl->muon_join[l], 0));
+  const bool gc = h->gradient_centralization != 0;
+  const EmaOut* outs = reinterpret_cast<const EmaOut*>(H.block + H.off_outs);
+  double* part = reinterpret_cast<double*>(H.block + H.off_part);
+  for (size_t b = 0; b < H.batches.size(); ++b) {
+    const MuonHost::Batch& B = H.batches[b];
+    if (B.n_mats == 0) continue;
+    cudaStream_t sl = lanes ? pl->muon_stream[b % NS_LANES] : s;
+    const int n_gen = gc ? B.n_all : B.n_rest;   // centralization takes the general form throughout
+    if (!gc && B.n_fast) {
+      const int grid = std::min((B.n_fast + ET / 32 - 1) / (ET / 32), pl->sm_count * 4);
+      ef<<<grid, ET, 0, sl>>>(v, reinterpret_cast<const Task*>(H.block + H.off_fast) + B.fast0, B.n_fast, w1, w1 - 1.0f, w1 < 0.5f, outs, part);
+      pl->launches += 1;
+    }
+    if (n_gen) {
+      const Task* list = gc ? reinterpret_cast<const Task*>(H.block + H.off_all) + B.all0 : reinterpret_cast<const Task*>(H.block + H.off_rest) + B.rest0;
+      ek<<<std::min(n_gen, pl->sm_count * 8), ET, 0, sl>>>(v, list, n_gen, w1, w1 - 1.0f, w1 < 0.5f, gc, outs, part);
+      pl->launches += 1;
+    }
+    ns_batch_scale(reinterpret_cast<const NsScale*>(H.block + H.off_scale) + (gc ? B.scale_a0 : B.scale_f0), B.n_mats, part, sl);
+    KAON_CUDA(cudaGetLastError());
+    long long nl = 1;
+    if (int rc = ns_batch_run(B.ns, H.block + B.ns_off, v.status, sl, &nl)) return rc;
+    pl->launches += nl;
+  }
+  if (lanes) {
+    for (int l = 0; l < NS_LANES; ++l) {
+      KAON_CUDA(cudaEventRecord(pl->muon_join[l], pl->muon_stream[l]));
+      KAON_CUDA(cudaStreamWaitEvent(s, pl->muon_join[l], 0));
+    }
   }
 
   // (3) second moment of O, clip, scale, cautious, weight write (and the whole 1-D branch)

@@ -150,10 +150,9 @@ struct kaon_plan {
   std::vector<kaon::DevTensor> h_tensors;   // host copy of the table
   std::vector<const void*> h_grads;         // host copy of the gradient-pointer column
   // AdaMuon only (built lazily by the first step)
-  kaon::Task* d_tasks_ema = nullptr;         // row-chunk items of the factored tensors, tensor by tensor
-  std::vector<int> ema_begin;                // [n_tensors + 1] ranges into d_tasks_ema
   const void** d_signal = nullptr;           // per-tensor pointer to O in the caller's workspace
   const void* signal_base = nullptr;         // workspace the pointers were computed for
+  void* muon = nullptr;                      // the batches' launch tables (adamuon.cu)
   bool muon_lanes_ready = false;             // internal streams of the per-matrix Newton-Schulz chains
   cudaStream_t muon_stream[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t muon_join[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -192,4 +191,5 @@ struct kaon_plan {
 namespace kaon {
 void pnm_free(kaon_plan* pl);
 void kp_free(kaon_plan* pl);
+void muon_free(kaon_plan* pl);
 }

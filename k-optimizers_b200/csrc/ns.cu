@@ -10,9 +10,15 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <cstring>
+#include <functional>
+#include <queue>
+#include <vector>
 
 #include "kaon_host.h"
+#include "ns_batch.h"
 #include "ns_gemm.cuh"
 
 namespace kaon {
@@ -66,10 +72,36 @@ __global__ void ns_gemm_simple_kernel(const __nv_bfloat16* A, int a_mn, long lon
   p.out[(long long)i * p.ld_out + j] = __float2bfloat16_rn(acc * alpha + beta * x);
 }
 
-static int g_gemm_sms[64] = {0};  // multiprocessors per device, once the kernel's shared-memory limit is set
+// always the shared memory of the widest tile: one CTA per SM, whose tensor-memory allocation (all 512
+// columns) then never waits for a neighbour
+constexpr size_t G2_SMEM = 1024 + (size_t)G2_STAGES * (G_A_BYTES + (size_t)G_MAX_BN * G_BK * 2);
+
+static std::atomic<int> g_gemm_sms[64];  // multiprocessors per device, once the kernel's shared-memory limit is set
+
+static int gemm_sms(int* out) {
+  int dev = 0;
+  KAON_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return fail(KAON_E_UNSUPPORTED, "device index %d", dev);
+  if (!g_gemm_sms[dev].load()) {
+    KAON_CUDA(cudaFuncSetAttribute((const void*)ns_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G2_SMEM));
+    KAON_CUDA(cudaFuncSetAttribute((const void*)ns_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G2_SMEM));
+    int sms = 0;
+    KAON_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    g_gemm_sms[dev].store(sms);
+  }
+  *out = g_gemm_sms[dev].load();
+  return KAON_OK;
+}
+
+static int operand_maps(NsProblem& pr, const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb) {
+  const GemmParams& p = pr.p;
+  int rc = p.a_mn ? make_map(&pr.a, A, p.M, p.K, lda, 64) : make_map(&pr.a, A, p.K, p.M, lda, G_BM);
+  if (rc) return rc;
+  return p.b_mn ? make_map(&pr.b, B, p.N, p.K, ldb, 64) : make_map(&pr.b, B, p.K, p.N, ldb, p.BN);
+}
 
 // out[M,N] = bf16(alpha * A(m,:) . B(n,:) + beta * aux)
-int launch_ns_gemm(const __nv_bfloat16* A, bool a_mn, long long lda, const __nv_bfloat16* B, bool b_mn, long long ldb,
+static int launch_ns_gemm(const __nv_bfloat16* A, bool a_mn, long long lda, const __nv_bfloat16* B, bool b_mn, long long ldb,
                    int M, int N, int K, float alpha, float beta, const float* dev_scale, const __nv_bfloat16* aux,
                    long long ld_aux, __nv_bfloat16* out, long long ld_out, unsigned* status, cudaStream_t stream,
                    long long* launches, bool sym = false) {
@@ -77,7 +109,7 @@ int launch_ns_gemm(const __nv_bfloat16* A, bool a_mn, long long lda, const __nv_
   p.sym = sym && M == N ? 1 : 0;
   p.M = M; p.N = N; p.K = K; p.a_mn = a_mn; p.b_mn = b_mn;
   p.alpha = alpha; p.beta = aux ? beta : 0.0f; p.dev_scale = dev_scale;
-  p.aux = aux; p.ld_aux = ld_aux; p.out = out; p.ld_out = ld_out; p.status = status;
+  p.aux = aux; p.ld_aux = ld_aux; p.out = out; p.ld_out = ld_out;
   const bool tma_ok = (lda % 8 == 0) && (ldb % 8 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)B % 16 == 0);
   if (launches) *launches += 1;
   if (!tma_ok) {
@@ -87,47 +119,16 @@ int launch_ns_gemm(const __nv_bfloat16* A, bool a_mn, long long lda, const __nv_
     return KAON_OK;
   }
   p.BN = N >= 256 ? 256 : (N > 64 ? 128 : 64);
-  if (p.sym && N >= 256) {
-    // Persistent CTAs share the computed tiles out evenly: take the tile width whose busiest SM has the
-    // least work (tiles per SM x width); narrower tiles balance better but feed the tensor cores worse,
-    // so 256 keeps a 10 % edge.
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    auto cost = [&](int bn) {
-      long long tiles = 0;
-      for (int m0 = 0; m0 < M; m0 += G_BM)
-        for (int n0 = 0; n0 < N; n0 += bn)
-          if (n0 + bn > m0) ++tiles;
-      return ((tiles + sms - 1) / sms) * (long long)bn;
-    };
-    if (cost(192) * 100 < cost(256) * 90) p.BN = 192;
-  }
-  CUtensorMap ma, mb;
-  int rc;
-  if (a_mn) rc = make_map(&ma, A, M, K, lda, 64); else rc = make_map(&ma, A, K, M, lda, G_BM);
-  if (rc) return rc;
-  if (b_mn) rc = make_map(&mb, B, N, K, ldb, 64); else rc = make_map(&mb, B, K, N, ldb, p.BN);
-  if (rc) return rc;
-  // always the shared memory of the widest tile: one CTA per SM, whose tensor-memory allocation (all 512
-  // columns) then never waits for a neighbour
-  const size_t smem = 1024 + (size_t)G2_STAGES * (G_A_BYTES + (size_t)G_MAX_BN * G_BK * 2);
-  int dev = 0;
-  KAON_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return fail(KAON_E_UNSUPPORTED, "device index %d", dev);
-  if (!g_gemm_sms[dev]) {
-    KAON_CUDA(cudaFuncSetAttribute((const void*)ns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(1024 + (size_t)G2_STAGES * (G_A_BYTES + (size_t)G_MAX_BN * G_BK * 2))));
-    int sms = 0;
-    KAON_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    g_gemm_sms[dev] = sms;
-  }
+  NsProblem pr{};
+  pr.p = p;
+  if (int rc = operand_maps(pr, A, lda, B, ldb)) return rc;
+  int sms = 0;
+  if (int rc = gemm_sms(&sms)) return rc;
   // computed tiles: all of them, or in symmetric mode those that reach the diagonal
   const int tm = (M + G_BM - 1) / G_BM, tn = (N + p.BN - 1) / p.BN;
   int total = 0;
   for (int mi = 0; mi < tm; ++mi) total += tn - (p.sym ? std::min(tn, (mi * G_BM) / p.BN) : 0);
-  const int grid = std::min(total, g_gemm_sms[dev]);
-  ns_gemm_kernel<<<grid, G2_THREADS, smem, stream>>>(ma, mb, p, total);
+  ns_gemm_kernel<false><<<std::min(total, sms), G2_THREADS, G2_SMEM, stream>>>(pr, NsWork{total, nullptr, nullptr, nullptr, status});
   KAON_CUDA(cudaGetLastError());
   return KAON_OK;
 }
@@ -163,14 +164,14 @@ __global__ void ns_scale_kernel(const double* partial, int n, float* scal) {
 
 constexpr int NS_PARTIALS = 296;
 
-size_t ns_workspace_bytes(long long R, long long C) {
+static size_t ns_workspace_bytes(long long R, long long C) {
   const long long r = std::min(R, C);
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   return up((size_t)R * C * 2) + 2 * up((size_t)r * r * 2) + up(NS_PARTIALS * 8) + 256;
 }
 
 // x_in [R,C] bf16 (unnormalised) -> out [R,C] bf16.  out may not alias x_in.  ws >= ns_workspace_bytes.
-int ns_run(const __nv_bfloat16* x_in, long long R, long long C, int steps, __nv_bfloat16* out, void* ws,
+static int ns_run(const __nv_bfloat16* x_in, long long R, long long C, int steps, __nv_bfloat16* out, void* ws,
            unsigned* status, cudaStream_t stream, long long* launches) {
   const bool tall = R > C;             // stored matrix is X^T (k rows, r columns)
   const long long r = tall ? C : R, k = tall ? R : C;
@@ -209,6 +210,179 @@ int ns_run(const __nv_bfloat16* x_in, long long R, long long C, int steps, __nv_
     if (rc) return rc;
     cur = nxt;
   }
+  return KAON_OK;
+}
+
+// ---------------------------------------------------------------------------------------------------
+// A batch of matrices: every matrix at the same stage of the iteration in one grouped launch.
+
+// scal of every matrix from its partial sums of squares: one CTA per matrix, partials in a fixed order.
+__global__ void __launch_bounds__(256) ns_batch_scale_kernel(const NsScale* mats, const double* part) {
+  __shared__ double red[8];
+  const NsScale m = mats[blockIdx.x];
+  double acc = 0.0;
+  for (int i = m.begin + threadIdx.x; i < m.end; i += 256) acc += part[i];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[w];
+    const float den = round_bf16(round_bf16((float)sqrt(t)) + 1e-7f);
+    const float s = 1.0f / den;
+    m.scal[0] = s * s; m.scal[1] = 0.0f; m.scal[2] = s; m.scal[3] = s;
+  }
+}
+
+void ns_batch_scale(const NsScale* mats, int n, const double* part, cudaStream_t s) {
+  ns_batch_scale_kernel<<<n, 256, 0, s>>>(mats, part);
+}
+
+static long long pad8(long long x) { return (x + 7) / 8 * 8; }
+
+size_t ns_scratch_bytes(long long R, long long C) {
+  const long long r = std::min(R, C);
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  return 2 * up((size_t)R * pad8(C) * 2) + 2 * up((size_t)r * pad8(r) * 2) + 256;
+}
+
+void ns_scratch_layout(NsMat& m, unsigned char* base) {
+  const long long r = std::min(m.R, m.C);
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  m.ld = pad8(m.C); m.lr = pad8(r);
+  m.x0 = reinterpret_cast<__nv_bfloat16*>(base); base += up((size_t)m.R * m.ld * 2);
+  m.xb = reinterpret_cast<__nv_bfloat16*>(base); base += up((size_t)m.R * m.ld * 2);
+  m.A = reinterpret_cast<__nv_bfloat16*>(base); base += up((size_t)r * m.lr * 2);
+  m.B = reinterpret_cast<__nv_bfloat16*>(base); base += up((size_t)r * m.lr * 2);
+  m.scal = reinterpret_cast<float*>(base);
+}
+
+// Tiles of one stage shared out over the CTAs, the longest first to the CTA with the least work.  The cost of a tile is
+// its bytes from L2 per k-block (128 + BN rows of 128 bytes: what a tile of up to 256 columns waits for, not the
+// tensor cores) times its k-blocks, plus its epilogue.  Returns the longest CTA's work.
+static long long share_out(const std::vector<NsProblem>& probs, int sms, std::vector<NsTile>* tiles, std::vector<int>* begin) {
+  struct T { long long cost; NsTile t; };
+  std::vector<T> all;
+  for (int i = 0; i < (int)probs.size(); ++i) {
+    const GemmParams& p = probs[i].p;
+    const int tm = (p.M + G_BM - 1) / G_BM, tn = (p.N + p.BN - 1) / p.BN;
+    const long long cost = (long long)((p.K + G_BK - 1) / G_BK) * (128 + p.BN) + 400 + p.BN;
+    for (int mi = 0; mi < tm; ++mi)
+      for (int ni = p.sym ? std::min(tn, mi * G_BM / p.BN) : 0; ni < tn; ++ni) all.push_back(T{cost, NsTile{i, (short)mi, (short)ni}});
+  }
+  std::stable_sort(all.begin(), all.end(), [](const T& a, const T& b) { return a.cost > b.cost; });
+  const int grid = std::min<int>(sms, (int)all.size());
+  typedef std::pair<long long, int> Load;
+  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> q;
+  for (int c = 0; c < grid; ++c) q.push(Load(0, c));
+  std::vector<std::vector<NsTile>> mine(grid);
+  long long most = 0;
+  for (const T& t : all) {
+    Load l = q.top(); q.pop();
+    l.first += t.cost;
+    most = std::max(most, l.first);
+    mine[l.second].push_back(t.t);
+    q.push(l);
+  }
+  if (tiles) {
+    for (int c = 0; c < grid; ++c) {
+      begin->push_back((int)tiles->size());
+      tiles->insert(tiles->end(), mine[c].begin(), mine[c].end());
+    }
+    begin->push_back((int)tiles->size());
+  }
+  return most;
+}
+
+// The launches of a batch's iterations.  Tile widths: the one of 256 / 192 / 128 / 64 columns (the same for a stage)
+// whose longest CTA has the least work: wide tiles need fewer bytes, narrow ones fill the machine.
+int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsBatch& out) {
+  out = NsBatch{};
+  if (mats.empty()) return KAON_OK;
+  int sms = 0;
+  if (int rc = gemm_sms(&sms)) return rc;
+  const float a = 3.4445f, b = -4.7750f, c = 2.0315f;
+  std::vector<NsProblem> probs;
+  std::vector<NsTile> tiles;
+  std::vector<int> begin;
+  for (int it = 0; it < steps; ++it) {
+    for (int stage = 0; stage < 3; ++stage) {
+      struct Op { const __nv_bfloat16 *A, *B; long long lda, ldb; };
+      std::vector<NsProblem> ps(mats.size());
+      std::vector<Op> ops(mats.size());
+      for (size_t i = 0; i < mats.size(); ++i) {
+        const NsMat& m = mats[i];
+        const bool tall = m.R > m.C;   // the stored matrix is X^T (k rows, r columns)
+        const int r = (int)std::min(m.R, m.C), k = (int)std::max(m.R, m.C);
+        // ping-pong; the last iteration lands in `out`
+        const bool last = it == steps - 1;
+        const __nv_bfloat16* cur = (it & 1) ? m.xb : m.x0;
+        __nv_bfloat16* nxt = last ? m.out : (it & 1) ? m.x0 : m.xb;
+        GemmParams p{};
+        Op op{};
+        if (stage == 0) {          // A = X X^T
+          op = Op{cur, cur, m.ld, m.ld};
+          p.M = r; p.N = r; p.K = k; p.a_mn = tall; p.b_mn = tall; p.alpha = 1.0f; p.sym = 1;
+          p.dev_scale = it == 0 ? m.scal : nullptr;
+          p.out = m.A; p.ld_out = m.lr;
+        } else if (stage == 1) {   // B = b A + c A A   (A symmetric: A A = A A^T, both operands K-major)
+          op = Op{m.A, m.A, m.lr, m.lr};
+          p.M = r; p.N = r; p.K = r; p.alpha = c; p.beta = b; p.sym = 1;
+          p.aux = m.A; p.ld_aux = m.lr; p.out = m.B; p.ld_out = m.lr;
+        } else {                   // X <- a X + B X; stored transposed: X^T <- a X^T + X^T B
+          op = tall ? Op{cur, m.B, m.ld, m.lr} : Op{m.B, cur, m.lr, m.ld};
+          p.M = tall ? k : r; p.N = tall ? r : k; p.K = r; p.b_mn = !tall; p.alpha = 1.0f; p.beta = a;
+          p.dev_scale = it == 0 ? m.scal + 2 : nullptr;
+          p.aux = cur; p.ld_aux = m.ld; p.out = nxt; p.ld_out = last ? m.C : m.ld;
+        }
+        ps[i].p = p;
+        ops[i] = op;
+      }
+      int best = 256;
+      long long least = 0;
+      for (int bn : {256, 192, 128, 64}) {
+        for (NsProblem& pr : ps) pr.p.BN = std::min(bn, (pr.p.N + 63) / 64 * 64);
+        const long long most = share_out(ps, sms, nullptr, nullptr);
+        if (least == 0 || most < least) { least = most; best = bn; }
+      }
+      for (size_t i = 0; i < ps.size(); ++i) {
+        ps[i].p.BN = std::min(best, (ps[i].p.N + 63) / 64 * 64);
+        if (int rc = operand_maps(ps[i], ops[i].A, ops[i].lda, ops[i].B, ops[i].ldb)) return rc;
+      }
+      std::vector<NsTile> tl;
+      std::vector<int> bg;
+      share_out(ps, sms, &tl, &bg);
+      out.stages.push_back(NsStage{(int)probs.size(), (int)tiles.size(), (int)begin.size(), (int)bg.size() - 1});
+      probs.insert(probs.end(), ps.begin(), ps.end());
+      tiles.insert(tiles.end(), tl.begin(), tl.end());
+      begin.insert(begin.end(), bg.begin(), bg.end());
+    }
+  }
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  const size_t o_t = up(sizeof(NsProblem) * probs.size()), o_b = o_t + up(sizeof(NsTile) * tiles.size());
+  out.bytes = o_b + up(sizeof(int) * begin.size());
+  out.host.assign(out.bytes, 0);
+  std::memcpy(out.host.data(), probs.data(), sizeof(NsProblem) * probs.size());
+  std::memcpy(out.host.data() + o_t, tiles.data(), sizeof(NsTile) * tiles.size());
+  std::memcpy(out.host.data() + o_b, begin.data(), sizeof(int) * begin.size());
+  out.off_tiles = o_t;
+  out.off_begin = o_b;
+  return KAON_OK;
+}
+
+// One grouped launch per stage, from the tables at `dev` (the bytes of NsBatch::host).
+int ns_batch_run(const NsBatch& b, const unsigned char* dev, unsigned* status, cudaStream_t s, long long* launches) {
+  const NsProblem none{};
+  for (const NsStage& st : b.stages) {
+    NsWork w{};
+    w.probs = reinterpret_cast<const NsProblem*>(dev) + st.prob0;
+    w.tiles = reinterpret_cast<const NsTile*>(dev + b.off_tiles) + st.tile0;
+    w.begin = reinterpret_cast<const int*>(dev + b.off_begin) + st.begin0;
+    w.status = status;
+    ns_gemm_kernel<true><<<st.grid, G2_THREADS, G2_SMEM, s>>>(none, w);
+    *launches += 1;
+  }
+  KAON_CUDA(cudaGetLastError());
   return KAON_OK;
 }
 

@@ -34,7 +34,6 @@ struct GemmParams {
   long long ld_aux;
   __nv_bfloat16* out;        // [M, ld_out]
   long long ld_out;
-  unsigned* status;          // device status word (bounded waits)
   int sym;                   // the product is symmetric (M == N, same operand on both sides): tiles that lie
                              // wholly below the diagonal are not computed; every computed tile also stores
                              // its transpose, which fills them
@@ -136,9 +135,27 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int tn, int c, 
   }
 }
 
+// One product of a grouped launch, in device memory.
+struct alignas(128) NsProblem {
+  CUtensorMap a, b;
+  GemmParams p;
+};
+struct NsTile { int prob; short mi, ni; };
+
+// What a launch works on.  One product (a Newton-Schulz call on its own): `one` is a kernel argument, CTA b takes tiles
+// b, b + grid, ...  GROUPED (every matrix of a batch at the same stage of the iteration): the products lie in device
+// memory and CTA b takes tiles[begin[b]] .. tiles[begin[b + 1]], shared out by the host so that all finish together.
+struct NsWork {
+  int total;
+  const NsProblem* probs;
+  const NsTile* tiles;
+  const int* begin;
+  unsigned* status;
+};
+
+template <bool GROUPED>
 __global__ void __launch_bounds__(G2_THREADS, 1)
-ns_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p,
-               int total_tiles) {
+ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ NsWork work) {
   extern __shared__ __align__(1024) unsigned char gsm[];
   __shared__ __align__(8) uint64_t full_bar[G2_STAGES];
   __shared__ __align__(8) uint64_t empty_bar[G2_STAGES];
@@ -147,12 +164,22 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __shared__ uint32_t tmem_base_s;
   __shared__ int fail_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int b_bytes = p.BN * G_BK * 2;
-  const int stage_bytes = G_A_BYTES + b_bytes;
+  constexpr int stage_bytes = G_A_BYTES + G_MAX_BN * G_BK * 2;
   // 1024-byte aligned tile base (the swizzle pattern is a function of address bits 4..9)
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gsm) + 1023) & ~uintptr_t(1023));
-  const int kblocks = (p.K + G_BK - 1) / G_BK;
-  const int tn = (p.N + p.BN - 1) / p.BN;
+  const int c_first = GROUPED ? work.begin[blockIdx.x] : (int)blockIdx.x;
+  const int c_end = GROUPED ? work.begin[blockIdx.x + 1] : work.total, c_step = GROUPED ? 1 : (int)gridDim.x;
+  // the product and the tile with number c
+  auto tile_of = [&](int c, int& mi, int& ni) -> const NsProblem* {
+    if constexpr (GROUPED) {
+      const NsTile t = work.tiles[c];
+      mi = t.mi; ni = t.ni;
+      return work.probs + t.prob;
+    } else {
+      tile_coords(one.p, (one.p.N + one.p.BN - 1) / one.p.BN, c, mi, ni);
+      return &one;
+    }
+  };
   volatile int* fail = &fail_s;
 
   if (tid == 0) {
@@ -173,27 +200,31 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // ---- TMA producer ----
     if (lane == 0) {
       unsigned it = 0;
-      for (int c = blockIdx.x; c < total_tiles && !*fail; c += gridDim.x) {
+      for (int c = c_first; c < c_end && !*fail; c += c_step) {
         int mi, ni;
-        tile_coords(p, tn, c, mi, ni);
-        const int m0 = mi * G_BM, n0 = ni * p.BN;
+        const NsProblem* pr = tile_of(c, mi, ni);
+        const CUtensorMap *mapA = &pr->a, *mapB = &pr->b;
+        const int kblocks = (pr->p.K + G_BK - 1) / G_BK, BN = pr->p.BN;
+        const bool a_mn = pr->p.a_mn != 0, b_mn = pr->p.b_mn != 0;
+        const unsigned tx = (unsigned)(G_A_BYTES + BN * G_BK * 2);
+        const int m0 = mi * G_BM, n0 = ni * BN;
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % G2_STAGES;
           const unsigned use = it / G2_STAGES;
           if (use > 0 && !mbar_wait_or_fail(&empty_bar[s], (use - 1u) & 1u, fail)) break;
           unsigned char* a_dst = tiles + (size_t)s * stage_bytes;
           unsigned char* b_dst = a_dst + G_A_BYTES;
-          mbar_expect_tx(&full_bar[s], (unsigned)stage_bytes);
+          mbar_expect_tx(&full_bar[s], tx);
           const int k0 = kb * G_BK;
-          if (p.a_mn) {
-            for (int j = 0; j < G_BM / 64; ++j) tma_load_2d(a_dst + j * 8192, &tmA, m0 + 64 * j, k0, &full_bar[s]);
+          if (a_mn) {
+            for (int j = 0; j < G_BM / 64; ++j) tma_load_2d(a_dst + j * 8192, mapA, m0 + 64 * j, k0, &full_bar[s]);
           } else {
-            tma_load_2d(a_dst, &tmA, k0, m0, &full_bar[s]);
+            tma_load_2d(a_dst, mapA, k0, m0, &full_bar[s]);
           }
-          if (p.b_mn) {
-            for (int j = 0; j < p.BN / 64; ++j) tma_load_2d(b_dst + j * 8192, &tmB, n0 + 64 * j, k0, &full_bar[s]);
+          if (b_mn) {
+            for (int j = 0; j < BN / 64; ++j) tma_load_2d(b_dst + j * 8192, mapB, n0 + 64 * j, k0, &full_bar[s]);
           } else {
-            tma_load_2d(b_dst, &tmB, k0, n0, &full_bar[s]);
+            tma_load_2d(b_dst, mapB, k0, n0, &full_bar[s]);
           }
         }
       }
@@ -201,9 +232,13 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else if (warp == 1) {
     // ---- MMA issuer ----
     if (lane == 0) {
-      const uint32_t idesc = umma_idesc(p.BN, p.a_mn != 0, p.b_mn != 0);
       unsigned it = 0, tcount = 0;
-      for (int c = blockIdx.x; c < total_tiles && !*fail; c += gridDim.x, ++tcount) {
+      for (int c = c_first; c < c_end && !*fail; c += c_step, ++tcount) {
+        int mi, ni;
+        const NsProblem* pr = tile_of(c, mi, ni);
+        const int kblocks = (pr->p.K + G_BK - 1) / G_BK;
+        const bool a_mn = pr->p.a_mn != 0, b_mn = pr->p.b_mn != 0;
+        const uint32_t idesc = umma_idesc(pr->p.BN, a_mn, b_mn);
         const unsigned buf = tcount & 1u, use = tcount >> 1;
         if (use > 0 && !mbar_wait_or_fail(&acce_bar[buf], (use - 1u) & 1u, fail)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -217,8 +252,8 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const uint32_t b_addr = a_addr + G_A_BYTES;
 #pragma unroll
           for (int k = 0; k < G_BK / 16; ++k) {
-            const uint64_t da = umma_desc(a_addr + (p.a_mn ? k * 2048 : k * 32), p.a_mn != 0);
-            const uint64_t db = umma_desc(b_addr + (p.b_mn ? k * 2048 : k * 32), p.b_mn != 0);
+            const uint64_t da = umma_desc(a_addr + (a_mn ? k * 2048 : k * 32), a_mn);
+            const uint64_t db = umma_desc(b_addr + (b_mn ? k * 2048 : k * 32), b_mn);
             umma_f16(tmem_acc, da, db, idesc, (kb | k) ? 1u : 0u);
           }
           umma_commit(&empty_bar[s]);  // frees the stage once these MMAs have read it
@@ -230,12 +265,13 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else {
     // ---- epilogue: warps 2..5; a warp may touch the 32 tensor-memory lanes of its quarter (warp % 4) ----
     const int quarter = warp & 3;
-    const float alpha = p.dev_scale ? p.alpha * p.dev_scale[0] : p.alpha;
-    const float beta = p.dev_scale ? p.beta * p.dev_scale[1] : p.beta;
     unsigned tcount = 0;
-    for (int c = blockIdx.x; c < total_tiles; c += gridDim.x, ++tcount) {
+    for (int c = c_first; c < c_end; c += c_step, ++tcount) {
       int mi, ni;
-      tile_coords(p, tn, c, mi, ni);
+      const NsProblem* pr = tile_of(c, mi, ni);
+      const GemmParams& p = pr->p;
+      const float alpha = p.dev_scale ? p.alpha * p.dev_scale[0] : p.alpha;
+      const float beta = p.dev_scale ? p.beta * p.dev_scale[1] : p.beta;
       const int m0 = mi * G_BM, n0 = ni * p.BN;
       const unsigned buf = tcount & 1u, use = tcount >> 1;
       if (!mbar_wait_or_fail(&accf_bar[buf], use & 1u, fail)) break;
@@ -293,7 +329,7 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (tid == 0 && fail_s) atomicCAS(p.status, 0u, 20001u);
+  if (tid == 0 && fail_s) atomicCAS(work.status, 0u, 20001u);
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * G2_ACC_COLS) : "memory");

@@ -397,7 +397,7 @@ int kaon_plan_destroy(kaon_plan* pl) {
   cudaFree(pl->d_flat_tensors);
   kaon::pnm_free(pl);
   kaon::kp_free(pl);
-  cudaFree(pl->d_tasks_ema);
+  kaon::muon_free(pl);
   cudaFree(pl->d_tasks_apply2);
   cudaFree(pl->d_tasks_na[0]);
   cudaFree(pl->d_tasks_na[1]);
