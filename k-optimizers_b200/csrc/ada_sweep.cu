@@ -19,110 +19,11 @@
 #include "adakaon_dev.h"
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
-#include "kaon_packed.cuh"
+#include "kaon_sweep.cuh"
 
 namespace kaon {
 
 constexpr int SWT = 256;   // threads per CTA
-
-// The cautious mask of one element as a factor: x > 0 as 1.0f / 0.0f by one saturating FMA, (big, add) = (2^127, 0);
-// mask off: 1.0f always, (0, 1).  A NaN gives 0.  A product below 2^-127 (subnormal) would come out in between; it
-// does not occur where both factors are normal gradients and updates.
-__device__ __forceinline__ float mask1(float x, float big, float add) {
-  float r;
-  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(big), "f"(add));
-  return r;
-}
-
-__device__ __forceinline__ void philox8(const AdaDev& hp, uint32_t tensor, uint64_t q, uint32_t tag, uint32_t out[4]) {
-  uint32_t c0 = (uint32_t)q, c1 = tensor, c2 = hp.step, c3 = tag | ((uint32_t)(q >> 32) << 8);
-#pragma unroll
-  for (int r = 0; r < KAON_PHILOX_ROUNDS; ++r) {
-    const unsigned long long p0 = (unsigned long long)0xD2511F53u * c0;
-    const unsigned long long p1 = (unsigned long long)0xCD9E8D57u * c2;
-    const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ hp.rk0[r];
-    const uint32_t n2 = (uint32_t)(p0 >> 32) ^ c3 ^ hp.rk1[r];
-    c1 = (uint32_t)p1;
-    c3 = (uint32_t)p0;
-    c0 = n0;
-    c2 = n2;
-  }
-  out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
-}
-
-// Eight weights on their way through a step: bf16 stays packed between the writes (four registers, not eight).
-template <typename PT>
-struct W8;
-
-template <>
-struct W8<__nv_bfloat16> {
-  uint32_t w[4];
-  __device__ __forceinline__ void load(const void* p) {
-    const uint4 q = *reinterpret_cast<const uint4*>(p);
-    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
-  }
-  __device__ __forceinline__ f32x2 pair(int j) const { return pack2(bf16lo(w[j]), bf16hi(w[j])); }
-  // stochastic rounding of w + D: 16 noise bits (the halves of nz[j], added by one dot-product instruction each) below
-  // the kept mantissa
-  __device__ __forceinline__ void add_sr(const f32x2 D[4], const uint32_t nz[4]) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const f32x2 r = add2(pair(j), D[j]);
-      w[j] = prmt(__dp2a_lo(nz[j], 0x00000001u, __float_as_uint(r.x)), __dp2a_lo(nz[j], 0x00000100u, __float_as_uint(r.y)), 0x7632u);
-    }
-  }
-  __device__ __forceinline__ void set(int j, f32x2 v) { w[j] = prmt(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632u); }
-  __device__ __forceinline__ void store(void* p, const Peers* pr) const {
-    const uint4 q = make_uint4(w[0], w[1], w[2], w[3]);
-    *reinterpret_cast<uint4*>(p) = q;
-    mirror16(pr, p, q);
-  }
-};
-
-template <>
-struct W8<float> {
-  f32x2 v[4];
-  __device__ __forceinline__ void load(const void* p) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-    v[0] = pack2(a.x, a.y); v[1] = pack2(a.z, a.w); v[2] = pack2(b.x, b.y); v[3] = pack2(b.z, b.w);
-  }
-  __device__ __forceinline__ f32x2 pair(int j) const { return v[j]; }
-  __device__ __forceinline__ void set(int j, f32x2 x) { v[j] = x; }
-  __device__ __forceinline__ void store(void* p, const Peers* pr) const {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      unsigned char* a = reinterpret_cast<unsigned char*>(p) + 16 * h;
-      const uint4 q = make_uint4(__float_as_uint(v[2 * h].x), __float_as_uint(v[2 * h].y),
-                                 __float_as_uint(v[2 * h + 1].x), __float_as_uint(v[2 * h + 1].y));
-      *reinterpret_cast<uint4*>(a) = q;
-      mirror16(pr, a, q);
-    }
-  }
-};
-
-// x less a row mean (bits as the row table holds them; 0 without centralization), rounded to x's dtype
-template <typename T>
-__device__ __forceinline__ void center(const W8<T>& x, float mu, f32x2 out[4]) {
-  if constexpr (Elems<T>::IS_BF16) {
-    const uint32_t m2 = __float_as_uint(mu);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t w = sub_bf16x2(x.w[j], m2);
-      out[j] = pack2(bf16lo(w), bf16hi(w));
-    }
-  } else {
-    const f32x2 M = pack2(mu, mu);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) out[j] = sub2(x.pair(j), M);
-  }
-}
-
-// The stored momentum of eight elements as it lies in memory.
-template <int MK> struct MRaw { };
-template <> struct MRaw<KAON_M_4BIT> { uint32_t w; float sc; };
-template <> struct MRaw<KAON_M_INT8> { uint2 w; };
-template <> struct MRaw<KAON_M_BF16> { W8<__nv_bfloat16> w; };
-template <> struct MRaw<KAON_M_F32> { W8<float> w; };
 
 // The vectors first, first + STRIDE, ... of a unit, 32 consecutive ones per warp (`first` includes the lane).  OWN: the
 // CTA itself has just written the row table and the column factors.
@@ -172,9 +73,8 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   MRaw<MK> mq;
   auto load = [&]() {
     gq.load(sp);
-    if constexpr (MK == KAON_M_4BIT) { mq.w = *reinterpret_cast<const uint32_t*>(mp); mq.sc = *msc; }
-    else if constexpr (MK == KAON_M_INT8) mq.w = *reinterpret_cast<const uint2*>(mp);
-    else if constexpr (MK != KAON_M_NONE) mq.w.load(mp);
+    if constexpr (MK != KAON_M_NONE) mq.load(mp);
+    if constexpr (MK == KAON_M_4BIT) mq.sc = *msc;
     if (need_p) P.load(pp);
   };
   // a climb of eight elements (reference src/kaon/msam.py:222-230); `wild`: a momentum that decodes to NaN or
@@ -189,20 +89,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
     }
   };
   auto add_noisy = [&](const f32x2 D[4], uint32_t tag) {
-    if constexpr (E::IS_BF16) {
-      uint32_t nz[4];
-      philox8(hp, d.tensor_id, q, tag, nz);
-      P.add_sr(D, nz);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) P.v[j] = add2(P.v[j], D[j]);
-    }
-  };
-  auto amax8 = [](const f32x2 M[4]) {
-    float a = max3f(fabsf(M[0].x), fabsf(M[0].y), fabsf(M[1].x));
-    a = max3f(a, fabsf(M[1].y), fabsf(M[2].x));
-    a = max3f(a, fabsf(M[2].y), fabsf(M[3].x));
-    return fmaxf(a, fabsf(M[3].y));
+    add_noisy8(hp, d, q, tag, P, D);
   };
   // the vector whose words are in gq, mq, P; `act`: this lane has one
   auto trip = [&](const bool act) {
@@ -216,29 +103,9 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
     center<ST>(gq, MUON ? 0.0f : f.x, G);
     // ---- stored momentum ----
     float sc_old = 1.0f;
-    if constexpr (MK == KAON_M_4BIT) {
-      sc_old = mq.sc;
-      const uint32_t wl = mq.w & 0x0F0F0F0Fu, wh = (mq.w >> 4) & 0x0F0F0F0Fu;
-      const f32x2 BIAS = pack2(-8388616.0f, -8388616.0f), SC = pack2(sc_old, sc_old);   // -(2^23 + 8)
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        MO[j] = mul2(add2(pack2(__uint_as_float(prmt(wl, 0x4B000000u, 0x7540u | (uint32_t)j)),
-                                __uint_as_float(prmt(wh, 0x4B000000u, 0x7540u | (uint32_t)j))), BIAS), SC);
-    } else if constexpr (MK == KAON_M_INT8) {
-      sc_old = f.z;
-      const uint32_t x0 = mq.w.x ^ 0x80808080u, x1 = mq.w.y ^ 0x80808080u;  // code + 128 in every byte
-      const f32x2 BIAS = pack2(-8388736.0f, -8388736.0f), SC = pack2(sc_old, sc_old);   // -(2^23 + 128)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t x = j < 2 ? x0 : x1;
-        const uint32_t b = (uint32_t)(2 * (j & 1));
-        MO[j] = mul2(add2(pack2(__uint_as_float(prmt(x, 0x4B000000u, 0x7540u | b)),
-                                __uint_as_float(prmt(x, 0x4B000000u, 0x7540u | (b + 1u)))), BIAS), SC);
-      }
-    } else if constexpr (MK != KAON_M_NONE) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) MO[j] = mq.w.pair(j);
-    }
+    if constexpr (MK == KAON_M_4BIT) sc_old = mq.sc;
+    if constexpr (MK == KAON_M_INT8) sc_old = f.z;
+    if constexpr (MK != KAON_M_NONE) mq.decode(sc_old, MO);
     if (MS && rem_here) {   // take the previous climb out (the mirrors get the step's last write only)
       f32x2 D[4];
       climb8(MO, hp.a_remove, hp.b_remove, CODED ? !(fabsf(sc_old) <= 3.0e38f) : true, D);
@@ -369,34 +236,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
         if (act) mq.w.store(mp, nullptr);
       }
       // ---- weights: p <- round(p - update), then the climb from the momentum as stored ----
-      if constexpr (E::IS_BF16) {
-        if (hp.sr) {
-          add_noisy(F, KAON_TAG_UPDATE);
-        } else if (hp.kahan) {
-          unsigned char* she = reinterpret_cast<unsigned char*>(d.shift) + q * 16;
-          W8<PT> SH;
-          if (act) SH.load(she); else SH.load(d.shift);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            f32x2 p = P.pair(j), sv = SH.pair(j);
-            kahan_step(p.x, sv.x, -F[j].x);
-            kahan_step(p.y, sv.y, -F[j].y);
-            P.set(j, p);
-            SH.set(j, sv);
-          }
-          if (act) SH.store(she, nullptr);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t fb = pack_bf16_rn(F[j].x, F[j].y);
-            const f32x2 s = add2(P.pair(j), pack2(bf16lo(fb), bf16hi(fb)));
-            P.w[j] = pack_bf16_rn(s.x, s.y);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) P.v[j] = add2(P.v[j], F[j]);
-      }
+      write8(hp, d, q, act, P, F);
       if (MS && hp.climb) {
         f32x2 D[4];
         climb8(MO, hp.a_climb, hp.b_climb, CODED ? !(sc <= 3.0e38f) : true, D);

@@ -6,12 +6,12 @@
 //   1. STATS + FINAL of the Adakaon kernels (row / column statistics of the centralised gradient, the
 //      factors r_i = rsqrt(row_i / mean(row)), c_j = rsqrt(col_j), the centralisation means) - the second
 //      moment is the same recurrence as Adakaon's (reference src/kaon/_factored.py:26-83).
-//   2. SUM: flat items of 8192 elements over every factored tensor: both momenta are decoded, the positive
-//      one takes the gradient, u = pn * ((r*c) * bc2); each item leaves its sum of u^2 (double), its count
+//   2. SUM: flat units over every factored tensor (a warp's, or items of 16 K for odd row lengths): both momenta are decoded, the positive
+//      one takes the gradient, u = pn * ((r*c) * bc2); each leaves its sum of u^2 (double), its count
 //      of u*g > 0 and, for int8 momentum, the row maxima of the new positive momentum.
-//   3. REDUCE: one CTA per factored tensor adds the item partials in item order: clip divisor, cautious
+//   3. REDUCE: one CTA per factored tensor adds the partials in order: clip divisor, cautious
 //      denominator.
-//   4. APPLY: the same flat items again: recompute, weight decay, clip, mask, weight write, store the
+//   4. APPLY: the same units again: recompute, weight decay, clip, mask, weight write, store the
 //      positive momentum through its codec.
 //   5. FLAT: one CTA per 1-D tensor (full second moment v, optional running maximum) doing 2-4 in place.
 // The two stored momenta swap roles every step (reference src/kaon/adapnm.py:588-596); `swap` selects.
@@ -29,6 +29,7 @@
 #include "kaon_host.h"
 #include "kaon_elem.cuh"
 #include "kaon_ops.cuh"
+#include "kaon_sweep.cuh"
 
 namespace kaon {
 
@@ -44,6 +45,7 @@ struct PnmDev {
   float clip;
   int has_wd, clip_on, cautious, gc, ams, sr, kahan, swap;
   uint32_t step, k0, k1;
+  uint32_t rk0[KAON_PHILOX_ROUNDS], rk1[KAON_PHILOX_ROUNDS];
 };
 
 struct PnmBufs {
@@ -53,12 +55,13 @@ struct PnmBufs {
 };
 
 struct PnmView {
-  const Task* items;      // flat items of the factored tensors, tensor by tensor
-  int n_items;
-  const int* item_begin;  // [n_tensors + 1] ranges into items
+  const Task* units;      // warp units of the factored tensors whose rows are a multiple of eight elements
+  const Task* items;      // flat items of the other factored tensors
+  int n_units, n_items;
+  const int* item_begin;  // [n_tensors + 1] ranges of units / items (Task::slot)
   const PnmBufs* bufs;    // [n_tensors]
-  double* part;           // [n_items] sum of u^2
-  unsigned* kpart;        // [n_items] count of u*g > 0
+  double* part;           // [slot] sum of u^2
+  unsigned* kpart;        // [slot] count of u*g > 0
   float* scal;            // [n_tensors][2] clip divisor, cautious denominator
   const int* fact;        // indices of the factored tensors
   int n_fact;
@@ -132,6 +135,151 @@ __device__ __forceinline__ void pnm_write(const PnmDev& hp, const DevTensor& d, 
 
 // ----------------------------------------------------------------------------- factored tensors
 
+// The two sweeps over tensors whose rows are a multiple of eight elements (4-bit blocks of 128): a warp per unit of up
+// to 4096 elements, nothing shared between warps.  Bound by instruction issue, so on packed pairs, the mask one
+// saturating FMA an element, rows and columns advanced by an addition.  (A CTA per 16 K-element item with guarded
+// elements and a scalar encode: SUM 409 us and APPLY 972 us on 269 M elements of 4-bit momentum.)
+template <typename PT, int MK, bool APPLY>
+__global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ PnmDev hp,
+                                                                  const __grid_constant__ PnmView x) {
+  using E = Elems<PT>;
+  constexpr int MV = MBytes<MK>::V;
+  const int lane = threadIdx.x & 31;
+  const int nw = gridDim.x * (PT_THREADS / 32);
+  for (int it = __shfl_sync(0xffffffffu, (int)(blockIdx.x * (PT_THREADS / 32) + (threadIdx.x >> 5)), 0); it < x.n_units; it += nw) {
+    const Task t = x.units[it];
+    const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
+    if (g == nullptr) continue;
+    const DevTensor& d = pv.tensors[t.tensor];
+    const PnmBufs& b = x.bufs[t.tensor];
+    const int nvec = t.n >> 3, nv = d.cols >> 3;
+    const float* rfac = pv.aux + aux_rfac(d);
+    const float* cfac = pv.aux + aux_cfac(d);
+    const float* mean = pv.aux + aux_mean(d);
+    unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
+    const unsigned char* gp = g + (t.e0 + lane * 8) * E::BYTES;
+    unsigned char* pp = reinterpret_cast<unsigned char*>(d.p) + (t.e0 + lane * 8) * E::BYTES;
+    unsigned char* pos = reinterpret_cast<unsigned char*>(b.m[hp.swap]) + ((t.e0 >> 3) + lane) * MV;
+    const unsigned char* neg = reinterpret_cast<const unsigned char*>(b.m[hp.swap ^ 1]) + ((t.e0 >> 3) + lane) * MV;
+    // 4-bit: the block's scale; int8: the row's (the positive buffer's as they were before this step)
+    const long long blk = (t.e0 >> 7) + (lane >> 4);
+    float* psc = b.sc[hp.swap] + (MK == KAON_M_4BIT ? blk : 0);
+    const float* nsc = b.sc[hp.swap ^ 1] + (MK == KAON_M_4BIT ? blk : 0);
+    const float* old = pv.aux + aux_oldsc(d);
+    uint64_t q = (uint64_t)(t.e0 >> 3) + (unsigned)lane;
+    int row = t.row0, cv = (t.pad >> 3) + lane;
+    if (cv >= nv) { const int k = cv / nv; row += k; cv -= k * nv; }
+    const int adv_r = 32 / nv, adv_c = 32 - adv_r * nv;
+    float div = 1.0f, denom = 1.0f;
+    if (APPLY) { div = x.scal[2 * t.tensor]; denom = hp.cautious ? x.scal[2 * t.tensor + 1] : 1.0f; }
+    const float rdiv = __frcp_rn(div), rdenom = __frcp_rn(denom);
+    double ss = 0.0;
+    f32x2 kept2 = pack2(0.0f, 0.0f);
+    for (int v = lane; v < nvec + lane; v += 32) {
+      const bool act = v < nvec;
+      W8<PT> gq, P;
+      MRaw<MK> mp, mn;
+      f32x2 Y[4], MP[4], MN[4], U[4];
+      gq.load(act ? gp : g);
+      mp.load(act ? pos : b.m[hp.swap]);
+      mn.load(act ? neg : b.m[hp.swap ^ 1]);
+      if constexpr (APPLY) P.load(act ? pp : d.p);
+      const int r = act ? row : 0, c = act ? cv : 0;
+      float sp = 1.0f, sn = 1.0f;
+      if constexpr (MK == KAON_M_4BIT) { sp = act ? *psc : 1.0f; sn = act ? *nsc : 1.0f; }
+      if constexpr (MK == KAON_M_INT8) { sp = old[r]; sn = nsc[r]; }
+      const float rf = rfac[r];
+      const float mu = hp.gc ? mean[r] : 0.0f;
+      const float4 ca = __ldg(reinterpret_cast<const float4*>(cfac) + 2 * c), cb = __ldg(reinterpret_cast<const float4*>(cfac) + 2 * c + 1);
+      const f32x2 CF[4] = {pack2(ca.x, ca.y), pack2(ca.z, ca.w), pack2(cb.x, cb.y), pack2(cb.z, cb.w)};
+      center<PT>(gq, E::IS_BF16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, Y);
+      mp.decode(sp, MP);
+      mn.decode(sn, MN);
+      const f32x2 RF = pack2(rf, rf);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        MP[j] = fma2(Y[j], pack2(hp.fw, hp.fw), mul2(MP[j], pack2(hp.fb, hp.fb)));
+        const f32x2 pn = mul2(fma2(MN[j], pack2(hp.c2, hp.c2), mul2(MP[j], pack2(hp.c1, hp.c1))), pack2(hp.c3, hp.c3));
+        U[j] = mul2(pn, mul2(mul2(RF, CF[j]), pack2(hp.bc2, hp.bc2)));
+      }
+      if constexpr (!APPLY) {
+        // the trip's eight squares in fp32, then one wide addition
+        const f32x2 s2 = fma2(U[3], U[3], fma2(U[2], U[2], fma2(U[1], U[1], mul2(U[0], U[0]))));
+        f32x2 K[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 X = mul2(U[j], Y[j]);
+          K[j] = pack2(mask1(X.x, 0x1p127f, 0.0f), mask1(X.y, 0x1p127f, 0.0f));
+        }
+        if (act) {
+          ss += (double)(s2.x + s2.y);
+          kept2 = add2(kept2, add2(add2(K[0], K[1]), add2(K[2], K[3])));
+        }
+        if constexpr (MK == KAON_M_INT8) {
+          unsigned bits = act ? __float_as_uint(amax8(MP)) : 0u;
+          const int row_l0 = __shfl_sync(0xffffffffu, row, 0);
+          if (__all_sync(0xffffffffu, !act || row == row_l0)) {
+            bits = __reduce_max_sync(0xffffffffu, bits);
+            if (lane == 0) atomicMax(rowmax + row_l0, bits);
+          } else if (act) {
+            atomicMax(rowmax + row, bits);
+          }
+        }
+      } else {
+        // -(u / div * lr), masked by its sign against the gradient's, over the kept share
+        f32x2 F[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          f32x2 u = U[j];
+          if (hp.clip_on) {
+            const f32x2 q0 = mul2(u, pack2(rdiv, rdiv));
+            u = fma2(fma2(q0, pack2(-div, -div), u), pack2(rdiv, rdiv), q0);
+          }
+          u = mul2(u, pack2(-hp.fstep, -hp.fstep));
+          if (hp.cautious) {
+            const f32x2 X = mul2(u, Y[j]);
+            const f32x2 q0 = mul2(u, pack2(rdenom, rdenom));
+            u = fma2(fma2(q0, pack2(-denom, -denom), u), pack2(rdenom, rdenom), q0);
+            u = mul2(u, pack2(mask1(X.x, -0x1p127f, 0.0f), mask1(X.y, -0x1p127f, 0.0f)));
+          }
+          F[j] = u;
+        }
+        if (hp.has_wd) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            f32x2 w = mul2(P.pair(j), pack2(hp.wdsc, hp.wdsc));
+            if constexpr (E::IS_BF16) w = pack2(round_bf16(w.x), round_bf16(w.y));
+            P.set(j, w);
+          }
+        }
+        write8(hp, d, q, act, P, F);
+        if (act) P.store(pp, &pv.peers);
+        float rm = 0.0f;
+        if constexpr (MK == KAON_M_INT8) rm = __uint_as_float(__ldcg(rowmax + r));
+        if constexpr (MK == KAON_M_BF16) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) MP[j] = pack2(round_bf16(MP[j].x), round_bf16(MP[j].y));
+        }
+        const float sc = store_m8<MK>(pos, MP, rm, act, lane);
+        if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(psc, sc); }
+        if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) psc[row] = sc; }
+      }
+      gp += 256 * E::BYTES; pp += 256 * E::BYTES; pos += 32 * MV; neg += 32 * MV;
+      if constexpr (MK == KAON_M_4BIT) { psc += 2; nsc += 2; }
+      q += 32;
+      row += adv_r; cv += adv_c;
+      if (cv >= nv) { cv -= nv; ++row; }
+    }
+    if constexpr (!APPLY) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const unsigned kept = __reduce_add_sync(0xffffffffu, (unsigned)(kept2.x + kept2.y + 0.5f));
+      if (lane == 0) { x.part[t.slot] = ss; x.kpart[t.slot] = kept; }
+    }
+  }
+}
+
+// The other factored tensors, eight elements a thread with every element guarded.
 template <typename PT, int MK, bool APPLY>
 __global__ void __launch_bounds__(PT_THREADS, 4) pnm_pass_kernel(PlanView pv, PnmDev hp, PnmView x) {
   using E = Elems<PT>;
@@ -295,8 +443,8 @@ __global__ void __launch_bounds__(PT_THREADS, 4) pnm_pass_kernel(PlanView pv, Pn
         double s = 0.0;
         unsigned kk = 0;
         for (int w = 0; w < PT_THREADS / 32; ++w) { s += red_d[w]; kk += red_u[w]; }
-        x.part[it] = s;
-        x.kpart[it] = kk;
+        x.part[t.slot] = s;
+        x.kpart[t.slot] = kk;
       }
     }
   }
@@ -490,6 +638,16 @@ static PnmPass pick_pass_pt(int mk) {
     default: return nullptr;
   }
 }
+template <typename PT, bool APPLY>
+static PnmPass pick_sweep_pt(int mk) {
+  switch (mk) {
+    case KAON_M_F32: return pnm_sweep_kernel<PT, KAON_M_F32, APPLY>;
+    case KAON_M_BF16: return pnm_sweep_kernel<PT, KAON_M_BF16, APPLY>;
+    case KAON_M_INT8: return pnm_sweep_kernel<PT, KAON_M_INT8, APPLY>;
+    case KAON_M_4BIT: return pnm_sweep_kernel<PT, KAON_M_4BIT, APPLY>;
+    default: return nullptr;
+  }
+}
 template <typename PT>
 static PnmPass pick_flat_pt(int mk) {
   switch (mk) {
@@ -515,12 +673,13 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   PnmHost* h = new PnmHost();
   pl->pnm = h;
   const int n = pl->n_tensors;
-  std::vector<Task> items, stats, fin;
+  std::vector<Task> units, items, stats, fin;
+  int slots = 0;
   std::vector<int> begin(n + 1, 0), fact, flat;
   std::vector<PnmBufs> bufs(n);
   for (int i = 0; i < n; ++i) {
     const DevTensor& t = pl->h_tensors[i];
-    begin[i] = (int)items.size();
+    begin[i] = slots;
     bufs[i].m[0] = t.m; bufs[i].sc[0] = t.m_scale;
     bufs[i].m[1] = const_cast<void*>(m_neg[i]);
     bufs[i].sc[1] = m_neg_scale ? m_neg_scale[i] : nullptr;
@@ -532,10 +691,18 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
       return fail(KAON_E_INVALID, "kaon_adapnm_attach: tensor %d: scales of the second momentum missing", i);
     if (t.rows <= 0) { flat.push_back(i); continue; }
     fact.push_back(i);
+    if ((t.cols & 7) == 0 && (pl->momentum_kind != KAON_M_4BIT || t.bshift == 7)) {
+      // a warp's unit: small tensors in more pieces (the tensor alone decides, so the order of its sums stays)
+      long long u = 512;
+      while (u < 4096 && u * 128 <= t.numel) u *= 2;
+      for (long long e = 0; e < t.numel; e += u)
+        units.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(u, t.numel - e), (int)(e / t.cols), slots++, (int)(e % t.cols)});
+      continue;
+    }
     for (long long e = 0; e < t.numel; e += PNM_ITEM)
-      items.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(PNM_ITEM, t.numel - e), 0, 0, 0});
+      items.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(PNM_ITEM, t.numel - e), 0, slots++, 0});
   }
-  begin[n] = (int)items.size();
+  begin[n] = slots;
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
@@ -556,9 +723,9 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   size_t o = 0;
   auto take = [&](size_t b) { size_t r = o; o += up(b); return r; };
-  const size_t o_items = take(sizeof(Task) * items.size()), o_begin = take(sizeof(int) * (n + 1));
-  const size_t o_bufs = take(sizeof(PnmBufs) * n), o_part = take(sizeof(double) * items.size());
-  const size_t o_kpart = take(sizeof(unsigned) * items.size()), o_scal = take(sizeof(float) * 2 * n);
+  const size_t o_items = take(sizeof(Task) * items.size()), o_units = take(sizeof(Task) * units.size()), o_begin = take(sizeof(int) * (n + 1));
+  const size_t o_bufs = take(sizeof(PnmBufs) * n), o_part = take(sizeof(double) * slots);
+  const size_t o_kpart = take(sizeof(unsigned) * slots), o_scal = take(sizeof(float) * 2 * n);
   const size_t o_fact = take(sizeof(int) * fact.size()), o_flat = take(sizeof(int) * flat.size());
   const size_t o_stats = take(sizeof(Task) * stats.size());
   const size_t o_fin = take(sizeof(Task) * fin.size());
@@ -569,6 +736,7 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
     return b ? cudaMemcpy(base + off, src, b, cudaMemcpyHostToDevice) : cudaSuccess;
   };
   KAON_CUDA(put(o_items, items.data(), sizeof(Task) * items.size()));
+  KAON_CUDA(put(o_units, units.data(), sizeof(Task) * units.size()));
   KAON_CUDA(put(o_begin, begin.data(), sizeof(int) * (n + 1)));
   KAON_CUDA(put(o_bufs, bufs.data(), sizeof(PnmBufs) * n));
   KAON_CUDA(put(o_fact, fact.data(), sizeof(int) * fact.size()));
@@ -578,6 +746,7 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   KAON_CUDA(cudaMemset(base + o_scal, 0, sizeof(float) * 2 * n));
   PnmView& x = h->view;
   x.items = reinterpret_cast<const Task*>(base + o_items); x.n_items = (int)items.size();
+  x.units = reinterpret_cast<const Task*>(base + o_units); x.n_units = (int)units.size();
   x.item_begin = reinterpret_cast<const int*>(base + o_begin);
   x.bufs = reinterpret_cast<const PnmBufs*>(base + o_bufs);
   x.part = reinterpret_cast<double*>(base + o_part);
@@ -637,6 +806,7 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
   hp.kahan = h->bf16_method == KAON_W_KAHAN && pl->param_dtype == KAON_DT_BF16;
   hp.swap = (h->group_step & 1u) ? 0 : 1;  // odd steps: "m_pos" is positive
   hp.step = step; hp.k0 = (uint32_t)seed; hp.k1 = (uint32_t)(seed >> 32);
+  philox_round_keys(hp);
   cudaStream_t s = (cudaStream_t)stream;
   const bool bf = pl->param_dtype == KAON_DT_BF16;
   const int mk = pl->momentum_kind;
@@ -657,6 +827,7 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
     // 2-4. the two sweeps over the flat items
     const int grid = std::min(x.n_items, pl->sm_count * 8);
+    const int gridu = std::min((x.n_units + PT_THREADS / 32 - 1) / (PT_THREADS / 32), pl->sm_count * 4);
     if (mk == KAON_M_INT8) {
       pnm_prep_kernel<<<x.n_fact, PT_THREADS, 0, s>>>(pl->view, hp, x);
       pl->launches += 1;
@@ -664,11 +835,13 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
     PnmPass sum = bf ? pick_pass_pt<__nv_bfloat16, false>(mk) : pick_pass_pt<float, false>(mk);
     PnmPass app = bf ? pick_pass_pt<__nv_bfloat16, true>(mk) : pick_pass_pt<float, true>(mk);
     if (!sum || !app) return fail(KAON_E_INVALID, "no AdaPNM kernel for this dtype combination");
-    sum<<<grid, PT_THREADS, 0, s>>>(pl->view, hp, x);
+    if (gridu > 0) (bf ? pick_sweep_pt<__nv_bfloat16, false>(mk) : pick_sweep_pt<float, false>(mk))<<<gridu, PT_THREADS, 0, s>>>(pl->view, hp, x);
+    if (grid > 0) sum<<<grid, PT_THREADS, 0, s>>>(pl->view, hp, x);
     pnm_reduce_kernel<<<x.n_fact, PT_THREADS, 0, s>>>(pl->view, hp, x);
-    app<<<grid, PT_THREADS, 0, s>>>(pl->view, hp, x);
+    if (gridu > 0) (bf ? pick_sweep_pt<__nv_bfloat16, true>(mk) : pick_sweep_pt<float, true>(mk))<<<gridu, PT_THREADS, 0, s>>>(pl->view, hp, x);
+    if (grid > 0) app<<<grid, PT_THREADS, 0, s>>>(pl->view, hp, x);
     KAON_CUDA(cudaGetLastError());
-    pl->launches += 3;
+    pl->launches += 1 + 2 * (gridu > 0) + 2 * (grid > 0);
   }
   if (x.n_flat > 0) {
     PnmPass fl = bf ? pick_flat_pt<__nv_bfloat16>(mk) : pick_flat_pt<float>(mk);

@@ -1,0 +1,253 @@
+// Building blocks of the warp sweeps: eight consecutive elements a lane and trip, packed pairs, rows a multiple of eight
+// elements, 4-bit blocks of 128 (so half a warp shares a scale).  Used by the Adakaon family, AdaMuon, AdaPNM and
+// KProdigy.
+#pragma once
+
+#include <cuda_bf16.h>
+
+#include "kaon_device.cuh"
+#include "kaon_ops.cuh"
+#include "kaon_packed.cuh"
+
+namespace kaon {
+
+// The cautious mask of one element as a factor: x > 0 as 1.0f / 0.0f by one saturating FMA, (big, add) = (2^127, 0);
+// mask off: 1.0f always, (0, 1).  A NaN gives 0.  A product below 2^-127 (subnormal) would come out in between; it
+// does not occur where both factors are normal gradients and updates.
+__device__ __forceinline__ float mask1(float x, float big, float add) {
+  float r;
+  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(big), "f"(add));
+  return r;
+}
+
+// Philox with the round keys from the host (HP: a hyper-parameter block with `step`, `rk0`, `rk1`)
+template <typename HP>
+__device__ __forceinline__ void philox8(const HP& hp, uint32_t tensor, uint64_t q, uint32_t tag, uint32_t out[4]) {
+  uint32_t c0 = (uint32_t)q, c1 = tensor, c2 = hp.step, c3 = tag | ((uint32_t)(q >> 32) << 8);
+#pragma unroll
+  for (int r = 0; r < KAON_PHILOX_ROUNDS; ++r) {
+    const unsigned long long p0 = (unsigned long long)0xD2511F53u * c0;
+    const unsigned long long p1 = (unsigned long long)0xCD9E8D57u * c2;
+    const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ hp.rk0[r];
+    const uint32_t n2 = (uint32_t)(p0 >> 32) ^ c3 ^ hp.rk1[r];
+    c1 = (uint32_t)p1;
+    c3 = (uint32_t)p0;
+    c0 = n0;
+    c2 = n2;
+  }
+  out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
+}
+
+// Eight weights on their way through a step: bf16 stays packed between the writes (four registers, not eight).
+template <typename PT>
+struct W8;
+
+template <>
+struct W8<__nv_bfloat16> {
+  uint32_t w[4];
+  __device__ __forceinline__ void load(const void* p) {
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
+    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
+  }
+  __device__ __forceinline__ f32x2 pair(int j) const { return pack2(bf16lo(w[j]), bf16hi(w[j])); }
+  // stochastic rounding of w + D: 16 noise bits (the halves of nz[j], added by one dot-product instruction each) below
+  // the kept mantissa
+  __device__ __forceinline__ void add_sr(const f32x2 D[4], const uint32_t nz[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const f32x2 r = add2(pair(j), D[j]);
+      w[j] = prmt(__dp2a_lo(nz[j], 0x00000001u, __float_as_uint(r.x)), __dp2a_lo(nz[j], 0x00000100u, __float_as_uint(r.y)), 0x7632u);
+    }
+  }
+  __device__ __forceinline__ void set(int j, f32x2 v) { w[j] = prmt(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632u); }
+  __device__ __forceinline__ void store(void* p, const Peers* pr) const {
+    const uint4 q = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(p) = q;
+    mirror16(pr, p, q);
+  }
+};
+
+template <>
+struct W8<float> {
+  f32x2 v[4];
+  __device__ __forceinline__ void load(const void* p) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = pack2(a.x, a.y); v[1] = pack2(a.z, a.w); v[2] = pack2(b.x, b.y); v[3] = pack2(b.z, b.w);
+  }
+  __device__ __forceinline__ f32x2 pair(int j) const { return v[j]; }
+  __device__ __forceinline__ void set(int j, f32x2 x) { v[j] = x; }
+  __device__ __forceinline__ void store(void* p, const Peers* pr) const {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      unsigned char* a = reinterpret_cast<unsigned char*>(p) + 16 * h;
+      const uint4 q = make_uint4(__float_as_uint(v[2 * h].x), __float_as_uint(v[2 * h].y),
+                                 __float_as_uint(v[2 * h + 1].x), __float_as_uint(v[2 * h + 1].y));
+      *reinterpret_cast<uint4*>(a) = q;
+      mirror16(pr, a, q);
+    }
+  }
+};
+
+// x less a row mean (bits as the row table holds them; 0 without centralization), rounded to x's dtype
+template <typename T>
+__device__ __forceinline__ void center(const W8<T>& x, float mu, f32x2 out[4]) {
+  if constexpr (Elems<T>::IS_BF16) {
+    const uint32_t m2 = __float_as_uint(mu);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w = sub_bf16x2(x.w[j], m2);
+      out[j] = pack2(bf16lo(w), bf16hi(w));
+    }
+  } else {
+    const f32x2 M = pack2(mu, mu);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[j] = sub2(x.pair(j), M);
+  }
+}
+
+// The stored momentum of eight elements as it lies in memory.
+template <int MK> struct MRaw { };
+template <> struct MRaw<KAON_M_4BIT> {
+  uint32_t w;
+  float sc;
+  __device__ __forceinline__ void load(const void* p) { w = *reinterpret_cast<const uint32_t*>(p); }
+  // nibble n as the float 2^23 + n by a byte permute, less 2^23 + 8
+  __device__ __forceinline__ void decode(float scale, f32x2 M[4]) const {
+    const uint32_t wl = w & 0x0F0F0F0Fu, wh = (w >> 4) & 0x0F0F0F0Fu;
+    const f32x2 BIAS = pack2(-8388616.0f, -8388616.0f), SC = pack2(scale, scale);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      M[j] = mul2(add2(pack2(__uint_as_float(prmt(wl, 0x4B000000u, 0x7540u | (uint32_t)j)),
+                             __uint_as_float(prmt(wh, 0x4B000000u, 0x7540u | (uint32_t)j))), BIAS), SC);
+  }
+};
+template <> struct MRaw<KAON_M_INT8> {
+  uint2 w;
+  __device__ __forceinline__ void load(const void* p) { w = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void decode(float scale, f32x2 M[4]) const {
+    const uint32_t x0 = w.x ^ 0x80808080u, x1 = w.y ^ 0x80808080u;  // code + 128 in every byte
+    const f32x2 BIAS = pack2(-8388736.0f, -8388736.0f), SC = pack2(scale, scale);   // -(2^23 + 128)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t x = j < 2 ? x0 : x1;
+      const uint32_t b = (uint32_t)(2 * (j & 1));
+      M[j] = mul2(add2(pack2(__uint_as_float(prmt(x, 0x4B000000u, 0x7540u | b)),
+                             __uint_as_float(prmt(x, 0x4B000000u, 0x7540u | (b + 1u)))), BIAS), SC);
+    }
+  }
+};
+template <typename T> struct MPlain {
+  W8<T> w;
+  __device__ __forceinline__ void load(const void* p) { w.load(p); }
+  __device__ __forceinline__ void decode(float, f32x2 M[4]) const {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) M[j] = w.pair(j);
+  }
+};
+template <> struct MRaw<KAON_M_BF16> : MPlain<__nv_bfloat16> { };
+template <> struct MRaw<KAON_M_F32> : MPlain<float> { };
+
+// bytes of eight stored momenta
+template <int MK> struct MBytes { static constexpr int V = MK == KAON_M_4BIT ? 4 : MK == KAON_M_INT8 ? 8 : MK == KAON_M_BF16 ? 16 : MK == KAON_M_F32 ? 32 : 0; };
+
+__device__ __forceinline__ float amax8(const f32x2 M[4]) {
+  float a = max3f(fabsf(M[0].x), fabsf(M[0].y), fabsf(M[1].x));
+  a = max3f(a, fabsf(M[1].y), fabsf(M[2].x));
+  a = max3f(a, fabsf(M[2].y), fabsf(M[3].x));
+  return fmaxf(a, fabsf(M[3].y));
+}
+
+// Store eight new momenta at mp (every lane of the warp calls it; `act`: this lane has eight).  bf16 momentum is
+// already rounded in M.  `amax`: int8 only, the finished maximum of the row; returns the scale (4-bit: the block's,
+// to be stored by the first lane of a half warp).  Codes are rounded from the correctly rounded quotient m' / scale.
+template <int MK>
+__device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax, const bool act, const int lane) {
+  if constexpr (MK == KAON_M_4BIT || MK == KAON_M_INT8) {
+    float sc;
+    if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(act ? amax8(M) : 0.0f, lane), 1e-12f));
+    else sc = div127_exact(fmaxf(amax, 1e-12f));
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
+    constexpr float MAGIC = MK == KAON_M_4BIT ? 12582920.0f : 12582912.0f;   // 1.5 * 2^23 (+ 8)
+    const f32x2 INV = pack2(inv, inv), MG = pack2(MAGIC, MAGIC), NSC = pack2(-sc, -sc);
+    f32x2 R[4];   // rint(m'/sc) + magic
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const f32x2 qq = mul2(M[j], INV);
+      R[j] = add2(fma2(fma2(qq, NSC, M[j]), INV, qq), MG);
+    }
+    if constexpr (MK == KAON_M_4BIT) {
+      f32x2 T[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) T[j] = sub2(MG, R[j]);
+      // sum_k (8 - t_k) 16^k = 0x8888 - (t0 + 16 t1 + 256 t2 + 4096 t3), exact in fp32; adding 2^23 leaves it in the low
+      // 16 mantissa bits
+      const f32x2 K256 = pack2(256.0f, 256.0f);
+      const f32x2 Xl = fma2(T[1], K256, T[0]), Yl = fma2(T[3], K256, T[2]);
+      const float lo4 = __fsub_rn(8423560.0f, __fmaf_rn(Xl.y, 16.0f, Xl.x));
+      const float hi4 = __fsub_rn(8423560.0f, __fmaf_rn(Yl.y, 16.0f, Yl.x));
+      if (act) stg_u32(mp, prmt(__float_as_uint(lo4), __float_as_uint(hi4), 0x5410u));
+    } else if (act) {  // the low byte of every R is the code in two's complement
+      const uint32_t w0 = prmt(prmt(__float_as_uint(R[0].x), __float_as_uint(R[0].y), 0x0040u),
+                               prmt(__float_as_uint(R[1].x), __float_as_uint(R[1].y), 0x0040u), 0x5410u);
+      const uint32_t w1 = prmt(prmt(__float_as_uint(R[2].x), __float_as_uint(R[2].y), 0x0040u),
+                               prmt(__float_as_uint(R[3].x), __float_as_uint(R[3].y), 0x0040u), 0x5410u);
+      *reinterpret_cast<uint2*>(mp) = make_uint2(w0, w1);
+    }
+    return sc;
+  } else {
+    MRaw<MK> o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.w.set(j, M[j]);
+    if (act) o.w.store(mp, nullptr);
+    return 1.0f;
+  }
+}
+
+// p <- p + D: bf16 by stochastic rounding, fp32 as is
+template <typename PT, typename HP>
+__device__ __forceinline__ void add_noisy8(const HP& hp, const DevTensor& d, uint64_t q, uint32_t tag, W8<PT>& P, const f32x2 D[4]) {
+  if constexpr (Elems<PT>::IS_BF16) {
+    uint32_t nz[4];
+    philox8(hp, d.tensor_id, q, tag, nz);
+    P.add_sr(D, nz);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) P.v[j] = add2(P.v[j], D[j]);
+  }
+}
+
+// The weight write p <- round(p + F) of vector q of a tensor: stochastic, Kahan-compensated or to nearest
+template <typename PT, typename HP>
+__device__ __forceinline__ void write8(const HP& hp, const DevTensor& d, uint64_t q, const bool act, W8<PT>& P, const f32x2 F[4]) {
+  if constexpr (Elems<PT>::IS_BF16) {
+    if (hp.sr) {
+      add_noisy8(hp, d, q, KAON_TAG_UPDATE, P, F);
+    } else if (hp.kahan) {
+      unsigned char* she = reinterpret_cast<unsigned char*>(d.shift) + q * 16;
+      W8<PT> SH;
+      if (act) SH.load(she); else SH.load(d.shift);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        f32x2 p = P.pair(j), sv = SH.pair(j);
+        kahan_step(p.x, sv.x, -F[j].x);
+        kahan_step(p.y, sv.y, -F[j].y);
+        P.set(j, p);
+        SH.set(j, sv);
+      }
+      if (act) SH.store(she, nullptr);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t fb = pack_bf16_rn(F[j].x, F[j].y);
+        const f32x2 s = add2(P.pair(j), pack2(bf16lo(fb), bf16hi(fb)));
+        P.w[j] = pack_bf16_rn(s.x, s.y);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) P.v[j] = add2(P.v[j], F[j]);
+  }
+}
+
+}  // namespace kaon
