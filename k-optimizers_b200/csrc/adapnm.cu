@@ -138,7 +138,7 @@ __device__ __forceinline__ void pnm_write(const PnmDev& hp, const DevTensor& d, 
 // The two sweeps over tensors whose rows are a multiple of eight elements (4-bit blocks of 128): a warp per unit of up
 // to 4096 elements, nothing shared between warps.  Bound by instruction issue, so on packed pairs, the mask one
 // saturating FMA an element, rows and columns advanced by an addition.  (A CTA per 16 K-element item with guarded
-// elements and a scalar encode: SUM 409 us and APPLY 972 us on 269 M elements of 4-bit momentum.)
+// elements and a scalar encode: SUM 409 us and APPLY 972 us on 269 M elements of 4-bit momentum; here 251 and 531 us.)
 template <typename PT, int MK, bool APPLY>
 __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ PnmDev hp,
                                                                   const __grid_constant__ PnmView x) {
@@ -175,8 +175,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_c
     const float rdiv = __frcp_rn(div), rdenom = __frcp_rn(denom);
     double ss = 0.0;
     f32x2 kept2 = pack2(0.0f, 0.0f);
-    for (int v = lane; v < nvec + lane; v += 32) {
-      const bool act = v < nvec;
+    auto trip = [&](const bool act) {
       W8<PT> gq, P;
       MRaw<MK> mp, mn;
       f32x2 Y[4], MP[4], MN[4], U[4];
@@ -264,12 +263,16 @@ __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_c
         if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(psc, sc); }
         if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) psc[row] = sc; }
       }
+    };
+    for (int full = nvec >> 5; full > 0; --full) {
+      trip(true);
       gp += 256 * E::BYTES; pp += 256 * E::BYTES; pos += 32 * MV; neg += 32 * MV;
       if constexpr (MK == KAON_M_4BIT) { psc += 2; nsc += 2; }
       q += 32;
       row += adv_r; cv += adv_c;
       if (cv >= nv) { cv -= nv; ++row; }
     }
+    if (nvec & 31) trip(lane < (nvec & 31));
     if constexpr (!APPLY) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);

@@ -6,10 +6,10 @@
 // Pass 1 of a plan:
 //   factored second moment: Adakaon's STATS and FINAL items (row / column EMA of g^2 + eps_factored, the
 //     factors r_i, c_j and the centralisation means into the scratch); full second moment with gradient
-//     centralisation: a row-mean launch (one warp per row) into the same scratch slot
-//   SWEEP over flat items of 8192 elements of EVERY tensor: the centralised gradient (plus coupled weight
+//     centralisation: a row-mean launch into the same scratch slot
+//   SWEEP over flat units of EVERY tensor (a warp's, or items of 16 K for odd row lengths): the centralised gradient (plus coupled weight
 //     decay), on every slice_p-th element the numerator term g*(p0 - p) and the s buffer with its |s| sum
-//     (per item, double, added per tensor in item order), the momentum through its codec (int8: only the
+//     (per unit, double, added per tensor in order), the momentum through its codec (int8: only the
 //     row maxima here, the codes in a second sweep), the full second moment v
 //   the per-tensor partial sums are copied to the host, which folds them in fp32 in tensor order.
 // Pass 2: [COUNT sweep + per-tensor reduce for the cautious mask] and the weight sweep.
@@ -25,6 +25,7 @@
 #include "kaon_elem.cuh"
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
+#include "kaon_sweep.cuh"
 
 namespace kaon {
 
@@ -43,6 +44,7 @@ struct KpDev {
   float floor_, cap, fdlr, fdecay;    // d*eps, 1/(d*eps), dlr, decay*dlr
   int has_decay, cautious, sr, kahan, store;  // store: the int8 second sweep of pass 1
   uint32_t step, k0, k1;
+  uint32_t rk0[KAON_PHILOX_ROUNDS], rk1[KAON_PHILOX_ROUNDS];
 };
 
 struct KpBufs {
@@ -51,46 +53,75 @@ struct KpBufs {
 };
 
 struct KpView {
-  const Task* items;      // flat items of every tensor, tensor by tensor
-  int n_items;
-  const int* item_begin;  // [n_tensors + 1]
+  const Task* units;      // warp units of the tensors kp_warp_kernel takes
+  const Task* items;      // flat items of the other tensors
+  int n_units, n_items;
+  const int* item_begin;  // [n_tensors + 1] ranges of units / items (Task::slot)
   const KpBufs* bufs;     // [n_tensors]
-  double* part;           // [n_items][2]: numerator term, |s| sum; pass 2: [n_items] kept counts as doubles
+  double* part;           // [slot][2]: numerator term, |s| sum; pass 2: kept counts as doubles
   float* sums;            // [n_tensors][2] per-tensor sums (pass 1), [n_tensors] cautious denominators (pass 2)
   unsigned* tmax;         // [n_tensors] 1-D int8: bits of the tensor's absmax of the new momentum
   float* told;            // [n_tensors] 1-D int8: the scalar scale before this step
-  const int* fact;        // indices of the >=2-D tensors
-  int n_fact;
-  const long long* row_begin;  // [n_fact + 1] rows before each >=2-D tensor
-  long long n_rows;
+  const Task* row_units;  // whole rows of the >=2-D tensors
+  int n_row_units;
 };
 
 // ----------------------------------------------------------------------------- row means (full second moment)
 
+// Row means, over units of whole rows (about 4096 elements).  Rows of up to 64 elements: a lane each; longer ones: the
+// warp, sixteen bytes a lane where the rows allow it.
 template <typename PT>
-__global__ void __launch_bounds__(KP_THREADS) kp_rowmean_kernel(PlanView pv, KpView x) {
+__global__ void __launch_bounds__(KP_THREADS) kp_rowmean_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ KpView x) {
   using E = Elems<PT>;
   const int lane = threadIdx.x & 31;
-  const long long warp0 = ((long long)blockIdx.x * KP_THREADS + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * KP_THREADS) >> 5;
-  for (long long gr = warp0; gr < x.n_rows; gr += nwarps) {
-    int lo = 0, hi = x.n_fact - 1;   // the tensor this row belongs to
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (x.row_begin[mid] <= gr) lo = mid; else hi = mid - 1;
-    }
-    const int ti = x.fact[lo];
-    const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[ti]);
+  const int nw = gridDim.x * (KP_THREADS / 32);
+  for (int it = __shfl_sync(0xffffffffu, (int)(blockIdx.x * (KP_THREADS / 32) + (threadIdx.x >> 5)), 0); it < x.n_row_units; it += nw) {
+    const Task t = x.row_units[it];   // n: rows
+    const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
     if (g == nullptr) continue;
-    const DevTensor d = pv.tensors[ti];
-    const long long r = gr - x.row_begin[lo];
-    const unsigned char* rowp = g + (size_t)r * d.cols * E::BYTES;
-    float s = 0.0f;
-    for (int i = lane; i < d.cols; i += 32) s += E::load1(rowp, i);
-    s = warp_sum(s);
-    if (lane == 0) {
-      const float mean = __fdiv_rn(s, (float)d.cols);
-      pv.aux[aux_mean(d) + r] = E::IS_BF16 ? round_bf16(mean) : mean;
+    const DevTensor& d = pv.tensors[t.tensor];
+    float* mean = pv.aux + aux_mean(d) + t.row0;
+    const int C = d.cols;
+    auto put = [&](int r, float s) {
+      const float m = __fdiv_rn(s, (float)C);
+      mean[r] = E::IS_BF16 ? round_bf16(m) : m;
+    };
+    if (C <= 64) {
+      for (int r = lane; r < t.n; r += 32) {
+        const unsigned char* rowp = g + (t.e0 + (long long)r * C) * E::BYTES;
+        float s = 0.0f;
+        if ((C & 7) == 0) {
+          f32x2 a = pack2(0.0f, 0.0f);
+          for (int v = 0; v < C; v += 8) {
+            W8<PT> w;
+            w.load(rowp + v * E::BYTES);
+            a = add2(a, add2(add2(w.pair(0), w.pair(1)), add2(w.pair(2), w.pair(3))));
+          }
+          s = a.x + a.y;
+        } else {
+          for (int i = 0; i < C; ++i) s += E::load1(rowp, i);
+        }
+        put(r, s);
+      }
+      continue;
+    }
+    for (int r = 0; r < t.n; ++r) {
+      const unsigned char* rowp = g + (t.e0 + (long long)r * C) * E::BYTES;
+      float s = 0.0f;
+      if ((C & 7) == 0) {
+        f32x2 a = pack2(0.0f, 0.0f);
+#pragma unroll 4
+        for (int v = lane * 8; v < C; v += 256) {
+          W8<PT> w;
+          w.load(rowp + v * E::BYTES);
+          a = add2(a, add2(add2(w.pair(0), w.pair(1)), add2(w.pair(2), w.pair(3))));
+        }
+        s = a.x + a.y;
+      } else {
+        for (int i = lane; i < C; i += 32) s += E::load1(rowp, i);
+      }
+      s = warp_sum(s);
+      if (lane == 0) put(r, s);
     }
   }
 }
@@ -113,8 +144,205 @@ __global__ void __launch_bounds__(KP_THREADS) kp_prep_kernel(PlanView pv, KpView
 
 // ----------------------------------------------------------------------------- the sweeps
 
+// The modes of both sweep kernels.
 // MODE 0: pass 1 (statistics, moments).  MODE 1: pass 1's second sweep for int8 (codes and scales).
 // MODE 2: pass 2 COUNT (cautious kept count).  MODE 3: pass 2 weight write.
+// The sweeps over tensors whose rows (1-D tensors: whose length) are a multiple of eight elements, with 4-bit blocks of
+// 128 and every element on the slice: a warp per unit of up to 4096 elements, vector accesses without guards, nothing
+// shared between warps.  Bound by HBM where the state is wide (MODE 0 reads and writes 28 bytes an element with the
+// full second moment: 1185 us for 269 M elements with bf16 momentum, 6.4 TB/s; MODE 3 522 us).  The guarded form, a
+// CTA per 16 K-element item, took 1976 and 1102 us.
+template <typename PT, int MK, int MODE>
+__global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ KpDev hp,
+                                                                              const __grid_constant__ KpView x) {
+  using E = Elems<PT>;
+  constexpr int MV = MBytes<MK>::V;
+  const int lane = threadIdx.x & 31;
+  const int nw = gridDim.x * (KP_THREADS / 32);
+  const bool need_p = MODE == 0 ? (hp.do_d || hp.has_wdc) : MODE == 1 ? hp.has_wdc != 0 : MODE == 2 ? hp.has_decay != 0 : true;
+  const bool read_m = MK != KAON_M_NONE && hp.has_m;
+  const bool need_g = MODE <= 2 || hp.cautious || !read_m;
+  const bool dstat = MODE == 0 && hp.do_d;
+  for (int it = __shfl_sync(0xffffffffu, (int)(blockIdx.x * (KP_THREADS / 32) + (threadIdx.x >> 5)), 0); it < x.n_units; it += nw) {
+    const Task t = x.units[it];
+    const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
+    if (g == nullptr) {
+      if ((MODE == 0 || MODE == 2) && lane == 0) { x.part[2 * t.slot] = 0.0; x.part[2 * t.slot + 1] = 0.0; }
+      continue;
+    }
+    const DevTensor& d = pv.tensors[t.tensor];
+    const bool two_d = d.rows > 0;
+    const bool gc = hp.gc && two_d, fac = hp.factored && two_d;
+    const int nvec = t.n >> 3, nv = two_d ? d.cols >> 3 : 0x40000000;
+    const float* mean = pv.aux + (two_d ? aux_mean(d) : 0);
+    const float* rfac = pv.aux + (two_d ? aux_rfac(d) : 0);
+    const float* cfac = pv.aux + (two_d ? aux_cfac(d) : 0);
+    unsigned* rowmax = two_d ? reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d)) : x.tmax + t.tensor;
+    const float* msc_rd = MK == KAON_M_INT8 && MODE <= 1 ? (two_d ? pv.aux + aux_oldsc(d) : x.told + t.tensor) : d.m_scale;
+    // (the unit's addresses are the warp's, a lane adds its vector's number)
+    const unsigned char* gp = g + t.e0 * E::BYTES;
+    unsigned char* pp = reinterpret_cast<unsigned char*>(d.p) + t.e0 * E::BYTES;
+    unsigned char* mp = MV ? reinterpret_cast<unsigned char*>(d.m) + (t.e0 >> 3) * MV : nullptr;
+    float* blk = MK == KAON_M_4BIT ? d.m_scale + (t.e0 >> 7) : nullptr;
+    float* vp = d.stat_a + t.e0;   // (read where the second moment is full)
+    float* sp = x.bufs[t.tensor].s + t.e0;
+    const float* p0p = x.bufs[t.tensor].p0;
+    if (p0p) p0p += t.e0;
+    int row = t.row0, cv = (t.pad >> 3) + lane;
+    if (cv >= nv) { const int k = cv / nv; row += k; cv -= k * nv; }
+    const int adv_r = two_d ? 32 / nv : 0, adv_c = 32 - (two_d ? adv_r * nv : 0);
+    const float denom = MODE == 3 && hp.cautious ? x.sums[t.tensor] : 1.0f;
+    const float rdenom = __frcp_rn(denom), rfd = __frcp_rn(hp.fd);
+    double acc_a = 0.0, acc_b = 0.0;
+    f32x2 kept2 = pack2(0.0f, 0.0f);
+    auto trip = [&](const unsigned v, const bool act) {
+      const unsigned o = act ? v : 0u;
+      W8<PT> gq, P;
+      W8<float> S, P0, V;
+      MRaw<MK == KAON_M_NONE ? KAON_M_BF16 : MK> mq;
+      f32x2 Y[4], M[4];
+      if (need_g) gq.load(gp + o * (8u * E::BYTES));
+      if (need_p) P.load(pp + o * (8u * E::BYTES));
+      if (read_m) mq.load(mp + o * (unsigned)MV);
+      if (!fac) V.load(vp + o * 8u);
+      if (dstat) {
+        S.load(sp + o * 8u);
+        if (p0p) P0.load(p0p + o * 8u);
+      }
+      const int r = act && two_d ? row : 0;
+      float sc_old = 1.0f;
+      if constexpr (MK == KAON_M_4BIT) sc_old = blk[o >> 4];
+      if constexpr (MK == KAON_M_INT8) sc_old = msc_rd[r];
+      if (need_g) {
+        const float mu = gc ? mean[r] : 0.0f;
+        center<PT>(gq, E::IS_BF16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, Y);
+      }
+      if (read_m) mq.decode(sc_old, M);
+      if constexpr (MODE <= 1) {
+        if (hp.has_wdc) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) Y[j] = fma2(P.pair(j), pack2(hp.fwd, hp.fwd), Y[j]);
+        }
+        if (dstat) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const f32x2 a = mul2(Y[j], p0p ? sub2(P0.v[j], P.pair(j)) : sub2(pack2(0.0f, 0.0f), P.pair(j)));
+            S.v[j] = fma2(Y[j], pack2(hp.fa, hp.fa), mul2(S.v[j], pack2(hp.fb3, hp.fb3)));
+            if (act) {
+              acc_a += (double)a.x; acc_a += (double)a.y;
+              acc_b += (double)fabsf(S.v[j].x); acc_b += (double)fabsf(S.v[j].y);
+            }
+          }
+          if (act) S.store(sp + v * 8u, nullptr);
+        }
+        if (MODE == 0 && !fac) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) V.v[j] = fma2(mul2(pack2(hp.fv, hp.fv), Y[j]), Y[j], mul2(V.v[j], pack2(hp.fb2, hp.fb2)));
+          if (act) V.store(vp + v * 8u, nullptr);
+        }
+        if (read_m) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if constexpr (MK == KAON_M_BF16) {
+              const f32x2 a = mul2(M[j], pack2(hp.fb1, hp.fb1));
+              const uint32_t ab = pack_bf16_rn(a.x, a.y), yb = pack_bf16_rn(Y[j].x, Y[j].y);
+              const f32x2 m = fma2(pack2(bf16lo(yb), bf16hi(yb)), pack2(hp.ftb, hp.ftb), pack2(bf16lo(ab), bf16hi(ab)));
+              M[j] = pack2(round_bf16(m.x), round_bf16(m.y));
+            } else if constexpr (MK == KAON_M_4BIT) {
+              const f32x2 u = hp.d_is_one ? Y[j] : mul2(Y[j], pack2(hp.fd, hp.fd));
+              M[j] = hp.small_w1 ? fma2(pack2(hp.w1, hp.w1), sub2(u, M[j]), M[j]) : fma2(pack2(hp.w1m1, hp.w1m1), sub2(u, M[j]), u);
+            } else {
+              M[j] = fma2(Y[j], pack2(hp.ft, hp.ft), mul2(M[j], pack2(hp.fb1, hp.fb1)));
+            }
+          }
+          if constexpr (MK == KAON_M_INT8 && MODE == 0) {   // the row maxima first; the codes in the second sweep
+            unsigned bits = act ? __float_as_uint(amax8(M)) : 0u;
+            const int row_l0 = __shfl_sync(0xffffffffu, row, 0);
+            if (__all_sync(0xffffffffu, !act || row == row_l0)) {
+              bits = __reduce_max_sync(0xffffffffu, bits);
+              if (lane == 0) atomicMax(rowmax + row_l0, bits);
+            } else if (act) {
+              atomicMax(rowmax + row, bits);
+            }
+          } else if constexpr (MK != KAON_M_NONE) {
+            float rm = 0.0f;
+            if constexpr (MK == KAON_M_INT8) rm = __uint_as_float(__ldcg(rowmax + r));
+            const float sc = store_m8<MK>(mp + o * (unsigned)MV, M, rm, act, lane);
+            if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(blk + (v >> 4), sc); }
+            if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) d.m_scale[row] = sc; }
+          }
+        }
+      } else {
+        f32x2 F[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) F[j] = read_m ? M[j] : Y[j];
+        if (fac) {
+          const float rf = rfac[r];
+          const float4 ca = __ldg(reinterpret_cast<const float4*>(cfac) + 2 * (act ? cv : 0)), cb = __ldg(reinterpret_cast<const float4*>(cfac) + 2 * (act ? cv : 0) + 1);
+          const f32x2 CF[4] = {pack2(ca.x, ca.y), pack2(ca.z, ca.w), pack2(cb.x, cb.y), pack2(cb.z, cb.w)};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const f32x2 a = mul2(pack2(rf, rf), CF[j]), q0 = mul2(a, pack2(rfd, rfd));
+            const f32x2 i = fma2(fma2(q0, pack2(-hp.fd, -hp.fd), a), pack2(rfd, rfd), q0);
+            F[j] = mul2(F[j], pack2(fminf(i.x, hp.cap), fminf(i.y, hp.cap)));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            F[j].x = __fdiv_rn(F[j].x, fmaxf(__fsqrt_rn(V.v[j].x), hp.floor_));
+            F[j].y = __fdiv_rn(F[j].y, fmaxf(__fsqrt_rn(V.v[j].y), hp.floor_));
+          }
+        }
+        // the update, negated: -(dlr numer / denominator + decay p)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) F[j] = mul2(F[j], pack2(-hp.fdlr, -hp.fdlr));
+        if (hp.has_decay) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) F[j] = fma2(P.pair(j), pack2(-hp.fdecay, -hp.fdecay), F[j]);
+        }
+        if (MODE == 2 || hp.cautious) {
+          f32x2 K[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const f32x2 X = mul2(F[j], Y[j]);
+            K[j] = pack2(mask1(X.x, -0x1p127f, 0.0f), mask1(X.y, -0x1p127f, 0.0f));
+          }
+          if constexpr (MODE == 2) {
+            if (act) kept2 = add2(kept2, add2(add2(K[0], K[1]), add2(K[2], K[3])));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const f32x2 q0 = mul2(F[j], pack2(rdenom, rdenom));
+              F[j] = mul2(fma2(fma2(q0, pack2(-denom, -denom), F[j]), pack2(rdenom, rdenom), q0), K[j]);
+            }
+          }
+        }
+        if constexpr (MODE == 3) {
+          write8(hp, d, (uint64_t)(t.e0 >> 3) + v, act, P, F);
+          if (act) P.store(pp + v * (8u * E::BYTES), &pv.peers);
+        }
+      }
+    };
+    int v0 = 0;
+    for (; v0 + 32 <= nvec; v0 += 32) {
+      trip((unsigned)(v0 + lane), true);
+      row += adv_r; cv += adv_c;
+      if (cv >= nv) { cv -= nv; ++row; }
+    }
+    if (v0 < nvec) trip((unsigned)(v0 + lane), v0 + lane < nvec);
+    if constexpr (MODE == 0 || MODE == 2) {
+      if (MODE == 2) acc_a = (double)(kept2.x + kept2.y);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        acc_a += __shfl_xor_sync(0xffffffffu, acc_a, o);
+        acc_b += __shfl_xor_sync(0xffffffffu, acc_b, o);
+      }
+      if (lane == 0) { x.part[2 * t.slot] = acc_a; x.part[2 * t.slot + 1] = acc_b; }
+    }
+  }
+}
+
+// The other tensors, eight elements a thread with every element guarded.
 template <typename PT, int MK, int MODE>
 __global__ void __launch_bounds__(KP_THREADS, 4) kp_sweep_kernel(PlanView pv, KpDev hp, KpView x) {
   using E = Elems<PT>;
@@ -156,7 +384,7 @@ __global__ void __launch_bounds__(KP_THREADS, 4) kp_sweep_kernel(PlanView pv, Kp
           float gx[8], mo[8], vv[8], sv[8], p0v[8];
           int cl[8];
           load8_guard<PT>(g + e * E::BYTES, cnt, gx);
-          const bool need_p = MODE == 0 ? (hp.do_d || hp.has_wdc) : (MODE >= 2);
+          const bool need_p = MODE == 0 ? (hp.do_d || hp.has_wdc) : MODE == 1 ? hp.has_wdc != 0 : true;
           if (need_p) load8_guard<PT>(reinterpret_cast<const unsigned char*>(d.p) + e * E::BYTES, cnt, pw);
           int r = 0, c = 0;
           if (two_d) {
@@ -342,8 +570,8 @@ __global__ void __launch_bounds__(KP_THREADS, 4) kp_sweep_kernel(PlanView pv, Kp
       if (tid == 0) {
         double a = 0.0, bb = 0.0;
         for (int w = 0; w < KP_THREADS / 32; ++w) { a += red_a[w]; bb += red_b[w]; }
-        x.part[2 * it] = a;
-        x.part[2 * it + 1] = bb;
+        x.part[2 * t.slot] = a;
+        x.part[2 * t.slot + 1] = bb;
       }
     }
   }
@@ -393,6 +621,17 @@ struct KpHost {
 typedef void (*KpSweep)(PlanView, KpDev, KpView);
 
 template <typename PT, int MODE>
+static KpSweep pick_warp_pt(int mk) {
+  switch (mk) {
+    case KAON_M_F32: return kp_warp_kernel<PT, KAON_M_F32, MODE>;
+    case KAON_M_BF16: return kp_warp_kernel<PT, KAON_M_BF16, MODE>;
+    case KAON_M_INT8: return kp_warp_kernel<PT, KAON_M_INT8, MODE>;
+    case KAON_M_4BIT: return kp_warp_kernel<PT, KAON_M_4BIT, MODE>;
+    case KAON_M_NONE: return kp_warp_kernel<PT, KAON_M_NONE, MODE>;
+    default: return nullptr;
+  }
+}
+template <typename PT, int MODE>
 static KpSweep pick_sweep_pt(int mk) {
   switch (mk) {
     case KAON_M_F32: return kp_sweep_kernel<PT, KAON_M_F32, MODE>;
@@ -403,9 +642,24 @@ static KpSweep pick_sweep_pt(int mk) {
     default: return nullptr;
   }
 }
+// The sweep of a mode over the plan's units and items.
 template <int MODE>
-static KpSweep pick_sweep(int pdt, int mk) {
-  return pdt == KAON_DT_BF16 ? pick_sweep_pt<__nv_bfloat16, MODE>(mk) : pick_sweep_pt<float, MODE>(mk);
+static int launch_sweep(kaon_plan* pl, const KpDev& hp, const KpView& x, cudaStream_t s) {
+  const bool bf = pl->param_dtype == KAON_DT_BF16;
+  const int mk = pl->momentum_kind;
+  KpSweep kw = bf ? pick_warp_pt<__nv_bfloat16, MODE>(mk) : pick_warp_pt<float, MODE>(mk);
+  KpSweep ki = bf ? pick_sweep_pt<__nv_bfloat16, MODE>(mk) : pick_sweep_pt<float, MODE>(mk);
+  if (!kw || !ki) return fail(KAON_E_INVALID, "no KProdigy kernel for this dtype combination");
+  if (x.n_units > 0) {
+    kw<<<std::min((x.n_units + KP_THREADS / 32 - 1) / (KP_THREADS / 32), pl->sm_count * (MODE == 0 ? 3 : 4)), KP_THREADS, 0, s>>>(pl->view, hp, x);
+    pl->launches += 1;
+  }
+  if (x.n_items > 0) {
+    ki<<<std::min(x.n_items, pl->sm_count * 8), KP_THREADS, 0, s>>>(pl->view, hp, x);
+    pl->launches += 1;
+  }
+  KAON_CUDA(cudaGetLastError());
+  return KAON_OK;
 }
 
 void kp_free(kaon_plan* pl) {
@@ -422,13 +676,13 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   pl->kp = h;
   h->slice_p = slice_p;
   const int n = pl->n_tensors;
-  std::vector<Task> items, stats, fin;
-  std::vector<int> begin(n + 1, 0), fact;
-  std::vector<long long> row_begin(1, 0);
+  std::vector<Task> units, items, rows, stats, fin;
+  std::vector<int> begin(n + 1, 0);
+  int slots = 0;
   std::vector<KpBufs> bufs(n);
   for (int i = 0; i < n; ++i) {
     const DevTensor& t = pl->h_tensors[i];
-    begin[i] = (int)items.size();
+    begin[i] = slots;
     bufs[i].s = s[i];
     bufs[i].p0 = p0 ? p0[i] : nullptr;
     if (t.numel == 0) continue;
@@ -437,13 +691,25 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
       return fail(KAON_E_UNSUPPORTED, "KProdigy: tensor %d: one 4-bit block over %lld elements", i, (long long)t.numel);
     if (t.rows > 0) {
       if (t.cols > CAP) return fail(KAON_E_UNSUPPORTED, "KProdigy: tensor %d: rows of %d elements exceed a work item of %d", i, t.cols, CAP);
-      fact.push_back(i);
-      row_begin.push_back(row_begin.back() + t.rows);
+      const long long nr = std::max<long long>(1, 4096 / t.cols);
+      for (long long r = 0; r < t.rows; r += nr)
+        rows.push_back(Task{i, PH_ADA_STATS, r * t.cols, (int)std::min<long long>(nr, t.rows - r), (int)r, 0, 0});
+    }
+    const uintptr_t ptrs = (uintptr_t)s[i] | (uintptr_t)bufs[i].p0 | (uintptr_t)t.stat_a;
+    if (((t.rows > 0 ? t.cols : t.numel) & 7) == 0 && (pl->momentum_kind != KAON_M_4BIT || t.bshift == 7) && slice_p == 1 &&
+        (ptrs & 15) == 0) {
+      // a warp's unit: small tensors in more pieces (the tensor alone decides, so the order of its sums stays)
+      long long u = 512;
+      while (u < 4096 && u * 128 <= t.numel) u *= 2;
+      for (long long e = 0; e < t.numel; e += u)
+        units.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(u, t.numel - e), t.rows > 0 ? (int)(e / t.cols) : 0, slots++,
+                             t.rows > 0 ? (int)(e % t.cols) : 0});
+      continue;
     }
     for (long long e = 0; e < t.numel; e += KP_ITEM)
-      items.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(KP_ITEM, t.numel - e), 0, 0, 0});
+      items.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(KP_ITEM, t.numel - e), 0, slots++, 0});
   }
-  begin[n] = (int)items.size();
+  begin[n] = slots;
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
@@ -460,10 +726,10 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   size_t o = 0;
   auto take = [&](size_t b) { size_t r = o; o += up(b); return r; };
-  const size_t o_items = take(sizeof(Task) * items.size()), o_begin = take(sizeof(int) * (n + 1));
-  const size_t o_bufs = take(sizeof(KpBufs) * n), o_part = take(sizeof(double) * 2 * items.size());
+  const size_t o_items = take(sizeof(Task) * items.size()), o_units = take(sizeof(Task) * units.size()), o_begin = take(sizeof(int) * (n + 1));
+  const size_t o_bufs = take(sizeof(KpBufs) * n), o_part = take(sizeof(double) * 2 * slots);
   const size_t o_sums = take(sizeof(float) * 2 * n), o_tmax = take(sizeof(unsigned) * n), o_told = take(sizeof(float) * n);
-  const size_t o_fact = take(sizeof(int) * fact.size()), o_rows = take(sizeof(long long) * row_begin.size());
+  const size_t o_rows = take(sizeof(Task) * rows.size());
   const size_t o_stats = take(sizeof(Task) * stats.size()), o_fin = take(sizeof(Task) * fin.size());
   KAON_CUDA(cudaMalloc(&h->block, std::max<size_t>(o, 256)));
   unsigned char* base = reinterpret_cast<unsigned char*>(h->block);
@@ -475,20 +741,20 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   KAON_CUDA(put(o_items, items.data(), sizeof(Task) * items.size()));
   KAON_CUDA(put(o_begin, begin.data(), sizeof(int) * (n + 1)));
   KAON_CUDA(put(o_bufs, bufs.data(), sizeof(KpBufs) * n));
-  KAON_CUDA(put(o_fact, fact.data(), sizeof(int) * fact.size()));
-  KAON_CUDA(put(o_rows, row_begin.data(), sizeof(long long) * row_begin.size()));
+  KAON_CUDA(put(o_units, units.data(), sizeof(Task) * units.size()));
+  KAON_CUDA(put(o_rows, rows.data(), sizeof(Task) * rows.size()));
   KAON_CUDA(put(o_stats, stats.data(), sizeof(Task) * stats.size()));
   KAON_CUDA(put(o_fin, fin.data(), sizeof(Task) * fin.size()));
   KpView& x = h->view;
   x.items = reinterpret_cast<const Task*>(base + o_items); x.n_items = (int)items.size();
+  x.units = reinterpret_cast<const Task*>(base + o_units); x.n_units = (int)units.size();
   x.item_begin = reinterpret_cast<const int*>(base + o_begin);
   x.bufs = reinterpret_cast<const KpBufs*>(base + o_bufs);
   x.part = reinterpret_cast<double*>(base + o_part);
   x.sums = reinterpret_cast<float*>(base + o_sums);
   x.tmax = reinterpret_cast<unsigned*>(base + o_tmax);
   x.told = reinterpret_cast<float*>(base + o_told);
-  x.fact = reinterpret_cast<const int*>(base + o_fact); x.n_fact = (int)fact.size();
-  x.row_begin = reinterpret_cast<const long long*>(base + o_rows); x.n_rows = row_begin.back();
+  x.row_units = reinterpret_cast<const Task*>(base + o_rows); x.n_row_units = (int)rows.size();
   h->d_stats = stats.empty() ? nullptr : reinterpret_cast<Task*>(base + o_stats); h->n_stats = (int)stats.size();
   h->d_final = reinterpret_cast<Task*>(base + o_fin); h->n_final = (int)fin.size();
   h->h_sums.assign((size_t)2 * n, 0.0f);
@@ -531,8 +797,7 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
   cudaStream_t s = (cudaStream_t)stream;
   const KpView& x = kh->view;
   const int mk = pl->momentum_kind;
-  const int grid = std::max(1, std::min(x.n_items, pl->sm_count * 8));
-  if (hp.factored && x.n_fact > 0) {
+  if (hp.factored && x.n_row_units > 0) {
     AdaDev ad{};
     ad.w2 = (float)(1.0 - h->beta2); ad.w2m1 = ad.w2 - 1.0f; ad.small_w2 = ad.w2 < 0.5f;
     ad.w1 = 1.0f; ad.eps1 = (float)h->eps_factored; ad.has_eps = h->eps_factored > 0.0; ad.clip = 1.0f;
@@ -545,24 +810,20 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
     v.tasks = kh->d_final; v.n_tasks = kh->n_final;
     if (int rc = launch_persistent(pl, v, ad, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
-  } else if (hp.gc && x.n_fact > 0) {
-    if (pl->param_dtype == KAON_DT_BF16) kp_rowmean_kernel<__nv_bfloat16><<<pl->sm_count * 8, KP_THREADS, 0, s>>>(pl->view, x);
-    else kp_rowmean_kernel<float><<<pl->sm_count * 8, KP_THREADS, 0, s>>>(pl->view, x);
+  } else if (hp.gc && x.n_row_units > 0) {
+    const int grid = std::min((x.n_row_units + KP_THREADS / 32 - 1) / (KP_THREADS / 32), pl->sm_count * 8);
+    if (pl->param_dtype == KAON_DT_BF16) kp_rowmean_kernel<__nv_bfloat16><<<grid, KP_THREADS, 0, s>>>(pl->view, x);
+    else kp_rowmean_kernel<float><<<grid, KP_THREADS, 0, s>>>(pl->view, x);
     pl->launches += 1;
   }
-  if (x.n_items > 0) {
+  if (x.n_units + x.n_items > 0) {
     if (mk == KAON_M_INT8) {
       kp_prep_kernel<<<pl->n_tensors, KP_THREADS, 0, s>>>(pl->view, x);
       pl->launches += 1;
     }
-    KpSweep k0 = pick_sweep<0>(pl->param_dtype, mk);
-    if (!k0) return fail(KAON_E_INVALID, "no KProdigy kernel for this dtype combination");
-    k0<<<grid, KP_THREADS, 0, s>>>(pl->view, hp, x);
-    pl->launches += 1;
-    if (mk == KAON_M_INT8) {
-      pick_sweep<1>(pl->param_dtype, mk)<<<grid, KP_THREADS, 0, s>>>(pl->view, hp, x);
-      pl->launches += 1;
-    }
+    if (int rc = launch_sweep<0>(pl, hp, x, s)) return rc;
+    if (mk == KAON_M_INT8)
+      if (int rc = launch_sweep<1>(pl, hp, x, s)) return rc;
     if (hp.do_d) {
       kp_reduce_kernel<false><<<pl->n_tensors, KP_THREADS, 0, s>>>(pl->view, x);
       pl->launches += 1;
@@ -595,18 +856,15 @@ extern "C" int kaon_kprodigy_pass2(kaon_plan* pl, const kaon_kprodigy_pass2_hpar
   hp.kahan = h->bf16_method == KAON_W_KAHAN && pl->param_dtype == KAON_DT_BF16;
   hp.slice_p = kh->slice_p;
   hp.step = step; hp.k0 = (uint32_t)seed; hp.k1 = (uint32_t)(seed >> 32);
+  philox_round_keys(hp);
   cudaStream_t s = (cudaStream_t)stream;
   const KpView& x = kh->view;
-  if (x.n_items == 0) return KAON_OK;
-  const int mk = pl->momentum_kind;
-  const int grid = std::max(1, std::min(x.n_items, pl->sm_count * 8));
+  if (x.n_units + x.n_items == 0) return KAON_OK;
   if (hp.cautious) {
-    pick_sweep<2>(pl->param_dtype, mk)<<<grid, KP_THREADS, 0, s>>>(pl->view, hp, x);
+    if (int rc = launch_sweep<2>(pl, hp, x, s)) return rc;
     kp_reduce_kernel<true><<<pl->n_tensors, KP_THREADS, 0, s>>>(pl->view, x);
-    pl->launches += 2;
+    pl->launches += 1;
   }
-  pick_sweep<3>(pl->param_dtype, mk)<<<grid, KP_THREADS, 0, s>>>(pl->view, hp, x);
-  KAON_CUDA(cudaGetLastError());
-  pl->launches += 1;
+  if (int rc = launch_sweep<3>(pl, hp, x, s)) return rc;
   return KAON_OK;
 }
