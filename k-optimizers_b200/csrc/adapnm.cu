@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_c
 #pragma unroll
           for (int j = 0; j < 4; ++j) MP[j] = pack2(round_bf16(MP[j].x), round_bf16(MP[j].y));
         }
-        const float sc = store_m8<MK>(pos, MP, rm, act, lane);
+        const float sc = store_m8<MK>(pos, MP, rm, act ? 8 : 0, lane);
         if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(psc, sc); }
         if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) psc[row] = sc; }
       }

@@ -157,14 +157,14 @@ __device__ __forceinline__ float amax8(const f32x2 M[4]) {
   return fmaxf(a, fabsf(M[3].y));
 }
 
-// Store eight new momenta at mp (every lane of the warp calls it; `act`: this lane has eight).  bf16 momentum is
+// Store eight new momenta at mp (every lane of the warp calls it; `cnt` of the lane's exist, 0..8, M is 0 beyond an odd end).  bf16 momentum is
 // already rounded in M.  `amax`: int8 only, the finished maximum of the row; returns the scale (4-bit: the block's,
 // to be stored by the first lane of a half warp).  Codes are rounded from the correctly rounded quotient m' / scale.
 template <int MK>
-__device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax, const bool act, const int lane) {
+__device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax, const int cnt, const int lane) {
   if constexpr (MK == KAON_M_4BIT || MK == KAON_M_INT8) {
     float sc;
-    if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(act ? amax8(M) : 0.0f, lane), 1e-12f));
+    if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(cnt > 0 ? amax8(M) : 0.0f, lane), 1e-12f));
     else sc = div127_exact(fmaxf(amax, 1e-12f));
     float inv;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
@@ -186,20 +186,32 @@ __device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax
       const f32x2 Xl = fma2(T[1], K256, T[0]), Yl = fma2(T[3], K256, T[2]);
       const float lo4 = __fsub_rn(8423560.0f, __fmaf_rn(Xl.y, 16.0f, Xl.x));
       const float hi4 = __fsub_rn(8423560.0f, __fmaf_rn(Yl.y, 16.0f, Yl.x));
-      if (act) stg_u32(mp, prmt(__float_as_uint(lo4), __float_as_uint(hi4), 0x5410u));
-    } else if (act) {  // the low byte of every R is the code in two's complement
+      const uint32_t w = prmt(__float_as_uint(lo4), __float_as_uint(hi4), 0x5410u);
+      if (cnt == 8) stg_u32(mp, w);
+      else
+        for (int b = 0; 2 * b < cnt; ++b)
+          reinterpret_cast<unsigned char*>(mp)[b] = (unsigned char)((w >> (8 * b)) & (2 * b + 1 < cnt ? 0xffu : 0xfu));
+    } else if (cnt > 0) {  // the low byte of every R is the code in two's complement
       const uint32_t w0 = prmt(prmt(__float_as_uint(R[0].x), __float_as_uint(R[0].y), 0x0040u),
                                prmt(__float_as_uint(R[1].x), __float_as_uint(R[1].y), 0x0040u), 0x5410u);
       const uint32_t w1 = prmt(prmt(__float_as_uint(R[2].x), __float_as_uint(R[2].y), 0x0040u),
                                prmt(__float_as_uint(R[3].x), __float_as_uint(R[3].y), 0x0040u), 0x5410u);
-      *reinterpret_cast<uint2*>(mp) = make_uint2(w0, w1);
+      *reinterpret_cast<uint2*>(mp) = make_uint2(w0, w1);   // (int8 rows are whole vectors)
     }
     return sc;
   } else {
     MRaw<MK> o;
 #pragma unroll
     for (int j = 0; j < 4; ++j) o.w.set(j, M[j]);
-    if (act) o.w.store(mp, nullptr);
+    if (cnt == 8) o.w.store(mp, nullptr);
+    else
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < cnt) {
+          const float x = k & 1 ? M[k >> 1].y : M[k >> 1].x;
+          if constexpr (MK == KAON_M_BF16) reinterpret_cast<uint16_t*>(mp)[k] = (uint16_t)(__float_as_uint(x) >> 16);
+          else reinterpret_cast<float*>(mp)[k] = x;
+        }
     return 1.0f;
   }
 }

@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
           } else if constexpr (MK != KAON_M_NONE) {
             float rm = 0.0f;
             if constexpr (MK == KAON_M_INT8) rm = __uint_as_float(__ldcg(rowmax + r));
-            const float sc = store_m8<MK>(mp + o * (unsigned)MV, M, rm, act, lane);
+            const float sc = store_m8<MK>(mp + o * (unsigned)MV, M, rm, act ? 8 : 0, lane);
             if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(blk + (v >> 4), sc); }
             if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) d.m_scale[row] = sc; }
           }

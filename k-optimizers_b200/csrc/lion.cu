@@ -14,16 +14,9 @@
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
 #include "kaon_packed.cuh"
+#include "lion_dev.h"
 
 namespace kaon {
-
-struct LionDev {
-  float lr, b1, w1, b2, w2, wd;
-  int cautious, gc, sr, has_wd;
-  uint32_t step, k0, k1;
-  uint32_t rk0[KAON_PHILOX_ROUNDS], rk1[KAON_PHILOX_ROUNDS];  // Philox round keys (k + r * Weyl), from the host
-  int kahan;
-};
 
 // Philox4x32-7 with the round keys read from the kernel's parameter block.
 __device__ __forceinline__ void philox_rk(const LionDev& hp, uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
@@ -847,9 +840,14 @@ extern "C" int kaon_lion_step(kaon_plan* pl, const kaon_lion_hparams* h, uint64_
   for (int r = 0; r < KAON_PHILOX_ROUNDS; ++r) { hp.rk0[r] = hp.k0 + 0x9E3779B9u * (uint32_t)r; hp.rk1[r] = hp.k1 + 0xBB67AE85u * (uint32_t)r; }
   cudaStream_t s = (cudaStream_t)stream;
   PlanView v = pl->view;
-  if (hp.cautious) { v.tasks = pl->d_tasks_full; v.n_tasks = pl->n_tasks_full; }
+  if (hp.cautious) { v.tasks = pl->d_tasks_full; v.n_tasks = pl->n_tasks_full; }   // (of the tensors without warp units)
   else { v.tasks = pl->d_tasks_main; v.n_tasks = pl->n_tasks_main; }
   KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
+  if (hp.cautious && pl->n_tasks_warp > 0) {
+    if (int rc = launch_lion_warp(pl, v, hp, s)) return rc;
+    v.task_counter = v.counters2;
+  }
+  if (v.n_tasks == 0) return KAON_OK;
   if (pl->n_flat_tensors > 0 && hp.gc) {  // row means of the tensors cut into flat runs
     if (pl->param_dtype == KAON_DT_BF16) lion_rowmean_kernel<__nv_bfloat16><<<pl->sm_count * 4, 256, 0, s>>>(v, pl->d_flat_tensors, pl->n_flat_tensors);
     else lion_rowmean_kernel<float><<<pl->sm_count * 4, 256, 0, s>>>(v, pl->d_flat_tensors, pl->n_flat_tensors);

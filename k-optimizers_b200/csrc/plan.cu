@@ -11,6 +11,7 @@
 
 #include "kaon_host.h"
 #include "kaon_plan.h"
+#include "lion_dev.h"
 
 namespace kaon {
 
@@ -316,12 +317,23 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   for (int i = 0; i < n; ++i)
     if (tens[i].m)
       for (const Task& t : per[i]) { Task a = t; a.phase = PH_AXPY; axpy_list.push_back(a); }
+  // Lion with the cautious mask: warp units for the tensors that can take them, the staged kernel for the others
+  std::vector<Task> warp_list;
+  if (optimizer == KAON_OPT_LION) {
+    std::vector<char> elig(n, 0);
+    for (int i = 0; i < n; ++i) elig[i] = lion_warp_tensor(tens[i], momentum_kind);
+    std::vector<int> units;
+    lion_warp_units(tens, elig, warp_list, units);
+    for (int i = 0; i < n; ++i) if (elig[i]) tens[i].n_main = units[i];
+    full_list.erase(std::remove_if(full_list.begin(), full_list.end(), [&](const Task& t) { return elig[t.tensor] != 0; }), full_list.end());
+  }
 
-  // One device allocation: tensors | grads | tasks(full) | tasks(main) | tasks(axpy) | tasks(small) | counters.
+  // One device allocation: tensors | grads | tasks(full) | tasks(main) | tasks(axpy) | tasks(small) | tasks(warp) | counters.
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   size_t o_t = 0, o_g = o_t + up(sizeof(DevTensor) * n), o_f = o_g + up(sizeof(void*) * n);
   size_t o_m = o_f + up(sizeof(Task) * full_list.size()), o_a = o_m + up(sizeof(Task) * main_list.size());
-  size_t o_s = o_a + up(sizeof(Task) * axpy_list.size()), o_c = o_s + up(sizeof(Task) * small_list.size());
+  size_t o_s = o_a + up(sizeof(Task) * axpy_list.size()), o_w = o_s + up(sizeof(Task) * small_list.size());
+  size_t o_c = o_w + up(sizeof(Task) * warp_list.size());
   pl->counters_bytes = sizeof(unsigned) * (size_t)(2 + 5 * n + 4);
   size_t tot = o_c + up(pl->counters_bytes);
   ce = cudaMalloc(&pl->d_block, tot);
@@ -351,6 +363,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   cudaMemcpy(base + o_g, grads.data(), sizeof(void*) * n, cudaMemcpyHostToDevice);
   cudaMemcpy(base + o_f, full_list.data(), sizeof(Task) * full_list.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(base + o_m, main_list.data(), sizeof(Task) * main_list.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(base + o_w, warp_list.data(), sizeof(Task) * warp_list.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(base + o_s, small_list.data(), sizeof(Task) * small_list.size(), cudaMemcpyHostToDevice);
   ce = cudaMemcpy(base + o_a, axpy_list.data(), sizeof(Task) * axpy_list.size(), cudaMemcpyHostToDevice);
   if (ce != cudaSuccess) { kaon_plan_destroy(pl); return cuda_fail(ce, "cudaMemcpy(plan tables)"); }
@@ -360,6 +373,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   pl->d_tasks_main = (Task*)(base + o_m); pl->n_tasks_main = (int)main_list.size();
   pl->d_tasks_axpy = (Task*)(base + o_a); pl->n_tasks_axpy = (int)axpy_list.size();
   pl->d_tasks_small = (Task*)(base + o_s); pl->n_tasks_small = (int)small_list.size();
+  pl->d_tasks_warp = (Task*)(base + o_w); pl->n_tasks_warp = (int)warp_list.size();
   pl->d_counters = (unsigned*)(base + o_c);
   PlanView& v = pl->view;
   v.tensors = (const DevTensor*)(base + o_t);
