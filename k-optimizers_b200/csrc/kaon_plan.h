@@ -141,7 +141,7 @@ struct kaon_plan {
   kaon::Task* d_tasks_main = nullptr;
   kaon::Task* d_tasks_axpy = nullptr;
   kaon::Task* d_tasks_warp = nullptr;   // Lion: warp units (lion_warp.cu), MAIN and APPLY in the order of claims
-  int n_tasks_warp = 0;
+  int n_tasks_warp = 0, n_tasks_warp_main = 0;   // (the latter: MAIN units at its head that are a launch of their own)
   void* d_block = nullptr;      // one allocation holding tables and counters
   unsigned char* d_codes = nullptr;
   float* d_aux = nullptr;

@@ -19,7 +19,7 @@ struct LionDev {
 // lion_warp.cu: the cautious step as warp units.  lion_warp_tensor: whether a tensor can take it; lion_warp_units: the
 // units of the plan's eligible tensors, MAIN and APPLY in the order they are claimed, and each one's number of MAIN units.
 bool lion_warp_tensor(const DevTensor& t, int momentum_kind);
-void lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<char>& elig, std::vector<Task>& out, std::vector<int>& n_main);
+int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<char>& elig, std::vector<Task>& out, std::vector<int>& n_main);
 int launch_lion_warp(kaon_plan* pl, const PlanView& base, const LionDev& hp, cudaStream_t s);
 
 }  // namespace kaon

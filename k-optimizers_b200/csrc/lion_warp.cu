@@ -4,7 +4,8 @@
 // new momentum, its codes, and two bits an element for APPLY (0 / 1 / 2: update sign -1 / 0 / +1; 3: masked out, where
 // there is weight decay; without it a masked element is 1).  APPLY unit: once every MAIN unit of the tensor has finished,
 // the weights with the tensor-wide rescale 1/max(kept/numel, 1e-8).  One launch: units are claimed in list order, a
-// tensor's APPLY some 32 M elements behind its MAIN, so that waits are rare and the two-bit codes are still in L2.
+// tensor's APPLY some 32 M elements behind its MAIN, so that waits are rare and the two-bit codes are still in L2 (large
+// lists: a launch each, see lion_warp_units).
 //
 // Bound by instruction issue (4-bit momentum) or HBM (wider states), so: packed pairs; the mask one saturating FMA an
 // element; both kinds of codes packed as small integers by FMAs; rows advanced by an addition; the next trip's words
@@ -93,7 +94,8 @@ __device__ __forceinline__ void row_means(const unsigned char* g, int C, int r0,
   }
 }
 
-template <typename PT, int MK, bool WD>
+// SIGNAL: APPLY units of the same launch wait for this one.
+template <typename PT, int MK, bool WD, bool SIGNAL>
 __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev& hp, const Task& t, const unsigned char* gbase,
                                                float* mean_s, const int lane) {
   using E = Elems<PT>;
@@ -268,21 +270,21 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
     else sweep(std::false_type{});
   }
   kept = __reduce_add_sync(0xffffffffu, kept);
-  if (lane == 0) {
-    if (kept) atomicAdd(pv.kept + t.tensor, kept);
+  if (lane == 0 && kept) atomicAdd(pv.kept + t.tensor, kept);
+  if constexpr (SIGNAL) {
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) signal_counter(pv.done + t.tensor, 1u);
   }
-  __threadfence();
-  __syncwarp();
-  if (lane == 0) signal_counter(pv.done + t.tensor, 1u);
 }
 
-template <typename PT, bool WD>
+template <typename PT, bool WD, bool WAIT>
 __device__ __forceinline__ void lion_apply_unit(const PlanView& pv, const LionDev& hp, const Task& t, float2* lut_s, const int lane) {
   using E = Elems<PT>;
   const DevTensor& d = pv.tensors[t.tensor];
   bool ok = true;
-  if (lane == 0) ok = wait_counter(pv.done + t.tensor, (unsigned)d.n_main, pv.status, 2001u, pv.spin_limit ? pv.spin_limit : KAON_SPIN_LIMIT);
-  if (!__all_sync(0xffffffffu, ok)) return;
+  if (WAIT && lane == 0) ok = wait_counter(pv.done + t.tensor, (unsigned)d.n_main, pv.status, 2001u, pv.spin_limit ? pv.spin_limit : KAON_SPIN_LIMIT);
+  if (WAIT && !__all_sync(0xffffffffu, ok)) return;
   // cautious rescale (reference src/kaon/_backend.py:127-134): mean(mask) = count / numel in fp32
   const float denom = fmaxf(__fdiv_rn((float)__ldcg(pv.kept + t.tensor), (float)d.numel), 1e-8f);
   const float rdenom = __frcp_rn(denom);
@@ -348,12 +350,10 @@ __device__ __forceinline__ void lion_apply_unit(const PlanView& pv, const LionDe
   __syncwarp();
 }
 
-template <typename PT, int MK, bool WD>
-__global__ void __launch_bounds__(LWT, 4) lion_warp_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ LionDev hp) {
-  __shared__ float mean_s[LWT / 32][LW_ROWS];
-  __shared__ float2 lut_s[LWT / 32][16];
+// Units in list order, each claimed while the one before it is worked on.
+template <typename Unit>
+__device__ __forceinline__ void claimed_units(const PlanView& pv, const int lane, Unit unit) {
   if (on_reserved_sm(pv.sm_reserve)) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   auto claim = [&]() -> int {
     int i = 0x7fffffff;
     if (lane == 0) {
@@ -367,12 +367,34 @@ __global__ void __launch_bounds__(LWT, 4) lion_warp_kernel(const __grid_constant
     const int next = claim();
     const Task t = pv.tasks[cur];
     const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
-    if (g != nullptr) {
-      if (t.phase == PH_LION_MAIN) lion_main_unit<PT, MK, WD>(pv, hp, t, g, mean_s[warp], lane);
-      else lion_apply_unit<PT, WD>(pv, hp, t, lut_s[warp], lane);
-    }
+    if (g != nullptr) unit(t, g);
     cur = __shfl_sync(0xffffffffu, next, 0);
   }
+}
+
+template <typename PT, int MK, bool WD>
+__global__ void __launch_bounds__(LWT, 4) lion_warp_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ LionDev hp) {
+  __shared__ float mean_s[LWT / 32][LW_ROWS];
+  __shared__ float2 lut_s[LWT / 32][16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  claimed_units(pv, lane, [&](const Task& t, const unsigned char* g) {
+    if (t.phase == PH_LION_MAIN) lion_main_unit<PT, MK, WD, true>(pv, hp, t, g, mean_s[warp], lane);
+    else lion_apply_unit<PT, WD, true>(pv, hp, t, lut_s[warp], lane);
+  });
+}
+
+template <typename PT, int MK, bool WD>
+__global__ void __launch_bounds__(LWT, 4) lion_main_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ LionDev hp) {
+  __shared__ float mean_s[LWT / 32][LW_ROWS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  claimed_units(pv, lane, [&](const Task& t, const unsigned char* g) { lion_main_unit<PT, MK, WD, false>(pv, hp, t, g, mean_s[warp], lane); });
+}
+
+template <typename PT, bool WD>
+__global__ void __launch_bounds__(LWT, 4) lion_apply_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ LionDev hp) {
+  __shared__ float2 lut_s[LWT / 32][16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  claimed_units(pv, lane, [&](const Task& t, const unsigned char*) { lion_apply_unit<PT, WD, false>(pv, hp, t, lut_s[warp], lane); });
 }
 
 // ----------------------------------------------------------------------------- host
@@ -387,8 +409,14 @@ bool lion_warp_tensor(const DevTensor& t, int momentum_kind) {
 // Units: about 4096 elements (small tensors in more pieces), starting on 128-element boundaries.  Whole rows where rows are a
 // multiple of 128; otherwise at least two rows' worth, since the rows at both ends are averaged by two units, and at most
 // LW_ROWS rows.
-void lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<char>& elig, std::vector<Task>& out, std::vector<int>& n_main) {
-  constexpr long long LAG = 32ll << 20;
+// Order: up to 64 M elements one launch, a tensor's APPLY LAG elements behind its MAIN.  Larger lists two launches, all of MAIN
+// first (returns the number of MAIN units; 0: one launch): the completion counters' fences cost the first level caches,
+// where the second reading of a row's gradient hits, more than the codes' way through HBM (2.6 B list: 5.23 ms in one).
+int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<char>& elig, std::vector<Task>& out, std::vector<int>& n_main) {
+  long long total = 0;
+  for (size_t i = 0; i < tensors.size(); ++i) if (elig[i]) total += tensors[i].numel;
+  const bool split = total > (64ll << 20);
+  const long long LAG = split ? total : 32ll << 20;
   const int n = (int)tensors.size();
   n_main.assign(n, 0);
   long long done = 0;
@@ -422,35 +450,46 @@ void lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<ch
     for (; waiting < i && end[waiting] + LAG <= done; ++waiting)
       if (elig[waiting]) apply(waiting);
   }
+  const int mains = split ? (int)out.size() : 0;
   for (; waiting < n; ++waiting)
     if (elig[waiting]) apply(waiting);
+  return mains;
 }
 
 typedef void (*LionWarp)(PlanView, LionDev);
 
 template <typename PT, bool WD>
-static LionWarp pick(int mk) {
+static LionWarp pick(int mk, bool split) {
   switch (mk) {
-    case KAON_M_4BIT: return lion_warp_kernel<PT, KAON_M_4BIT, WD>;
-    case KAON_M_BF16: return lion_warp_kernel<PT, KAON_M_BF16, WD>;
-    case KAON_M_F32: return lion_warp_kernel<PT, KAON_M_F32, WD>;
+    case KAON_M_4BIT: return split ? lion_main_kernel<PT, KAON_M_4BIT, WD> : lion_warp_kernel<PT, KAON_M_4BIT, WD>;
+    case KAON_M_BF16: return split ? lion_main_kernel<PT, KAON_M_BF16, WD> : lion_warp_kernel<PT, KAON_M_BF16, WD>;
+    case KAON_M_F32: return split ? lion_main_kernel<PT, KAON_M_F32, WD> : lion_warp_kernel<PT, KAON_M_F32, WD>;
     default: return nullptr;
   }
 }
 
 int launch_lion_warp(kaon_plan* pl, const PlanView& base, const LionDev& hp, cudaStream_t s) {
-  PlanView v = base;
-  v.tasks = pl->d_tasks_warp;
-  v.n_tasks = pl->n_tasks_warp;
-  const bool bf = pl->param_dtype == KAON_DT_BF16;
-  LionWarp k = hp.has_wd ? (bf ? pick<__nv_bfloat16, true>(pl->momentum_kind) : pick<float, true>(pl->momentum_kind))
-                         : (bf ? pick<__nv_bfloat16, false>(pl->momentum_kind) : pick<float, false>(pl->momentum_kind));
+  const bool bf = pl->param_dtype == KAON_DT_BF16, split = pl->n_tasks_warp_main > 0;
+  const int mk = pl->momentum_kind;
+  LionWarp k = hp.has_wd ? (bf ? pick<__nv_bfloat16, true>(mk, split) : pick<float, true>(mk, split))
+                         : (bf ? pick<__nv_bfloat16, false>(mk, split) : pick<float, false>(mk, split));
+  LionWarp ka = hp.has_wd ? (bf ? lion_apply_kernel<__nv_bfloat16, true> : lion_apply_kernel<float, true>)
+                          : (bf ? lion_apply_kernel<__nv_bfloat16, false> : lion_apply_kernel<float, false>);
   if (!k) return fail(KAON_E_INVALID, "no Lion kernel for this dtype combination");
-  const int most = pl->sm_count * 4;
-  const int grid = base.sm_reserve ? most : std::max(1, std::min((v.n_tasks + LWT / 32 - 1) / (LWT / 32), most));
-  k<<<grid, LWT, 0, s>>>(v, hp);
+  auto run = [&](LionWarp kernel, const Task* tasks, int n, unsigned* counter) {
+    PlanView v = base;
+    v.tasks = tasks;
+    v.n_tasks = n;
+    v.task_counter = counter;
+    const int most = pl->sm_count * 4;
+    const int grid = base.sm_reserve ? most : std::max(1, std::min((n + LWT / 32 - 1) / (LWT / 32), most));
+    kernel<<<grid, LWT, 0, s>>>(v, hp);
+    pl->launches += 1;
+  };
+  const int first = split ? pl->n_tasks_warp_main : pl->n_tasks_warp;
+  run(k, pl->d_tasks_warp, first, base.task_counter);
+  if (split) run(ka, pl->d_tasks_warp + first, pl->n_tasks_warp - first, base.counters2 + 1);
   KAON_CUDA(cudaGetLastError());
-  pl->launches += 1;
   return KAON_OK;
 }
 

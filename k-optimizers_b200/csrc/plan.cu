@@ -323,7 +323,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
     std::vector<char> elig(n, 0);
     for (int i = 0; i < n; ++i) elig[i] = lion_warp_tensor(tens[i], momentum_kind);
     std::vector<int> units;
-    lion_warp_units(tens, elig, warp_list, units);
+    pl->n_tasks_warp_main = lion_warp_units(tens, elig, warp_list, units);
     for (int i = 0; i < n; ++i) if (elig[i]) tens[i].n_main = units[i];
     full_list.erase(std::remove_if(full_list.begin(), full_list.end(), [&](const Task& t) { return elig[t.tensor] != 0; }), full_list.end());
   }
