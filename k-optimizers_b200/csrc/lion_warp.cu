@@ -1,8 +1,8 @@
 // The cautious Lion step, a warp per unit of up to 4096 consecutive elements, nothing shared between warps.
 //
 // MAIN unit: the means of the rows it touches, then per eight elements of a lane the direction sign(b1*m + (1-b1)*g), the
-// new momentum, its codes, and two bits an element for APPLY (0 / 1 / 2: update sign -1 / 0 / +1; 3: masked out, where
-// there is weight decay; without it a masked element is 1).  APPLY unit: once every MAIN unit of the tensor has finished,
+// new momentum, its codes, and two bits an element for APPLY (element e, o of a pair: nibble kept_e | kept_o << 1 |
+// neg_e << 2 | neg_o << 3; with weight decay (w_e + 1) + 4 (w_o + 1), w the update's sign or 2 where masked out).  APPLY unit: once every MAIN unit of the tensor has finished,
 // the weights with the tensor-wide rescale 1/max(kept/numel, 1e-8).  One launch: units are claimed in list order, a
 // tensor's APPLY some 32 M elements behind its MAIN, so that waits are rare and the two-bit codes are still in L2 (large
 // lists: a launch each, see lion_warp_units).
@@ -17,6 +17,7 @@
 
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
+#include "kaon_elem.cuh"
 #include "kaon_sweep.cuh"
 #include "lion_dev.h"
 
@@ -47,13 +48,29 @@ __device__ __forceinline__ void load_some(MRaw<KAON_M_4BIT>& w, const void* p, i
 template <typename T>
 __device__ __forceinline__ void load_some(MPlain<T>& w, const void* p, int cnt) { load_some(w.w, p, cnt); }
 
+// A lane's part of the sum of a row of whole vectors
+template <typename PT>
+__device__ __forceinline__ float row_part(const unsigned char* rowp, int C, int lane) {
+  f32x2 a = pack2(0.0f, 0.0f), b = pack2(0.0f, 0.0f);
+#pragma unroll 4
+  for (int v = lane * 8; v < C; v += 256) {
+    W8<PT> w;
+    w.load(rowp + v * Elems<PT>::BYTES);
+    a = add2(a, add2(w.pair(0), w.pair(1)));
+    b = add2(b, add2(w.pair(2), w.pair(3)));
+  }
+  a = add2(a, b);
+  return a.x + a.y;
+}
+
 // Means of rows r0 .. r0 + n (as the gradient's dtype holds them) into mean_s: rows of up to 64 elements a lane each, longer ones
 // the whole warp.
 template <typename PT>
 __device__ __forceinline__ void row_means(const unsigned char* g, int C, int r0, int n, float* mean_s, int lane) {
   using E = Elems<PT>;
   const bool vec = (C & 7) == 0;
-  auto put = [&](int r, float s) { mean_s[r] = round_to(__fdiv_rn(s, (float)C), PT()); };
+  const float fC = (float)C, rC = __frcp_rn(fC);
+  auto put = [&](int r, float s) { mean_s[r] = round_to(div_by(s, fC, rC), PT()); };
   if (C <= 64) {
     for (int r = lane; r < n; r += 32) {
       const unsigned char* rowp = g + (long long)(r0 + r) * C * E::BYTES;
@@ -77,14 +94,7 @@ __device__ __forceinline__ void row_means(const unsigned char* g, int C, int r0,
     const unsigned char* rowp = g + (long long)(r0 + r) * C * E::BYTES;
     float s = 0.0f;
     if (vec) {
-      f32x2 a = pack2(0.0f, 0.0f);
-#pragma unroll 4
-      for (int v = lane * 8; v < C; v += 256) {
-        W8<PT> w;
-        w.load(rowp + v * E::BYTES);
-        a = add2(a, add2(add2(w.pair(0), w.pair(1)), add2(w.pair(2), w.pair(3))));
-      }
-      s = a.x + a.y;
+      s = row_part<PT>(rowp, C, lane);
     } else {
 #pragma unroll 8
       for (int i = lane; i < C; i += 32) s += E::load1(rowp, i);
@@ -105,7 +115,9 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
   const int C = d.cols;
   // rows that start on vector and block boundaries go one by one (mean and sweep of a row back to back: the second
   // reading hits L1); others with the whole unit's means first
-  const int seg = gc && (C & 127) == 0 && C >= 512 ? C : t.n;
+  const bool by_row = gc && (C & 127) == 0 && C >= 512;
+  const int seg = by_row ? C : t.n;
+  const float fC = (float)C, rC = __frcp_rn(fC);
   unsigned kept = 0;
   for (int s0 = 0; s0 < t.n; s0 += seg) {
     const int n = min(seg, t.n - s0);
@@ -127,29 +139,30 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
       if constexpr (WD) P.load(pp + v * (8u * E::BYTES));
     };
     if (lane < nvec) load((unsigned)lane);   // in flight over the means
-    const int row0 = seg == t.n ? t.row0 : t.row0 + s0 / C;
-    const int col0 = seg == t.n ? t.pad : 0;
-    if (gc) {
+    float mean = 0.0f;   // by_row: the segment's
+    if (by_row) {
+      mean = round_to(div_by(warp_sum(row_part<PT>(gp, C, lane)), fC, rC), PT());
+    } else if (gc) {
       __syncwarp();
-      row_means<PT>(gbase, C, row0, (col0 + n + C - 1) / C, mean_s, lane);
+      row_means<PT>(gbase, C, t.row0, (t.pad + n + C - 1) / C, mean_s, lane);
       __syncwarp();
     }
+    const float mean_bits = E::IS_BF16 ? __uint_as_float(pack_bf16_rn(mean, mean)) : mean;
     // row (of the unit's) and column of the lane's next vector; a trip advances by 256 elements
-    int lr = 0, col = col0 + lane * 8;
-    if (gc && col >= C) { const int k = col / C; lr = k; col -= k * C; }
+    int lr = 0, col = t.pad + lane * 8;
+    if (gc && !by_row && col >= C) { const int k = col / C; lr = k; col -= k * C; }
     const int adv_r = gc ? 256 / C : 0, adv_c = 256 - adv_r * C;
 
     // the vector in g, m, p; `cnt` of its elements exist (8 but at the end of a tensor)
-    auto trip = [&](const W8<PT>& g, const MRaw<MK>& m, const W8<PT>& p, const unsigned v, const int cnt, auto rag_tag) {
-      constexpr bool RAG = decltype(rag_tag)::value;
-      f32x2 G[4], MO[4], CD[4], N[4], W[4];
-      if (!gc) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) G[j] = g.pair(j);
-      } else if constexpr (!RAG) {
+    auto trip = [&](const W8<PT>& g, const MRaw<MK>& m, const W8<PT>& p, const unsigned v, const int cnt, auto rows_tag) {
+      constexpr int ROWS = decltype(rows_tag)::value;   // 0: one mean, 1: a row per vector, 2: rows end inside vectors
+      f32x2 G[4], MO[4], CD[4], N[4];
+      if constexpr (ROWS == 0) {
+        center<PT>(g, mean_bits, G);
+      } else if constexpr (ROWS == 1) {
         const float mu = mean_s[lr];
         center<PT>(g, E::IS_BF16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, G);
-      } else {   // rows end inside a vector
+      } else {
         float mu[8];
         if (C >= 8) {
           const float a = mean_s[lr], b = mean_s[min(lr + 1, LW_ROWS - 1)];
@@ -185,24 +198,39 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
         // kept: direction and gradient have the same sign; the update's sign is then the gradient's
         float x[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const f32x2 X = mul2(CD[j], G[j]);
-          x[2 * j] = X.x; x[2 * j + 1] = X.y;
-          W[j] = pack2(mask1(X.x, 0x1p127f, 0.0f), mask1(X.y, 0x1p127f, 0.0f));
-        }
+        for (int j = 0; j < 4; ++j) unpack2(mul2(CD[j], G[j]), x[2 * j], x[2 * j + 1]);
         float low = min3f(fabsf(x[0]), fabsf(x[1]), fabsf(x[2]));
         low = min3f(low, fabsf(x[3]), fabsf(x[4]));
         low = min3f(low, fabsf(x[5]), fabsf(x[6]));
         low = fminf(low, fabsf(x[7]));
-        if (!(low >= 0x1p-126f)) {   // a zero, or a product that underflows: by comparisons
+        // bytes 0xFF where the product is negative (masked out), where the gradient is negative
+        auto signs = [](float a, float b, float c, float d) {
+          return prmt(prmt(__float_as_uint(a), __float_as_uint(b), 0x00FBu), prmt(__float_as_uint(c), __float_as_uint(d), 0x00FBu), 0x5410u);
+        };
+        const uint32_t a_lo = signs(x[0], x[1], x[2], x[3]), a_hi = signs(x[4], x[5], x[6], x[7]);
+        const uint32_t g_lo = signs(G[0].x, G[0].y, G[1].x, G[1].y), g_hi = signs(G[2].x, G[2].y, G[3].x, G[3].y);
+        // element b of each four lives in byte b: kept bits 0,1,4,5 and neg bits 2,3,6,7 of the code byte, all disjoint, so
+        // that the sum of the bytes (top byte of t * 0x01010101) is their OR
+        const uint32_t t_lo = ~a_lo & ((g_lo & 0x80400804u) | 0x20100201u);
+        const uint32_t t_hi = ~a_hi & ((g_hi & 0x80400804u) | 0x20100201u);
+        code = prmt(t_lo * 0x01010101u, t_hi * 0x01010101u, 0x0073u) & 0xffffu;
+        if (!(low > 0.0f)) {   // a zero, or a product that underflows: by comparisons
+          code = 0u;
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            W[j] = pack2((CD[j].x > 0.0f && G[j].x > 0.0f) || (CD[j].x < 0.0f && G[j].x < 0.0f) ? 1.0f : 0.0f,
-                         (CD[j].y > 0.0f && G[j].y > 0.0f) || (CD[j].y < 0.0f && G[j].y < 0.0f) ? 1.0f : 0.0f);
+          for (int k = 0; k < 8; ++k) {
+            const float c = k & 1 ? CD[k >> 1].y : CD[k >> 1].x, gr = k & 1 ? G[k >> 1].y : G[k >> 1].x;
+            const uint32_t bit = 1u << (4 * (k >> 1) + (k & 1));
+            if (c > 0.0f && gr > 0.0f) code |= bit;
+            if (c < 0.0f && gr < 0.0f) code |= 5u * bit;
+          }
         }
+        if (cnt < 8) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) W[j] = pack2(copysignf(W[j].x, G[j].x), copysignf(W[j].y, G[j].y));
+          for (int k = 0; k < 8; ++k) if (k >= cnt) code &= ~(5u << (4 * (k >> 1) + (k & 1)));
+        }
+        kept += __popc(code & 0x3333u);
       } else {
+        f32x2 W[4];
         auto one = [&](float c, float gr, float w) {
           const float s = c > 0.0f ? 1.0f : (c < 0.0f ? -1.0f : 0.0f);
           return __fmul_rn(__fmaf_rn(w, hp.wd, s), gr) > 0.0f ? s : 2.0f;
@@ -212,21 +240,18 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
           const f32x2 w = p.pair(j);
           W[j] = pack2(one(CD[j].x, G[j].x, w.x), one(CD[j].y, G[j].y, w.y));
         }
-      }
-      // sum of (w_k + 1) 4^k, exact in fp32, in the low 16 mantissa bits
-      {
+        // sum of (w_k + 1) 4^k, exact in fp32, in the low 16 mantissa bits
         const f32x2 K16 = pack2(16.0f, 16.0f);
         const f32x2 D = fma2(fma2(W[3], K16, W[2]), pack2(256.0f, 256.0f), fma2(W[1], K16, W[0]));
         code = __float_as_uint(__fadd_rn(__fmaf_rn(D.y, 4.0f, D.x), 8388608.0f + 21845.0f)) & 0xffffu;
+        if (cnt < 8) code |= 0xffffu & ~((1u << (2 * cnt)) - 1u);
+        kept += 8u - __popc(code & (code >> 1) & 0x5555u);
       }
       if (cnt < 8) {
-        const uint32_t there = (1u << (2 * cnt)) - 1u;
-        code = (code & there) | ((WD ? 0xffffu : 0x5555u) & ~there);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
           if (k >= cnt) { if (k & 1) N[k >> 1].y = 0.0f; else N[k >> 1].x = 0.0f; }
       }
-      kept += 8u - __popc((WD ? code & (code >> 1) : code) & 0x5555u);
       if constexpr (MK == KAON_M_BF16) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) N[j] = pack2(round_bf16(N[j].x), round_bf16(N[j].y));
@@ -235,7 +260,7 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
       if constexpr (MK == KAON_M_4BIT) { if (cnt > 0 && (lane & 15) == 0) stg_f32(scp + (v >> 4), sc); }
       if (cnt > 0) stg_u16(cp + v, code);
     };
-    auto sweep = [&](auto rag_tag) {
+    auto sweep = [&](auto rows_tag) {
       int v0 = 0;
       for (; v0 + 32 <= nvec; v0 += 32) {
         const W8<PT> g = gq;
@@ -243,10 +268,12 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
         const W8<PT> p = P;
         const unsigned v = (unsigned)(v0 + lane);
         if (v + 32u < (unsigned)nvec) load(v + 32u);
-        trip(g, m, p, v, 8, rag_tag);
-        lr += adv_r;
-        col += adv_c;
-        if (gc && col >= C) { col -= C; ++lr; }
+        trip(g, m, p, v, 8, rows_tag);
+        if constexpr (decltype(rows_tag)::value != 0) {
+          lr += adv_r;
+          col += adv_c;
+          if (col >= C) { col -= C; ++lr; }
+        }
       }
       if (v0 * 8 < n) {   // the last trip of the unit
         const unsigned v = (unsigned)(v0 + lane);
@@ -263,11 +290,12 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
           if constexpr (MK == KAON_M_4BIT) mq.sc = 1.0f;
           lr = 0;
         }
-        trip(gq, mq, P, v, cnt, rag_tag);
+        trip(gq, mq, P, v, cnt, rows_tag);
       }
     };
-    if (gc && (C & 7)) sweep(std::true_type{});
-    else sweep(std::false_type{});
+    if (!gc || by_row) sweep(std::integral_constant<int, 0>{});
+    else if (C & 7) sweep(std::integral_constant<int, 2>{});
+    else sweep(std::integral_constant<int, 1>{});
   }
   kept = __reduce_add_sync(0xffffffffu, kept);
   if (lane == 0 && kept) atomicAdd(pv.kept + t.tensor, kept);
@@ -291,8 +319,8 @@ __device__ __forceinline__ void lion_apply_unit(const PlanView& pv, const LionDe
   const float vpos = __fmul_rn(__fdiv_rn(1.0f, denom), hp.lr);  // |update| of a kept element, no weight decay
   // the pair a nibble of the codes stands for: minus the updates, or (weight decay) the signs, 2 where masked out
   if (lane < 16) {
-    const float e = (float)(lane & 3) - 1.0f, o = (float)(lane >> 2) - 1.0f;
-    lut_s[lane] = WD ? make_float2(e, o) : make_float2(-e * vpos, -o * vpos);
+    if (WD) lut_s[lane] = make_float2((float)(lane & 3) - 1.0f, (float)(lane >> 2) - 1.0f);
+    else lut_s[lane] = make_float2((lane & 1) ? ((lane & 4) ? vpos : -vpos) : 0.0f, (lane & 2) ? ((lane & 8) ? vpos : -vpos) : 0.0f);
   }
   __syncwarp();
   unsigned char* pp = reinterpret_cast<unsigned char*>(d.p) + t.e0 * E::BYTES;
