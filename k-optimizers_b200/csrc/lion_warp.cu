@@ -96,8 +96,11 @@ __device__ __forceinline__ void row_means(const unsigned char* g, int C, int r0,
     if (vec) {
       s = row_part<PT>(rowp, C, lane);
     } else {
-#pragma unroll 8
-      for (int i = lane; i < C; i += 32) s += E::load1(rowp, i);
+      // whole vectors, and a lane each for the elements before the first and after the last
+      const long long e = (long long)(r0 + r) * C, a = (e + 7) / 8 * 8, b = (e + C) / 8 * 8;
+      s = row_part<PT>(g + a * E::BYTES, (int)(b - a), lane);
+      const long long i = lane < 8 ? e + lane : b + lane - 8;
+      if (lane < 8 ? i < a : i < e + C) s += E::load1(g, i);
     }
     s = warp_sum(s);
     if (lane == 0) put(r, s);
