@@ -2,10 +2,9 @@
 //
 // MAIN unit: the means of the rows it touches, then per eight elements of a lane the direction sign(b1*m + (1-b1)*g), the
 // new momentum, its codes, and two bits an element for APPLY (element e, o of a pair: nibble kept_e | kept_o << 1 |
-// neg_e << 2 | neg_o << 3; with weight decay (w_e + 1) + 4 (w_o + 1), w the update's sign or 2 where masked out).  APPLY unit: once every MAIN unit of the tensor has finished,
-// the weights with the tensor-wide rescale 1/max(kept/numel, 1e-8).  One launch: units are claimed in list order, a
-// tensor's APPLY some 32 M elements behind its MAIN, so that waits are rare and the two-bit codes are still in L2 (large
-// lists: a launch each, see lion_warp_units).
+// neg_e << 2 | neg_o << 3; with weight decay (w_e + 1) + 4 (w_o + 1), w the update's sign or 2 where masked out).  APPLY unit: once every MAIN
+// unit of the tensor has finished, the weights with the tensor-wide rescale 1/max(kept/numel, 1e-8).  Units are claimed in
+// list order, all of MAIN first; small lists are one launch, large ones a launch each (see lion_warp_units).
 //
 // Bound by instruction issue (4-bit momentum) or HBM (wider states), so: packed pairs; the mask one saturating FMA an
 // element; both kinds of codes packed as small integers by FMAs; rows advanced by an addition; the next trip's words
@@ -303,8 +302,7 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
   kept = __reduce_add_sync(0xffffffffu, kept);
   if (lane == 0 && kept) atomicAdd(pv.kept + t.tensor, kept);
   if constexpr (SIGNAL) {
-    __threadfence();
-    __syncwarp();
+    __syncwarp();   // orders the other lanes' stores before the release
     if (lane == 0) signal_counter(pv.done + t.tensor, 1u);
   }
 }
@@ -440,19 +438,16 @@ bool lion_warp_tensor(const DevTensor& t, int momentum_kind) {
 // Units: about 4096 elements (small tensors in more pieces), starting on 128-element boundaries.  Whole rows where rows are a
 // multiple of 128; otherwise at least two rows' worth, since the rows at both ends are averaged by two units, and at most
 // LW_ROWS rows.
-// Order: up to 64 M elements one launch, a tensor's APPLY LAG elements behind its MAIN.  Larger lists two launches, all of MAIN
-// first (returns the number of MAIN units; 0: one launch): the completion counters' fences cost the first level caches,
-// where the second reading of a row's gradient hits, more than the codes' way through HBM (2.6 B list: 5.23 ms in one).
+// Order: all MAIN units, then all APPLY units (APPLY units between them would empty the first level caches by their acquiring
+// reads, where the second reading of a row's gradient hits).  Up to 64 M elements one launch; larger lists two (returns
+// the number of MAIN units; 0: one launch), without the counters, whose fences then cost more than a launch (2.6 B list:
+// 4.59 ms, in one launch 4.98).
 int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<char>& elig, std::vector<Task>& out, std::vector<int>& n_main) {
   long long total = 0;
   for (size_t i = 0; i < tensors.size(); ++i) if (elig[i]) total += tensors[i].numel;
   const bool split = total > (64ll << 20);
-  const long long LAG = split ? total : 32ll << 20;
   const int n = (int)tensors.size();
   n_main.assign(n, 0);
-  long long done = 0;
-  std::vector<long long> end(n, 0);
-  int waiting = 0;   // the first tensor whose APPLY units are not listed yet
   auto apply = [&](int i) {
     const DevTensor& t = tensors[i];
     long long u = 512;
@@ -461,7 +456,6 @@ int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<cha
       out.push_back(Task{i, PH_LION_APPLY, e, (int)std::min<long long>(u, t.numel - e), 0, 0, 0});
   };
   for (int i = 0; i < n; ++i) {
-    end[i] = done;
     if (!elig[i]) continue;
     const DevTensor& t = tensors[i];
     const long long C = t.cols;
@@ -476,14 +470,10 @@ int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<cha
                          t.rows > 0 ? (int)(e % C) : 0});
       ++n_main[i];
     }
-    done += t.numel;
-    end[i] = done;
-    for (; waiting < i && end[waiting] + LAG <= done; ++waiting)
-      if (elig[waiting]) apply(waiting);
   }
   const int mains = split ? (int)out.size() : 0;
-  for (; waiting < n; ++waiting)
-    if (elig[waiting]) apply(waiting);
+  for (int i = 0; i < n; ++i)
+    if (elig[i]) apply(i);
   return mains;
 }
 
