@@ -6,6 +6,7 @@
 #include <cuda_bf16.h>
 
 #include "kaon_device.cuh"
+#include "kaon_elem.cuh"
 #include "kaon_ops.cuh"
 #include "kaon_packed.cuh"
 
@@ -259,6 +260,68 @@ __device__ __forceinline__ void write8(const HP& hp, const DevTensor& d, uint64_
   } else {
 #pragma unroll
     for (int j = 0; j < 4; ++j) P.v[j] = add2(P.v[j], F[j]);
+  }
+}
+
+__device__ __forceinline__ float round_to(float x, __nv_bfloat16) { return round_bf16(x); }
+__device__ __forceinline__ float round_to(float x, float) { return x; }
+
+// A lane's part of the sum of a row of whole vectors
+template <typename PT>
+__device__ __forceinline__ float row_part(const unsigned char* rowp, int C, int lane) {
+  f32x2 a = pack2(0.0f, 0.0f), b = pack2(0.0f, 0.0f);
+#pragma unroll 4
+  for (int v = lane * 8; v < C; v += 256) {
+    W8<PT> w;
+    w.load(rowp + v * Elems<PT>::BYTES);
+    a = add2(a, add2(w.pair(0), w.pair(1)));
+    b = add2(b, add2(w.pair(2), w.pair(3)));
+  }
+  a = add2(a, b);
+  return a.x + a.y;
+}
+
+// put(i, mean of row r0 + i), i < n, means as the gradient's dtype holds them, by one warp: rows of up to 64 elements a lane
+// each, longer ones the whole warp (put is then lane 0's).  g: element 0 of row 0, 16-byte aligned.
+template <typename PT, typename Put>
+__device__ __forceinline__ void row_means(const unsigned char* g, int C, int r0, int n, int lane, Put out) {
+  using E = Elems<PT>;
+  const bool vec = (C & 7) == 0;
+  const float fC = (float)C, rC = __frcp_rn(fC);
+  auto put = [&](int r, float s) { out(r, round_to(div_by(s, fC, rC), PT())); };
+  if (C <= 64) {
+    for (int r = lane; r < n; r += 32) {
+      const unsigned char* rowp = g + (long long)(r0 + r) * C * E::BYTES;
+      float s = 0.0f;
+      if (vec) {
+        f32x2 a = pack2(0.0f, 0.0f);
+        for (int v = 0; v < C; v += 8) {
+          W8<PT> w;
+          w.load(rowp + v * E::BYTES);
+          a = add2(a, add2(add2(w.pair(0), w.pair(1)), add2(w.pair(2), w.pair(3))));
+        }
+        s = a.x + a.y;
+      } else {
+        for (int i = 0; i < C; ++i) s += E::load1(rowp, i);
+      }
+      put(r, s);
+    }
+    return;
+  }
+  for (int r = 0; r < n; ++r) {
+    const unsigned char* rowp = g + (long long)(r0 + r) * C * E::BYTES;
+    float s = 0.0f;
+    if (vec) {
+      s = row_part<PT>(rowp, C, lane);
+    } else {
+      // whole vectors, and a lane each for the elements before the first and after the last
+      const long long e = (long long)(r0 + r) * C, a = (e + 7) / 8 * 8, b = (e + C) / 8 * 8;
+      s = row_part<PT>(g + a * E::BYTES, (int)(b - a), lane);
+      const long long i = lane < 8 ? e + lane : b + lane - 8;
+      if (lane < 8 ? i < a : i < e + C) s += E::load1(g, i);
+    }
+    s = warp_sum(s);
+    if (lane == 0) put(r, s);
   }
 }
 

@@ -14,6 +14,7 @@
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
 #include "kaon_packed.cuh"
+#include "kaon_sweep.cuh"
 #include "lion_dev.h"
 
 namespace kaon {
@@ -352,36 +353,12 @@ __device__ void lion_main(const PlanView& pv, const LionDev& hp, const Task& t, 
     }
   } else if (do_gc) {
     const int warp = tid >> 5, lane = tid & 31;
-    for (int r = warp; r < nrows; r += NTHREADS / 32) {
-      const unsigned char* rowp = g_s + (size_t)r * C * E::BYTES;
-      float s = 0.0f;
-      if ((C & 7) == 0) {
-        if constexpr (E::IS_BF16) {
-          f32x2 acc = pack2(0.0f, 0.0f), acc2 = pack2(0.0f, 0.0f);
-          for (int v = lane; v < (C >> 3); v += 32) {
-            const uint4 q = *reinterpret_cast<const uint4*>(rowp + (size_t)v * 16);
-            acc = add2(acc, add2(pack2(bf16lo(q.x), bf16hi(q.x)), pack2(bf16lo(q.y), bf16hi(q.y))));
-            acc2 = add2(acc2, add2(pack2(bf16lo(q.z), bf16hi(q.z)), pack2(bf16lo(q.w), bf16hi(q.w))));
-          }
-          acc = add2(acc, acc2);
-          s = acc.x + acc.y;
-        } else {
-          for (int v = lane; v < (C >> 3); v += 32) {
-            float x[8];
-            E::load8(rowp + (size_t)v * 8 * E::BYTES, x);
-            s += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
-          }
-        }
-      } else {
-        for (int i = lane; i < C; i += 32) s += E::load1(rowp, i);
-      }
-      s = warp_sum(s);
-      if (lane == 0) {
-        float mean = __fdiv_rn(s, (float)C);
-        if (mean_packed) reinterpret_cast<uint32_t*>(mean_s)[r] = pack_bf16_rn(mean, mean);
-        else mean_s[r] = E::IS_BF16 ? round_bf16(mean) : mean;
-      }
-    }
+    // (in the order of additions of the warp units, lion_warp.cu: both kernels give the same bits)
+    const int per = (nrows + NTHREADS / 32 - 1) / (NTHREADS / 32), r0 = warp * per;
+    row_means<PT>(g_s, C, r0, min(per, nrows - r0), lane, [&](int i, float mean) {
+      if (mean_packed) reinterpret_cast<uint32_t*>(mean_s)[r0 + i] = pack_bf16_rn(mean, mean);
+      else mean_s[r0 + i] = mean;
+    });
   }
   if constexpr (MK == KAON_M_4BIT) {  // old block scales of the chunk (the fast path reads them from here)
     if (fast) {
@@ -748,7 +725,6 @@ __global__ void __launch_bounds__(NTHREADS, 4) lion_kernel(PlanView pv, LionDev 
 // the plan's scratch: bf16-rounded for bf16 gradients, as the staged rows' means are.
 template <typename PT>
 __global__ void lion_rowmean_kernel(PlanView pv, const int* tensor_ids, int n_ids) {
-  using E = Elems<PT>;
   const int lane = threadIdx.x & 31;
   const long long warp0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -756,25 +732,9 @@ __global__ void lion_rowmean_kernel(PlanView pv, const int* tensor_ids, int n_id
     const DevTensor d = pv.tensors[tensor_ids[k]];
     const unsigned char* g = reinterpret_cast<const unsigned char*>(pv.grads[tensor_ids[k]]);
     if (g == nullptr) continue;
-    const int C = d.cols;
-    for (long long r = warp0; r < d.rows; r += nwarps) {
-      const unsigned char* rowp = g + (size_t)r * C * E::BYTES;
-      float s = 0.0f;
-      if ((C & 7) == 0 && ((reinterpret_cast<uintptr_t>(rowp) & 15) == 0)) {
-        for (int v = lane; v < (C >> 3); v += 32) {
-          float x[8];
-          E::load8(rowp + (size_t)v * 8 * E::BYTES, x);
-          s += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
-        }
-      } else {
-        for (int i = lane; i < C; i += 32) s += E::load1(rowp, i);
-      }
-      s = warp_sum(s);
-      if (lane == 0) {
-        const float mean = __fdiv_rn(s, (float)C);
-        pv.aux[d.aux_off + r] = E::IS_BF16 ? round_bf16(mean) : mean;
-      }
-    }
+    const long long per = d.cols <= 64 ? 32 : 1;
+    for (long long r = warp0 * per; r < d.rows; r += nwarps * per)
+      row_means<PT>(g, d.cols, (int)r, (int)min(per, d.rows - r), lane, [&](int i, float mean) { pv.aux[d.aux_off + r + i] = mean; });
   }
 }
 

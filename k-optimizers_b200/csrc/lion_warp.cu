@@ -16,7 +16,6 @@
 
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
-#include "kaon_elem.cuh"
 #include "kaon_sweep.cuh"
 #include "lion_dev.h"
 
@@ -25,9 +24,6 @@ namespace kaon {
 constexpr int LWT = 256;            // threads per CTA
 constexpr int LW_ROWS = 64;         // rows a unit may touch
 constexpr int LW_MAX_COLS = 16384;  // longer rows: the staged kernel, whose row means come from a launch of their own
-
-__device__ __forceinline__ float round_to(float x, __nv_bfloat16) { return round_bf16(x); }
-__device__ __forceinline__ float round_to(float x, float) { return x; }
 
 // Eight consecutive elements of which `cnt` exist (the end of a tensor whose length is no multiple of eight)
 template <typename T>
@@ -46,65 +42,6 @@ __device__ __forceinline__ void load_some(MRaw<KAON_M_4BIT>& w, const void* p, i
 }
 template <typename T>
 __device__ __forceinline__ void load_some(MPlain<T>& w, const void* p, int cnt) { load_some(w.w, p, cnt); }
-
-// A lane's part of the sum of a row of whole vectors
-template <typename PT>
-__device__ __forceinline__ float row_part(const unsigned char* rowp, int C, int lane) {
-  f32x2 a = pack2(0.0f, 0.0f), b = pack2(0.0f, 0.0f);
-#pragma unroll 4
-  for (int v = lane * 8; v < C; v += 256) {
-    W8<PT> w;
-    w.load(rowp + v * Elems<PT>::BYTES);
-    a = add2(a, add2(w.pair(0), w.pair(1)));
-    b = add2(b, add2(w.pair(2), w.pair(3)));
-  }
-  a = add2(a, b);
-  return a.x + a.y;
-}
-
-// Means of rows r0 .. r0 + n (as the gradient's dtype holds them) into mean_s: rows of up to 64 elements a lane each, longer ones
-// the whole warp.
-template <typename PT>
-__device__ __forceinline__ void row_means(const unsigned char* g, int C, int r0, int n, float* mean_s, int lane) {
-  using E = Elems<PT>;
-  const bool vec = (C & 7) == 0;
-  const float fC = (float)C, rC = __frcp_rn(fC);
-  auto put = [&](int r, float s) { mean_s[r] = round_to(div_by(s, fC, rC), PT()); };
-  if (C <= 64) {
-    for (int r = lane; r < n; r += 32) {
-      const unsigned char* rowp = g + (long long)(r0 + r) * C * E::BYTES;
-      float s = 0.0f;
-      if (vec) {
-        f32x2 a = pack2(0.0f, 0.0f);
-        for (int v = 0; v < C; v += 8) {
-          W8<PT> w;
-          w.load(rowp + v * E::BYTES);
-          a = add2(a, add2(add2(w.pair(0), w.pair(1)), add2(w.pair(2), w.pair(3))));
-        }
-        s = a.x + a.y;
-      } else {
-        for (int i = 0; i < C; ++i) s += E::load1(rowp, i);
-      }
-      put(r, s);
-    }
-    return;
-  }
-  for (int r = 0; r < n; ++r) {
-    const unsigned char* rowp = g + (long long)(r0 + r) * C * E::BYTES;
-    float s = 0.0f;
-    if (vec) {
-      s = row_part<PT>(rowp, C, lane);
-    } else {
-      // whole vectors, and a lane each for the elements before the first and after the last
-      const long long e = (long long)(r0 + r) * C, a = (e + 7) / 8 * 8, b = (e + C) / 8 * 8;
-      s = row_part<PT>(g + a * E::BYTES, (int)(b - a), lane);
-      const long long i = lane < 8 ? e + lane : b + lane - 8;
-      if (lane < 8 ? i < a : i < e + C) s += E::load1(g, i);
-    }
-    s = warp_sum(s);
-    if (lane == 0) put(r, s);
-  }
-}
 
 // SIGNAL: APPLY units of the same launch wait for this one.
 template <typename PT, int MK, bool WD, bool SIGNAL>
@@ -146,7 +83,7 @@ __device__ __forceinline__ void lion_main_unit(const PlanView& pv, const LionDev
       mean = round_to(div_by(warp_sum(row_part<PT>(gp, C, lane)), fC, rC), PT());
     } else if (gc) {
       __syncwarp();
-      row_means<PT>(gbase, C, t.row0, (t.pad + n + C - 1) / C, mean_s, lane);
+      row_means<PT>(gbase, C, t.row0, (t.pad + n + C - 1) / C, lane, [&](int r, float mean) { mean_s[r] = mean; });
       __syncwarp();
     }
     const float mean_bits = E::IS_BF16 ? __uint_as_float(pack_bf16_rn(mean, mean)) : mean;
