@@ -55,9 +55,10 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   const float4 scal = __ldcg(reinterpret_cast<const float4*>(pv.aux + aux_scal(d)));
   const float div = scal.y, rcp_div = scal.w;       // the clip divisor
   const bool clipped = div != 1.0f;
-  float nrcp_denom = -1.0f;                         // minus the reciprocal of the kept share
+  float denom = 1.0f;                               // the kept share
   if (APPLY && hp.cautious)
-    nrcp_denom = -__fdiv_rn(1.0f, fmaxf(__fdiv_rn((float)__ldcg(pv.kept + t.tensor), (float)d.numel), 1e-8f));
+    denom = fmaxf(__fdiv_rn((float)__ldcg(pv.kept + t.tensor), (float)d.numel), 1e-8f);
+  const float nrcp_denom = -__fdiv_rn(1.0f, denom);
   const float4* rowtab = reinterpret_cast<const float4*>(pv.aux + aux_rowtab(d));
   const float* cfac = pv.aux + aux_cfac(d);
   unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
@@ -182,7 +183,10 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) F[j] = mul2(mul2(F[j], K[j]), pack2(nrcp_denom, nrcp_denom));
+      for (int j = 0; j < 4; ++j) {   // minus the correctly rounded quotient
+        const f32x2 NR = pack2(nrcp_denom, nrcp_denom), qq = mul2(F[j], NR);
+        F[j] = mul2(fma2(fma2(qq, pack2(denom, denom), F[j]), NR, qq), K[j]);
+      }
       // ---- store the new momentum; MO <- the momentum as stored ----
       float sc = 1.0f;
       if constexpr (CODED) {

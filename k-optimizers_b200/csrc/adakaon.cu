@@ -71,8 +71,12 @@ __device__ __forceinline__ float div_shared(float x, float d, float rcp) {
   return __fmaf_rn(r, rcp, q0);
 }
 
-// a warp's sum of fp32 values, taken in double: a row statistic one ulp off moves codes of the row
-__device__ __forceinline__ float warp_sum_d(float v) {
+// A warp's sum of fp32 values, taken in double: a row statistic one ulp off moves codes of the row.  `plain`: in fp32.
+// Weights with a Kahan compensation keep the order of additions of the package's first versions (plain sums here and in
+// FINAL, larger STATS runs in the plan): the compensation stores rounding differences at the size of a bf16 step, so
+// a statistic that moves by an ulp shows there at full scale, and a resumed run should not see it.
+__device__ __forceinline__ float warp_sum_d(float v, bool plain) {
+  if (plain) return warp_sum(v);
   double t = (double)v;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
@@ -186,7 +190,7 @@ __device__ __forceinline__ const unsigned char* m_ptr(const DevTensor& d, long l
 
 // Row means of the staged chunk for gradient centralization (0 when it is off).
 template <typename PT>
-__device__ __forceinline__ float row_mean(const unsigned char* rowp, int C, int lane) {
+__device__ __forceinline__ float row_mean(const unsigned char* rowp, int C, int lane, bool plain) {
   using E = Elems<PT>;
   float s = 0.0f;
   if ((C & 7) == 0) {
@@ -198,7 +202,7 @@ __device__ __forceinline__ float row_mean(const unsigned char* rowp, int C, int 
   } else {
     for (int i = lane; i < C; i += 32) s += E::load1(rowp, i);
   }
-  s = warp_sum_d(s);
+  s = warp_sum_d(s, plain);
   float mean = __fdiv_rn(s, (float)C);
   return E::IS_BF16 ? round_bf16(mean) : mean;
 }
@@ -207,7 +211,7 @@ __device__ __forceinline__ float row_mean(const unsigned char* rowp, int C, int 
 // (SQ = false, for the centralization mean) or the sum of (x - mu)^2 + eps1 (SQ = true).
 template <typename PT, bool SQ>
 __device__ __forceinline__ float row_part(const unsigned char* rowp, int C, int part, int G, int lane,
-                                          float mu, bool gc, bool has_eps, float eps1) {
+                                          float mu, bool gc, bool has_eps, float eps1, bool plain) {
   using E = Elems<PT>;
   float s = 0.0f;
   auto term = [&](float x) -> float {
@@ -226,7 +230,7 @@ __device__ __forceinline__ float row_part(const unsigned char* rowp, int C, int 
   } else {
     for (int i = part * 32 + lane; i < C; i += G * 32) s += term(E::load1(rowp, i));
   }
-  return warp_sum_d(s);
+  return warp_sum_d(s, plain);
 }
 
 template <typename PT>
@@ -295,7 +299,7 @@ __device__ void ada_stats(const PlanView& pv, const AdaDev& hp, const Task& t, S
       const bool act = r < nrc;
       const unsigned char* rowp = st.g_s + (size_t)(act ? r : 0) * C * E::BYTES;
       if (gc) {
-        const float ps = act ? row_part<PT, false>(rowp, C, part, G, lane, 0.0f, false, false, 0.0f) : 0.0f;
+        const float ps = act ? row_part<PT, false>(rowp, C, part, G, lane, 0.0f, false, false, 0.0f, d.shift != nullptr) : 0.0f;
         if (lane == 0) sm.part_s[warp] = ps;
         __syncthreads();
         if (tid < nrc) {
@@ -311,7 +315,7 @@ __device__ void ada_stats(const PlanView& pv, const AdaDev& hp, const Task& t, S
         sm.mean_s[tid] = 0.0f;
       }
       const float mu = (gc && act) ? sm.mean_s[r] : 0.0f;
-      const float ps2 = act ? row_part<PT, true>(rowp, C, part, G, lane, mu, gc, hp.has_eps != 0, hp.eps1) : 0.0f;
+      const float ps2 = act ? row_part<PT, true>(rowp, C, part, G, lane, mu, gc, hp.has_eps != 0, hp.eps1, d.shift != nullptr) : 0.0f;
       if (lane == 0) sm.part_s[warp] = ps2;
       __syncthreads();
       if (tid < nrc) {
@@ -327,7 +331,7 @@ __device__ void ada_stats(const PlanView& pv, const AdaDev& hp, const Task& t, S
     } else
     for (int r = warp; r < nrc; r += AT / 32) {
       const unsigned char* rowp = st.g_s + (size_t)r * C * E::BYTES;
-      const float mu = gc ? row_mean<PT>(rowp, C, lane) : 0.0f;
+      const float mu = gc ? row_mean<PT>(rowp, C, lane, d.shift != nullptr) : 0.0f;
       float s = 0.0f;
       if ((C & 7) == 0) {
         for (int v = lane; v < (C >> 3); v += 32) {
@@ -349,7 +353,7 @@ __device__ void ada_stats(const PlanView& pv, const AdaDev& hp, const Task& t, S
           s += sq;
         }
       }
-      s = warp_sum_d(s);
+      s = warp_sum_d(s, d.shift != nullptr);
       if (lane == 0) {
         const int row = t.row0 + c0 + r;
         const float mean = __fdiv_rn(s, (float)C);
@@ -477,7 +481,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
             a0 = add2(a0, add2(pairs(q0.x), pairs(q0.y)));
             a1v = add2(a1v, add2(pairs(q0.z), pairs(q0.w)));
           }
-          const float s = warp_sum_d((a0.x + a0.y) + (a1v.x + a1v.y));
+          const float s = warp_sum_d((a0.x + a0.y) + (a1v.x + a1v.y), d.shift != nullptr);
           mu = round_bf16(__fdiv_rn(s, (float)C));
         }
         const uint32_t mu2 = pack_bf16_rn(mu, mu);
@@ -501,7 +505,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
           b0 = add2(b0, add2(sq2(q0.x), sq2(q0.y)));
           b1 = add2(b1, add2(sq2(q0.z), sq2(q0.w)));
         }
-        s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y));
+        s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y), d.shift != nullptr);
       } else {
         if (gc) {
           float s = 0.0f;
@@ -510,7 +514,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
             E::load8(rowp + (size_t)v * 8 * E::BYTES, x);
             s += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
           }
-          s = warp_sum_d(s);
+          s = warp_sum_d(s, d.shift != nullptr);
           mu = __fdiv_rn(s, (float)C);
         }
         for (int v = lane; v < nv; v += 32) {
@@ -525,7 +529,7 @@ __device__ void ada_stats_stream(const PlanView& pv, const AdaDev& hp, const Tas
           }
           s2 += ((sq[0] + sq[1]) + (sq[2] + sq[3])) + ((sq[4] + sq[5]) + (sq[6] + sq[7]));
         }
-        s2 = warp_sum_d(s2);
+        s2 = warp_sum_d(s2, d.shift != nullptr);
       }
       if (lane == 0) {
         const float mean = __fdiv_rn(s2, (float)C);
@@ -696,7 +700,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
             a0 = add2(a0, add2(pairs(q0.x), pairs(q0.y)));
             a1 = add2(a1, add2(pairs(q0.z), pairs(q0.w)));
           }
-          mu = round_bf16(__fdiv_rn(warp_sum_d((a0.x + a0.y) + (a1.x + a1.y)), (float)C));
+          mu = round_bf16(__fdiv_rn(warp_sum_d((a0.x + a0.y) + (a1.x + a1.y), d.shift != nullptr), (float)C));
         }
         const uint32_t mu2 = pack_bf16_rn(mu, mu);
         auto sq2 = [&](uint32_t w) {
@@ -718,7 +722,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
           b0 = add2(b0, add2(sq2(q0.x), sq2(q0.y)));
           b1 = add2(b1, add2(sq2(q0.z), sq2(q0.w)));
         }
-        const float s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y));
+        const float s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y), d.shift != nullptr);
         if (lane == 0) {
           const float rn = lerp_torch(old, __fdiv_rn(s2, (float)C), hp.w2, hp.w2m1, hp.small_w2 != 0);
           d.stat_a[row] = rn;
@@ -857,6 +861,7 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
   double tl = 0.0;
   for (int j = tid; j < nc; j += AT) {
     double s1 = 0.0, s2 = 0.0;
+    auto add = [&](double a, float x) { return d.shift ? (double)((float)a + x) : a + (double)x; };   // (see warp_sum_d)
     int s = 0;
     for (; s + 8 <= d.n_stats; s += 8) {  // eight slots' loads in flight; the sums keep the slot order
       float x1[8], x2[8];
@@ -866,11 +871,11 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
         x2[u] = __ldcg(part + 2ll * (s + u) * C + C + j0 + j);
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) { s1 += (double)x1[u]; s2 += (double)x2[u]; }
+      for (int u = 0; u < 8; ++u) { s1 = add(s1, x1[u]); s2 = add(s2, x2[u]); }
     }
     for (; s < d.n_stats; ++s) {
-      s1 += (double)__ldcg(part + 2ll * s * C + j0 + j);
-      s2 += (double)__ldcg(part + 2ll * s * C + C + j0 + j);
+      s1 = add(s1, __ldcg(part + 2ll * s * C + j0 + j));
+      s2 = add(s2, __ldcg(part + 2ll * s * C + C + j0 + j));
     }
     const float mean = __fdiv_rn((float)s1, (float)d.rows);
     const float cn = lerp_torch(d.stat_b[j0 + j], mean, hp.w2, hp.w2m1, hp.small_w2 != 0);
