@@ -1,4 +1,4 @@
-// The cautious Lion step, a warp per unit of up to 4096 consecutive elements, nothing shared between warps.
+// The cautious Lion step, a warp per unit of 512 to 16384 consecutive elements, nothing shared between warps.
 //
 // MAIN unit: the means of the rows it touches, then per eight elements of a lane the direction sign(b1*m + (1-b1)*g), the
 // new momentum, its codes, and two bits an element for APPLY (element e, o of a pair: nibble kept_e | kept_o << 1 |
@@ -372,7 +372,7 @@ bool lion_warp_tensor(const DevTensor& t, int momentum_kind) {
   return t.numel > 0 && (t.rows <= 0 || (t.cols >= 3 && t.cols <= LW_MAX_COLS));
 }
 
-// Units: about 4096 elements (small tensors in more pieces), starting on 128-element boundaries.  Whole rows where rows are a
+// Units: about 4096 elements (small tensors in more pieces, large lists in fewer), starting on 128-element boundaries.  Whole rows where rows are a
 // multiple of 128; otherwise at least two rows' worth, since the rows at both ends are averaged by two units, and at most
 // LW_ROWS rows.
 // Order: all MAIN units, then all APPLY units (APPLY units between them would empty the first level caches by their acquiring
@@ -385,10 +385,12 @@ int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<cha
   const bool split = total > (64ll << 20);
   const int n = (int)tensors.size();
   n_main.assign(n, 0);
+  out.reserve((size_t)(total / 2048) + 64 * (size_t)n);
+  const long long most = split ? 8192 : 4096;   // (large lists: a shorter list of units to build and to claim)
   auto apply = [&](int i) {
     const DevTensor& t = tensors[i];
     long long u = 512;
-    while (u < 4096 && u * 128 <= t.numel) u *= 2;
+    while (u < (split ? 2 : 1) * most && u * 128 <= t.numel) u *= 2;
     for (long long e = 0; e < t.numel; e += u)
       out.push_back(Task{i, PH_LION_APPLY, e, (int)std::min<long long>(u, t.numel - e), 0, 0, 0});
   };
@@ -397,7 +399,7 @@ int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<cha
     const DevTensor& t = tensors[i];
     const long long C = t.cols;
     long long u = 512;
-    while (u < 4096 && u * 128 <= t.numel) u *= 2;
+    while (u < most && u * 128 <= t.numel) u *= 2;
     if (t.rows > 0) {
       if (C % 128 == 0) u = std::min<long long>(std::max<long long>(1, u / C), LW_ROWS) * C;
       else u = std::min(std::max(u, (2 * C + 127) / 128 * 128), (LW_ROWS - 2) * C / 128 * 128);
