@@ -1,13 +1,15 @@
 // Per-step host work over a parameter list, in native code: the CPython module kaon_b200._kaon_host.
 //
 // A step has to look at every tensor of every parameter group: does it have a gradient, where is it, is it of a
-// kind the kernels read, have the weights moved, does the tensor still have its optimizer state.  In Python that
+// kind the kernels read, have the weights moved, is it still the tensor and the state the plan was built for.  In Python that
 // costs about 0.6 us a tensor (a 720-tensor adapter list: 440 us of host time beside 60 us of device work); here
 // about 10 ns.  Anything unusual is only reported: the Python path then runs and raises or rebuilds.
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
 #include <cstring>
+#include <new>
+#include <unordered_map>
 #include <vector>
 
 namespace {
@@ -60,6 +62,60 @@ PyObject* scan(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return PyLong_FromLong(mask);
 }
 
+// entries(state, params, pos): pos[i] (int64 array at an address) = where PyDict_Next finds params[i] in the dict `state`,
+// -1 where it is no key.
+PyObject* entries(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 3 || !PyDict_Check(args[0]) || !PyList_CheckExact(args[1])) {
+    PyErr_SetString(PyExc_TypeError, "entries(state: dict, params: list, pos: int)");
+    return nullptr;
+  }
+  int64_t* pos = reinterpret_cast<int64_t*>(PyLong_AsUnsignedLongLong(args[2]));
+  if (PyErr_Occurred()) return nullptr;
+  try {
+    std::unordered_map<PyObject*, int64_t> at;
+    PyObject *k, *v;
+    for (Py_ssize_t next = 0, here = 0; PyDict_Next(args[0], &next, &k, &v); here = next) at[k] = here;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[1]); ++i) {
+      const auto it = at.find(PyList_GET_ITEM(args[1], i));
+      pos[i] = it == at.end() ? -1 : it->second;
+    }
+  } catch (const std::bad_alloc&) {
+    return PyErr_NoMemory();
+  }
+  Py_RETURN_NONE;
+}
+
+// settled(params, seen, state, states, pos): whether a group is what its plans were built for: the live list `params`
+// holds the tensors of `seen` in their order, and the live dict `state` maps each that has a dict in `states` (not
+// None) to that very dict; the others have no gradient.  pos: as `entries` left it.  A key occurs once in a dict, so finding
+// (tensor, dict) at the position noted proves the mapping, without hashing the tensor (a call back into Python); a
+// dict that was rearranged since only looks changed.
+PyObject* settled(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 5 || !PyList_CheckExact(args[1]) || !PyList_CheckExact(args[3]) ||
+      PyList_GET_SIZE(args[1]) != PyList_GET_SIZE(args[3])) {
+    PyErr_SetString(PyExc_TypeError, "settled(params, seen: list, state, states: list, pos: int)");
+    return nullptr;
+  }
+  const int64_t* pos = reinterpret_cast<const int64_t*>(PyLong_AsUnsignedLongLong(args[4]));
+  if (PyErr_Occurred()) return nullptr;
+  const Py_ssize_t n = PyList_GET_SIZE(args[1]);
+  if (!PyList_CheckExact(args[0]) || PyList_GET_SIZE(args[0]) != n || !PyDict_Check(args[2])) Py_RETURN_FALSE;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject *p = PyList_GET_ITEM(args[1], i), *st = PyList_GET_ITEM(args[3], i);
+    if (PyList_GET_ITEM(args[0], i) != p) Py_RETURN_FALSE;
+    if (st == Py_None) {
+      const at::Tensor* t = plain(p);
+      if (!t || t->grad().defined()) Py_RETURN_FALSE;
+      continue;
+    }
+    Py_ssize_t at = static_cast<Py_ssize_t>(pos[i]);
+    PyObject *k, *v;
+    if (at < 0 || !PyDict_Next(args[2], &at, &k, &v) || k != p || v != st) Py_RETURN_FALSE;
+    if (!PyDict_CheckExact(st) || PyDict_GET_SIZE(st) == 0) Py_RETURN_FALSE;
+  }
+  Py_RETURN_TRUE;
+}
+
 // grads_present(params): 0 no tensor of the list has a gradient, 1 some have, 2 all have (an empty list: 0); -1: unusual.
 PyObject* grads_present(PyObject*, PyObject* list) {
   if (!PyList_CheckExact(list)) return PyLong_FromLong(-1);
@@ -100,6 +156,8 @@ PyObject* bump(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 
 PyMethodDef methods[] = {
     {"scan", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(scan)), METH_FASTCALL, nullptr},
+    {"entries", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(entries)), METH_FASTCALL, nullptr},
+    {"settled", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(settled)), METH_FASTCALL, nullptr},
     {"grads_present", grads_present, METH_O, nullptr},
     {"bump", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(bump)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};

@@ -6,11 +6,13 @@ per tensor (weights, momentum, scales, statistics, shape), a work list and scrat
 reused every step.  Only the gradient-pointer column is refreshed per step, because
 ``zero_grad(set_to_none=True)`` reallocates gradients (the stale-pointer hazard the reference guards
 against in src/kaon/_fused_triton.py:1229-1245).  Plans are dropped whenever optimizer state is
-replaced (``load_state_dict``) or the set of stepped parameters changes.
+replaced (``load_state_dict``, ``opt.state[p] = {}``) or the set of stepped parameters changes.
 """
 from __future__ import annotations
 
 import ctypes as C
+import operator
+from collections.abc import Iterable
 from typing import Any
 
 import torch
@@ -18,6 +20,11 @@ import torch
 from . import _lib as L
 
 _PARAM_DT = {torch.float32: L.DT_F32, torch.bfloat16: L.DT_BF16}
+
+
+def _same(a: list, b: list) -> bool:
+    """Whether two lists hold the same objects (tensors compare element by element, so not ``==``)."""
+    return len(a) == len(b) and all(map(operator.is_, a, b))
 
 
 def fourbit_block_size(numel: int, block: int) -> int:
@@ -70,6 +77,7 @@ class GroupPlan:
             raise NotImplementedError(f"kaon_b200: parameter dtype {p0.dtype} (float32 and bfloat16 are supported)")
         self.device = p0.device
         self.params = params
+        self.momentum_dtype = momentum_dtype
         self.n = len(params)
         self.param_ptrs = [p.data_ptr() for p in params]
         mk = L.M_NONE if momentum_dtype is None else L.MOMENTUM_KIND[momentum_dtype]
@@ -206,9 +214,9 @@ class FusedStepMixin:
 
     def _fused_init(self) -> None:
         self._plans: dict[tuple, GroupPlan] = {}
-        self._plan_members: dict[tuple, tuple[int, ...]] = {}
-        self._group_buckets: dict[int, tuple] = {}   # per group: (params list, its length, momentum dtype, buckets)
-        self._steady: dict[int, tuple] = {}          # per group: what its next step is checked against, and its plans
+        # per group: what its next step is checked against (momentum dtype, tensors, their states, where those lie in
+        # ``state``), and its plans
+        self._steady: dict[int, tuple] = {}
         self._t = 0                 # completed steps; the SR stream uses the 1-based index
         self.sr_seed: int | None = None  # None -> torch.initial_seed() at the first step
         self._mirrors: tuple[int, int, list[int]] | None = None
@@ -232,8 +240,6 @@ class FusedStepMixin:
         for pl in self._plans.values():
             pl.destroy()
         self._plans.clear()
-        self._plan_members.clear()
-        self._group_buckets.clear()
         self._steady.clear()
 
     def _seed(self) -> int:
@@ -257,15 +263,14 @@ class FusedStepMixin:
     def _plans_to_step(self, gi: int, group: dict[str, Any]) -> list[tuple[GroupPlan, int]]:
         """(plan, stream) of every plan of the group with a gradient to step, its gradient column refreshed.
 
-        A group that looks as it did at its last step (same list, state, momentum dtype; no gradient on a tensor
-        that has no state yet) needs one native pass per plan; everything else takes ``_group_plans``."""
+        A group that looks as it did at its last step (the same tensors in its list, each with the state dict its plan
+        was built for; the same momentum dtype; no gradient on a tensor without state) needs two native passes;
+        everything else takes ``_group_plans``."""
         params, md = group["params"], self._momentum_dtype(group)
         steady = self._steady.get(gi)
-        if (steady is not None and steady[0] is params and steady[1] == len(params) and steady[2] == md
-                and steady[3] is self.state and steady[4] == len(self.state)
-                and (not steady[5] or L.host().grads_present(steady[5]) == 0)):
+        if steady is not None and steady[0] == md and L.host().settled(params, steady[1], self.state, steady[2], C.addressof(steady[3])):
             out = []
-            for pl in steady[6]:
+            for pl in steady[4]:
                 stream = L.raw_stream(pl.device.index)
                 some = pl.refresh(stream)
                 if some is None:
@@ -278,20 +283,27 @@ class FusedStepMixin:
         out = []
         plans = self._group_plans(gi, group)
         for pl in plans:
-            with torch.cuda.device(pl.device):
+            with L.on_device(pl.device):
                 stream = L.raw_stream(pl.device.index)
                 if pl.set_grads(stream):
                     out.append((pl, stream))
         if plans:
-            rest = [p for p in params if p not in self.state or not self.state[p]]
-            self._steady[gi] = (params, len(params), md, self.state, len(self.state), rest, plans)
+            seen = list(params)
+            states = [self.state[p] if p in self.state and self.state[p] else None for p in seen]
+            pos = (C.c_int64 * len(seen))()
+            L.host().entries(self.state, seen, C.addressof(pos))
+            self._steady[gi] = (md, seen, states, pos, plans)
         return out
+
+    def _drop_plans(self, gi: int, keep: Iterable[tuple] = ()) -> None:
+        """Give up the group's plans but those under the keys of ``keep``."""
+        for key in [k for k in self._plans if k[0] == gi and k not in keep]:
+            self._plans.pop(key).destroy()
 
     def _group_plans(self, gi: int, group: dict[str, Any]) -> list[GroupPlan]:
         """Plans covering every parameter of the group that has a gradient now or had one before."""
-        state_of = lambda p: self.state[p]  # noqa: E731
         params = group["params"]
-        fresh = active = False
+        active = False
         for p in params:
             g = p.grad
             if g is None:
@@ -299,46 +311,40 @@ class FusedStepMixin:
             active = True
             if g.is_sparse:
                 raise RuntimeError(f"{type(self).__name__} does not support sparse gradients")
-            st = state_of(p)
+            st = self.state[p]
             if not st:
+                self._drop_plans(gi)   # (also where an emptied dict is filled again: the plans hold its old tensors)
                 self._init_state(p, st, group)
-                fresh = True
         if not active:
             return []
-        # The buckets of the group (which tensors, in which plan) change only when a tensor gets its first
-        # state, the group's list is replaced or resized, the momentum dtype changes or the plans are
-        # dropped (load_state_dict, new mirrors): kept between steps, so a step of an unchanged group
-        # costs one pass over the gradients.
         md = self._momentum_dtype(group)
-        cached = self._group_buckets.get(gi)
-        if cached is None or fresh or cached[0] is not params or cached[1] != len(params) or cached[2] != md:
+        buckets: dict[tuple, tuple[list[torch.Tensor], list[dict[str, Any]]]] = {}
+        for p in params:
             # tensors stepped now or before (a lookup must not create state for the others); an empty tensor
             # has state, as in the reference, but nothing to step and no address
-            members = [p for p in params if p in self.state and state_of(p) and p.numel() > 0]
-            buckets: dict[tuple, list[torch.Tensor]] = {}
-            for p in members:
-                buckets.setdefault((gi, p.device, p.dtype), []).append(p)
-            cached = (params, len(params), md,
-                      [(key, plist, tuple(id(p) for p in plist) + (md,)) for key, plist in buckets.items()])
-            self._group_buckets[gi] = cached
+            st = self.state[p] if p in self.state else None
+            if st and p.numel() > 0:
+                ps, sts = buckets.setdefault((gi, p.device, p.dtype), ([], []))
+                ps.append(p)
+                sts.append(st)
+        self._drop_plans(gi, keep=buckets)
         plans = []
         ids = None
-        for key, plist, sig in cached[3]:
+        for key, (plist, slist) in buckets.items():
             pl = self._plans.get(key)
-            if pl is None or fresh or self._plan_members.get(key) != sig or pl.params_moved():
+            if (pl is None or pl.momentum_dtype != md or not _same(pl.params, plist) or not _same(pl.states, slist)
+                    or pl.params_moved()):
                 if pl is not None:
                     pl.destroy()
                 if ids is None:
                     ids = self._tensor_ids()
-                pl = GroupPlan(self._OPT_KIND, plist, [state_of(p) for p in plist],
-                               [ids[id(p)] for p in plist], md, self._M_KEY)
-                self._plan_created(pl, plist, [state_of(p) for p in plist])
+                pl = GroupPlan(self._OPT_KIND, plist, slist, [ids[id(p)] for p in plist], md, self._M_KEY)
+                self._plan_created(pl, plist, slist)
                 if self._mirrors is not None:
                     pl.set_peers(*self._mirrors)
                 if self.sm_limit is not None:
                     L.check(L.lib().kaon_plan_set_sm_limit(pl.handle, int(self.sm_limit)))
                 self._plans[key] = pl
-                self._plan_members[key] = sig
             plans.append(pl)
         return plans
 
