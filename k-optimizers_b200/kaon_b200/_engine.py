@@ -130,7 +130,8 @@ class GroupPlan:
         if mask & L.SCAN_UNUSUAL:
             return None
         if mask & L.SCAN_CHANGED:
-            self._upload(stream)
+            with L.on_device(self.device):
+                self._upload(stream)
         return bool(mask & L.SCAN_ANY)
 
     def _upload(self, stream: int) -> None:

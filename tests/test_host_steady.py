@@ -1,5 +1,5 @@
 """What a step notices between steps of an unchanged group: a state dict or a tensor of the list that is not the one of the
-step before.  On CPU tensors, with plans that only record what they are given."""
+step before, gradients that moved (their addresses go up under the plan's device).  On CPU tensors, with plans that only record what they are given."""
 import contextlib
 import ctypes as C
 
@@ -12,6 +12,7 @@ from kaon_b200 import _lib as L
 
 class RecordingPlan(_engine.GroupPlan):
     """The host half of a plan: no library handle, no device memory."""
+    guarded = 0        # depth of the device guard
     def __init__(self, kind, params, states, ids, momentum_dtype, m_key="m"):
         self.device = params[0].device
         self.params, self.states, self.n = params, states, len(params)
@@ -23,12 +24,15 @@ class RecordingPlan(_engine.GroupPlan):
         self._param_addr, self.grad_addr = C.addressof(self._param_arr), C.addressof(self.grad_arr)
 
     def _upload(self, stream):
+        assert RecordingPlan.guarded > 0, "gradient pointers uploaded outside the plan's device"
         self.uploads += 1
 
 
 @contextlib.contextmanager
 def _guard(device):
+    RecordingPlan.guarded += 1
     yield
+    RecordingPlan.guarded -= 1
 
 
 @pytest.fixture
@@ -96,7 +100,7 @@ def test_a_replaced_list_entry_is_stepped(stepped, known):
     assert _is_live(opt, stepped[-1])
 
 
-def test_an_unchanged_group_keeps_its_plan_and_uploads_moved_gradients(stepped):
+def test_an_unchanged_group_keeps_its_plan_and_uploads_moved_gradients_on_its_device(stepped):
     ps, opt = _make(Lion)
     opt.step()
     plan, = opt._plans.values()
