@@ -47,6 +47,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+// A tensor map in global memory is read through a proxy of its own: what was written there since (the host's copy of
+// the next tables into the same allocation) has to be acquired before a block's first load with it.
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, unsigned parity) {
   for (unsigned i = 0; i < G_WAIT_LIMIT; ++i)
     if (mbar_try_wait(bar, parity)) return true;
@@ -200,10 +206,16 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
     // ---- TMA producer ----
     if (lane == 0) {
       unsigned it = 0;
+      const NsProblem* last = nullptr;
       for (int c = c_first; c < c_end && !*fail; c += c_step) {
         int mi, ni;
         const NsProblem* pr = tile_of(c, mi, ni);
         const CUtensorMap *mapA = &pr->a, *mapB = &pr->b;
+        if (GROUPED && pr != last) {   // (the one product's maps are kernel parameters)
+          tensormap_acquire(mapA);
+          tensormap_acquire(mapB);
+          last = pr;
+        }
         const int kblocks = (pr->p.K + G_BK - 1) / G_BK, BN = pr->p.BN;
         const bool a_mn = pr->p.a_mn != 0, b_mn = pr->p.b_mn != 0;
         const unsigned tx = (unsigned)(G_A_BYTES + BN * G_BK * 2);

@@ -133,6 +133,51 @@ def _chain_vs_oracle(md, method, wd, dtype, kind, gc):
                 assert bad.mean() < 1e-3 and np.abs(got - want).max() < 3e-3, (step, i, SHAPES[i], bad.sum())
 
 
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_another_set_of_gradients_or_iterations_between_steps(dtype):
+    """Products and tensor maps follow the set of gradients and ns_steps: matrices without a gradient are left alone, and
+    the others' factors are those of this step's momentum.  No synchronisation between the steps."""
+    import kaon_b200
+    from _gpu import to_bits
+    tdt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    gen = torch.Generator().manual_seed(17)
+    host = [(torch.randn(s, generator=gen) * 0.02).to(tdt) for s in SHAPES]
+    params = [torch.nn.Parameter(h.clone().cuda()) for h in host]
+    kw = dict(lr=1e-3, betas=(0.95, 0.999), momentum_dtype="bfloat16", bf16_method="none")
+    opt = kaon_b200.AdaMuon(params, **kw)
+    plan_steps = [(set(), 2), ({1}, 2), (set(), 2), (set(), 3), ({0, 3, 5}, 3), (set(), 2), ({0, 1, 3, 4, 5}, 2), (set(), 2)]
+    drawn = [[(torch.randn(s, generator=gen) * 1e-3).to(tdt) for s in SHAPES] for _ in plan_steps]
+    on_gpu = [[g.cuda() for g in gs] for gs in drawn]
+    seen = []
+    for (without, iters), gs in zip(plan_steps, on_gpu):
+        for i, p in enumerate(params):
+            p.grad = None if i in without else gs[i]
+        opt.param_groups[0]["ns_steps"] = iters
+        opt.step()
+        seen.append(([None if i in without else opt.orthogonalised(p) for i, p in enumerate(params)],
+                     [p.detach().clone() for p in params]))
+    torch.cuda.synchronize()
+    opt.check_device_status()
+    orc = ko.OracleAdaMuon([to_bits(h) for h in host], SHAPES, ns_steps=2, **kw)
+    for k, ((without, iters), gs, (ortho, weights)) in enumerate(zip(plan_steps, drawn, seen)):
+        override = [None if o is None else o.float().cpu().numpy() for o in ortho]
+        orc.hp["ns_steps"] = iters
+        orc.step([None if i in without else to_bits(g) for i, g in enumerate(gs)], ns_override=override, capture_ns_in=True)
+        for i, (w, ot) in enumerate(zip(weights, orc.tensors)):
+            if i in without:
+                assert torch.equal(w, seen[k - 1][1][i]), (k, i)
+                continue
+            if ot.rows:   # (one bf16 chain against another: the tolerance of the tests above)
+                own = ko.newton_schulz(orc.ns_in[i].reshape(ot.rows, ot.cols), iters)
+                np.testing.assert_allclose(override[i], own, rtol=2e-2, atol=2e-2, err_msg=str((k, i)))
+            got, want = to_bits(w), ot.p
+            if dtype == "bf16":   # (as above: values within rounding of a boundary)
+                assert np.mean(got != want) < 5e-3, (k, i)
+            else:
+                bad = np.abs(got - want) > 2e-5 * np.abs(want) + 1e-9
+                assert bad.mean() < 1e-3, (k, i)
+
+
 def test_zeropower_function_matches_module_api():
     import kaon_b200.adamuon as am
     gen = torch.Generator().manual_seed(3)

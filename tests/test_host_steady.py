@@ -13,6 +13,7 @@ from kaon_b200 import _lib as L
 class RecordingPlan(_engine.GroupPlan):
     """The host half of a plan: no library handle, no device memory."""
     guarded = 0        # depth of the device guard
+
     def __init__(self, kind, params, states, ids, momentum_dtype, m_key="m"):
         self.device = params[0].device
         self.params, self.states, self.n = params, states, len(params)
