@@ -47,7 +47,7 @@ PyObject* scan(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     PyObject* st = PyList_GET_ITEM(args[1], i);
     if (!p || !PyDict_CheckExact(st) || PyDict_GET_SIZE(st) == 0 || reinterpret_cast<int64_t>(p->const_data_ptr()) != was[i])
       return PyLong_FromLong(UNUSUAL);
-    const at::Tensor& g = p->grad();
+    const at::Tensor& g = p->unsafeGetTensorImpl()->grad();   // (Tensor::grad() asks whether it is a leaf, to warn)
     if (g.defined()) {
       if (g.layout() != at::kStrided || g.scalar_type() != p->scalar_type() || !g.is_contiguous())
         return PyLong_FromLong(UNUSUAL);
