@@ -13,8 +13,6 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
-#include <functional>
-#include <queue>
 #include <vector>
 
 #include "kaon_host.h"
@@ -125,7 +123,7 @@ static int launch_ns_gemm(const __nv_bfloat16* A, bool a_mn, long long lda, cons
   int sms = 0;
   if (int rc = gemm_sms(&sms)) return rc;
   // computed tiles: all of them, or in symmetric mode those that reach the diagonal
-  const int tm = (M + G_BM - 1) / G_BM, tn = (N + p.BN - 1) / p.BN;
+  const int tm = ns_tiles(M, G_BM), tn = ns_tiles(N, p.BN);
   int total = 0;
   for (int mi = 0; mi < tm; ++mi) total += tn - (p.sym ? std::min(tn, (mi * G_BM) / p.BN) : 0);
   ns_gemm_kernel<false><<<std::min(total, sms), G2_THREADS, G2_SMEM, stream>>>(pr, NsWork{total, nullptr, nullptr, nullptr, status});
@@ -257,45 +255,7 @@ void ns_scratch_layout(NsMat& m, unsigned char* base) {
   m.scal = reinterpret_cast<float*>(base);
 }
 
-// Tiles of one stage shared out over the CTAs, the longest first to the CTA with the least work.  The cost of a tile is
-// its bytes from L2 per k-block (128 + BN rows of 128 bytes: what a tile of up to 256 columns waits for, not the
-// tensor cores) times its k-blocks, plus its epilogue.  Returns the longest CTA's work.
-static long long share_out(const std::vector<NsProblem>& probs, int sms, std::vector<NsTile>* tiles, std::vector<int>* begin) {
-  struct T { long long cost; NsTile t; };
-  std::vector<T> all;
-  for (int i = 0; i < (int)probs.size(); ++i) {
-    const GemmParams& p = probs[i].p;
-    const int tm = (p.M + G_BM - 1) / G_BM, tn = (p.N + p.BN - 1) / p.BN;
-    const long long cost = (long long)((p.K + G_BK - 1) / G_BK) * (128 + p.BN) + 400 + p.BN;
-    for (int mi = 0; mi < tm; ++mi)
-      for (int ni = p.sym ? std::min(tn, mi * G_BM / p.BN) : 0; ni < tn; ++ni) all.push_back(T{cost, NsTile{i, (short)mi, (short)ni}});
-  }
-  std::stable_sort(all.begin(), all.end(), [](const T& a, const T& b) { return a.cost > b.cost; });
-  const int grid = std::min<int>(sms, (int)all.size());
-  typedef std::pair<long long, int> Load;
-  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> q;
-  for (int c = 0; c < grid; ++c) q.push(Load(0, c));
-  std::vector<std::vector<NsTile>> mine(grid);
-  long long most = 0;
-  for (const T& t : all) {
-    Load l = q.top(); q.pop();
-    l.first += t.cost;
-    most = std::max(most, l.first);
-    mine[l.second].push_back(t.t);
-    q.push(l);
-  }
-  if (tiles) {
-    for (int c = 0; c < grid; ++c) {
-      begin->push_back((int)tiles->size());
-      tiles->insert(tiles->end(), mine[c].begin(), mine[c].end());
-    }
-    begin->push_back((int)tiles->size());
-  }
-  return most;
-}
-
-// The launches of a batch's iterations.  Tile widths: the one of 256 / 192 / 128 / 64 columns (the same for a stage)
-// whose longest CTA has the least work: wide tiles need fewer bytes, narrow ones fill the machine.
+// The launches of a batch's iterations, their tiles shared out by ns_share_out.
 int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsBatch& out) {
   out = NsBatch{};
   if (mats.empty()) return KAON_OK;
@@ -338,24 +298,17 @@ int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsBatch& out) {
         ps[i].p = p;
         ops[i] = op;
       }
-      int best = 256;
-      long long least = 0;
-      for (int bn : {256, 192, 128, 64}) {
-        for (NsProblem& pr : ps) pr.p.BN = std::min(bn, (pr.p.N + 63) / 64 * 64);
-        const long long most = share_out(ps, sms, nullptr, nullptr);
-        if (least == 0 || most < least) { least = most; best = bn; }
-      }
+      std::vector<NsShape> shapes;
+      for (const NsProblem& pr : ps) shapes.push_back(NsShape{pr.p.M, pr.p.N, pr.p.K, pr.p.sym != 0});
+      const NsShare sh = ns_share_out(shapes, sms);
       for (size_t i = 0; i < ps.size(); ++i) {
-        ps[i].p.BN = std::min(best, (ps[i].p.N + 63) / 64 * 64);
+        ps[i].p.BN = ns_tile_cols(sh.bn, ps[i].p.N);
         if (int rc = operand_maps(ps[i], ops[i].A, ops[i].lda, ops[i].B, ops[i].ldb)) return rc;
       }
-      std::vector<NsTile> tl;
-      std::vector<int> bg;
-      share_out(ps, sms, &tl, &bg);
-      out.stages.push_back(NsStage{(int)probs.size(), (int)tiles.size(), (int)begin.size(), (int)bg.size() - 1});
+      out.stages.push_back(NsStage{(int)probs.size(), (int)tiles.size(), (int)begin.size(), (int)sh.begin.size() - 1});
       probs.insert(probs.end(), ps.begin(), ps.end());
-      tiles.insert(tiles.end(), tl.begin(), tl.end());
-      begin.insert(begin.end(), bg.begin(), bg.end());
+      tiles.insert(tiles.end(), sh.tiles.begin(), sh.tiles.end());
+      begin.insert(begin.end(), sh.begin.begin(), sh.begin.end());
     }
   }
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };

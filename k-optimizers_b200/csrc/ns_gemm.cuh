@@ -13,15 +13,14 @@
 #include <stdint.h>
 
 #include "kaon_stage.cuh"
+#include "ns_share.h"
 
 namespace kaon {
 
-constexpr int G_BM = 128;          // rows of the output tile = UMMA M
-constexpr int G_BK = 64;           // K elements per stage (one 128-byte swizzle atom of bf16)
-constexpr int G_STAGES = 2;
+constexpr int G_BM = NS_TILE_M;    // rows of the output tile = UMMA M
+constexpr int G_BK = NS_TILE_K;    // K elements per stage (one 128-byte swizzle atom of bf16)
 constexpr int G_A_BYTES = G_BM * G_BK * 2;  // 16 KiB
 constexpr int G_MAX_BN = 256;
-constexpr int G_THREADS = 128;
 constexpr unsigned G_WAIT_LIMIT = 1u << 22;
 
 struct GemmParams {
@@ -51,12 +50,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 // the next tables into the same allocation) has to be acquired before a block's first load with it.
 __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, unsigned parity) {
-  for (unsigned i = 0; i < G_WAIT_LIMIT; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
 }
 
 // 64-bit shared-memory matrix descriptor, 128-byte swizzle.
@@ -103,7 +96,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t v[32]) {
 
 // ---- persistent, warp-specialised kernel ----
 // One CTA per SM walks the output tiles (128 x BN) in a fixed stride.  Warp 0 (one lane) feeds a ring of
-// G_STAGES shared-memory stages by TMA; warp 1 (one lane) issues the MMAs into one of two accumulators in
+// G2_STAGES shared-memory stages by TMA; warp 1 (one lane) issues the MMAs into one of two accumulators in
 // tensor memory (2 x 256 columns, allocated once per CTA); warps 2-5 drain the other accumulator
 // (tcgen05.ld, fused epilogue, bf16 stores), so that a tile's epilogue runs under the next tile's MMAs.
 // In symmetric mode only the tiles that reach the diagonal are enumerated.
@@ -146,7 +139,6 @@ struct alignas(128) NsProblem {
   CUtensorMap a, b;
   GemmParams p;
 };
-struct NsTile { int prob; short mi, ni; };
 
 // What a launch works on.  One product (a Newton-Schulz call on its own): `one` is a kernel argument, CTA b takes tiles
 // b, b + grid, ...  GROUPED (every matrix of a batch at the same stage of the iteration): the products lie in device
@@ -182,7 +174,7 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
       mi = t.mi; ni = t.ni;
       return work.probs + t.prob;
     } else {
-      tile_coords(one.p, (one.p.N + one.p.BN - 1) / one.p.BN, c, mi, ni);
+      tile_coords(one.p, ns_tiles(one.p.N, one.p.BN), c, mi, ni);
       return &one;
     }
   };
@@ -216,7 +208,7 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
           tensormap_acquire(mapB);
           last = pr;
         }
-        const int kblocks = (pr->p.K + G_BK - 1) / G_BK, BN = pr->p.BN;
+        const int kblocks = ns_tiles(pr->p.K, G_BK), BN = pr->p.BN;
         const bool a_mn = pr->p.a_mn != 0, b_mn = pr->p.b_mn != 0;
         const unsigned tx = (unsigned)(G_A_BYTES + BN * G_BK * 2);
         const int m0 = mi * G_BM, n0 = ni * BN;
@@ -248,7 +240,7 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
       for (int c = c_first; c < c_end && !*fail; c += c_step, ++tcount) {
         int mi, ni;
         const NsProblem* pr = tile_of(c, mi, ni);
-        const int kblocks = (pr->p.K + G_BK - 1) / G_BK;
+        const int kblocks = ns_tiles(pr->p.K, G_BK);
         const bool a_mn = pr->p.a_mn != 0, b_mn = pr->p.b_mn != 0;
         const uint32_t idesc = umma_idesc(pr->p.BN, a_mn, b_mn);
         const unsigned buf = tcount & 1u, use = tcount >> 1;
@@ -289,16 +281,16 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
       if (!mbar_wait_or_fail(&accf_bar[buf], use & 1u, fail)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_acc = tmem_base + buf * G2_ACC_COLS;
-      const int row = m0 + quarter * 32 + lane;
+      const unsigned row = (unsigned)m0 + quarter * 32 + lane;   // (beyond 2^31 in the last tile of the tallest matrix)
       for (int c0 = 0; c0 < p.BN; c0 += 32) {
         uint32_t v[32];
         tmem_ld32(tmem_acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        const int col = n0 + c0;
-        if (row < p.M && col < p.N) {
+        const unsigned col = (unsigned)n0 + c0, M = p.M, N = p.N;
+        if (row < M && col < N) {
           __nv_bfloat16* orow = p.out + (long long)row * p.ld_out + col;
           const __nv_bfloat16* arow = p.aux ? p.aux + (long long)row * p.ld_aux + col : nullptr;
-          const bool full = (col + 32 <= p.N) && ((reinterpret_cast<uintptr_t>(orow) & 15) == 0) &&
+          const bool full = (col + 32 <= N) && ((reinterpret_cast<uintptr_t>(orow) & 15) == 0) &&
                             (!arow || (reinterpret_cast<uintptr_t>(arow) & 15) == 0);
           if (full) {
 #pragma unroll
@@ -324,7 +316,10 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
               }
             }
           } else {
-            for (int e = 0; e < 32 && col + e < p.N; ++e) {
+            const int left = (int)min(32u, N - col);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              if (e >= left) break;
               const float x = arow ? __bfloat162float(arow[e]) : 0.0f;
               const __nv_bfloat16 r = __float2bfloat16_rn(__uint_as_float(v[e]) * alpha + beta * x);
               orow[e] = r;

@@ -1,0 +1,92 @@
+// The tiles of a batch's grouped products and how they are shared out over the CTAs of a launch (ns.cu).  Host code,
+// compiled without CUDA too.
+#pragma once
+
+#include <algorithm>
+#include <functional>
+#include <queue>
+#include <utility>
+#include <vector>
+
+#ifdef __CUDACC__
+#define NS_HD __host__ __device__
+#else
+#define NS_HD
+#endif
+
+namespace kaon {
+
+constexpr int NS_TILE_M = 128, NS_TILE_K = 64;   // rows of an output tile, K elements of a pipeline stage
+
+// (tile coordinates are int: a matrix of 2^31 - 1 rows, the most a plan takes, has 2^24 row tiles)
+struct NsTile { int prob, mi, ni; };
+
+// one product: out[M, N], K deep; sym: only the tiles that reach the diagonal are computed
+struct NsShape { int M, N, K; bool sym; };
+
+// A stage's tiles: CTA b takes tiles[begin[b]] .. tiles[begin[b + 1]].
+struct NsShare {
+  int bn = 0;                // width of the stage's tiles (a narrower matrix: its own, see ns_tile_cols)
+  long long most = 0;        // the longest CTA's work
+  std::vector<NsTile> tiles;
+  std::vector<int> begin;
+};
+
+NS_HD inline int ns_tiles(int extent, int tile) { return (extent - 1) / tile + 1; }   // (extent >= 1; no sum that overflows)
+inline int ns_tile_cols(int bn, int N) { return std::min(bn, ns_tiles(N, 64) * 64); }
+inline int ns_first_col(const NsShape& p, int bn, int mi) {
+  return p.sym ? std::min(ns_tiles(p.N, bn), (int)((long long)mi * NS_TILE_M / bn)) : 0;
+}
+
+// Tiles of one stage shared out over at most `ctas` CTAs, the longest first to the CTA with the least work.  The cost of
+// a tile is its bytes from L2 per k-block (128 + BN rows of 128 bytes: what a tile of up to 256 columns waits for, not
+// the tensor cores) times its k-blocks, plus its epilogue.  Tile widths: the one of 256 / 192 / 128 / 64 columns (the
+// same for a stage) whose longest CTA has the least work: wide tiles need fewer bytes, narrow ones fill the machine.
+inline NsShare ns_share_out(const std::vector<NsShape>& ps, int ctas) {
+  NsShare best;
+  for (int bn : {256, 192, 128, 64}) {
+    struct P { long long cost; int prob; };
+    std::vector<P> order;
+    long long count = 0;
+    for (int i = 0; i < (int)ps.size(); ++i) {
+      const int w = ns_tile_cols(bn, ps[i].N), tm = ns_tiles(ps[i].M, NS_TILE_M), tn = ns_tiles(ps[i].N, w);
+      const long long cost = (long long)ns_tiles(ps[i].K, NS_TILE_K) * (128 + w) + 400 + w;
+      long long c = (long long)tm * tn;
+      for (int mi = 0; ps[i].sym && mi < tm; ++mi) c -= ns_first_col(ps[i], w, mi);
+      order.push_back(P{cost, i});
+      count += c;
+    }
+    const int grid = (int)std::min<long long>(ctas, count);
+    std::stable_sort(order.begin(), order.end(), [](const P& a, const P& b) { return a.cost > b.cost; });
+    typedef std::pair<long long, int> Load;
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> q;
+    for (int c = 0; c < grid; ++c) q.push(Load(0, c));
+    std::vector<std::vector<NsTile>> mine(grid);
+    long long most = 0;
+    for (const P& o : order) {
+      const NsShape& p = ps[o.prob];
+      const int w = ns_tile_cols(bn, p.N), tm = ns_tiles(p.M, NS_TILE_M), tn = ns_tiles(p.N, w);
+      for (int mi = 0; mi < tm; ++mi)
+        for (int ni = ns_first_col(p, w, mi); ni < tn; ++ni) {
+          Load l = q.top();
+          q.pop();
+          l.first += o.cost;
+          most = std::max(most, l.first);
+          mine[l.second].push_back(NsTile{o.prob, mi, ni});
+          q.push(l);
+        }
+    }
+    if (best.bn && most >= best.most) continue;
+    best = NsShare();
+    best.bn = bn;
+    best.most = most;
+    for (int c = 0; c < grid; ++c) {
+      best.begin.push_back((int)best.tiles.size());
+      best.tiles.insert(best.tiles.end(), mine[c].begin(), mine[c].end());
+    }
+    best.begin.push_back((int)best.tiles.size());
+  }
+  return best;
+}
+
+}  // namespace kaon

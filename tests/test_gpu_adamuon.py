@@ -178,6 +178,29 @@ def test_another_set_of_gradients_or_iterations_between_steps(dtype):
                 assert bad.mean() < 1e-3, (k, i)
 
 
+def test_a_matrix_of_more_row_tiles_than_15_bits():
+    """32 770 row tiles; every block of the factor against the iteration in fp64 (bf16 chain: a few 2^-8 of an entry's
+    size, as between two implementations elsewhere in this file)."""
+    import kaon_b200
+    rows, cols = 128 * 32770 - 5, 8
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    p = torch.nn.Parameter((torch.randn(rows, cols, device="cuda", generator=gen) * 0.02).bfloat16())
+    p.grad = (torch.randn(rows, cols, device="cuda", generator=gen) * 1e-3).bfloat16()
+    opt = kaon_b200.AdaMuon([p], lr=1e-3, betas=(0.0, 0.999), bf16_method="none")   # no momentum: X is the gradient
+    opt.step()
+    torch.cuda.synchronize()
+    opt.check_device_status()
+    got = opt.orthogonalised(p).double()
+    x = p.grad.double()
+    x /= x.norm() + 1e-7
+    for _ in range(2):
+        a = x.T @ x
+        x = 3.4445 * x + x @ (-4.7750 * a + 2.0315 * a @ a)
+    for lo in range(0, rows, 128 * 1024):
+        want, have = x[lo:lo + 128 * 1024], got[lo:lo + 128 * 1024]
+        assert ((have - want).norm() / want.norm()).item() < 2e-2, lo
+
+
 def test_zeropower_function_matches_module_api():
     import kaon_b200.adamuon as am
     gen = torch.Generator().manual_seed(3)
