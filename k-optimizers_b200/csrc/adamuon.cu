@@ -411,8 +411,8 @@ static MuonLayout muon_layout(const kaon_plan* pl) {
   return L;
 }
 
-// What a plan keeps between steps: the batches' launch tables, rebuilt when the workspace, the number of iterations or
-// the set of matrices with a gradient changes.
+// What a plan keeps between steps: the batches' launch tables, rebuilt when the workspace or the number of iterations
+// changes.  They cover every matrix; one without a gradient is passed over by the kernels.
 struct MuonHost {
   MuonLayout layout;
   struct Batch {
@@ -421,10 +421,10 @@ struct MuonHost {
     int fast0 = 0, n_fast = 0;            // EMA units, general items of the tensors without units, items of all
     int rest0 = 0, n_rest = 0;
     int all0 = 0, n_all = 0;
-    int scale_f0 = 0, scale_a0 = 0, n_mats = 0;
+    int scale_f0 = 0, scale_a0 = 0;
+    std::vector<int> tensors;
   };
   std::vector<Batch> batches;
-  std::vector<char> key;                  // which tensors have a gradient
   const void* base = nullptr;
   int steps = 0;
   unsigned char* block = nullptr;
@@ -439,12 +439,13 @@ void muon_free(kaon_plan* pl) {
   pl->muon = nullptr;
 }
 
-static int muon_build(kaon_plan* pl, MuonHost& h, unsigned char* ws, int steps, const std::vector<char>& key, cudaStream_t s) {
+static int muon_build(kaon_plan* pl, MuonHost& h, unsigned char* ws, int steps, cudaStream_t s) {
   const int n = pl->n_tensors;
   const MuonLayout& L = h.layout;
   std::vector<Task> fast, rest, all;
   std::vector<EmaOut> outs(n, EmaOut{nullptr, 0});
   std::vector<NsScale> scales;
+  NsShares shares;
   h.batches.assign(L.n_batches, MuonHost::Batch());
   int slots = 0;
   size_t tab = 0;
@@ -454,13 +455,15 @@ static int muon_build(kaon_plan* pl, MuonHost& h, unsigned char* ws, int steps, 
     std::vector<NsMat> mats;
     std::vector<NsScale> sf, sa;
     for (int i = 0; i < n; ++i) {
-      if (L.batch[i] != b || !key[i]) continue;
+      if (L.batch[i] != b) continue;
       const DevTensor& t = pl->h_tensors[i];
       NsMat m{};
       m.R = t.rows; m.C = t.cols;
       ns_scratch_layout(m, ws + L.scratch_off + (size_t)(b % NS_LANES) * L.lane_stride + L.s_off[i]);
       m.out = reinterpret_cast<__nv_bfloat16*>(ws + L.o_off[i]);
+      m.tensor = i;
       mats.push_back(m);
+      B.tensors.push_back(i);
       outs[i] = EmaOut{m.x0, m.ld};
       // general items: runs of whole rows
       const int a0 = slots;
@@ -484,10 +487,9 @@ static int muon_build(kaon_plan* pl, MuonHost& h, unsigned char* ws, int steps, 
       sf.push_back(NsScale{f0, slots, m.scal});
     }
     B.n_fast = (int)fast.size() - B.fast0; B.n_rest = (int)rest.size() - B.rest0; B.n_all = (int)all.size() - B.all0;
-    B.n_mats = (int)mats.size();
     B.scale_f0 = (int)scales.size(); scales.insert(scales.end(), sf.begin(), sf.end());
     B.scale_a0 = (int)scales.size(); scales.insert(scales.end(), sa.begin(), sa.end());
-    if (int rc = ns_batch_build(mats, steps, B.ns)) return rc;
+    if (int rc = ns_batch_build(mats, steps, shares, B.ns)) return rc;
     B.ns_off = tab;
     tab += up256(B.ns.bytes);
   }
@@ -518,7 +520,6 @@ static int muon_build(kaon_plan* pl, MuonHost& h, unsigned char* ws, int steps, 
   // pageable source: staged before the call returns, ordered on the step's stream after the steps before it
   KAON_CUDA(cudaMemcpyAsync(h.block, img.data(), uploaded, cudaMemcpyHostToDevice, s));
   for (MuonHost::Batch& B : h.batches) { B.ns.host.clear(); B.ns.host.shrink_to_fit(); }
-  h.key = key;
   h.base = ws;
   h.steps = steps;
   return KAON_OK;
@@ -563,17 +564,13 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
   const int n = pl->n_tensors;
 
-  // one-time: the O column; per workspace, iteration count and set of gradients: the batches' tables
+  // one-time: the O column; per workspace and iteration count: the batches' tables
   if (!pl->d_signal) {
     KAON_CUDA(cudaMalloc((void**)&pl->d_signal, sizeof(void*) * (size_t)n));
     pl->device_bytes += (int64_t)(sizeof(void*) * n);
   }
-  {
-    std::vector<char> key(n, 0);
-    for (int i = 0; i < n; ++i) key[i] = L.batch[i] >= 0 && pl->h_grads[i] != nullptr;
-    if (H.base != workspace || H.steps != h->ns_steps || H.key != key)
-      if (int rc = muon_build(pl, H, ws, h->ns_steps, key, s)) { H.base = nullptr; return rc; }
-  }
+  if (H.base != workspace || H.steps != h->ns_steps)
+    if (int rc = muon_build(pl, H, ws, h->ns_steps, s)) { H.base = nullptr; return rc; }
   if (pl->signal_base != workspace) {
     std::vector<const void*> sig(n, nullptr);
     for (int i = 0; i < n; ++i)
@@ -611,7 +608,9 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
   double* part = reinterpret_cast<double*>(H.block + H.off_part);
   for (size_t b = 0; b < H.batches.size(); ++b) {
     const MuonHost::Batch& B = H.batches[b];
-    if (B.n_mats == 0) continue;
+    const int n_mats = (int)B.tensors.size();
+    const int live = (int)std::count_if(B.tensors.begin(), B.tensors.end(), [&](int i) { return pl->h_grads[i] != nullptr; });
+    if (live == 0) continue;
     cudaStream_t sl = lanes ? pl->muon_stream[b % NS_LANES] : s;
     const int n_gen = gc ? B.n_all : B.n_rest;   // centralization takes the general form throughout
     if (!gc && B.n_fast) {
@@ -624,10 +623,10 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
       ek<<<std::min(n_gen, pl->sm_count * 8), ET, 0, sl>>>(v, list, n_gen, w1, w1 - 1.0f, w1 < 0.5f, gc, outs, part);
       pl->launches += 1;
     }
-    ns_batch_scale(reinterpret_cast<const NsScale*>(H.block + H.off_scale) + (gc ? B.scale_a0 : B.scale_f0), B.n_mats, part, sl);
+    ns_batch_scale(reinterpret_cast<const NsScale*>(H.block + H.off_scale) + (gc ? B.scale_a0 : B.scale_f0), n_mats, part, sl);
     KAON_CUDA(cudaGetLastError());
     long long nl = 1;
-    if (int rc = ns_batch_run(B.ns, H.block + B.ns_off, v.status, sl, &nl)) return rc;
+    if (int rc = ns_batch_run(B.ns, H.block + B.ns_off, live < n_mats ? v.grads : nullptr, v.status, sl, &nl)) return rc;
     pl->launches += nl;
   }
   if (lanes) {

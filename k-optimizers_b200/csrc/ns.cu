@@ -126,7 +126,7 @@ static int launch_ns_gemm(const __nv_bfloat16* A, bool a_mn, long long lda, cons
   const int tm = ns_tiles(M, G_BM), tn = ns_tiles(N, p.BN);
   int total = 0;
   for (int mi = 0; mi < tm; ++mi) total += tn - (p.sym ? std::min(tn, (mi * G_BM) / p.BN) : 0);
-  ns_gemm_kernel<false><<<std::min(total, sms), G2_THREADS, G2_SMEM, stream>>>(pr, NsWork{total, nullptr, nullptr, nullptr, status});
+  ns_gemm_kernel<false><<<std::min(total, sms), G2_THREADS, G2_SMEM, stream>>>(pr, NsWork{total, nullptr, nullptr, nullptr, nullptr, status});
   KAON_CUDA(cudaGetLastError());
   return KAON_OK;
 }
@@ -255,60 +255,62 @@ void ns_scratch_layout(NsMat& m, unsigned char* base) {
   m.scal = reinterpret_cast<float*>(base);
 }
 
-// The launches of a batch's iterations, their tiles shared out by ns_share_out.
-int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsBatch& out) {
+// The launches of a batch's iterations: products and tensor maps per iteration, tiles per stage.
+int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsShares& shares, NsBatch& out) {
   out = NsBatch{};
   if (mats.empty()) return KAON_OK;
   int sms = 0;
   if (int rc = gemm_sms(&sms)) return rc;
+  NsShares::Key key;
+  for (const NsMat& m : mats) key.push_back({m.R, m.C});
+  const std::array<NsShare, 3>& share = shares.get(key, sms);
   const float a = 3.4445f, b = -4.7750f, c = 2.0315f;
   std::vector<NsProblem> probs;
   std::vector<NsTile> tiles;
   std::vector<int> begin;
+  int tile0[3], begin0[3];
+  for (int stage = 0; stage < 3; ++stage) {
+    tile0[stage] = (int)tiles.size();
+    begin0[stage] = (int)begin.size();
+    tiles.insert(tiles.end(), share[stage].tiles.begin(), share[stage].tiles.end());
+    begin.insert(begin.end(), share[stage].begin.begin(), share[stage].begin.end());
+  }
   for (int it = 0; it < steps; ++it) {
     for (int stage = 0; stage < 3; ++stage) {
-      struct Op { const __nv_bfloat16 *A, *B; long long lda, ldb; };
-      std::vector<NsProblem> ps(mats.size());
-      std::vector<Op> ops(mats.size());
-      for (size_t i = 0; i < mats.size(); ++i) {
-        const NsMat& m = mats[i];
+      out.stages.push_back(NsStage{(int)probs.size(), tile0[stage], begin0[stage], (int)share[stage].begin.size() - 1});
+      for (const NsMat& m : mats) {
         const bool tall = m.R > m.C;   // the stored matrix is X^T (k rows, r columns)
-        const int r = (int)std::min(m.R, m.C), k = (int)std::max(m.R, m.C);
         // ping-pong; the last iteration lands in `out`
         const bool last = it == steps - 1;
         const __nv_bfloat16* cur = (it & 1) ? m.xb : m.x0;
         __nv_bfloat16* nxt = last ? m.out : (it & 1) ? m.x0 : m.xb;
-        GemmParams p{};
-        Op op{};
+        const NsShape sh = ns_stage_shape(stage, m.R, m.C);
+        NsProblem pr{};
+        GemmParams& p = pr.p;
+        p.M = sh.M; p.N = sh.N; p.K = sh.K; p.sym = sh.sym;
+        p.BN = ns_tile_cols(share[stage].bn, sh.N);
+        pr.tensor = m.tensor;
+        const __nv_bfloat16 *A, *B;
+        long long lda, ldb;
         if (stage == 0) {          // A = X X^T
-          op = Op{cur, cur, m.ld, m.ld};
-          p.M = r; p.N = r; p.K = k; p.a_mn = tall; p.b_mn = tall; p.alpha = 1.0f; p.sym = 1;
+          A = B = cur; lda = ldb = m.ld;
+          p.a_mn = tall; p.b_mn = tall; p.alpha = 1.0f;
           p.dev_scale = it == 0 ? m.scal : nullptr;
           p.out = m.A; p.ld_out = m.lr;
         } else if (stage == 1) {   // B = b A + c A A   (A symmetric: A A = A A^T, both operands K-major)
-          op = Op{m.A, m.A, m.lr, m.lr};
-          p.M = r; p.N = r; p.K = r; p.alpha = c; p.beta = b; p.sym = 1;
+          A = B = m.A; lda = ldb = m.lr;
+          p.alpha = c; p.beta = b;
           p.aux = m.A; p.ld_aux = m.lr; p.out = m.B; p.ld_out = m.lr;
         } else {                   // X <- a X + B X; stored transposed: X^T <- a X^T + X^T B
-          op = tall ? Op{cur, m.B, m.ld, m.lr} : Op{m.B, cur, m.lr, m.ld};
-          p.M = tall ? k : r; p.N = tall ? r : k; p.K = r; p.b_mn = !tall; p.alpha = 1.0f; p.beta = a;
+          A = tall ? cur : m.B; lda = tall ? m.ld : m.lr;
+          B = tall ? m.B : cur; ldb = tall ? m.lr : m.ld;
+          p.b_mn = !tall; p.alpha = 1.0f; p.beta = a;
           p.dev_scale = it == 0 ? m.scal + 2 : nullptr;
           p.aux = cur; p.ld_aux = m.ld; p.out = nxt; p.ld_out = last ? m.C : m.ld;
         }
-        ps[i].p = p;
-        ops[i] = op;
+        if (int rc = operand_maps(pr, A, lda, B, ldb)) return rc;
+        probs.push_back(pr);
       }
-      std::vector<NsShape> shapes;
-      for (const NsProblem& pr : ps) shapes.push_back(NsShape{pr.p.M, pr.p.N, pr.p.K, pr.p.sym != 0});
-      const NsShare sh = ns_share_out(shapes, sms);
-      for (size_t i = 0; i < ps.size(); ++i) {
-        ps[i].p.BN = ns_tile_cols(sh.bn, ps[i].p.N);
-        if (int rc = operand_maps(ps[i], ops[i].A, ops[i].lda, ops[i].B, ops[i].ldb)) return rc;
-      }
-      out.stages.push_back(NsStage{(int)probs.size(), (int)tiles.size(), (int)begin.size(), (int)sh.begin.size() - 1});
-      probs.insert(probs.end(), ps.begin(), ps.end());
-      tiles.insert(tiles.end(), sh.tiles.begin(), sh.tiles.end());
-      begin.insert(begin.end(), sh.begin.begin(), sh.begin.end());
     }
   }
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
@@ -323,14 +325,16 @@ int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsBatch& out) {
   return KAON_OK;
 }
 
-// One grouped launch per stage, from the tables at `dev` (the bytes of NsBatch::host).
-int ns_batch_run(const NsBatch& b, const unsigned char* dev, unsigned* status, cudaStream_t s, long long* launches) {
+// One grouped launch per stage, from the tables at `dev` (the bytes of NsBatch::host).  `grads`: the gradient column where
+// some matrix of the batch has none (its products are passed over), null where all have one.
+int ns_batch_run(const NsBatch& b, const unsigned char* dev, const void* const* grads, unsigned* status, cudaStream_t s, long long* launches) {
   const NsProblem none{};
   for (const NsStage& st : b.stages) {
     NsWork w{};
     w.probs = reinterpret_cast<const NsProblem*>(dev) + st.prob0;
     w.tiles = reinterpret_cast<const NsTile*>(dev + b.off_tiles) + st.tile0;
     w.begin = reinterpret_cast<const int*>(dev + b.off_begin) + st.begin0;
+    w.grads = grads;
     w.status = status;
     ns_gemm_kernel<true><<<st.grid, G2_THREADS, G2_SMEM, s>>>(none, w);
     *launches += 1;

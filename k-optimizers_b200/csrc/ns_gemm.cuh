@@ -138,16 +138,19 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int tn, int c, 
 struct alignas(128) NsProblem {
   CUtensorMap a, b;
   GemmParams p;
+  int tensor;   // whose gradient decides whether it is computed (NsWork::grads)
 };
 
 // What a launch works on.  One product (a Newton-Schulz call on its own): `one` is a kernel argument, CTA b takes tiles
 // b, b + grid, ...  GROUPED (every matrix of a batch at the same stage of the iteration): the products lie in device
-// memory and CTA b takes tiles[begin[b]] .. tiles[begin[b + 1]], shared out by the host so that all finish together.
+// memory and CTA b takes tiles[begin[b]] .. tiles[begin[b + 1]], shared out by the host so that all finish together; with
+// `grads` set, the tiles of matrices without a gradient are passed over.
 struct NsWork {
   int total;
   const NsProblem* probs;
   const NsTile* tiles;
   const int* begin;
+  const void* const* grads;
   unsigned* status;
 };
 
@@ -178,6 +181,7 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
       return &one;
     }
   };
+  auto passed_over = [&](const NsProblem* pr) { return GROUPED && work.grads && work.grads[pr->tensor] == nullptr; };
   volatile int* fail = &fail_s;
 
   if (tid == 0) {
@@ -202,6 +206,7 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
       for (int c = c_first; c < c_end && !*fail; c += c_step) {
         int mi, ni;
         const NsProblem* pr = tile_of(c, mi, ni);
+        if (passed_over(pr)) continue;
         const CUtensorMap *mapA = &pr->a, *mapB = &pr->b;
         if (GROUPED && pr != last) {   // (the one product's maps are kernel parameters)
           tensormap_acquire(mapA);
@@ -237,13 +242,15 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
     // ---- MMA issuer ----
     if (lane == 0) {
       unsigned it = 0, tcount = 0;
-      for (int c = c_first; c < c_end && !*fail; c += c_step, ++tcount) {
+      for (int c = c_first; c < c_end && !*fail; c += c_step) {
         int mi, ni;
         const NsProblem* pr = tile_of(c, mi, ni);
+        if (passed_over(pr)) continue;
         const int kblocks = ns_tiles(pr->p.K, G_BK);
         const bool a_mn = pr->p.a_mn != 0, b_mn = pr->p.b_mn != 0;
         const uint32_t idesc = umma_idesc(pr->p.BN, a_mn, b_mn);
         const unsigned buf = tcount & 1u, use = tcount >> 1;
+        ++tcount;
         if (use > 0 && !mbar_wait_or_fail(&acce_bar[buf], (use - 1u) & 1u, fail)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_acc = tmem_base + buf * G2_ACC_COLS;
@@ -270,14 +277,16 @@ ns_gemm_kernel(const __grid_constant__ NsProblem one, const __grid_constant__ Ns
     // ---- epilogue: warps 2..5; a warp may touch the 32 tensor-memory lanes of its quarter (warp % 4) ----
     const int quarter = warp & 3;
     unsigned tcount = 0;
-    for (int c = c_first; c < c_end; c += c_step, ++tcount) {
+    for (int c = c_first; c < c_end; c += c_step) {
       int mi, ni;
       const NsProblem* pr = tile_of(c, mi, ni);
+      if (passed_over(pr)) continue;
       const GemmParams& p = pr->p;
       const float alpha = p.dev_scale ? p.alpha * p.dev_scale[0] : p.alpha;
       const float beta = p.dev_scale ? p.beta * p.dev_scale[1] : p.beta;
       const int m0 = mi * G_BM, n0 = ni * p.BN;
       const unsigned buf = tcount & 1u, use = tcount >> 1;
+      ++tcount;
       if (!mbar_wait_or_fail(&accf_bar[buf], use & 1u, fail)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_acc = tmem_base + buf * G2_ACC_COLS;

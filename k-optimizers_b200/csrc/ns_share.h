@@ -3,7 +3,9 @@
 #pragma once
 
 #include <algorithm>
+#include <array>
 #include <functional>
+#include <map>
 #include <queue>
 #include <utility>
 #include <vector>
@@ -42,12 +44,14 @@ inline int ns_first_col(const NsShape& p, int bn, int mi) {
 // a tile is its bytes from L2 per k-block (128 + BN rows of 128 bytes: what a tile of up to 256 columns waits for, not
 // the tensor cores) times its k-blocks, plus its epilogue.  Tile widths: the one of 256 / 192 / 128 / 64 columns (the
 // same for a stage) whose longest CTA has the least work: wide tiles need fewer bytes, narrow ones fill the machine.
+// A width whose mean work is no less than the longest CTA's so far cannot win and is not shared out: of a large batch
+// only the widest is.
 inline NsShare ns_share_out(const std::vector<NsShape>& ps, int ctas) {
   NsShare best;
   for (int bn : {256, 192, 128, 64}) {
     struct P { long long cost; int prob; };
     std::vector<P> order;
-    long long count = 0;
+    long long count = 0, work = 0;
     for (int i = 0; i < (int)ps.size(); ++i) {
       const int w = ns_tile_cols(bn, ps[i].N), tm = ns_tiles(ps[i].M, NS_TILE_M), tn = ns_tiles(ps[i].N, w);
       const long long cost = (long long)ns_tiles(ps[i].K, NS_TILE_K) * (128 + w) + 400 + w;
@@ -55,8 +59,10 @@ inline NsShare ns_share_out(const std::vector<NsShape>& ps, int ctas) {
       for (int mi = 0; ps[i].sym && mi < tm; ++mi) c -= ns_first_col(ps[i], w, mi);
       order.push_back(P{cost, i});
       count += c;
+      work += c * cost;
     }
     const int grid = (int)std::min<long long>(ctas, count);
+    if (best.bn && work >= best.most * grid) continue;
     std::stable_sort(order.begin(), order.end(), [](const P& a, const P& b) { return a.cost > b.cost; });
     typedef std::pair<long long, int> Load;
     std::priority_queue<Load, std::vector<Load>, std::greater<Load>> q;
@@ -88,5 +94,31 @@ inline NsShare ns_share_out(const std::vector<NsShape>& ps, int ctas) {
   }
   return best;
 }
+
+// The three products of an iteration on a matrix stored [R, C] (r, k: its smaller and larger side):
+// A = X X^T [r, r], B = b A + c A A [r, r], X <- a X + B X as stored.
+inline NsShape ns_stage_shape(int stage, long long R, long long C) {
+  const int r = (int)std::min(R, C), k = (int)std::max(R, C);
+  if (stage == 0) return NsShape{r, r, k, true};
+  if (stage == 1) return NsShape{r, r, r, true};
+  return R > C ? NsShape{k, r, r, false} : NsShape{r, k, r, false};
+}
+
+// Share-outs by the shapes of a batch: all iterations of a batch have the same, and most batches of a list too.
+struct NsShares {
+  typedef std::vector<std::pair<long long, long long>> Key;   // the matrices' [R, C]
+  std::map<Key, std::array<NsShare, 3>> known;
+  const std::array<NsShare, 3>& get(const Key& key, int ctas) {
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    std::array<NsShare, 3> a;
+    for (int stage = 0; stage < 3; ++stage) {
+      std::vector<NsShape> shapes;
+      for (const auto& m : key) shapes.push_back(ns_stage_shape(stage, m.first, m.second));
+      a[stage] = ns_share_out(shapes, ctas);
+    }
+    return known.emplace(key, std::move(a)).first->second;
+  }
+};
 
 }  // namespace kaon

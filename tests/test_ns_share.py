@@ -67,3 +67,22 @@ def program(tmp_path_factory):
 def test_every_tile_once(program, shapes, ctas):
     out = subprocess.run([program, str(ctas), *(str(x) for s in shapes for x in s)], capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, (out.returncode, out.stderr)
+
+
+def test_stages_of_a_batch_are_shared_out_once(tmp_path):
+    """Batches of the same shapes get the same share-out, and its shapes are those of the iteration's products."""
+    (tmp_path / "m.cpp").write_text(r"""
+#include "ns_share.h"
+using namespace kaon;
+int main() {
+  NsShares s;
+  const NsShares::Key wide{{320, 1280}, {64, 64}}, tall{{1280, 320}, {64, 64}};
+  const auto* a = &s.get(wide, 148);
+  const auto* b = &s.get(tall, 148);
+  if (a != &s.get(wide, 148) || b == a || s.known.size() != 2) return 1;
+  const NsShape x = ns_stage_shape(2, 320, 1280), y = ns_stage_shape(2, 1280, 320), z = ns_stage_shape(0, 1280, 320);
+  return x.M == 320 && x.N == 1280 && x.K == 320 && y.M == 1280 && y.N == 320 && y.K == 320 && z.M == 320 && z.K == 1280 && z.sym ? 0 : 2;
+}
+""")
+    subprocess.check_call(["g++", "-std=c++17", f"-I{CSRC}", str(tmp_path / "m.cpp"), "-o", str(tmp_path / "m")])
+    assert subprocess.run([str(tmp_path / "m")]).returncode == 0
