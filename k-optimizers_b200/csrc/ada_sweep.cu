@@ -10,7 +10,7 @@
 // consecutive elements and streams it, eight elements a lane and trip, with nothing shared between warps: no staging, no
 // barrier.  What is per row is one 16-byte table entry (left by FINAL), what is per column two vector loads that hit
 // L1; rows and columns advance by an addition, without a division.  Arithmetic is on packed pairs in the
-// reference's order of roundings; the mask is one saturating FMA an element; codes are rounded from the correctly
+// reference's order of roundings; the mask is one comparison an element; codes are rounded from the correctly
 // rounded quotient m' / scale (reciprocal and residual), so no vector needs a second look.
 #include <algorithm>
 #include <type_traits>
@@ -166,11 +166,10 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const f32x2 X = mul2(F[j], G[j]);
-      K[j] = pack2(mask1(X.x, hp.mask_big, hp.mask_add), mask1(X.y, hp.mask_big, hp.mask_add));
+      K[j] = pack2(gt0_or(X.x, hp.mask_off), gt0_or(X.y, hp.mask_off));
     }
     if constexpr (!APPLY) {
-      const f32x2 k2 = add2(add2(K[0], K[1]), add2(K[2], K[3]));
-      if (act) kept2 = add2(kept2, k2);
+      if (act) kept2 = add2(kept2, add2(add2(K[0], K[1]), add2(K[2], K[3])));
       if constexpr (MK == KAON_M_INT8) {
         unsigned bits = act ? __float_as_uint(amax8(MN)) : 0u;
         const int row_l0 = __shfl_sync(0xffffffffu, row, 0);

@@ -17,8 +17,8 @@ struct AdaDev {
   float a_remove, b_remove, a_climb, b_climb;
   uint32_t step, k0, k1;
   uint32_t rk0[KAON_PHILOX_ROUNDS], rk1[KAON_PHILOX_ROUNDS];  // Philox round keys (k + r * Weyl), from the host
+  int mask_off;          // !cautious
   int stats_only;        // second moment only (AdaPNM, KProdigy)
-  float mask_big, mask_add;   // the cautious mask as one saturating FMA (mask1 in kaon_sweep.cuh)
 };
 
 // Philox round keys of a hyper-parameter block from its k0, k1
@@ -27,12 +27,11 @@ inline void philox_round_keys(HP& hp) {
   for (int r = 0; r < KAON_PHILOX_ROUNDS; ++r) { hp.rk0[r] = hp.k0 + 0x9E3779B9u * (uint32_t)r; hp.rk1[r] = hp.k1 + 0xBB67AE85u * (uint32_t)r; }
 }
 
-// round keys and mask constants from k0, k1 and cautious
+// round keys from k0, k1; no eps is an eps of 0
 inline void ada_finish(AdaDev& hp) {
   philox_round_keys(hp);
   if (!hp.has_eps) hp.eps1 = 0.0f;
-  hp.mask_big = hp.cautious ? 0x1p127f : 0.0f;
-  hp.mask_add = hp.cautious ? 0.0f : 1.0f;
+  hp.mask_off = !hp.cautious;
 }
 
 int launch_persistent(kaon_plan* pl, const PlanView& v, const AdaDev& hp, cudaStream_t s);

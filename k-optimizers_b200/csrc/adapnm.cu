@@ -137,7 +137,7 @@ __device__ __forceinline__ void pnm_write(const PnmDev& hp, const DevTensor& d, 
 
 // The two sweeps over tensors whose rows are a multiple of eight elements (4-bit blocks of 128): a warp per unit of up
 // to 4096 elements, nothing shared between warps.  Bound by instruction issue, so on packed pairs, the mask one
-// saturating FMA an element, rows and columns advanced by an addition.  (A CTA per 16 K-element item with guarded
+// comparison an element, rows and columns advanced by an addition.  (A CTA per 16 K-element item with guarded
 // elements and a scalar encode: SUM 409 us and APPLY 972 us on 269 M elements of 4-bit momentum; here 251 and 531 us.)
 template <typename PT, int MK, bool APPLY>
 __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ PnmDev hp,
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_c
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const f32x2 X = mul2(U[j], Y[j]);
-          K[j] = pack2(mask1(X.x, 0x1p127f, 0.0f), mask1(X.y, 0x1p127f, 0.0f));
+          K[j] = pack2(gt0(X.x), gt0(X.y));
         }
         if (act) {
           ss += (double)(s2.x + s2.y);
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_c
             const f32x2 X = mul2(u, Y[j]);
             const f32x2 q0 = mul2(u, pack2(rdenom, rdenom));
             u = fma2(fma2(q0, pack2(-denom, -denom), u), pack2(rdenom, rdenom), q0);
-            u = mul2(u, pack2(mask1(X.x, -0x1p127f, 0.0f), mask1(X.y, -0x1p127f, 0.0f)));
+            u = mul2(u, pack2(lt0(X.x), lt0(X.y)));
           }
           F[j] = u;
         }

@@ -12,12 +12,23 @@
 
 namespace kaon {
 
-// The cautious mask of one element as a factor: x > 0 as 1.0f / 0.0f by one saturating FMA, (big, add) = (2^127, 0);
-// mask off: 1.0f always, (0, 1).  A NaN gives 0.  A product below 2^-127 (subnormal) would come out in between; it
-// does not occur where both factors are normal gradients and updates.
-__device__ __forceinline__ float mask1(float x, float big, float add) {
+// The cautious mask of one element as a factor: x > 0 (x < 0) as 1.0f / 0.0f in one instruction, by comparison, so that a
+// product in the subnormal range decides like any other.  A NaN gives 0.
+__device__ __forceinline__ float gt0(float x) {
   float r;
-  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(big), "f"(add));
+  asm("set.gt.f32.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float lt0(float x) {
+  float r;
+  asm("set.lt.f32.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// gt0, or 1.0f where `off`
+__device__ __forceinline__ float gt0_or(float x, int off) {
+  float r;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tset.gt.or.f32.f32 %0, %1, 0f00000000, p;\n\t}" : "=f"(r) : "f"(x), "r"(off));
   return r;
 }
 

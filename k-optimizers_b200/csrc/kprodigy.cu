@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const f32x2 X = mul2(F[j], Y[j]);
-            K[j] = pack2(mask1(X.x, -0x1p127f, 0.0f), mask1(X.y, -0x1p127f, 0.0f));
+            K[j] = pack2(lt0(X.x), lt0(X.y));
           }
           if constexpr (MODE == 2) {
             if (act) kept2 = add2(kept2, add2(add2(K[0], K[1]), add2(K[2], K[3])));
