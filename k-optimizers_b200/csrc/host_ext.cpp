@@ -12,7 +12,13 @@
 #include <unordered_map>
 #include <vector>
 
+#ifndef KAON_HOST_ABI
+#error "KAON_HOST_ABI: the torch and Python this is compiled for (kaon_b200/_build.py)"
+#endif
+
 namespace {
+
+const char g_abi[] = "kaon host module for " KAON_HOST_ABI;   // _build.py looks for it in the file
 
 enum : long { ANY_GRAD = 1, GRADS_CHANGED = 2, UNUSUAL = 4 };
 
@@ -177,5 +183,7 @@ PyMODINIT_FUNC PyInit__kaon_host() {
   g_tensor = type_of("torch", "Tensor");
   g_parameter = type_of("torch.nn", "Parameter");
   if (!g_tensor || !g_parameter) return nullptr;
-  return PyModule_Create(&module);
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "abi", g_abi + sizeof("kaon host module for ") - 1) < 0) Py_CLEAR(m);
+  return m;
 }

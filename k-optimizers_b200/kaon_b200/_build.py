@@ -51,8 +51,18 @@ def needs_build() -> bool:
     return any(os.path.getmtime(d) > t for d in sources() + headers())
 
 
+def host_abi() -> str:
+    """What the host module is compiled for: it reads tensor objects by torch's layout of them."""
+    import torch
+    return f"torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}"
+
+
 def _host_stale() -> bool:
-    return not os.path.exists(HOST_LIB) or os.path.getmtime(HOST_LIB) < os.path.getmtime(HOST_SRC)
+    """Missing, older than its source, or compiled for another torch or Python (its `abi` string, as the file holds it)."""
+    if not os.path.exists(HOST_LIB) or os.path.getmtime(HOST_LIB) < os.path.getmtime(HOST_SRC):
+        return True
+    with open(HOST_LIB, "rb") as f:
+        return f"kaon host module for {host_abi()}\0".encode() not in f.read()
 
 
 def _build_host(env: dict) -> None:
@@ -62,7 +72,7 @@ def _build_host(env: dict) -> None:
     from torch.utils.cpp_extension import include_paths
     libs = os.path.join(os.path.dirname(torch.__file__), "lib")
     subprocess.check_call(
-        ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+        ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f'-DKAON_HOST_ABI="{host_abi()}"', f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
          *[f"-I{p}" for p in include_paths()], f"-I{sysconfig.get_paths()['include']}", HOST_SRC, "-o", HOST_LIB,
          f"-L{libs}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", f"-Wl,-rpath,{libs}"], env=env)
 

@@ -119,6 +119,11 @@ def host():
         except ImportError as e:
             raise KaonError(f"the host module _kaon_host cannot be loaded ({e}): build it with "
                             "`python -m kaon_b200._build`") from e
+        from ._build import host_abi
+        abi = getattr(_kaon_host, "abi", "another torch")
+        if abi != host_abi():   # it reads tensor objects by the layout it was compiled for
+            raise KaonError(f"the host module _kaon_host was compiled for {abi}, this is {host_abi()}: "
+                            "build it again with `python -m kaon_b200._build`")
         _host = _kaon_host
     return _host
 

@@ -65,3 +65,14 @@ def test_grads_present(have, want):
     for p, h in zip(ps, have):
         p.grad = torch.zeros(2) if h else None
     assert L.host().grads_present(ps) == want
+
+
+def test_a_module_compiled_for_another_torch_is_not_used(monkeypatch):
+    """It reads tensor objects by torch's layout of them: built again by a build, refused by a step."""
+    from kaon_b200 import _build
+    assert not _build._host_stale() and L.host().abi == _build.host_abi()
+    monkeypatch.setattr(torch, "__version__", "2.0.0")
+    monkeypatch.setattr(L, "_host", None)
+    assert _build._host_stale() and _build.needs_build()
+    with pytest.raises(L.KaonError, match="build it again"):
+        L.host()
