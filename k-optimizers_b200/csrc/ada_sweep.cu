@@ -363,11 +363,12 @@ __global__ void __launch_bounds__(SWT, 4) ada_small_kernel(const __grid_constant
   for (int r0 = 0; r0 < R; r0 += per) {
     const int r = r0 + rr;
     const bool act = r < R;
+    const int vecs = act ? nv : 0;   // (a thread without a row reads none: its owner writes it back meanwhile)
     unsigned char* rowp = g_s + (size_t)(act ? r : 0) * C * S::BYTES;
     float mu = 0.0f;
     if (gc) {
       float s = 0.0f;
-      for (int v = sub; v < nv; v += T) {
+      for (int v = sub; v < vecs; v += T) {
         W8<ST> x;
         x.load(rowp + (size_t)v * 8 * S::BYTES);
         const f32x2 a = add2(add2(x.pair(0), x.pair(1)), add2(x.pair(2), x.pair(3)));
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(SWT, 4) ada_small_kernel(const __grid_constant
     }
     const float mb = S::IS_BF16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu;
     float s2 = 0.0f;
-    for (int v = sub; v < nv; v += T) {
+    for (int v = sub; v < vecs; v += T) {
       W8<ST> x;
       f32x2 y[4];
       x.load(rowp + (size_t)v * 8 * S::BYTES);
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(SWT, 4) ada_small_kernel(const __grid_constant
         x.set(j, y[j]);
       }
       s2 += a.x + a.y;
-      if (act) x.store(rowp + (size_t)v * 8 * S::BYTES, nullptr);
+      x.store(rowp + (size_t)v * 8 * S::BYTES, nullptr);
     }
     s2 = row_sum(s2);
     if (act && sub == 0) {
