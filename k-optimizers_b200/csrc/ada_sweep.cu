@@ -10,8 +10,8 @@
 // consecutive elements and streams it, eight elements a lane and trip, with nothing shared between warps: no staging, no
 // barrier.  What is per row is one 16-byte table entry (left by FINAL), what is per column two vector loads that hit
 // L1; rows and columns advance by an addition, without a division.  Arithmetic is on packed pairs in the
-// reference's order of roundings; the mask is one comparison an element; codes are rounded from the correctly
-// rounded quotient m' / scale (reciprocal and residual), so no vector needs a second look.
+// reference's order of roundings; the mask is one comparison an element; codes are rounded from m' / scale
+// as corrected by its exact residual (see store_m8), so no vector needs a second look.
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -193,7 +193,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
         else sc = div127_exact(fmaxf(__uint_as_float(__ldcg(rowmax + row)), 1e-12f));
         float inv;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
-        // R = rint(m'/sc) + magic, from the correctly rounded quotient; T = -rint(m'/sc)
+        // R = rint(m'/sc) + magic; T = -rint(m'/sc)
         constexpr float MAGIC = MK == KAON_M_4BIT ? 12582920.0f : 12582912.0f;   // 1.5 * 2^23 (+ 8)
         const f32x2 INV = pack2(inv, inv), MG = pack2(MAGIC, MAGIC), NSC = pack2(-sc, -sc);
         f32x2 T[4], R[4];

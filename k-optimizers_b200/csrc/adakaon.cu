@@ -72,9 +72,12 @@ __device__ __forceinline__ float div_shared(float x, float d, float rcp) {
 }
 
 // A warp's sum of fp32 values, taken in double: a row statistic one ulp off moves codes of the row.  `plain`: in fp32.
-// Weights with a Kahan compensation keep the order of additions of the package's first versions (plain sums here and in
-// FINAL, larger STATS runs in the plan): the compensation stores rounding differences at the size of a bf16 step, so
-// a statistic that moves by an ulp shows there at full scale, and a resumed run should not see it.
+// The rule for every kernel: a tensor with a Kahan compensation (DevTensor::shift) that is shared out over STATS runs adds
+// in fp32 (here and in FINAL), in runs of at least 40 rows and 128 K elements (plan.cu); every other tensor, and any that
+// one CTA steps (ada_small_kernel), adds in double.  What the exception is for: the compensation stores rounding
+// differences at the size of a bf16 step, so a statistic that moves by an ulp shows there at full scale (double sums for
+// such tensors too: elements of the compensation off by a quarter of its size), and a run resumed from a checkpoint
+// of before should go on as it was.  Its price on the 269 M list: 1351 us a step against 1310.
 __device__ __forceinline__ float warp_sum_d(float v, bool plain) {
   if (plain) return warp_sum(v);
   double t = (double)v;

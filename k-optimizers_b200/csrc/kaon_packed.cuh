@@ -63,15 +63,14 @@ __device__ __forceinline__ void stg_f32(void* p, float v) {
   asm volatile("st.global.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v));
 }
 // a / 7 correctly rounded without the division unit: quotient estimate, exact residual, one correction.
-// Equal to the IEEE quotient for every a in [1e-12, FNTHREADS_MAX] (checked exhaustively on the host).
+// Equal to the IEEE quotient for every a in [1e-12, FLT_MAX] (tests/test_packed_division.py: all mantissas).
 __device__ __forceinline__ float div7_exact(float a) {
   const float r7 = 0.142857149243354797363281250f;  // RN(1/7)
   const float q0 = __fmul_rn(a, r7);
   return __fmaf_rn(__fmaf_rn(-7.0f, q0, a), r7, q0);
 }
 
-
-// a / 127 correctly rounded, as div7_exact (same exhaustive check)
+// a / 127 correctly rounded, as div7_exact (same test)
 __device__ __forceinline__ float div127_exact(float a) {
   const float r127 = 0.007874015718698501586914062500f;  // RN(1/127)
   const float q0 = __fmul_rn(a, r127);

@@ -1,6 +1,6 @@
 // Building blocks of the warp sweeps: eight consecutive elements a lane and trip, packed pairs, rows a multiple of eight
-// elements, 4-bit blocks of 128 (so half a warp shares a scale).  Used by the Adakaon family, AdaMuon, AdaPNM and
-// KProdigy.
+// elements, 4-bit blocks of 128 (so half a warp shares a scale).  Used by Lion, the Adakaon family, AdaMuon's EMA, AdaPNM
+// and KProdigy.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -171,7 +171,9 @@ __device__ __forceinline__ float amax8(const f32x2 M[4]) {
 
 // Store eight new momenta at mp (every lane of the warp calls it; `cnt` of the lane's exist, 0..8, M is 0 beyond an odd end).  bf16 momentum is
 // already rounded in M.  `amax`: int8 only, the finished maximum of the row; returns the scale (4-bit: the block's,
-// to be stored by the first lane of a half warp).  Codes are rounded from the correctly rounded quotient m' / scale.
+// to be stored by the first lane of a half warp).  Codes are rounded from m' / scale by an approximate reciprocal (within an
+// ulp) and one correction with the exact residual: the correctly rounded quotient but where m' / scale lies within
+// 2^-21 ulp of the middle between two floats.
 template <int MK>
 __device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax, const int cnt, const int lane) {
   if constexpr (MK == KAON_M_4BIT || MK == KAON_M_INT8) {

@@ -262,7 +262,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
       // how a list is split.
       const long long run_elems = std::max<long long>(8192, std::min<long long>(131072, t.numel / 32));
       long long run_rows = std::max<long long>(t.numel >= (1ll << 22) ? 20 : 8, (run_elems + C - 1) / C);
-      if (t.shift) run_rows = std::max<long long>(40, (131072 + C - 1) / C);   // (see warp_sum_d in adakaon.cu)
+      if (t.shift) run_rows = std::max<long long>(40, (131072 + C - 1) / C);   // (the rule at warp_sum_d in adakaon.cu)
       run_rows = (run_rows + t.chunk_rows - 1) / t.chunk_rows * t.chunk_rows;
       stages[i].resize(4);
       int slot = 0;
