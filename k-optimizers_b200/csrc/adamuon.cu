@@ -13,7 +13,7 @@
 #include "adakaon_dev.h"
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
-#include "kaon_packed.cuh"
+#include "kaon_sweep.cuh"
 #include "ns_batch.h"
 
 namespace kaon {
@@ -208,6 +208,7 @@ template <typename PT, int MK>
 __global__ void __launch_bounds__(ET, 4) muon_ema_fast_kernel(const __grid_constant__ PlanView pv, const Task* tasks, int n_tasks,
                                                               float w1, float w1m1, int small_w1, const EmaOut* outs, double* part) {
   using E = Elems<PT>;
+  constexpr int MV = MBytes<MK>::V;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (ET / 32);
   for (int i = __shfl_sync(0xffffffffu, (int)(blockIdx.x * (ET / 32) + (threadIdx.x >> 5)), 0); i < n_tasks; i += nw) {
@@ -226,57 +227,28 @@ __global__ void __launch_bounds__(ET, 4) muon_ema_fast_kernel(const __grid_const
       // the new momentum of vector v
       auto fresh = [&](int v, f32x2 MN[4]) {
         const long long e = e0 + v * 8ll;
-        float gx[8], mo[8];
-        E::load8(g + e * E::BYTES, gx);
-        if constexpr (MK == KAON_M_4BIT) {
-          const uint32_t w = *reinterpret_cast<const uint32_t*>(m + (e >> 1));
-          const uint32_t wl = w & 0x0F0F0F0Fu, wh = (w >> 4) & 0x0F0F0F0Fu;
-          const float sc = d.m_scale[e >> 7];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const f32x2 x = mul2(add2(pack2(__uint_as_float(prmt(wl, 0x4B000000u, 0x7540u | (uint32_t)j)),
-                                            __uint_as_float(prmt(wh, 0x4B000000u, 0x7540u | (uint32_t)j))),
-                                      pack2(-8388616.0f, -8388616.0f)), pack2(sc, sc));
-            mo[2 * j] = x.x; mo[2 * j + 1] = x.y;
-          }
-        } else if constexpr (MK == KAON_M_INT8) {
-          const uint2 w = *reinterpret_cast<const uint2*>(m + e);
-          const uint32_t x0 = w.x ^ 0x80808080u, x1 = w.y ^ 0x80808080u;  // code + 128 in every byte
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t x = j < 2 ? x0 : x1, b = (uint32_t)(2 * (j & 1));
-            const f32x2 y = mul2(add2(pack2(__uint_as_float(prmt(x, 0x4B000000u, 0x7540u | b)),
-                                            __uint_as_float(prmt(x, 0x4B000000u, 0x7540u | (b + 1u)))),
-                                      pack2(-8388736.0f, -8388736.0f)), pack2(row_sc, row_sc));
-            mo[2 * j] = y.x; mo[2 * j + 1] = y.y;
-          }
-        } else if constexpr (MK == KAON_M_BF16) {
-          Elems<__nv_bfloat16>::load8(m + e * 2, mo);
-        } else if constexpr (MK == KAON_M_F32) {
-          Elems<float>::load8(m + e * 4, mo);
+        W8<PT> gq;
+        MRaw<MK> mq;
+        f32x2 MO[4];
+        gq.load(g + e * E::BYTES);
+        if constexpr (MK != KAON_M_NONE) {
+          mq.load(m + (e >> 3) * MV);
+          mq.decode(MK == KAON_M_4BIT ? d.m_scale[e >> 7] : row_sc, MO);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          f32x2 G = pack2(gx[2 * j], gx[2 * j + 1]);
+          f32x2 G = gq.pair(j);
           if constexpr (MK == KAON_M_NONE) {
             MN[j] = G;
           } else {
-            const f32x2 M = pack2(mo[2 * j], mo[2 * j + 1]);
             if constexpr (MK == KAON_M_BF16) G = pack2(round_bf16(G.x), round_bf16(G.y));
-            MN[j] = small_w1 ? fma2(pack2(w1, w1), sub2(G, M), M) : fma2(pack2(w1m1, w1m1), sub2(G, M), G);
+            MN[j] = small_w1 ? fma2(pack2(w1, w1), sub2(G, MO[j]), MO[j]) : fma2(pack2(w1m1, w1m1), sub2(G, MO[j]), G);
             if constexpr (MK == KAON_M_BF16) MN[j] = pack2(round_bf16(MN[j].x), round_bf16(MN[j].y));
           }
         }
       };
-      auto amax8 = [](const f32x2 M[4]) {
-        float a = max3f(fabsf(M[0].x), fabsf(M[0].y), fabsf(M[1].x));
-        a = max3f(a, fabsf(M[1].y), fabsf(M[2].x));
-        a = max3f(a, fabsf(M[2].y), fabsf(M[3].x));
-        return fmaxf(a, fabsf(M[3].y));
-      };
-      float sc = 1.0f;
+      float amax = 0.0f;
       if constexpr (MK == KAON_M_INT8) {
-        float amax = 0.0f;
 #pragma unroll 2
         for (int v = lane; v < nv; v += 32) {
           f32x2 MN[4];
@@ -285,7 +257,6 @@ __global__ void __launch_bounds__(ET, 4) muon_ema_fast_kernel(const __grid_const
         }
         __syncwarp();
         amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
-        sc = div127_exact(fmaxf(amax, 1e-12f));
       }
       for (int v0 = 0; v0 < nv; v0 += 32) {
         const int v = v0 + lane;
@@ -293,41 +264,15 @@ __global__ void __launch_bounds__(ET, 4) muon_ema_fast_kernel(const __grid_const
         f32x2 MN[4];
         fresh(act ? v : 0, MN);
         const long long e = e0 + v * 8ll;
-        if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(act ? amax8(MN) : 0.0f, lane), 1e-12f));
-        if (!act) continue;
-        if constexpr (MK == KAON_M_4BIT || MK == KAON_M_INT8) {
-          // rint(m'/sc) + magic, from the correctly rounded quotient
-          float inv;
-          asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
-          constexpr float MAGIC = MK == KAON_M_4BIT ? 12582920.0f : 12582912.0f;
-          uint32_t R[8];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const f32x2 INV = pack2(inv, inv), qq = mul2(MN[j], INV);
-            const f32x2 x = add2(fma2(fma2(qq, pack2(-sc, -sc), MN[j]), INV, qq), pack2(MAGIC, MAGIC));
-            R[2 * j] = __float_as_uint(x.x); R[2 * j + 1] = __float_as_uint(x.y);
-          }
-          if constexpr (MK == KAON_M_4BIT) {
-            uint32_t w = 0u;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) w |= (R[k] & 0xFu) << (4 * k);
-            *reinterpret_cast<uint32_t*>(m + (e >> 1)) = w;
-            if ((lane & 15) == 0) d.m_scale[e >> 7] = sc;
-          } else {
-            *reinterpret_cast<uint2*>(m + e) = make_uint2(prmt(prmt(R[0], R[1], 0x0040u), prmt(R[2], R[3], 0x0040u), 0x5410u),
-                                                          prmt(prmt(R[4], R[5], 0x0040u), prmt(R[6], R[7], 0x0040u), 0x5410u));
-            if (v == 0) d.m_scale[t.row0 + r] = sc;
-          }
+        if constexpr (MK != KAON_M_NONE) {
+          const float sc = store_m8<MK>(m + (e >> 3) * MV, MN, amax, act ? 8 : 0, lane);
+          if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) d.m_scale[e >> 7] = sc; }
+          if constexpr (MK == KAON_M_INT8) { if (v == 0) d.m_scale[t.row0 + r] = sc; }
         }
+        if (!act) continue;
         const uint4 x = make_uint4(pack_bf16_rn(MN[0].x, MN[0].y), pack_bf16_rn(MN[1].x, MN[1].y),
                                    pack_bf16_rn(MN[2].x, MN[2].y), pack_bf16_rn(MN[3].x, MN[3].y));
         *reinterpret_cast<uint4*>(x_out + e) = x;   // bf16 of the momentum before requantisation
-        if constexpr (MK == KAON_M_BF16) *reinterpret_cast<uint4*>(m + e * 2) = x;
-        if constexpr (MK == KAON_M_F32) {
-          float4* md = reinterpret_cast<float4*>(m + e * 4);
-          md[0] = make_float4(MN[0].x, MN[0].y, MN[1].x, MN[1].y);
-          md[1] = make_float4(MN[2].x, MN[2].y, MN[3].x, MN[3].y);
-        }
         const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
         f32x2 q = pack2(0.0f, 0.0f);
 #pragma unroll
