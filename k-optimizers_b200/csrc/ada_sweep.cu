@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(SWT, 4) ada_sweep_kernel(const __grid_constant
 // A factored tensor of at most ADA_SMALL_MAX elements in ONE CTA: row statistics, column statistics, clip divisor,
 // COUNT and APPLY with barriers in between.  A list of adapter matrices has hundreds of them, each far too small to
 // share out; as items of the stages above they spent the step waiting for one another (720 matrices of 10 240
-// elements: 700 us, here 51).  The gradient is kept in shared memory for the statistics.  Sums in a fixed order.
+// elements: 700 us, here 62 of the step's 69).  The gradient is kept in shared memory for the statistics.  Sums in a fixed order.
 __device__ __forceinline__ double small_sum(double v, double* red, int tid) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -138,7 +138,7 @@ __device__ __forceinline__ void pnm_write(const PnmDev& hp, const DevTensor& d, 
 // The two sweeps over tensors whose rows are a multiple of eight elements (4-bit blocks of 128): a warp per unit of up
 // to 4096 elements, nothing shared between warps.  Bound by instruction issue, so on packed pairs, the mask one
 // comparison an element, rows and columns advanced by an addition.  (A CTA per 16 K-element item with guarded
-// elements and a scalar encode: SUM 409 us and APPLY 972 us on 269 M elements of 4-bit momentum; here 251 and 531 us.)
+// elements and a scalar encode: SUM 409 us and APPLY 972 us on 269 M elements of 4-bit momentum; here 260 and 550 us.)
 template <typename PT, int MK, bool APPLY>
 __global__ void __launch_bounds__(PT_THREADS, 4) pnm_sweep_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ PnmDev hp,
                                                                   const __grid_constant__ PnmView x) {

@@ -6,9 +6,9 @@
 // unit of the tensor has finished, the weights with the tensor-wide rescale 1/max(kept/numel, 1e-8).  Units are claimed in
 // list order, all of MAIN first; small lists are one launch, large ones a launch each (see lion_warp_units).
 //
-// Bound by instruction issue (4-bit momentum) or HBM (wider states), so: packed pairs; the mask one saturating FMA an
-// element; both kinds of codes packed as small integers by FMAs; rows advanced by an addition; the next trip's words
-// loaded ahead; no staging and no barrier.  (Rows staged in shared memory by a CTA per 16 K-element item: 5.30 ms on the
+// Bound by instruction issue (4-bit momentum: MAIN 69 % of the slots, 224 warp instructions per 256 elements) or HBM (wider
+// states; APPLY 5.3 TB/s), so: packed pairs; the mask from the sign bytes of the products; momentum codes packed as small
+// integers by FMAs; rows advanced by an addition; the next trip's words loaded ahead; no staging and no barrier.  (Rows staged in shared memory by a CTA per 16 K-element item: 5.30 ms on the
 // 2.6 B-parameter list with 4-bit momentum, 267 us on ragged fp32 lists.)
 #include <algorithm>
 #include <type_traits>
@@ -377,8 +377,8 @@ bool lion_warp_tensor(const DevTensor& t, int momentum_kind) {
 // LW_ROWS rows.
 // Order: all MAIN units, then all APPLY units (APPLY units between them would empty the first level caches by their acquiring
 // reads, where the second reading of a row's gradient hits).  Up to 64 M elements one launch; larger lists two (returns
-// the number of MAIN units; 0: one launch), without the counters, whose fences then cost more than a launch (2.6 B list:
-// 4.59 ms, in one launch 4.98).
+// the number of MAIN units; 0: one launch), without the counters, whose fences then cost more than a launch (2.6 B list in
+// units of 4096: 4.59 ms, in one launch 4.98; in units of 8192 4.40).
 int lion_warp_units(const std::vector<DevTensor>& tensors, const std::vector<char>& elig, std::vector<Task>& out, std::vector<int>& n_main) {
   long long total = 0;
   for (size_t i = 0; i < tensors.size(); ++i) if (elig[i]) total += tensors[i].numel;

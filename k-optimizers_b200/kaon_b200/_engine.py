@@ -269,9 +269,9 @@ class FusedStepMixin:
         everything else takes ``_group_plans``."""
         params, md = group["params"], self._momentum_dtype(group)
         steady = self._steady.get(gi)
-        if steady is not None and steady[0] == md and L.host().settled(params, steady[1], self.state, steady[2], C.addressof(steady[3])):
+        if steady is not None and steady[0] == md and L.host().settled(params, steady[1], self.state, steady[2], steady[3]):
             out = []
-            for pl in steady[4]:
+            for pl in steady[5]:
                 stream = L.raw_stream(pl.device.index)
                 some = pl.refresh(stream)
                 if some is None:
@@ -293,7 +293,7 @@ class FusedStepMixin:
             states = [self.state[p] if p in self.state and self.state[p] else None for p in seen]
             pos = (C.c_int64 * len(seen))()
             L.host().entries(self.state, seen, C.addressof(pos))
-            self._steady[gi] = (md, seen, states, pos, plans)
+            self._steady[gi] = (md, seen, states, C.addressof(pos), pos, plans)
         return out
 
     def _drop_plans(self, gi: int, keep: Iterable[tuple] = ()) -> None:

@@ -1,8 +1,8 @@
 """Adakaon (conv-aware factored second moment, quantised momentum) on the fused sm_100a step.
 
 Same constructor, param-group keys, state layout and errors as the reference class
-(src/kaon/adakaon.py:195-292, 318-335); ``step()`` launches one persistent CUDA kernel per parameter
-group instead of the foreach buckets (src/kaon/adakaon.py:339-383, 793-1014).  ``foreach*``, ``fused`` and
+(src/kaon/adakaon.py:195-292, 318-335); ``step()`` launches a short chain of CUDA kernels per parameter
+group (statistics, count, write) instead of the foreach buckets (src/kaon/adakaon.py:339-383, 793-1014).  ``foreach*``, ``fused`` and
 ``fused_tile_cap`` are accepted and ignored.
 """
 from __future__ import annotations

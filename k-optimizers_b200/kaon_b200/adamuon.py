@@ -2,7 +2,7 @@
 
 Same constructor, param-group keys, state layout and errors as the reference class
 (src/kaon/adamuon.py:216-325); ``step()`` runs, per parameter group, the EMA pre-pass, the Newton-Schulz
-iteration as tcgen05 GEMMs and one persistent kernel for everything after it, instead of the foreach
+iteration as grouped tcgen05 GEMMs and Adakaon's kernels for everything after it, instead of the foreach
 buckets and ``torch.bmm`` (src/kaon/adamuon.py:327-352, 393-615).  ``foreach*`` and ``compile`` are
 accepted and ignored.
 """

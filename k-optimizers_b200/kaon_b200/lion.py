@@ -1,7 +1,7 @@
 """Lion (sign momentum, one quantised buffer) on the fused sm_100a step.
 
 Same constructor, param-group keys, state layout and errors as the reference class
-(src/kaon/lion.py:152-208); ``step()`` launches one persistent CUDA kernel per parameter group instead of
+(src/kaon/lion.py:152-208); ``step()`` launches one or two CUDA kernels per parameter group instead of
 the foreach buckets (src/kaon/lion.py:322-485).  ``foreach*`` knobs are accepted and ignored: they are
 numerically neutral in the reference (tests/test_lion.py:190-239) and have no meaning here.
 """
