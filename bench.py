@@ -38,20 +38,20 @@ ADAMUON_KW = dict(lr=1e-3, ns_steps=2, cautious=True, momentum_dtype="int8")
 #  Adakaon-int8 (config 3): g 2 + p 2+2 + m 1+1 + row scales, row/col stats, 1-D v; 1 % of grads x100
 #  Nekaon-4bit (config 4): as Lion-4bit + stats; climb and removal ride on the same weight access
 #  AdaMuon-int8 (config 5): the non-NS passes move 8.006 B/param; Newton-Schulz is 3.24e14 flop per step
-# traffic_bpp: DRAM bytes per parameter of one step (all its launches), from the ncu launch list of the
-# *_mid workload (a list of 269 M parameters with every tensor shape of the big one, 15x L2) summarised in
-# profiles/lion_kernel_bf16_4bit_unet_mid.md and profiles/adakaon_kernels_bf16_unet_mid.md.
+# traffic_bpp: DRAM bytes per parameter of one step (all its launches), from ncu captures of the *_mid workload's
+# launches (a list of 269 M parameters with every tensor shape of the big one, 15x L2) summarised in
+# profiles/lion_kernels_unet_mid.md and profiles/adakaon_kernels_unet_mid.md.
 WORKLOADS = {
-    "lion4bit_unet2p6b": ("Lion", LION_KW, "unet_2p6b", 7.0625, {"traffic_bpp": 7.22}),
+    "lion4bit_unet2p6b": ("Lion", LION_KW, "unet_2p6b", 7.0625, {"traffic_bpp": 7.48}),
     "lion4bit_sample": ("Lion", LION_KW, "unet_sample", 7.0625, {}),
     "lion4bit_mid": ("Lion", LION_KW, "unet_mid", 7.0625, {}),
     "lion4bit_nogc_unet2p6b": ("Lion", dict(LION_KW, gradient_centralization=False), "unet_2p6b", 7.0625, {}),
-    "adakaon_int8_unet2p6b": ("Adakaon", ADAKAON_KW, "unet_2p6b", 8.015, {"outlier": True, "traffic_bpp": 13.78}),
+    "adakaon_int8_unet2p6b": ("Adakaon", ADAKAON_KW, "unet_2p6b", 8.015, {"outlier": True, "traffic_bpp": 13.86}),
     "adakaon_int8_sample": ("Adakaon", ADAKAON_KW, "unet_sample", 8.015, {"outlier": True}),
     "adakaon_int8_mid": ("Adakaon", ADAKAON_KW, "unet_mid", 8.015, {"outlier": True}),
     "adakaon_int8_mid_odd": ("Adakaon", ADAKAON_KW, "unet_mid_odd", 8.015, {"outlier": True}),
     "nekaon4bit_unet2p6b": ("Nekaon", NEKAON_KW, "unet_2p6b", 7.073, {"cosine": (1e-4, 1e-5, 50), "steps": 50,
-                                                                       "traffic_bpp": 14.38}),
+                                                                       "traffic_bpp": 16.30}),
     "nekaon4bit_sample": ("Nekaon", NEKAON_KW, "unet_sample", 7.073, {"cosine": (1e-4, 1e-5, 50)}),
     "nekaon4bit_mid": ("Nekaon", NEKAON_KW, "unet_mid", 7.073, {"cosine": (1e-4, 1e-5, 50)}),
     "adamuon_int8_dit11b": ("AdaMuon", ADAMUON_KW, "dit_11b", 8.006, {"one_grad_set": True, "steps": 10}),
@@ -65,9 +65,10 @@ WORKLOADS = {
 E2E_GROUPS = 16   # parameter groups of the end-to-end pipeline
 HEADLINE = "lion4bit_unet2p6b"
 RECORD = ["adakaon_int8_unet2p6b", "nekaon4bit_unet2p6b", "adamuon_int8_dit11b"]
-KERNEL_NAME = {"AdaMuon": "ns_gemm_kernel", "Lion": "lion_kernel<bf16,4bit>", "Adakaon": "adakaon_kernel<bf16,int8>",
-               "Nekaon": "adakaon_kernel<bf16,4bit>", "AdaPNM": "pnm_pass_kernel<bf16,4bit>",
-               "KProdigy": "kp_sweep_kernel<bf16,bf16>"}
+KERNEL_NAME = {"AdaMuon": "ns_gemm_kernel (grouped)", "Lion": "lion_main_kernel + lion_apply_kernel <bf16,4bit>",
+               "Adakaon": "ada_stats_kernel + adakaon_kernel + ada_sweep_kernel (COUNT, APPLY) <bf16,int8>",
+               "Nekaon": "ada_stats_kernel + adakaon_kernel + ada_sweep_kernel (COUNT, APPLY) <bf16,4bit>",
+               "AdaPNM": "pnm_sweep_kernel<bf16,4bit>", "KProdigy": "kp_warp_kernel<bf16,bf16>"}
 
 
 def host_cores() -> int:
@@ -665,18 +666,15 @@ def measure(ctx: Ctx, workload: str, steps: int, warmup: int, e2e_steps: int = 0
                              "peak": 770.0, "unit": "GB/s", "floor_ms": max(t_hbm, t_link) * 1e3,
                              "frac_of_floor": max(t_hbm, t_link) * 1e3 / kern_ms}
         if ns_info is not None:
-            rest_ms = max(kern_ms - ns_info["total"]["ms_per_step"], 1e-6)
-            res["hbm_passes"] = dict(res["roofline"], achieved=alg_bytes / (rest_ms * 1e-3) / 1e9,
-                                     frac=alg_bytes / (rest_ms * 1e-3) / 1e9 / peak, ms=rest_ms,
-                                     note="everything of the step that is not a Newton-Schulz GEMM: step time minus "
-                                          "the GEMM chains timed alone")
-            res["hbm_passes"].pop("frac_of_nominal_8TBs", None)
-            res["roofline"] = {"bound": "tensor", "achieved": ns_info["total"]["tflops"], "peak": tpeak,
-                               "unit": "TFLOP/s", "frac": ns_info["total"]["tflops"] / tpeak, "traffic": None,
-                               "peak_kind": f"{peak_kind} cuBLAS bf16 burst", "kernel": "ns_gemm_kernel",
-                               "note": "Newton-Schulz GEMM chain of one matrix timed alone per shape (CUDA events); inside a step "
-                                       "the chains of different matrices overlap on three streams: newton_schulz.whole_step_tflops "
-                                       "is the same flops over the whole step time"}
+            # The step runs the products of all matrices of a batch in grouped launches; a Newton-Schulz call on its own
+            # (timed per shape above) launches one product at a time, so the two cannot be subtracted from each other.
+            tf = ns_info["total"]["flop_per_step"] / (kern_ms * 1e-3) / 1e12
+            res["roofline"] = {"bound": "tensor", "achieved": tf, "peak": tpeak,
+                               "unit": "TFLOP/s", "frac": tf / tpeak, "traffic": None,
+                               "peak_kind": f"{peak_kind} cuBLAS bf16 burst", "kernel": KERNEL_NAME[opt_name],
+                               "note": "Newton-Schulz flops (full products) over the whole step: grouped products, the "
+                                       "momentum pre-pass, second-moment statistics and the weight sweeps, batches "
+                                       "alternating over two streams; newton_schulz has one call on its own per shape"}
             ns_info["whole_step_tflops"] = ns_info["total"]["flop_per_step"] / (kern_ms * 1e-3) / 1e12
             res["newton_schulz"] = ns_info
     return res
@@ -717,7 +715,7 @@ def run_ours(args):
                 "ms_per_step": head["ms_per_step"], "higher_is_better": True, "scaling": "strong",
                 "vs_baseline": None, "dtype": "f32", "data": "synthetic"}
         for k in ("config", "step_kernel_ms", "publish_ms", "compute_only_ms", "incl_publish_ms",
-                  "gradient_reduce_scatter", "roofline", "e2e", "gpu_launches", "clocks", "nvlink", "hbm_passes",
+                  "gradient_reduce_scatter", "roofline", "e2e", "gpu_launches", "clocks", "nvlink",
                   "newton_schulz"):
             if k in head:
                 line[k] = head[k]
