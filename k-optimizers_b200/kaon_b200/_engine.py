@@ -336,7 +336,7 @@ class FusedStepMixin:
             if (pl is None or pl.momentum_dtype != md or not _same(pl.params, plist) or not _same(pl.states, slist)
                     or pl.params_moved()):
                 if pl is not None:
-                    pl.destroy()
+                    self._plans.pop(key).destroy()   # (gone also where building the next one raises)
                 if ids is None:
                     ids = self._tensor_ids()
                 pl = GroupPlan(self._OPT_KIND, plist, slist, [ids[id(p)] for p in plist], md, self._M_KEY)

@@ -128,3 +128,21 @@ def test_a_plan_whose_tensors_changed_dtype_is_given_up(stepped):
         p.grad = torch.randn(6, 8).bfloat16()
     opt.step()
     assert [key[2] for key in opt._plans] == [torch.bfloat16]
+
+
+def test_a_plan_that_cannot_be_built_leaves_none_behind(stepped, monkeypatch):
+    ps, opt = _make(Lion)
+    opt.step()
+    ps[0].data = ps[0].data.clone()
+
+    class Refused(RecordingPlan):
+        def __init__(self, *args):
+            raise NotImplementedError("refused")
+
+    monkeypatch.setattr(_engine, "GroupPlan", Refused)
+    with pytest.raises(NotImplementedError):
+        opt.step()
+    assert not opt._plans
+    monkeypatch.setattr(_engine, "GroupPlan", RecordingPlan)
+    opt.step()
+    assert len(stepped[-1]) == len(ps) and _is_live(opt, stepped[-1])
