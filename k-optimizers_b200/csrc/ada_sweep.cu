@@ -188,55 +188,12 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
       }
       // ---- store the new momentum; MO <- the momentum as stored ----
       float sc = 1.0f;
-      if constexpr (CODED) {
-        if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(act ? amax8(MN) : 0.0f, lane), 1e-12f));
-        else sc = div127_exact(fmaxf(__uint_as_float(__ldcg(rowmax + row)), 1e-12f));
-        float inv;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(sc));
-        // R = rint(m'/sc) + magic; T = -rint(m'/sc)
-        constexpr float MAGIC = MK == KAON_M_4BIT ? 12582920.0f : 12582912.0f;   // 1.5 * 2^23 (+ 8)
-        const f32x2 INV = pack2(inv, inv), MG = pack2(MAGIC, MAGIC), NSC = pack2(-sc, -sc);
-        f32x2 T[4], R[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const f32x2 qq = mul2(MN[j], INV);
-          R[j] = add2(fma2(fma2(qq, NSC, MN[j]), INV, qq), MG);
-        }
-        if constexpr (MK == KAON_M_4BIT) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) T[j] = sub2(MG, R[j]);
-          // sum_k (8 - t_k) 16^k = 0x8888 - (t0 + 16 t1 + 256 t2 + 4096 t3), exact in fp32; adding 2^23 leaves it
-          // in the low 16 mantissa bits
-          const f32x2 K256 = pack2(256.0f, 256.0f);
-          const f32x2 Xl = fma2(T[1], K256, T[0]), Yl = fma2(T[3], K256, T[2]);
-          const float lo4 = __fsub_rn(8423560.0f, __fmaf_rn(Xl.y, 16.0f, Xl.x));
-          const float hi4 = __fsub_rn(8423560.0f, __fmaf_rn(Yl.y, 16.0f, Yl.x));
-          if (act) {
-            stg_u32(mp, prmt(__float_as_uint(lo4), __float_as_uint(hi4), 0x5410u));
-            if ((lane & 15) == 0) stg_f32(msc, sc);
-          }
-        } else {
-          if (MS && hp.climb) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) T[j] = sub2(MG, R[j]);
-          }
-          if (act) {  // the low byte of every R is the code in two's complement
-            const uint32_t w0 = prmt(prmt(__float_as_uint(R[0].x), __float_as_uint(R[0].y), 0x0040u),
-                                     prmt(__float_as_uint(R[1].x), __float_as_uint(R[1].y), 0x0040u), 0x5410u);
-            const uint32_t w1 = prmt(prmt(__float_as_uint(R[2].x), __float_as_uint(R[2].y), 0x0040u),
-                                     prmt(__float_as_uint(R[3].x), __float_as_uint(R[3].y), 0x0040u), 0x5410u);
-            *reinterpret_cast<uint2*>(mp) = make_uint2(w0, w1);
-            if (cv == 0) msc[row] = sc;
-          }
-        }
-        if (MS && hp.climb) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) MO[j] = mul2(T[j], NSC);
-        }
-      } else if constexpr (MK != KAON_M_NONE) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { MO[j] = MN[j]; mq.w.set(j, MN[j]); }
-        if (act) mq.w.store(mp, nullptr);
+      if constexpr (MK != KAON_M_NONE) {
+        float amax = 0.0f;
+        if constexpr (MK == KAON_M_INT8) amax = __uint_as_float(__ldcg(rowmax + row));
+        sc = store_m8<MK>(mp, MN, amax, act ? 8 : 0, lane, MS ? MO : nullptr);
+        if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(msc, sc); }
+        if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) msc[row] = sc; }
       }
       // ---- weights: p <- round(p - update), then the climb from the momentum as stored ----
       write8(hp, d, q, act, P, F);

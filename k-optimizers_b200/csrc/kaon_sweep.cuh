@@ -174,8 +174,9 @@ __device__ __forceinline__ float amax8(const f32x2 M[4]) {
 // to be stored by the first lane of a half warp).  Codes are rounded from m' / scale by an approximate reciprocal (within an
 // ulp) and one correction with the exact residual: the correctly rounded quotient but where m' / scale lies within
 // 2^-21 ulp of the middle between two floats.
+// `stored`, where given: the momenta as they were stored.
 template <int MK>
-__device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax, const int cnt, const int lane) {
+__device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax, const int cnt, const int lane, f32x2* stored = nullptr) {
   if constexpr (MK == KAON_M_4BIT || MK == KAON_M_INT8) {
     float sc;
     if constexpr (MK == KAON_M_4BIT) sc = div7_exact(fmaxf(half_warp_max(cnt > 0 ? amax8(M) : 0.0f, lane), 1e-12f));
@@ -190,10 +191,13 @@ __device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax
       const f32x2 qq = mul2(M[j], INV);
       R[j] = add2(fma2(fma2(qq, NSC, M[j]), INV, qq), MG);
     }
-    if constexpr (MK == KAON_M_4BIT) {
-      f32x2 T[4];
+    f32x2 T[4];   // -rint(m'/sc)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) T[j] = sub2(MG, R[j]);
+    for (int j = 0; j < 4; ++j) {
+      T[j] = sub2(MG, R[j]);
+      if (stored) stored[j] = mul2(T[j], NSC);
+    }
+    if constexpr (MK == KAON_M_4BIT) {
       // sum_k (8 - t_k) 16^k = 0x8888 - (t0 + 16 t1 + 256 t2 + 4096 t3), exact in fp32; adding 2^23 leaves it in the low
       // 16 mantissa bits
       const f32x2 K256 = pack2(256.0f, 256.0f);
@@ -216,7 +220,10 @@ __device__ __forceinline__ float store_m8(void* mp, const f32x2 M[4], float amax
   } else {
     MRaw<MK> o;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) o.w.set(j, M[j]);
+    for (int j = 0; j < 4; ++j) {
+      o.w.set(j, M[j]);
+      if (stored) stored[j] = M[j];
+    }
     if (cnt == 8) o.w.store(mp, nullptr);
     else
 #pragma unroll
