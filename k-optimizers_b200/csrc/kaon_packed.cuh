@@ -40,6 +40,12 @@ __device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
   asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
+// a + b, as sub_bf16x2
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 // maximum over the 16 lanes of this thread's half warp (every lane of the warp calls it; v >= 0, so
 // the ordering of the bit patterns is that of the values): two whole-warp reductions, one per half
 __device__ __forceinline__ float half_warp_max(float v, int tid) {

@@ -261,21 +261,16 @@ __device__ __forceinline__ void write8(const HP& hp, const DevTensor& d, uint64_
       W8<PT> SH;
       if (act) SH.load(she); else SH.load(d.shift);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f32x2 p = P.pair(j), sv = SH.pair(j);
-        kahan_step(p.x, sv.x, -F[j].x);
-        kahan_step(p.y, sv.y, -F[j].y);
-        P.set(j, p);
-        SH.set(j, sv);
+      for (int j = 0; j < 4; ++j) {   // kahan_step in bf16 arithmetic: 5 instructions a pair for 28
+        const uint32_t s1 = add_bf16x2(SH.w[j], pack_bf16_rn(F[j].x, F[j].y));
+        const uint32_t pn = add_bf16x2(P.w[j], s1);
+        SH.w[j] = add_bf16x2(s1, sub_bf16x2(P.w[j], pn));
+        P.w[j] = pn;
       }
       if (act) SH.store(she, nullptr);
     } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t fb = pack_bf16_rn(F[j].x, F[j].y);
-        const f32x2 s = add2(P.pair(j), pack2(bf16lo(fb), bf16hi(fb)));
-        P.w[j] = pack_bf16_rn(s.x, s.y);
-      }
+      for (int j = 0; j < 4; ++j) P.w[j] = add_bf16x2(P.w[j], pack_bf16_rn(F[j].x, F[j].y));
     }
   } else {
 #pragma unroll
