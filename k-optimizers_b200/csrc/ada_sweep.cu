@@ -29,7 +29,8 @@ constexpr int SWT = 256;   // threads per CTA
 // CTA itself has just written the row table and the column factors.
 // MUON (AdaMuon's factored tensors): the signal is the orthogonalised matrix (bf16, `pv.signal`), the chain carries no
 // momentum, and the mask compares with the raw gradient.  MS: the build with the Nekaon climb.
-template <typename PT, int MKP, bool MUON, bool MS, bool APPLY, int STRIDE, bool OWN>
+// CP (COUNT): with weight decay, where the mask looks at the weights.
+template <typename PT, int MKP, bool MUON, bool MS, bool APPLY, bool CP, int STRIDE, bool OWN>
 __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp, const Task& t, const unsigned char* gbase,
                                            const int first, const int lane) {
   using E = Elems<PT>;
@@ -39,7 +40,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   constexpr bool CODED = MK == KAON_M_INT8 || MK == KAON_M_4BIT;
   constexpr int MBITS = MK == KAON_M_4BIT ? 4 : MK == KAON_M_INT8 ? 8 : MK == KAON_M_BF16 ? 16 : MK == KAON_M_F32 ? 32 : 0;
   // with weight decay the mask looks at the weights after the removal: COUNT writes them, APPLY finds them
-  const bool count_p = hp.has_wd && hp.cautious;
+  const bool count_p = APPLY ? hp.has_wd && hp.cautious : CP;
   const bool rem_here = MS && hp.remove && (APPLY ? !count_p : count_p);
   const bool need_p = APPLY || count_p;
   const DevTensor& d = pv.tensors[t.tensor];
@@ -68,15 +69,24 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   if (cv >= nv) { const int k = cv / nv; row += k; cv -= k * nv; }
   const int adv_r = STRIDE / nv, adv_c = STRIDE - adv_r * nv;
   f32x2 kept2 = pack2(0.0f, 0.0f);
+  // int8 COUNT: every trip lies in one row (rows and the unit's start are whole trips); the running maximum of the row's codes
+  const bool whole = !OWN && ((nv | (t.pad >> 3) | nvec) & 31) == 0;
+  unsigned run = 0u;
 
+  // int8 momentum: a trip's signal and momentum are loaded by the trip before it, as soon as that has unpacked its own (no
+  // register but the words' own), its weights, which are used last, at its start.  (2.6 B list: COUNT 2110 -> 1740 us, APPLY 3921
+  // -> 3510.)  Otherwise all at its start: with 4-bit and bf16 momentum the words' registers are short (COUNT 256 -> 278 us on
+  // 269 M elements of bf16 momentum when loaded ahead).
+  constexpr bool AHEAD = !OWN && MK == KAON_M_INT8;
   W8<ST> gq;
-  W8<PT> P;
+  W8<PT> P, rq;
   MRaw<MK> mq;
-  auto load = [&]() {
-    gq.load(sp);
-    if constexpr (MK != KAON_M_NONE) mq.load(mp);
-    if constexpr (MK == KAON_M_4BIT) mq.sc = *msc;
-    if (need_p) P.load(pp);
+  auto load = [&](auto ahead) {
+    constexpr int A = decltype(ahead)::value;   // trips ahead
+    gq.load(sp + A * STRIDE * 8 * S::BYTES);
+    if constexpr (MK != KAON_M_NONE) mq.load(mp + A * STRIDE * MBITS);
+    if constexpr (MK == KAON_M_4BIT) mq.sc = msc[A * STRIDE / 16];
+    if constexpr (MUON) rq.load(rawp + A * STRIDE * 8 * E::BYTES);
   };
   // a climb of eight elements (reference src/kaon/msam.py:222-230); `wild`: a momentum that decodes to NaN or
   // infinity (a corrupt scale) keeps the reference's nan_to_num
@@ -92,9 +102,11 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   auto add_noisy = [&](const f32x2 D[4], uint32_t tag) {
     add_noisy8(hp, d, q, tag, P, D);
   };
-  // the vector whose words are in gq, mq, P; `act`: this lane has one
-  auto trip = [&](const bool act) {
-    const float4 f = __ldcg(rowtab + row);   // {mean, r_i, int8: scale of the stored codes, -}
+  // the vector whose words are in gq, mq; `act`: this lane has one; `more`: and one in the next trip
+  auto trip = [&](const bool act, const bool more) {
+    if (!AHEAD && act) load(std::integral_constant<int, 0>{});
+    const float4 f = OWN ? rowtab[row] : __ldg(rowtab + row);   // {mean, r_i, int8: scale of the stored codes, r_i / div * scale}
+    if (need_p) P.load(act ? pp : reinterpret_cast<unsigned char*>(d.p));
     f32x2 CF[4], G[4], MO[4];
     {
       const float4* cp = reinterpret_cast<const float4*>(cfac) + 2 * cv;
@@ -102,11 +114,14 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
       CF[0] = pack2(a.x, a.y); CF[1] = pack2(a.z, a.w); CF[2] = pack2(b.x, b.y); CF[3] = pack2(b.z, b.w);
     }
     center<ST>(gq, MUON ? 0.0f : f.x, G);
+    f32x2 GM[4];   // MUON: the raw gradient, which the mask compares with
+    if constexpr (MUON) center<PT>(rq, f.x, GM);
     // ---- stored momentum ----
     float sc_old = 1.0f;
     if constexpr (MK == KAON_M_4BIT) sc_old = mq.sc;
     if constexpr (MK == KAON_M_INT8) sc_old = f.z;
     if constexpr (MK != KAON_M_NONE) mq.decode(sc_old, MO);
+    if (AHEAD && more) load(std::integral_constant<int, 1>{});
     if (MS && rem_here) {   // take the previous climb out (the mirrors get the step's last write only)
       f32x2 D[4];
       climb8(MO, hp.a_remove, hp.b_remove, CODED ? !(fabsf(sc_old) <= 3.0e38f) : true, D);
@@ -114,21 +129,27 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
       if (!APPLY && act) P.store(pp, nullptr);
     }
     // ---- u = ((g r) c) / div * scale (reference src/kaon/adakaon.py:885-888), m' = lerp(m, u) ----
+    // A COUNT that only counts takes r / div * scale as one factor (three roundings fewer); where codes, row maxima or a
+    // compensation come of u, the reference's order of roundings stays (an ulp moves codes, and with them the next scales)
     f32x2 MN[4], F[4];
-    const f32x2 RF = pack2(f.y, f.y);
+    const bool folded = !APPLY && MK != KAON_M_INT8 && !hp.kahan;
+    const f32x2 RF = folded ? pack2(f.w, f.w) : pack2(f.y, f.y);
 #pragma unroll
     for (int j = 0; j < 4; ++j) MN[j] = mul2(mul2(G[j], RF), CF[j]);
-    if (clipped) {
-      const f32x2 DIVN = pack2(-div, -div), RCPD = pack2(rcp_div, rcp_div);
+    if (!folded) {
+      if (clipped) {
+        const f32x2 DIVN = pack2(-div, -div), RCPD = pack2(rcp_div, rcp_div);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const f32x2 qq = mul2(MN[j], RCPD);
-        MN[j] = fma2(fma2(qq, DIVN, MN[j]), RCPD, qq);
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 qq = mul2(MN[j], RCPD);
+          MN[j] = fma2(fma2(qq, DIVN, MN[j]), RCPD, qq);
+        }
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) MN[j] = mul2(MN[j], pack2(hp.upd_scale, hp.upd_scale));
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      MN[j] = mul2(MN[j], pack2(hp.upd_scale, hp.upd_scale));
       if constexpr (MK == KAON_M_BF16) {
         const uint32_t ub = pack_bf16_rn(MN[j].x, MN[j].y);
         MN[j] = pack2(bf16lo(ub), bf16hi(ub));
@@ -153,25 +174,29 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
     // ---- delta = m' + (lr wd) p; the mask; APPLY: the update, negated: -(delta if kept else 0) / (kept / numel) ----
 #pragma unroll
     for (int j = 0; j < 4; ++j) F[j] = MN[j];
-    if (hp.has_wd && need_p) {
+    if (APPLY ? hp.has_wd != 0 : CP) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) F[j] = fma2(P.pair(j), pack2(hp.lrwd, hp.lrwd), F[j]);
-    }
-    if constexpr (MUON) {
-      W8<PT> rq;
-      rq.load(act ? rawp : gbase);
-      center<PT>(rq, f.x, G);
     }
     f32x2 K[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const f32x2 X = mul2(F[j], G[j]);
+      const f32x2 X = mul2(F[j], MUON ? GM[j] : G[j]);
       K[j] = pack2(gt0_or(X.x, hp.mask_off), gt0_or(X.y, hp.mask_off));
     }
     if constexpr (!APPLY) {
       if (act) kept2 = add2(kept2, add2(add2(K[0], K[1]), add2(K[2], K[3])));
       if constexpr (MK == KAON_M_INT8) {
         unsigned bits = act ? __float_as_uint(amax8(MN)) : 0u;
+        if (whole) {   // to the row's atomic when it ends
+          run = max(run, bits);
+          if (cv + adv_c >= nv || adv_r > 0 || !more) {
+            run = __reduce_max_sync(0xffffffffu, run);
+            if (lane == 0) atomicMax(rowmax + row, run);
+            run = 0u;
+          }
+          return;
+        }
         const int row_l0 = __shfl_sync(0xffffffffu, row, 0);
         if (__all_sync(0xffffffffu, !act || row == row_l0)) {
           bits = __reduce_max_sync(0xffffffffu, bits);
@@ -190,7 +215,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
       float sc = 1.0f;
       if constexpr (MK != KAON_M_NONE) {
         float amax = 0.0f;
-        if constexpr (MK == KAON_M_INT8) amax = __uint_as_float(__ldcg(rowmax + row));
+        if constexpr (MK == KAON_M_INT8) amax = __uint_as_float(OWN ? __ldcg(rowmax + row) : __ldg(rowmax + row));
         sc = store_m8<MK>(mp, MN, amax, act ? 8 : 0, lane, MS ? MO : nullptr);
         if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(msc, sc); }
         if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) msc[row] = sc; }
@@ -219,21 +244,15 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   const int left = nvec - (first - lane);                 // vectors from the warp's first on
   int full = left >= 32 ? (left - 32) / STRIDE + 1 : 0;   // trips of the whole warp
   const int tail = left - full * STRIDE;
+  const bool act = lane < tail;                           // in a tensor's last vectors
+  if (AHEAD && (full > 0 || act)) load(std::integral_constant<int, 0>{});
   for (; full > 0; --full) {
-    load();
-    trip(true);
+    trip(true, full > 1 || act);
     advance();
   }
-  if (tail > 0) {   // a tensor's last vectors
-    const bool act = lane < tail;
-    if (!act) {   // (in bounds, and of no consequence)
-      row = t.row0; cv = 0;
-      sp = sig; pp = reinterpret_cast<unsigned char*>(d.p);
-      if constexpr (MBITS > 0) mp = reinterpret_cast<unsigned char*>(d.m);
-      if constexpr (MK == KAON_M_4BIT) msc = d.m_scale;
-    }
-    load();
-    trip(act);
+  if (tail > 0) {
+    if (!act) { row = t.row0; cv = 0; }   // (in bounds; what such a lane computes is of no consequence)
+    trip(act, false);
   }
   if constexpr (!APPLY) {
     const unsigned kept = __reduce_add_sync(0xffffffffu, (unsigned)(kept2.x + kept2.y + 0.5f));
@@ -241,8 +260,10 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   }
 }
 
-template <typename PT, int MKP, bool MUON, bool MS, bool APPLY>
+template <typename PT, int MKP, bool MUON, bool MS, bool APPLY, bool CP>
 __global__ void __launch_bounds__(SWT, 4) ada_sweep_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+  early_launch();
+  after_launch_before();
   if (on_reserved_sm(pv.sm_reserve)) return;
   const int lane = threadIdx.x & 31;
   // The first unit is the warp's own number (with reserved multiprocessors, whose warps leave, a claimed one), the
@@ -262,7 +283,7 @@ __global__ void __launch_bounds__(SWT, 4) ada_sweep_kernel(const __grid_constant
     const int next = claim();
     const Task t = pv.tasks[cur];
     const unsigned char* gbase = reinterpret_cast<const unsigned char*>(pv.grads[t.tensor]);
-    if (gbase != nullptr) sweep_unit<PT, MKP, MUON, MS, APPLY, 32, false>(pv, hp, t, gbase, lane, lane);
+    if (gbase != nullptr) sweep_unit<PT, MKP, MUON, MS, APPLY, CP, 32, false>(pv, hp, t, gbase, lane, lane);
     cur = __shfl_sync(0xffffffffu, next, 0);
   }
 }
@@ -415,40 +436,42 @@ __global__ void __launch_bounds__(SWT, 4) ada_small_kernel(const __grid_constant
   for (int r = tid; r < R; r += SWT) {
     const float rf = rsqrt_torch(__fdiv_rn(d.stat_a[r], rowmean));
     rowtab[r].y = rf;
+    rowtab[r].w = __fmul_rn(rf, update_factor(hp, div));
     pv.aux[aux_rfac(d) + r] = rf;
   }
   if (hp.stats_only) return;
   __syncthreads();
   const Task t{ti, 0, 0, n, 0, 0, 0};
   if (hp.cautious || hp.int8) {
-    sweep_unit<PT, MKP, MUON, MS, false, SWT, true>(pv, hp, t, g, tid, lane);
+    if (hp.has_wd && hp.cautious) sweep_unit<PT, MKP, MUON, MS, false, true, SWT, true>(pv, hp, t, g, tid, lane);
+    else sweep_unit<PT, MKP, MUON, MS, false, false, SWT, true>(pv, hp, t, g, tid, lane);
     __threadfence_block();
     __syncthreads();
   }
-  sweep_unit<PT, MKP, MUON, MS, true, SWT, true>(pv, hp, t, g, tid, lane);
+  sweep_unit<PT, MKP, MUON, MS, true, false, SWT, true>(pv, hp, t, g, tid, lane);
 }
 
 // ----------------------------------------------------------------------------- host
 
 typedef void (*SweepKernel)(PlanView, AdaDev);
 
-template <typename PT, bool MS, bool APPLY>
+template <typename PT, bool MS, bool APPLY, bool CP>
 static SweepKernel pick_sweep_pt(int mk) {
   switch (mk) {
-    case KAON_M_F32: return ada_sweep_kernel<PT, KAON_M_F32, false, MS, APPLY>;
-    case KAON_M_BF16: return ada_sweep_kernel<PT, KAON_M_BF16, false, MS, APPLY>;
-    case KAON_M_INT8: return ada_sweep_kernel<PT, KAON_M_INT8, false, MS, APPLY>;
-    case KAON_M_4BIT: return ada_sweep_kernel<PT, KAON_M_4BIT, false, MS, APPLY>;
-    case KAON_M_NONE: return ada_sweep_kernel<PT, KAON_M_NONE, false, false, APPLY>;
+    case KAON_M_F32: return ada_sweep_kernel<PT, KAON_M_F32, false, MS, APPLY, CP>;
+    case KAON_M_BF16: return ada_sweep_kernel<PT, KAON_M_BF16, false, MS, APPLY, CP>;
+    case KAON_M_INT8: return ada_sweep_kernel<PT, KAON_M_INT8, false, MS, APPLY, CP>;
+    case KAON_M_4BIT: return ada_sweep_kernel<PT, KAON_M_4BIT, false, MS, APPLY, CP>;
+    case KAON_M_NONE: return ada_sweep_kernel<PT, KAON_M_NONE, false, false, APPLY, CP>;
     default: return nullptr;
   }
 }
-template <bool APPLY>
+template <bool APPLY, bool CP>
 static SweepKernel pick_sweep(int pdt, int mk, bool muon, bool ms) {
   const bool bf = pdt == KAON_DT_BF16;
-  if (muon) return bf ? ada_sweep_kernel<__nv_bfloat16, KAON_M_NONE, true, false, APPLY> : ada_sweep_kernel<float, KAON_M_NONE, true, false, APPLY>;
-  if (ms) return bf ? pick_sweep_pt<__nv_bfloat16, true, APPLY>(mk) : pick_sweep_pt<float, true, APPLY>(mk);
-  return bf ? pick_sweep_pt<__nv_bfloat16, false, APPLY>(mk) : pick_sweep_pt<float, false, APPLY>(mk);
+  if (muon) return bf ? ada_sweep_kernel<__nv_bfloat16, KAON_M_NONE, true, false, APPLY, CP> : ada_sweep_kernel<float, KAON_M_NONE, true, false, APPLY, CP>;
+  if (ms) return bf ? pick_sweep_pt<__nv_bfloat16, true, APPLY, CP>(mk) : pick_sweep_pt<float, true, APPLY, CP>(mk);
+  return bf ? pick_sweep_pt<__nv_bfloat16, false, APPLY, CP>(mk) : pick_sweep_pt<float, false, APPLY, CP>(mk);
 }
 
 typedef void (*SmallKernel)(PlanView, AdaDev);
@@ -515,13 +538,13 @@ int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cu
   const int grid = base.sm_reserve ? most : std::max(1, std::min(want, most));
   if (hp.cautious || hp.int8) {
     va.task_counter = base.counters2 + 1;
-    pick_sweep<false>(pl->param_dtype, pl->momentum_kind, muon, ms)<<<grid, SWT, 0, s>>>(va, hp);
-    KAON_CUDA(cudaGetLastError());
+    SweepKernel k = hp.has_wd && hp.cautious ? pick_sweep<false, true>(pl->param_dtype, pl->momentum_kind, muon, ms)
+                                             : pick_sweep<false, false>(pl->param_dtype, pl->momentum_kind, muon, false);
+    KAON_CUDA(launch_early(k, grid, SWT, s, va, hp));
     pl->launches += 1;
   }
   va.task_counter = base.counters2 + 2;
-  pick_sweep<true>(pl->param_dtype, pl->momentum_kind, muon, ms)<<<grid, SWT, 0, s>>>(va, hp);
-  KAON_CUDA(cudaGetLastError());
+  KAON_CUDA(launch_early(pick_sweep<true, false>(pl->param_dtype, pl->momentum_kind, muon, ms), grid, SWT, s, va, hp));
   pl->launches += 1;
   return KAON_OK;
 }

@@ -18,6 +18,7 @@
 // leave it: COUNT and APPLY run as launches of their own (ada_sweep.cu), STATS of bf16 rows of at least 256
 // elements too (ada_stats_kernel below; other such rows stream through ada_stats_stream here), and tensors of at most
 // ADA_SMALL_MAX elements are stepped whole by one CTA each (ada_small_kernel).
+#include <algorithm>
 #include <map>
 #include <vector>
 #include <mutex>
@@ -25,6 +26,7 @@
 #include <type_traits>
 
 #include "adakaon_dev.h"
+#include "kaon_elem.cuh"
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
 #include "kaon_packed.cuh"
@@ -656,6 +658,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
   __shared__ double red[STT / 32];
   __shared__ int next_s[2];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  early_launch();
   if (on_reserved_sm(pv.sm_reserve)) return;
   auto claim_next = [&](int slot) {
     if (tid == 0) {
@@ -679,14 +682,21 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
     const bool ok = g != nullptr;
     const int C = d.cols, nv = C >> 3, nrows = t.n / C;
     double rowsum = 0.0;
+    float *stat = d.stat_a + t.row0, *mean = pv.aux + aux_mean(d) + t.row0;
+    const bool plain = d.shift != nullptr;
+    const float fC = (float)C, rC = __frcp_rn(fC);
     const uint4* gitem = reinterpret_cast<const uint4*>(g + (ok ? t.e0 * 2 : 0));
+    // a run of rows on its way to L2 while the one before it is worked on
+    auto ahead = [&](int ra, int rb) {
+      if (tid == 0 && ra < rb)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gitem + (size_t)ra * nv), "r"((unsigned)(rb - ra) * (unsigned)nv * 16u) : "memory");
+    };
     float* slot = pv.aux + d.aux_off + 2ll * t.slot * C;
     // row statistics of rows [ra, rb) of the item, one warp per row
     auto rows_phase = [&](const int ra, const int rb) {
       for (int r = ra + warp; r < rb; r += STT / 32) {
         const uint4* rowq = gitem + (size_t)r * nv;
-        const int row = t.row0 + r;
-        const float old = d.stat_a[row];
+        const float old = stat[r];
         float mu = 0.0f;
         if (gc) {
           f32x2 a0 = pack2(0.0f, 0.0f), a1 = pack2(0.0f, 0.0f);
@@ -703,13 +713,12 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
             a0 = add2(a0, add2(pairs(q0.x), pairs(q0.y)));
             a1 = add2(a1, add2(pairs(q0.z), pairs(q0.w)));
           }
-          mu = round_bf16(__fdiv_rn(warp_sum_d((a0.x + a0.y) + (a1.x + a1.y), d.shift != nullptr), (float)C));
+          mu = round_bf16(div_by(warp_sum_d((a0.x + a0.y) + (a1.x + a1.y), plain), fC, rC));
         }
         const uint32_t mu2 = pack_bf16_rn(mu, mu);
         auto sq2 = [&](uint32_t w) {
           const f32x2 y = pairs(gc ? sub_bf16x2(w, mu2) : w);
-          const f32x2 q = mul2(y, y);
-          return hp.has_eps ? add2(q, EPS) : q;
+          return fma2(y, y, EPS);   // (the square is exact: one rounding either way)
         };
         f32x2 b0 = pack2(0.0f, 0.0f), b1 = pack2(0.0f, 0.0f);
         int v = lane;
@@ -725,12 +734,12 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
           b0 = add2(b0, add2(sq2(q0.x), sq2(q0.y)));
           b1 = add2(b1, add2(sq2(q0.z), sq2(q0.w)));
         }
-        const float s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y), d.shift != nullptr);
+        const float s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y), plain);
         if (lane == 0) {
-          const float rn = lerp_torch(old, __fdiv_rn(s2, (float)C), hp.w2, hp.w2m1, hp.small_w2 != 0);
-          d.stat_a[row] = rn;
+          const float rn = lerp_torch(old, div_by(s2, fC, rC), hp.w2, hp.w2m1, hp.small_w2 != 0);
+          stat[r] = rn;
           mean2_s[r] = mu2;
-          if (gc) pv.aux[aux_mean(d) + row] = mu;
+          if (gc) mean[r] = mu;
           rinv_s[r] = __fdiv_rn(1.0f, rn);
           rowsum += (double)rn;
         }
@@ -745,7 +754,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
       for (int w = 0; w < 4; ++w) {
         const f32x2 y = pairs(gc ? sub_bf16x2(ww[w], mu2) : ww[w]);
         const f32x2 sq = mul2(y, y);
-        A1[w] = add2(A1[w], hp.has_eps ? add2(sq, EPS) : sq);
+        A1[w] = add2(A1[w], fma2(y, y, EPS));
         A2[w] = add2(A2[w], mul2(sq, RI));
       }
     };
@@ -762,6 +771,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
       for (int w = 0; w < 4; ++w) { A1[w] = pack2(0.0f, 0.0f); A2[w] = pack2(0.0f, 0.0f); }
       for (int ra = 0; ra < nrows; ra += sg) {
         const int rb = min(nrows, ra + sg);
+        ahead(rb, min(nrows, rb + sg));
         rows_phase(ra, rb);
         __syncthreads();
         if (q < Q) {
@@ -846,6 +856,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
     slot_i ^= 1;
     cur = next_s[slot_i];
   }
+  after_launch_before();   // (what follows this launch may rely on the one beside it, too)
 }
 
 // ----------------------------------------------------------------------------- FINAL
@@ -912,18 +923,19 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
       scal[2] = rms;
       scal[3] = __fdiv_rn(1.0f, scal[1]);
       sm.part_s[0] = rowmean;
+      sm.part_s[1] = update_factor(hp, scal[1]);
     }
   }
   last = __syncthreads_or(last);
   if (last) {  // the whole CTA: r_i of every row, then release COUNT / APPLY
-    const float rowmean = sm.part_s[0];
+    const float rowmean = sm.part_s[0], uf = sm.part_s[1];
     float* rfac = pv.aux + aux_rfac(d);
     float4* rowtab = reinterpret_cast<float4*>(pv.aux + aux_rowtab(d));
     for (int r = tid; r < d.rows; r += AT) {
       const float rf = rsqrt_torch(__fdiv_rn(__ldcg(d.stat_a + r), rowmean));
       rfac[r] = rf;
       const float mu = hp.gc ? __ldcg(pv.aux + aux_mean(d) + r) : 0.0f;
-      rowtab[r] = make_float4(pv.param_bf16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, rf, hp.int8 ? d.m_scale[r] : 1.0f, 0.0f);
+      rowtab[r] = make_float4(pv.param_bf16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, rf, hp.int8 ? d.m_scale[r] : 1.0f, __fmul_rn(rf, uf));
     }
     if (hp.int8) {  // int8 momentum: COUNT starts from zeroed row maxima; APPLY decodes with the old scales
       unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
@@ -1575,6 +1587,7 @@ __global__ void __launch_bounds__(AT, 1) adakaon_kernel(PlanView pv, AdaDev hp, 
   // COUNT/APPLY/FLAT put cfac / the flat buffer after them.
   AdaSmem sm_stats{mean_s, rfac_s, rowmax_s, scale_s, reinterpret_cast<float*>(mbase), red, part_s};
   AdaSmem sm_rows{mean_s, rfac_s, rowmax_s, scale_s, reinterpret_cast<float*>(mbase + (size_t)nbuf * mcap), red, part_s};
+  early_launch();
   if (on_reserved_sm(pv.sm_reserve)) return;
   auto claim_next = [&](int slot) {
     if (tid == 0) {
@@ -1772,15 +1785,22 @@ int ensure_apply2(kaon_plan* pl) {
   sweep_units(pl, elig, items);
   // the persistent kernel's lists and the STATS launch's
   const bool stats_dtype = muon || pl->param_dtype == KAON_DT_BF16;
-  std::vector<Task> stats;
+  std::vector<Task> stats, strips;
+  // FINAL leaves with STATS, unless stages that stay wait for it
+  std::vector<char> leaves((size_t)pl->n_tensors, 0);
+  bool flat_only[2] = {false, false};
   pl->long_rows_ok = true;
   for (int variant = 0; variant < 2; ++variant) {   // 0: from the list without COUNT items; 1: from the full list
     const Task* src = variant ? pl->d_tasks_full : pl->d_tasks_main;
     const int ns = variant ? pl->n_tasks_full : pl->n_tasks_main;
     std::vector<Task> h((size_t)ns), keep;
     KAON_CUDA(cudaMemcpy(h.data(), src, sizeof(Task) * h.size(), cudaMemcpyDeviceToHost));
+    if (variant == 0)
+      for (const Task& t : h)
+        if (t.phase == PH_ADA_STATS && stats_dtype && elig[t.tensor] && stats_item_ok(pl, t)) leaves[t.tensor] = 1;
     for (const Task& t : h) {
       const bool el = elig[t.tensor] != 0;
+      if (t.phase == PH_ADA_FINAL && leaves[t.tensor]) continue;
       if ((t.phase == PH_ADA_APPLY || t.phase == PH_ADA_COUNT) && el) continue;
       if (t.phase == PH_ADA_STATS && stats_dtype && stats_item_ok(pl, t)) {
         if (variant == 0) stats.push_back(t);
@@ -1793,12 +1813,27 @@ int ensure_apply2(kaon_plan* pl) {
     KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_na[variant], sizeof(Task) * std::max<size_t>(keep.size(), 1)));
     KAON_CUDA(cudaMemcpy(pl->d_tasks_na[variant], keep.data(), sizeof(Task) * keep.size(), cudaMemcpyHostToDevice));
     pl->n_tasks_na[variant] = (int)keep.size();
+    flat_only[variant] = std::all_of(keep.begin(), keep.end(), [](const Task& t) { return t.phase == PH_ADA_FLAT; });
     pl->device_bytes += (int64_t)(sizeof(Task) * keep.size());
+  }
+  // The persistent kernel's short lists run beside STATS: a few 1-D tensors, or any list where both launches find room.  (Its
+  // blocks fill a multiprocessor each: beside a STATS that needs the whole machine, a list with stages that wait for one
+  // another cost 40 us more than the two in turn, and the 540 1-D tensors of the 2.6 B list gained nothing.)
+  for (int variant = 0; variant < 2; ++variant) {
+    const int n = pl->n_tasks_na[variant];
+    pl->na_beside[variant] = n > 0 && n <= pl->sm_count / 2 && (flat_only[variant] || n + (int)stats.size() / 4 <= pl->sm_count);
   }
   if (!stats.empty()) {
     KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_stats, sizeof(Task) * stats.size()));
     KAON_CUDA(cudaMemcpy(pl->d_tasks_stats, stats.data(), sizeof(Task) * stats.size(), cudaMemcpyHostToDevice));
     pl->n_tasks_stats = (int)stats.size();
+    final_items(pl, leaves, strips, pl->n_tasks_strips);
+    if (!strips.empty()) {
+      KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_final, sizeof(Task) * strips.size()));
+      KAON_CUDA(cudaMemcpy(pl->d_tasks_final, strips.data(), sizeof(Task) * strips.size(), cudaMemcpyHostToDevice));
+      pl->n_tasks_final = (int)strips.size();
+      pl->device_bytes += (int64_t)(sizeof(Task) * strips.size());
+    }
     pl->device_bytes += (int64_t)(sizeof(Task) * stats.size());
   }
   KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_apply2, sizeof(Task) * items.size()));
@@ -1821,30 +1856,25 @@ int launch_persistent(kaon_plan* pl, const PlanView& v, const AdaDev& hp, cudaSt
   return KAON_OK;
 }
 
-// STATS as a launch of its own over the plan's qualifying STATS items (the persistent kernel's lists
-// do not hold them); KAON_OK also when there are none.
-int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s) {
-  if (pl->n_tasks_stats == 0) return KAON_OK;
-  return launch_stats_tasks(pl, base, hp, pl->d_tasks_stats, pl->n_tasks_stats, s);
-}
-
 bool stats_item_ok(const kaon_plan* pl, const Task& t) {
   const DevTensor& dt = pl->h_tensors[t.tensor];
   return dt.cols >= 256 && (dt.cols & 7) == 0 && t.n / dt.cols <= ST_MAXROWS && (dt.aux_off & 3) == 0;
 }
 
-int launch_stats_tasks(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* tasks, int n, cudaStream_t s) {
+int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* tasks, int n, bool beside, cudaStream_t s) {
+  if (n == 0) return KAON_OK;
   if (pl->stats_grid == 0) {
     int per_sm = 0;
     KAON_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)ada_stats_kernel, STT, 0));
     pl->stats_grid = pl->sm_count * std::max(per_sm, 1);
   }
-  PlanView vs = base;
-  vs.tasks = tasks;
-  vs.n_tasks = n;
-  vs.task_counter = base.counters2;
-  if (n == 0) return KAON_OK;
-  ada_stats_kernel<<<base.sm_reserve ? pl->stats_grid : std::min(pl->stats_grid, n), STT, 0, s>>>(vs, hp);
+  PlanView v = base;
+  v.tasks = tasks;
+  v.n_tasks = n;
+  v.task_counter = base.counters2;
+  const int grid = v.sm_reserve ? pl->stats_grid : std::min(pl->stats_grid, n);
+  if (beside) KAON_CUDA(launch_early(ada_stats_kernel, grid, STT, s, v, hp));
+  else ada_stats_kernel<<<grid, STT, 0, s>>>(v, hp);
   KAON_CUDA(cudaGetLastError());
   pl->launches += 1;
   return KAON_OK;
@@ -1899,9 +1929,11 @@ extern "C" int kaon_adakaon_step(kaon_plan* pl, const kaon_adakaon_hparams* h, u
   else if (hp.cautious) { v.tasks = pl->d_tasks_full; v.n_tasks = pl->n_tasks_full; }
   else { v.tasks = pl->d_tasks_main; v.n_tasks = pl->n_tasks_main; }
   KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-  if (two)
-    if (int rc = launch_stats(pl, pl->view, hp, s)) return rc;
   if (int rc = launch_persistent(pl, v, hp, s)) return rc;
+  if (two) {
+    if (int rc = launch_stats(pl, pl->view, hp, pl->d_tasks_stats, pl->n_tasks_stats, pl->na_beside[hp.cautious ? 1 : 0], s)) return rc;
+    if (int rc = launch_final(pl, pl->view, hp, pl->d_tasks_final, pl->n_tasks_strips, pl->n_tasks_final, s)) return rc;
+  }
   if (int rc = launch_small(pl, pl->view, hp, s)) return rc;
   if (two) {
     if (int rc = launch_count_apply(pl, pl->view, hp, s)) return rc;

@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "kaon_device.cuh"
 #include "kaon_plan.h"
 
@@ -34,15 +36,23 @@ inline void ada_finish(AdaDev& hp) {
   hp.mask_off = !hp.cautious;
 }
 
+#ifdef __CUDACC__
+// what r_i is multiplied by for a COUNT that takes the clip divisor and the step's scale with it
+__device__ __forceinline__ float update_factor(const AdaDev& hp, float div) { return (float)((double)hp.upd_scale / (double)div); }
+#endif
+
 int launch_persistent(kaon_plan* pl, const PlanView& v, const AdaDev& hp, cudaStream_t s);
 // COUNT and APPLY as launches of their own (ada_sweep.cu), for the factored tensors whose rows stream
 void sweep_units(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out);
 int ensure_apply2(kaon_plan* pl);
 int launch_small(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
 int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
-int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
-// the STATS launch over a caller's list of STATS items (all of which pass stats_item_ok); KAON_OK or an error
+// the STATS launch over a caller's list of STATS items (all of which pass stats_item_ok); `beside`: the launch before it on the
+// stream is the persistent kernel's, and the two may run at the same time
 bool stats_item_ok(const kaon_plan* pl, const Task& t);
-int launch_stats_tasks(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* tasks, int n, cudaStream_t s);
+int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* tasks, int n, bool beside, cudaStream_t s);
+// FINAL as launches of its own (ada_final.cu)
+void final_items(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out, int& n_strips);
+int launch_final(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* items, int n_strips, int n, cudaStream_t s);
 
 }  // namespace kaon

@@ -622,9 +622,10 @@ __global__ void __launch_bounds__(PT_THREADS) pnm_flat_kernel(PlanView pv, PnmDe
 struct PnmHost {
   PnmView view{};
   void* block = nullptr;
-  Task* d_stats = nullptr;   // STATS items the small-CTA launch takes, or null
+  Task* d_stats = nullptr;   // STATS items the launch of its own takes
   Task* d_final = nullptr;   // the other STATS items and the FINAL items, for the persistent kernel
-  int n_stats = 0, n_final = 0;
+  Task* d_strips = nullptr;  // and their FINAL strips and row-table runs
+  int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0;
   bool attached = false;
   int64_t bytes = 0;
 };
@@ -676,7 +677,7 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   PnmHost* h = new PnmHost();
   pl->pnm = h;
   const int n = pl->n_tensors;
-  std::vector<Task> units, items, stats, fin;
+  std::vector<Task> units, items, stats, strips, fin;
   int slots = 0;
   std::vector<int> begin(n + 1, 0), fact, flat;
   std::vector<PnmBufs> bufs(n);
@@ -708,20 +709,22 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   begin[n] = slots;
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
+    std::vector<char> leaves(n, 0);   // tensors whose STATS and FINAL are launches of their own
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
     // STATS items the small-CTA launch can take go there, the others stay with FINAL in the persistent
     // kernel (which stages whole rows, so it cannot take rows longer than a work item)
     const bool bf16 = pl->param_dtype == KAON_DT_BF16;
     for (const Task& t : hm) {
       if (t.phase == PH_ADA_STATS) {
-        if (bf16 && stats_item_ok(pl, t)) stats.push_back(t);
+        if (bf16 && stats_item_ok(pl, t)) { stats.push_back(t); leaves[t.tensor] = 1; }
         else if (pl->h_tensors[t.tensor].cols > CAP)
           return fail(KAON_E_UNSUPPORTED, "AdaPNM: tensor %d: rows longer than %d elements need bf16 weights and a row length that is a multiple of 8", t.tensor, CAP);
         else fin.push_back(t);
-      } else if (t.phase == PH_ADA_FINAL) {
+      } else if (t.phase == PH_ADA_FINAL && !leaves[t.tensor]) {
         fin.push_back(t);
       }
     }
+    final_items(pl, leaves, strips, h->n_strips);
   }
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   size_t o = 0;
@@ -730,7 +733,7 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   const size_t o_bufs = take(sizeof(PnmBufs) * n), o_part = take(sizeof(double) * slots);
   const size_t o_kpart = take(sizeof(unsigned) * slots), o_scal = take(sizeof(float) * 2 * n);
   const size_t o_fact = take(sizeof(int) * fact.size()), o_flat = take(sizeof(int) * flat.size());
-  const size_t o_stats = take(sizeof(Task) * stats.size());
+  const size_t o_strips = take(sizeof(Task) * strips.size()), o_stats = take(sizeof(Task) * stats.size());
   const size_t o_fin = take(sizeof(Task) * fin.size());
   KAON_CUDA(cudaMalloc(&h->block, std::max<size_t>(o, 256)));
   unsigned char* base = reinterpret_cast<unsigned char*>(h->block);
@@ -744,6 +747,7 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   KAON_CUDA(put(o_bufs, bufs.data(), sizeof(PnmBufs) * n));
   KAON_CUDA(put(o_fact, fact.data(), sizeof(int) * fact.size()));
   KAON_CUDA(put(o_flat, flat.data(), sizeof(int) * flat.size()));
+  KAON_CUDA(put(o_strips, strips.data(), sizeof(Task) * strips.size()));
   KAON_CUDA(put(o_stats, stats.data(), sizeof(Task) * stats.size()));
   KAON_CUDA(put(o_fin, fin.data(), sizeof(Task) * fin.size()));
   KAON_CUDA(cudaMemset(base + o_scal, 0, sizeof(float) * 2 * n));
@@ -757,7 +761,8 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   x.scal = reinterpret_cast<float*>(base + o_scal);
   x.fact = reinterpret_cast<const int*>(base + o_fact); x.n_fact = (int)fact.size();
   x.flat = reinterpret_cast<const int*>(base + o_flat); x.n_flat = (int)flat.size();
-  h->d_stats = stats.empty() ? nullptr : reinterpret_cast<Task*>(base + o_stats); h->n_stats = (int)stats.size();
+  h->d_stats = reinterpret_cast<Task*>(base + o_stats); h->n_stats = (int)stats.size();
+  h->d_strips = reinterpret_cast<Task*>(base + o_strips); h->n_final_items = (int)strips.size();
   h->d_final = reinterpret_cast<Task*>(base + o_fin); h->n_final = (int)fin.size();
   h->attached = true;
   pl->device_bytes += h->bytes;
@@ -823,10 +828,10 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
     ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-    if (ph->d_stats != nullptr)
-      if (int rc = launch_stats_tasks(pl, pl->view, ad, ph->d_stats, ph->n_stats, s)) return rc;
     v.tasks = ph->d_final; v.n_tasks = ph->n_final;
     if (int rc = launch_persistent(pl, v, ad, s)) return rc;
+    if (int rc = launch_stats(pl, pl->view, ad, ph->d_stats, ph->n_stats, false, s)) return rc;
+    if (int rc = launch_final(pl, pl->view, ad, ph->d_strips, ph->n_strips, ph->n_final_items, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
     // 2-4. the two sweeps over the flat items
     const int grid = std::min(x.n_items, pl->sm_count * 8);

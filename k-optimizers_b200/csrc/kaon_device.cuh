@@ -136,6 +136,13 @@ __device__ __forceinline__ void kahan_step(float& p, float& shift, float d) {
   p = pn;
 }
 
+// ----------------------------------------------------------------------------- launches that overlap
+
+// Lets a launch_early launch after this one begin once every block of this one has come here (or left).
+__device__ __forceinline__ void early_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
+// The launch before this one on the stream has completed and its writes are visible (at once where it was launched without).
+__device__ __forceinline__ void after_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------- warp helpers
 
 __device__ __forceinline__ float warp_sum(float v) {

@@ -24,4 +24,21 @@ int check_device(const kaon_plan* pl);
     if (e__ != cudaSuccess) return ::kaon::cuda_fail(e__, #call);    \
   } while (0)
 
+// A launch that may begin while the launch before it on the stream drains (programmatic stream serialization): the kernel calls
+// after_launch_before() ahead of the first access to what that launch writes, or, where the two have nothing to do with
+// each other, at its end.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), int grid, int block, cudaStream_t s, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace kaon

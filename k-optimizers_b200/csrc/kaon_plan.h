@@ -56,7 +56,7 @@ struct DevTensor {
   int n_count;          // COUNT items
   long long aux_off;    // float index of this tensor's scratch in `aux`:
                         //   colpart[n_stats][2][cols] | cfac[cols] | rowpart[n_stats] (double) |
-                        //   tpart[n_strips] (double) | scal[4] = {rowmean, divisor, rms, 1 / divisor} | rowmax[rows] | mean[rows]
+                        //   tpart[ceil(cols / 128)] (double) | scal[4] = {rowmean, divisor, rms, 1 / divisor} | rowmax[rows] | mean[rows]
   void* shift;          // Kahan compensation buffer (bf16 [numel]) or null
 };
 
@@ -68,7 +68,7 @@ __host__ __device__ inline int blk_lanes(const DevTensor& d) { return d.bshift >
 __host__ __device__ inline long long aux_cfac(const DevTensor& d) { return d.aux_off + 2ll * d.n_stats * d.cols; }
 __host__ __device__ inline long long aux_rowpart(const DevTensor& d) { return (aux_cfac(d) + d.cols + 1) / 2 * 2; }
 __host__ __device__ inline long long aux_tpart(const DevTensor& d) { return aux_rowpart(d) + 2ll * d.n_stats; }
-__host__ __device__ inline long long aux_scal(const DevTensor& d) { return (aux_tpart(d) + 2ll * d.n_strips + 3) / 4 * 4; }
+__host__ __device__ inline long long aux_scal(const DevTensor& d) { return (aux_tpart(d) + 2ll * ((d.cols + 127) / 128) + 3) / 4 * 4; }
 // int8 momentum: bits of each row's absmax of the new momentum, left by COUNT for APPLY
 __host__ __device__ inline long long aux_rowmax(const DevTensor& d) { return aux_scal(d) + 4; }
 // centralization mean of every row, left by STATS for COUNT / APPLY
@@ -80,7 +80,7 @@ __host__ __device__ inline long long aux_rfac(const DevTensor& d) { return aux_o
 // scratch of a 1-D tensor stepped from global memory: 8 floats | n floats (padded) | one word per 4-bit block (>= 32 elements)
 __host__ __device__ inline long long flat_long_pad(long long n) { return (n + 63) / 64 * 64; }
 __host__ __device__ inline long long flat_long_size(long long n) { return 8 + flat_long_pad(n) + ((n + 31) / 32 + 1 + 63) / 64 * 64; }
-// {mean (bf16 weights: two bf16 copies), r_i, int8: old scale, -} of every row, for COUNT / APPLY (16-byte aligned)
+// {mean (bf16 weights: two bf16 copies), r_i, int8: old scale, r_i / clip divisor * update scale} of every row, for COUNT / APPLY (16-byte aligned)
 __host__ __device__ inline long long aux_rowtab(const DevTensor& d) { return (aux_rfac(d) + d.rows + 3) / 4 * 4; }
 __host__ __device__ inline long long aux_size(const DevTensor& d) { return aux_rowtab(d) + 4ll * d.rows - d.aux_off; }
 
@@ -167,12 +167,15 @@ struct kaon_plan {
   // the persistent kernel's lists beside those launches: [0] without COUNT items, [1] with them
   kaon::Task* d_tasks_na[2] = {nullptr, nullptr};
   int n_tasks_na[2] = {0, 0};
+  bool na_beside[2] = {false, false};        // the list may run beside the STATS launch
   bool long_rows_ok = false;                 // every tensor whose rows exceed a work item left the persistent kernel
   kaon::Task* d_tasks_small = nullptr;       // factored tensors one CTA steps on its own
   int n_tasks_small = 0, small_max = 0;      // and the elements of the largest
   // STATS as a launch of its own: the STATS items that qualify
   kaon::Task* d_tasks_stats = nullptr;
   int n_tasks_stats = 0, stats_grid = 0;
+  kaon::Task* d_tasks_final = nullptr;       // the FINAL launch's strips of those tensors, then the row-table launch's runs
+  int n_tasks_final = 0, n_tasks_strips = 0;
   unsigned* d_counters = nullptr;  // task_counter, status, done[n], kept[n] (contiguous; memset per step)
   size_t counters_bytes = 0;
   int64_t device_bytes = 0;

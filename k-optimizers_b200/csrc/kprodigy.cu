@@ -610,9 +610,10 @@ __global__ void __launch_bounds__(KP_THREADS) kp_reduce_kernel(PlanView pv, KpVi
 struct KpHost {
   KpView view{};
   void* block = nullptr;
-  Task* d_stats = nullptr;
+  Task* d_stats = nullptr;   // STATS items the launch of its own takes
   Task* d_final = nullptr;
-  int n_stats = 0, n_final = 0;
+  Task* d_strips = nullptr;  // and their FINAL strips and row-table runs
+  int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0;
   long long slice_p = 1;
   std::vector<float> h_sums;
   int64_t bytes = 0;
@@ -676,7 +677,7 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   pl->kp = h;
   h->slice_p = slice_p;
   const int n = pl->n_tensors;
-  std::vector<Task> units, items, rows, stats, fin;
+  std::vector<Task> units, items, rows, stats, strips, fin;
   std::vector<int> begin(n + 1, 0);
   int slots = 0;
   std::vector<KpBufs> bufs(n);
@@ -712,16 +713,18 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   begin[n] = slots;
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
+    std::vector<char> leaves(n, 0);   // tensors whose STATS and FINAL are launches of their own
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
     const bool bf16 = pl->param_dtype == KAON_DT_BF16;
     for (const Task& t : hm) {
       if (t.phase == PH_ADA_STATS) {
-        if (bf16 && stats_item_ok(pl, t)) stats.push_back(t);
+        if (bf16 && stats_item_ok(pl, t)) { stats.push_back(t); leaves[t.tensor] = 1; }
         else fin.push_back(t);
-      } else if (t.phase == PH_ADA_FINAL) {
+      } else if (t.phase == PH_ADA_FINAL && !leaves[t.tensor]) {
         fin.push_back(t);
       }
     }
+    final_items(pl, leaves, strips, h->n_strips);
   }
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   size_t o = 0;
@@ -730,7 +733,7 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   const size_t o_bufs = take(sizeof(KpBufs) * n), o_part = take(sizeof(double) * 2 * slots);
   const size_t o_sums = take(sizeof(float) * 2 * n), o_tmax = take(sizeof(unsigned) * n), o_told = take(sizeof(float) * n);
   const size_t o_rows = take(sizeof(Task) * rows.size());
-  const size_t o_stats = take(sizeof(Task) * stats.size()), o_fin = take(sizeof(Task) * fin.size());
+  const size_t o_strips = take(sizeof(Task) * strips.size()), o_stats = take(sizeof(Task) * stats.size()), o_fin = take(sizeof(Task) * fin.size());
   KAON_CUDA(cudaMalloc(&h->block, std::max<size_t>(o, 256)));
   unsigned char* base = reinterpret_cast<unsigned char*>(h->block);
   KAON_CUDA(cudaMemset(base, 0, std::max<size_t>(o, 256)));
@@ -743,6 +746,7 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   KAON_CUDA(put(o_bufs, bufs.data(), sizeof(KpBufs) * n));
   KAON_CUDA(put(o_units, units.data(), sizeof(Task) * units.size()));
   KAON_CUDA(put(o_rows, rows.data(), sizeof(Task) * rows.size()));
+  KAON_CUDA(put(o_strips, strips.data(), sizeof(Task) * strips.size()));
   KAON_CUDA(put(o_stats, stats.data(), sizeof(Task) * stats.size()));
   KAON_CUDA(put(o_fin, fin.data(), sizeof(Task) * fin.size()));
   KpView& x = h->view;
@@ -755,7 +759,8 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   x.tmax = reinterpret_cast<unsigned*>(base + o_tmax);
   x.told = reinterpret_cast<float*>(base + o_told);
   x.row_units = reinterpret_cast<const Task*>(base + o_rows); x.n_row_units = (int)rows.size();
-  h->d_stats = stats.empty() ? nullptr : reinterpret_cast<Task*>(base + o_stats); h->n_stats = (int)stats.size();
+  h->d_stats = reinterpret_cast<Task*>(base + o_stats); h->n_stats = (int)stats.size();
+  h->d_strips = reinterpret_cast<Task*>(base + o_strips); h->n_final_items = (int)strips.size();
   h->d_final = reinterpret_cast<Task*>(base + o_fin); h->n_final = (int)fin.size();
   h->h_sums.assign((size_t)2 * n, 0.0f);
   pl->device_bytes += h->bytes;
@@ -805,10 +810,10 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
     ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-    if (kh->d_stats != nullptr)
-      if (int rc = launch_stats_tasks(pl, pl->view, ad, kh->d_stats, kh->n_stats, s)) return rc;
     v.tasks = kh->d_final; v.n_tasks = kh->n_final;
     if (int rc = launch_persistent(pl, v, ad, s)) return rc;
+    if (int rc = launch_stats(pl, pl->view, ad, kh->d_stats, kh->n_stats, false, s)) return rc;
+    if (int rc = launch_final(pl, pl->view, ad, kh->d_strips, kh->n_strips, kh->n_final_items, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
   } else if (hp.gc && x.n_row_units > 0) {
     const int grid = std::min((x.n_row_units + KP_THREADS / 32 - 1) / (KP_THREADS / 32), pl->sm_count * 8);

@@ -417,6 +417,7 @@ int kaon_plan_destroy(kaon_plan* pl) {
   cudaFree(pl->d_tasks_na[0]);
   cudaFree(pl->d_tasks_na[1]);
   cudaFree(pl->d_tasks_stats);
+  cudaFree(pl->d_tasks_final);
   cudaFree((void*)pl->d_signal);
   if (pl->muon_lanes_ready) {
     for (int l = 0; l < 4; ++l) {

@@ -1,0 +1,72 @@
+"""FINAL as launches of its own, at the edges of its strips (128 columns) and of the row table's runs (256 rows): one strip
+exactly two wide, a last strip of eight columns, one row beyond a run, fewer runs of rows than warps; int8 momentum over rows
+that are whole trips of a warp (their maxima wait for the row's end) and over rows that are not.  Two steps against the CPU
+oracle: statistics, scales and codes, weights."""
+import numpy as np
+import pytest
+import torch
+
+import kaon_oracle as ko
+
+pytestmark = pytest.mark.gpu
+
+EDGES = [(65, 256), (257, 264), (40, 1032), (1025, 512), (13, 4096), (300,)]
+
+
+@pytest.mark.parametrize("name,kw", [
+    ("Adakaon", dict(momentum_dtype="int8")),
+    ("Adakaon", dict(momentum_dtype="int8", cautious=False, weight_decay=0.1)),
+    ("Adakaon", dict(momentum_dtype="4bit", weight_decay=0.1, bf16_method="none")),
+    ("Adakaon", dict(bf16_method="kahan", weight_decay=0.1)),
+    ("Nekaon", dict(momentum_dtype="int8")),
+    ("AdaPNM", dict(momentum_dtype="4bit")),
+    ("KProdigy", dict(second_moment="factored", cautious=True)),
+])
+def test_final_edges_vs_oracle(name, kw):
+    import kaon_b200
+    from _gpu import state_np, to_bits
+    kw = dict(kw) if name == "KProdigy" else dict(kw, lr=1e-3)
+    gen = torch.Generator().manual_seed(47)
+    host = [(torch.randn(s, generator=gen) * 0.02).bfloat16() for s in EDGES]
+    params = [torch.nn.Parameter(h.clone().cuda()) for h in host]
+    opt = getattr(kaon_b200, name)(params, **kw)
+    opt.sr_seed = 5
+    inner = getattr(opt, "base_optimizer", opt)
+    orc = getattr(ko, "Oracle" + name)([to_bits(h) for h in host], EDGES, seed=5, **kw)
+    for step in range(2):
+        grads = [(torch.randn(s, generator=gen) * 1e-3).bfloat16() for s in EDGES]
+        for p, g in zip(params, grads):
+            p.grad = g.cuda()
+        opt.step()
+        torch.cuda.synchronize()
+        opt.check_device_status()
+        orc.step([to_bits(g) for g in grads])
+        bad = total = bad_codes = codes = 0
+        for i, p in enumerate(params):
+            at = (step, EDGES[i])
+            for key, want in orc.tensors[i].state.items():
+                got = state_np(inner.state[p], key)
+                if not isinstance(want, np.ndarray) or got is None or want.size == 0 or key == "shift":
+                    continue
+                got, want = got.reshape(-1), want.reshape(-1)
+                if got.dtype.kind == "f":       # sums in another order: an ulp or two of a statistic
+                    assert np.abs(got - want).max() <= 2e-6 * np.abs(want).max(), (at, key)
+                else:                           # codes, packed codes, bf16 bits: a neighbour where the quotient lies on a boundary
+                    diff = np.nonzero(got != want)[0]
+                    bad_codes += diff.size
+                    codes += got.size
+                    if got.dtype == np.uint16 or got.dtype == np.int16:
+                        # bf16 momentum: a neighbour of the update (2^-7 of it at most) enters by w1 < 1; in steps of the momentum
+                        # itself that can be several, where it is small
+                        val = lambda b: (b.view(np.uint16).astype(np.uint32) << 16).view(np.float32)  # noqa: E731
+                        assert np.abs(val(got) - val(want)).max() <= 2.0 ** -7 * np.abs(val(want)).max(), (at, key)
+                        continue
+                    for x, y in zip(got[diff].tolist(), want[diff].tolist()):
+                        step_of = max(abs((x & 15) - (y & 15)), abs((x >> 4) - (y >> 4))) if got.dtype == np.uint8 else abs(x - y)
+                        assert step_of == 1, (at, key)
+            diff = np.abs(to_bits(p).astype(np.int32) - orc.tensors[i].p.reshape(-1).astype(np.int32))
+            assert diff.max() <= (2 if name == "Nekaon" else 1), at   # the other bf16 neighbour at most; Nekaon rounds twice (update, climb)
+            bad += int((diff != 0).sum())
+            total += diff.size
+        assert bad <= 1e-3 * total, (step, bad, total)
+        assert bad_codes <= 2 + 1e-4 * codes, (step, bad_codes, codes)
