@@ -72,7 +72,7 @@ __global__ void ns_gemm_simple_kernel(const __nv_bfloat16* A, int a_mn, long lon
 
 // always the shared memory of the widest tile: one CTA per SM, whose tensor-memory allocation (all 512
 // columns) then never waits for a neighbour
-constexpr size_t G2_SMEM = 1024 + (size_t)G2_STAGES * (G_A_BYTES + (size_t)G_MAX_BN * G_BK * 2);
+constexpr size_t G2_SMEM = 1024 + (size_t)G2_RING + (size_t)G2_EPI_WARPS * G2_STAGE_OUT;
 
 static std::atomic<int> g_gemm_sms[64];  // multiprocessors per device, once the kernel's shared-memory limit is set
 
@@ -83,6 +83,7 @@ static int gemm_sms(int* out) {
   if (!g_gemm_sms[dev].load()) {
     KAON_CUDA(cudaFuncSetAttribute((const void*)ns_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G2_SMEM));
     KAON_CUDA(cudaFuncSetAttribute((const void*)ns_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G2_SMEM));
+    KAON_CUDA(cudaFuncSetAttribute((const void*)ns_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G2_SMEM));
     int sms = 0;
     KAON_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     g_gemm_sms[dev].store(sms);
@@ -91,11 +92,12 @@ static int gemm_sms(int* out) {
   return KAON_OK;
 }
 
-static int operand_maps(NsProblem& pr, const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb) {
+// (a pair's CTA loads half of a tile's columns)
+static int operand_maps(NsProblem& pr, const __nv_bfloat16* A, long long lda, const __nv_bfloat16* B, long long ldb, bool pair = false) {
   const GemmParams& p = pr.p;
   int rc = p.a_mn ? make_map(&pr.a, A, p.M, p.K, lda, 64) : make_map(&pr.a, A, p.K, p.M, lda, G_BM);
   if (rc) return rc;
-  return p.b_mn ? make_map(&pr.b, B, p.N, p.K, ldb, 64) : make_map(&pr.b, B, p.K, p.N, ldb, p.BN);
+  return p.b_mn ? make_map(&pr.b, B, p.N, p.K, ldb, 64) : make_map(&pr.b, B, p.K, p.N, ldb, pair ? p.BN / 2 : p.BN);
 }
 
 // out[M,N] = bf16(alpha * A(m,:) . B(n,:) + beta * aux)
@@ -277,7 +279,7 @@ int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsShares& shares, 
   }
   for (int it = 0; it < steps; ++it) {
     for (int stage = 0; stage < 3; ++stage) {
-      out.stages.push_back(NsStage{(int)probs.size(), tile0[stage], begin0[stage], (int)share[stage].begin.size() - 1});
+      out.stages.push_back(NsStage{(int)probs.size(), tile0[stage], begin0[stage], (int)share[stage].begin.size() - 1, share[stage].pair});
       for (const NsMat& m : mats) {
         const bool tall = m.R > m.C;   // the stored matrix is X^T (k rows, r columns)
         // ping-pong; the last iteration lands in `out`
@@ -288,7 +290,7 @@ int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsShares& shares, 
         NsProblem pr{};
         GemmParams& p = pr.p;
         p.M = sh.M; p.N = sh.N; p.K = sh.K; p.sym = sh.sym;
-        p.BN = ns_tile_cols(share[stage].bn, sh.N);
+        p.BN = ns_tile_cols(share[stage].bn, sh.N, share[stage].pair);
         pr.tensor = m.tensor;
         const __nv_bfloat16 *A, *B;
         long long lda, ldb;
@@ -308,7 +310,7 @@ int ns_batch_build(const std::vector<NsMat>& mats, int steps, NsShares& shares, 
           p.dev_scale = it == 0 ? m.scal + 2 : nullptr;
           p.aux = cur; p.ld_aux = m.ld; p.out = nxt; p.ld_out = last ? m.C : m.ld;
         }
-        if (int rc = operand_maps(pr, A, lda, B, ldb)) return rc;
+        if (int rc = operand_maps(pr, A, lda, B, ldb, share[stage].pair)) return rc;
         probs.push_back(pr);
       }
     }
@@ -336,7 +338,8 @@ int ns_batch_run(const NsBatch& b, const unsigned char* dev, const void* const* 
     w.begin = reinterpret_cast<const int*>(dev + b.off_begin) + st.begin0;
     w.grads = grads;
     w.status = status;
-    ns_gemm_kernel<true><<<st.grid, G2_THREADS, G2_SMEM, s>>>(none, w);
+    if (st.pair) ns_pair_kernel<<<2 * st.grid, G2_THREADS, G2_SMEM, s>>>(w);
+    else ns_gemm_kernel<true><<<st.grid, G2_THREADS, G2_SMEM, s>>>(none, w);
     *launches += 1;
   }
   KAON_CUDA(cudaGetLastError());

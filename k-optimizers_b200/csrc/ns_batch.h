@@ -21,7 +21,7 @@ struct NsMat {
 
 struct NsScale { int begin, end; float* scal; };   // partial sums of squares of one matrix
 
-struct NsStage { int prob0, tile0, begin0, grid; };
+struct NsStage { int prob0, tile0, begin0, grid; bool pair; };   // (grid: CTAs, or pairs of CTAs)
 
 struct NsBatch {
   std::vector<NsStage> stages;        // three per iteration (iterations share their tiles)
