@@ -293,7 +293,9 @@ __global__ void __launch_bounds__(SWT, 4) ada_sweep_kernel(const __grid_constant
 // A factored tensor of at most ADA_SMALL_MAX elements in ONE CTA: row statistics, column statistics, clip divisor,
 // COUNT and APPLY with barriers in between.  A list of adapter matrices has hundreds of them, each far too small to
 // share out; as items of the stages above they spent the step waiting for one another (720 matrices of 10 240
-// elements: 700 us, here 62 of the step's 69).  The gradient is kept in shared memory for the statistics.  Sums in a fixed order.
+// elements: 700 us).  The gradient is kept in shared memory for the statistics.  Sums in a fixed order.
+// Bound by the latency of a matrix's phases, so five blocks an SM, in 48 registers: those 720 matrices are then one round
+// of blocks instead of one and a fifth (a step 70 -> 65 us with what the registers spill).
 __device__ __forceinline__ double small_sum(double v, double* red, int tid) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -307,7 +309,7 @@ __device__ __forceinline__ double small_sum(double v, double* red, int tid) {
 }
 
 template <typename PT, int MKP, bool MUON, bool MS>
-__global__ void __launch_bounds__(SWT, 4) ada_small_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+__global__ void __launch_bounds__(SWT, 5) ada_small_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
   using ST = typename std::conditional<MUON, __nv_bfloat16, PT>::type;
   using S = Elems<ST>;
   extern __shared__ __align__(128) unsigned char g_s[];
@@ -321,6 +323,14 @@ __global__ void __launch_bounds__(SWT, 4) ada_small_kernel(const __grid_constant
   const unsigned char* sig = MUON ? reinterpret_cast<const unsigned char*>(pv.signal[ti]) : g;
   const int n = (int)d.numel, R = d.rows, C = d.cols;
   const bool gc = hp.gc != 0 && !MUON;   // AdaMuon's statistics are of a matrix that is not centralised
+  if (tid == 0 && !hp.stats_only) {   // what the sweeps will read, on its way to L2 meanwhile
+    auto ahead = [](const void* p, long long bytes) {
+      if (p != nullptr && bytes >= 16) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"((unsigned)bytes & ~15u) : "memory");
+    };
+    ahead(d.p, (long long)n * Elems<PT>::BYTES);
+    if constexpr (!MUON && MKP != KAON_M_NONE) ahead(d.m, (long long)(n >> 3) * MBytes<MKP>::V);
+  }
+#pragma unroll 4
   for (int k = tid; k < n * S::BYTES / 16; k += SWT)
     reinterpret_cast<uint4*>(g_s)[k] = reinterpret_cast<const uint4*>(sig)[k];
   __syncthreads();
