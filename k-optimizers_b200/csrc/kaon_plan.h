@@ -25,7 +25,9 @@ enum : int { PH_LION_MAIN = 0, PH_LION_APPLY = 1, PH_AXPY = 2,
               // run of rows; FINAL = column statistics, clip divisor (one item per column strip);
               // COUNT = cautious kept count; APPLY = momentum store + weight write.  FLAT = a whole 1-D
               // tensor in one item.
-              PH_ADA_STATS = 10, PH_ADA_FINAL = 11, PH_ADA_COUNT = 12, PH_ADA_APPLY = 13, PH_ADA_FLAT = 14 };
+              PH_ADA_STATS = 10, PH_ADA_FINAL = 11, PH_ADA_COUNT = 12, PH_ADA_APPLY = 13, PH_ADA_FLAT = 14,
+              // KProdigy: a warp's unit of whole rows, which takes their means itself
+              PH_KP_ROWS = 20 };
 
 constexpr int ADA_THREADS = 512;
 constexpr int FINAL_STRIP = 512;   // columns per FINAL item: one per thread

@@ -62,7 +62,7 @@ struct KpView {
   float* sums;            // [n_tensors][2] per-tensor sums (pass 1), [n_tensors] cautious denominators (pass 2)
   unsigned* tmax;         // [n_tensors] 1-D int8: bits of the tensor's absmax of the new momentum
   float* told;            // [n_tensors] 1-D int8: the scalar scale before this step
-  const Task* row_units;  // whole rows of the >=2-D tensors
+  const Task* row_units;  // whole rows of the >=2-D tensors whose units do not take their means themselves
   int n_row_units;
 };
 
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
     const bool two_d = d.rows > 0;
     const bool gc = hp.gc && two_d, fac = hp.factored && two_d;
     const int nvec = t.n >> 3, nv = two_d ? d.cols >> 3 : 0x40000000;
-    const float* mean = pv.aux + (two_d ? aux_mean(d) : 0);
+    float* mean = pv.aux + (two_d ? aux_mean(d) : 0);
     const float* rfac = pv.aux + (two_d ? aux_rfac(d) : 0);
     const float* cfac = pv.aux + (two_d ? aux_cfac(d) : 0);
     unsigned* rowmax = two_d ? reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d)) : x.tmax + t.tensor;
@@ -195,6 +195,10 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
     const float rdenom = __frcp_rn(denom), rfd = __frcp_rn(hp.fd);
     double acc_a = 0.0, acc_b = 0.0;
     f32x2 kept2 = pack2(0.0f, 0.0f);
+    // Pass 1 with the full second moment takes the means of a unit of whole rows itself, row by row (the second reading of the
+    // gradient hits a cache: a launch of their own read all of it once more, 133 us on 269 M elements of bf16)
+    const bool own_mean = MODE == 0 && gc && !fac && t.phase == PH_KP_ROWS;
+    float mu_row = 0.0f;
     auto trip = [&](const unsigned v, const bool act) {
       const unsigned o = act ? v : 0u;
       W8<PT> gq, P;
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
       if constexpr (MK == KAON_M_4BIT) sc_old = blk[o >> 4];
       if constexpr (MK == KAON_M_INT8) sc_old = msc_rd[r];
       if (need_g) {
-        const float mu = gc ? mean[r] : 0.0f;
+        const float mu = own_mean ? mu_row : gc ? mean[r] : 0.0f;
         center<PT>(gq, E::IS_BF16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, Y);
       }
       if (read_m) mq.decode(sc_old, M);
@@ -323,13 +327,33 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
         }
       }
     };
-    int v0 = 0;
-    for (; v0 + 32 <= nvec; v0 += 32) {
-      trip((unsigned)(v0 + lane), true);
-      row += adv_r; cv += adv_c;
-      if (cv >= nv) { cv -= nv; ++row; }
+    {
+      // (one place for the trip: it is long, and the compiler spills where it has it twice)
+      const int seg = own_mean ? nv : nvec;
+      for (int v0 = 0; v0 < nvec; v0 += seg) {
+        if (own_mean) {
+          const unsigned char* rowp = gp + (unsigned)v0 * (8u * E::BYTES);
+          f32x2 a = pack2(0.0f, 0.0f);
+#pragma unroll 4
+          for (int v = lane; v < nv; v += 32) {
+            W8<PT> w;
+            w.load(rowp + (unsigned)v * (8u * E::BYTES));
+            a = add2(a, add2(add2(w.pair(0), w.pair(1)), add2(w.pair(2), w.pair(3))));
+          }
+          mu_row = round_to(__fdiv_rn(warp_sum(a.x + a.y), (float)d.cols), PT());
+          if (lane == 0) mean[row] = mu_row;   // (for the sweeps to come)
+        }
+        for (int v = lane; v - lane < seg; v += 32) {
+          trip((unsigned)(v0 + v), v < seg);
+          cv += adv_c;
+          if (!own_mean) {
+            row += adv_r;
+            if (cv >= nv) { cv -= nv; ++row; }
+          }
+        }
+        if (own_mean) { ++row; cv = lane; }
+      }
     }
-    if (v0 < nvec) trip((unsigned)(v0 + lane), v0 + lane < nvec);
     if constexpr (MODE == 0 || MODE == 2) {
       if (MODE == 2) acc_a = (double)(kept2.x + kept2.y);
 #pragma unroll
@@ -615,6 +639,7 @@ struct KpHost {
   Task* d_strips = nullptr;  // and their FINAL strips and row-table runs
   int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0;
   long long slice_p = 1;
+  bool any_rows = false;     // a tensor of two dimensions or more
   std::vector<float> h_sums;
   int64_t bytes = 0;
 };
@@ -692,25 +717,35 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
       return fail(KAON_E_UNSUPPORTED, "KProdigy: tensor %d: one 4-bit block over %lld elements", i, (long long)t.numel);
     if (t.rows > 0) {
       if (t.cols > CAP) return fail(KAON_E_UNSUPPORTED, "KProdigy: tensor %d: rows of %d elements exceed a work item of %d", i, t.cols, CAP);
+      h->any_rows = true;
+    }
+    bool rowwise = false;
+    const uintptr_t ptrs = (uintptr_t)s[i] | (uintptr_t)bufs[i].p0 | (uintptr_t)t.stat_a;
+    if (((t.rows > 0 ? t.cols : t.numel) & 7) == 0 && (pl->momentum_kind != KAON_M_4BIT || t.bshift == 7) && slice_p == 1 &&
+        (ptrs & 15) == 0) {
+      // a warp's unit: small tensors in more pieces (the tensor alone decides, so the order of its sums stays); whole rows
+      // where a row is long beside its mean's latency (of a list of width 448, 250 us a step with flat units, 256 with its
+      // rows; 4-bit: and rows of whole blocks)
+      long long u = 512;
+      while (u < 4096 && u * 128 <= t.numel) u *= 2;
+      rowwise = t.rows > 0 && t.cols >= 1024 && (pl->momentum_kind != KAON_M_4BIT || t.cols % 128 == 0);
+      if (rowwise) u = std::max<long long>(1, u / t.cols) * t.cols;
+      for (long long e = 0; e < t.numel; e += u)
+        units.push_back(Task{i, rowwise ? PH_KP_ROWS : PH_ADA_APPLY, e, (int)std::min<long long>(u, t.numel - e), t.rows > 0 ? (int)(e / t.cols) : 0, slots++,
+                             t.rows > 0 ? (int)(e % t.cols) : 0});
+    } else {
+      for (long long e = 0; e < t.numel; e += KP_ITEM)
+        items.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(KP_ITEM, t.numel - e), 0, slots++, 0});
+    }
+    if (t.rows > 0 && !rowwise) {   // row means by a launch of their own
       const long long nr = std::max<long long>(1, 4096 / t.cols);
       for (long long r = 0; r < t.rows; r += nr)
         rows.push_back(Task{i, PH_ADA_STATS, r * t.cols, (int)std::min<long long>(nr, t.rows - r), (int)r, 0, 0});
     }
-    const uintptr_t ptrs = (uintptr_t)s[i] | (uintptr_t)bufs[i].p0 | (uintptr_t)t.stat_a;
-    if (((t.rows > 0 ? t.cols : t.numel) & 7) == 0 && (pl->momentum_kind != KAON_M_4BIT || t.bshift == 7) && slice_p == 1 &&
-        (ptrs & 15) == 0) {
-      // a warp's unit: small tensors in more pieces (the tensor alone decides, so the order of its sums stays)
-      long long u = 512;
-      while (u < 4096 && u * 128 <= t.numel) u *= 2;
-      for (long long e = 0; e < t.numel; e += u)
-        units.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(u, t.numel - e), t.rows > 0 ? (int)(e / t.cols) : 0, slots++,
-                             t.rows > 0 ? (int)(e % t.cols) : 0});
-      continue;
-    }
-    for (long long e = 0; e < t.numel; e += KP_ITEM)
-      items.push_back(Task{i, PH_ADA_APPLY, e, (int)std::min<long long>(KP_ITEM, t.numel - e), 0, slots++, 0});
   }
   begin[n] = slots;
+  // the long units first (rows of 11 520 elements at a list's end were a last wave of their own)
+  std::stable_sort(units.begin(), units.end(), [](const Task& a, const Task& b) { return a.n > b.n; });
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
     std::vector<char> leaves(n, 0);   // tensors whose STATS and FINAL are launches of their own
@@ -802,7 +837,7 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
   cudaStream_t s = (cudaStream_t)stream;
   const KpView& x = kh->view;
   const int mk = pl->momentum_kind;
-  if (hp.factored && x.n_row_units > 0) {
+  if (hp.factored && kh->any_rows) {
     AdaDev ad{};
     ad.w2 = (float)(1.0 - h->beta2); ad.w2m1 = ad.w2 - 1.0f; ad.small_w2 = ad.w2 < 0.5f;
     ad.w1 = 1.0f; ad.eps1 = (float)h->eps_factored; ad.has_eps = h->eps_factored > 0.0; ad.clip = 1.0f;
