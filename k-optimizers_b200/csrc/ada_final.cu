@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(FS_THREADS) ada_rowtab_kernel(const __grid_con
   const DevTensor& d = pv.tensors[t.tensor];
   const int r = t.row0 + threadIdx.x;
   if ((int)threadIdx.x >= t.n) return;
-  const float rn = __ldg(d.stat_a + r), mu = hp.gc ? __ldg(pv.aux + aux_mean(d) + r) : 0.0f, sc = hp.int8 ? __ldg(d.m_scale + r) : 1.0f;
-  const float4 scal = __ldg(reinterpret_cast<const float4*>(pv.aux + aux_scal(d)));
+  const float rn = __ldcg(d.stat_a + r), mu = hp.gc ? __ldcg(pv.aux + aux_mean(d) + r) : 0.0f, sc = hp.int8 ? __ldcg(d.m_scale + r) : 1.0f;
+  const float4 scal = __ldcg(reinterpret_cast<const float4*>(pv.aux + aux_scal(d)));
   const float rf = rsqrt_torch(__fdiv_rn(rn, scal.x));
   pv.aux[aux_rfac(d) + r] = rf;
   reinterpret_cast<float4*>(pv.aux + aux_rowtab(d))[r] =

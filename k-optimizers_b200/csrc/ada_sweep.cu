@@ -60,6 +60,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   if (APPLY && hp.cautious)
     denom = fmaxf(__fdiv_rn((float)__ldcg(pv.kept + t.tensor), (float)d.numel), 1e-8f);
   const float nrcp_denom = -__fdiv_rn(1.0f, denom);
+  // (plain loads, not the read-only ones: a launch that began early must not have them ahead of its wait)
   const float4* rowtab = reinterpret_cast<const float4*>(pv.aux + aux_rowtab(d));
   const float* cfac = pv.aux + aux_cfac(d);
   unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));
@@ -105,12 +106,12 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   // the vector whose words are in gq, mq; `act`: this lane has one; `more`: and one in the next trip
   auto trip = [&](const bool act, const bool more) {
     if (!AHEAD && act) load(std::integral_constant<int, 0>{});
-    const float4 f = OWN ? rowtab[row] : __ldg(rowtab + row);   // {mean, r_i, int8: scale of the stored codes, r_i / div * scale}
+    const float4 f = rowtab[row];   // {mean, r_i, int8: scale of the stored codes, r_i / div * scale}
     if (need_p) P.load(act ? pp : reinterpret_cast<unsigned char*>(d.p));
     f32x2 CF[4], G[4], MO[4];
     {
       const float4* cp = reinterpret_cast<const float4*>(cfac) + 2 * cv;
-      const float4 a = OWN ? cp[0] : __ldg(cp), b = OWN ? cp[1] : __ldg(cp + 1);
+      const float4 a = cp[0], b = cp[1];
       CF[0] = pack2(a.x, a.y); CF[1] = pack2(a.z, a.w); CF[2] = pack2(b.x, b.y); CF[3] = pack2(b.z, b.w);
     }
     center<ST>(gq, MUON ? 0.0f : f.x, G);
@@ -215,7 +216,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
       float sc = 1.0f;
       if constexpr (MK != KAON_M_NONE) {
         float amax = 0.0f;
-        if constexpr (MK == KAON_M_INT8) amax = __uint_as_float(OWN ? __ldcg(rowmax + row) : __ldg(rowmax + row));
+        if constexpr (MK == KAON_M_INT8) amax = __uint_as_float(OWN ? __ldcg(rowmax + row) : rowmax[row]);
         sc = store_m8<MK>(mp, MN, amax, act ? 8 : 0, lane, MS ? MO : nullptr);
         if constexpr (MK == KAON_M_4BIT) { if (act && (lane & 15) == 0) stg_f32(msc, sc); }
         if constexpr (MK == KAON_M_INT8) { if (act && cv == 0) msc[row] = sc; }
