@@ -16,7 +16,8 @@
 //
 // This kernel's stages handle any shape.  Tensors whose rows are a multiple of 8 elements (4-bit blocks of 128)
 // leave it: COUNT and APPLY run as launches of their own (ada_sweep.cu), STATS of bf16 rows of at least 256
-// elements too (ada_stats_kernel below; other such rows stream through ada_stats_stream here), and tensors of at most
+// elements too (ada_stats_kernel below; other such rows stream through ada_stats_stream here), and with STATS its FINAL
+// (ada_final.cu); tensors of at most
 // ADA_SMALL_MAX elements are stepped whole by one CTA each (ada_small_kernel).
 #include <algorithm>
 #include <map>
@@ -79,7 +80,8 @@ __device__ __forceinline__ float div_shared(float x, float d, float rcp) {
 // one CTA steps (ada_small_kernel), adds in double.  What the exception is for: the compensation stores rounding
 // differences at the size of a bf16 step, so a statistic that moves by an ulp shows there at full scale (double sums for
 // such tensors too: elements of the compensation off by a quarter of its size), and a run resumed from a checkpoint
-// of before should go on as it was.  Its price on the 269 M list: 1351 us a step against 1310.
+// of before should go on as it was.  Its price on the 269 M list, before FINAL was a launch of its own:
+// 1351 us a step against 1310.
 __device__ __forceinline__ float warp_sum_d(float v, bool plain) {
   if (plain) return warp_sum(v);
   double t = (double)v;
@@ -1756,7 +1758,7 @@ int configure_launch_adakaon(kaon_plan* pl, const cudaDeviceProp& prop, int max_
 // One-time set-up of the launches beside the persistent kernel.  Per factored tensor: its COUNT and
 // APPLY items go to the COUNT / APPLY launches (ada_sweep.cu) when its rows stream (a multiple of 8 elements; 4-bit
 // block 128), and its STATS items to the STATS launch when they qualify
-// (stats_item_ok, bf16 gradients or AdaMuon's bf16 signal).  Everything else - FINAL, the 1-D tensors,
+// (stats_item_ok, bf16 gradients or AdaMuon's bf16 signal), and FINAL with them.  Everything else - the 1-D tensors,
 // the stages of tensors that do not qualify - stays in the persistent kernel, whose two lists (with
 // COUNT items for the cautious mask, without them otherwise) are the plan's lists minus what left.
 int ensure_apply2(kaon_plan* pl) {
@@ -1923,8 +1925,8 @@ extern "C" int kaon_adakaon_step(kaon_plan* pl, const kaon_adakaon_hparams* h, u
                 "a tensor's rows exceed a work item of %d elements: such rows are stepped by the streaming launches "
                 "only (bf16 weights, a row length that is a multiple of 8 (16 with int8 momentum), 4-bit block 128, "
                 "int8 momentum with the cautious mask on)", CAP);
-  // the persistent kernel: FINAL, the 1-D tensors and the stages of tensors that do not stream; beside it
-  // the STATS launch before and the COUNT / APPLY launches after
+  // the persistent kernel: the 1-D tensors and the stages of tensors that do not stream; STATS, FINAL, COUNT and APPLY of the
+  // others as launches after it
   if (two) { v.tasks = pl->d_tasks_na[hp.cautious ? 1 : 0]; v.n_tasks = pl->n_tasks_na[hp.cautious ? 1 : 0]; }
   else if (hp.cautious) { v.tasks = pl->d_tasks_full; v.n_tasks = pl->n_tasks_full; }
   else { v.tasks = pl->d_tasks_main; v.n_tasks = pl->n_tasks_main; }
