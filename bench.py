@@ -65,9 +65,9 @@ WORKLOADS = {
 E2E_GROUPS = 16   # parameter groups of the end-to-end pipeline
 HEADLINE = "lion4bit_unet2p6b"
 RECORD = ["adakaon_int8_unet2p6b", "nekaon4bit_unet2p6b", "adamuon_int8_dit11b"]
-KERNEL_NAME = {"AdaMuon": "ns_gemm_kernel (grouped)", "Lion": "lion_main_kernel + lion_apply_kernel <bf16,4bit>",
-               "Adakaon": "ada_stats_kernel + adakaon_kernel + ada_sweep_kernel (COUNT, APPLY) <bf16,int8>",
-               "Nekaon": "ada_stats_kernel + adakaon_kernel + ada_sweep_kernel (COUNT, APPLY) <bf16,4bit>",
+KERNEL_NAME = {"AdaMuon": "ns_pair_kernel (grouped)", "Lion": "lion_main_kernel + lion_apply_kernel <bf16,4bit>",
+               "Adakaon": "ada_stats_kernel + ada_final_kernel + ada_sweep_kernel (COUNT, APPLY) <bf16,int8>",
+               "Nekaon": "ada_stats_kernel + ada_final_kernel + ada_sweep_kernel (COUNT, APPLY) <bf16,4bit>",
                "AdaPNM": "pnm_sweep_kernel<bf16,4bit>", "KProdigy": "kp_warp_kernel<bf16,bf16>"}
 
 
