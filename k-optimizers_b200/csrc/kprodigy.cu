@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(KP_THREADS) kp_prep_kernel(PlanView pv, KpView
 // The sweeps over tensors whose rows (1-D tensors: whose length) are a multiple of eight elements, with 4-bit blocks of
 // 128 and every element on the slice: a warp per unit of up to 4096 elements, vector accesses without guards, nothing
 // shared between warps.  Bound by HBM where the state is wide (MODE 0 reads and writes 28 bytes an element with the
-// full second moment: 1185 us for 269 M elements with bf16 momentum, 6.4 TB/s; MODE 3 522 us).  The guarded form, a
+// full second moment: 1243 us for 269 M elements with bf16 momentum, the row means in it, 6.0 TB/s; MODE 3 524 us).  The guarded form, a
 // CTA per 16 K-element item, took 1976 and 1102 us.
 template <typename PT, int MK, int MODE>
 __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ KpDev hp,
@@ -724,11 +724,12 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
     if (((t.rows > 0 ? t.cols : t.numel) & 7) == 0 && (pl->momentum_kind != KAON_M_4BIT || t.bshift == 7) && slice_p == 1 &&
         (ptrs & 15) == 0) {
       // a warp's unit: small tensors in more pieces (the tensor alone decides, so the order of its sums stays); whole rows
-      // where a row is long beside its mean's latency (of a list of width 448, 250 us a step with flat units, 256 with its
-      // rows; 4-bit: and rows of whole blocks)
+      // where rows are long beside their mean's latency and the tensor has warps enough of them (with rows from 256 elements on, a
+      // list of width 448 took 256 us a step for 250, and adapters of four rows of 1088 elements 111 for 108; 4-bit: and rows of
+      // whole blocks)
       long long u = 512;
       while (u < 4096 && u * 128 <= t.numel) u *= 2;
-      rowwise = t.rows > 0 && t.cols >= 1024 && (pl->momentum_kind != KAON_M_4BIT || t.cols % 128 == 0);
+      rowwise = t.numel >= (1ll << 19) && t.rows > 0 && t.cols >= 1024 && (pl->momentum_kind != KAON_M_4BIT || t.cols % 128 == 0);
       if (rowwise) u = std::max<long long>(1, u / t.cols) * t.cols;
       for (long long e = 0; e < t.numel; e += u)
         units.push_back(Task{i, rowwise ? PH_KP_ROWS : PH_ADA_APPLY, e, (int)std::min<long long>(u, t.numel - e), t.rows > 0 ? (int)(e / t.cols) : 0, slots++,
