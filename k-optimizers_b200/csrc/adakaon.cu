@@ -26,6 +26,7 @@
 #include <utility>
 #include <type_traits>
 
+#include "ada_lists.h"
 #include "adakaon_dev.h"
 #include "kaon_elem.cuh"
 #include "kaon_host.h"
@@ -646,11 +647,9 @@ __device__ __forceinline__ bool stats_stream_ok(const DevTensor& d, const void* 
 // centralization means, the item's column partial sums and row-statistic sum), taken with packed-pair
 // arithmetic.  Phase 1: one warp per row, the row streamed twice (mean, then sum of squares).  Phase 2:
 // thread-owned columns over the item's rows, which are in L2 by then; rows narrower than the CTA are
-// shared out over row groups whose partial sums are combined in a fixed order.  FINAL runs in the
-// following launch, so the order of the stream stands in for waiting on the completion counter (which
-// is still raised: the FINAL items look at it).
+// shared out over row groups whose partial sums are combined in a fixed order.  FINAL runs in a launch
+// after this one; the completion counter is raised for those FINAL items that are the persistent kernel's.
 constexpr int STT = 256;
-constexpr int ST_MAXROWS = 1024;   // rows of one STATS item at most
 constexpr int ST_VPT = 2;          // column vectors a thread accumulates at a time
 
 __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev hp) {
@@ -1755,93 +1754,38 @@ int configure_launch_adakaon(kaon_plan* pl, const cudaDeviceProp& prop, int max_
   return KAON_OK;
 }
 
-// One-time set-up of the launches beside the persistent kernel.  Per factored tensor: its COUNT and
-// APPLY items go to the COUNT / APPLY launches (ada_sweep.cu) when its rows stream (a multiple of 8 elements; 4-bit
-// block 128), and its STATS items to the STATS launch when they qualify
-// (stats_item_ok, bf16 gradients or AdaMuon's bf16 signal), and FINAL with them.  Everything else - the 1-D tensors,
-// the stages of tensors that do not qualify - stays in the persistent kernel, whose two lists (with
-// COUNT items for the cautious mask, without them otherwise) are the plan's lists minus what left.
+// One-time set-up of the launches beside the persistent kernel: the lists of ada_lists.h on the device.
 int ensure_apply2(kaon_plan* pl) {
   if (pl->apply2 != 0) return KAON_OK;
   pl->apply2 = -1;
-  const bool muon = pl->optimizer == KAON_OPT_ADAMUON;
-  const int mk = muon ? KAON_M_NONE : pl->momentum_kind;
-  std::vector<Task> items;
-  std::vector<char> elig((size_t)pl->n_tensors, 0);
-  std::vector<char> small((size_t)pl->n_tensors, 0);
-  {
-    std::vector<Task> h((size_t)pl->n_tasks_small);
-    if (!h.empty()) KAON_CUDA(cudaMemcpy(h.data(), pl->d_tasks_small, sizeof(Task) * h.size(), cudaMemcpyDeviceToHost));
-    for (const Task& t : h) small[t.tensor] = 1;
-  }
-  bool any = false;
-  for (int i = 0; i < pl->n_tensors; ++i) {
-    const DevTensor& t = pl->h_tensors[i];
-    if (t.rows <= 0 || t.numel == 0 || (t.cols & 7) != 0) continue;
-    if (mk == KAON_M_4BIT && t.block != 128u) continue;
-    if (small[i]) continue;
-    elig[i] = 1;
-    any = true;
-  }
-  if (!any) return KAON_OK;
-  sweep_units(pl, elig, items);
-  // the persistent kernel's lists and the STATS launch's
-  const bool stats_dtype = muon || pl->param_dtype == KAON_DT_BF16;
-  std::vector<Task> stats, strips;
-  // FINAL leaves with STATS, unless stages that stay wait for it
-  std::vector<char> leaves((size_t)pl->n_tensors, 0);
-  bool flat_only[2] = {false, false};
-  pl->long_rows_ok = true;
-  for (int variant = 0; variant < 2; ++variant) {   // 0: from the list without COUNT items; 1: from the full list
-    const Task* src = variant ? pl->d_tasks_full : pl->d_tasks_main;
-    const int ns = variant ? pl->n_tasks_full : pl->n_tasks_main;
-    std::vector<Task> h((size_t)ns), keep;
-    KAON_CUDA(cudaMemcpy(h.data(), src, sizeof(Task) * h.size(), cudaMemcpyDeviceToHost));
-    if (variant == 0)
-      for (const Task& t : h)
-        if (t.phase == PH_ADA_STATS && stats_dtype && elig[t.tensor] && stats_item_ok(pl, t)) leaves[t.tensor] = 1;
-    for (const Task& t : h) {
-      const bool el = elig[t.tensor] != 0;
-      if (t.phase == PH_ADA_FINAL && leaves[t.tensor]) continue;
-      if ((t.phase == PH_ADA_APPLY || t.phase == PH_ADA_COUNT) && el) continue;
-      if (t.phase == PH_ADA_STATS && stats_dtype && stats_item_ok(pl, t)) {
-        if (variant == 0) stats.push_back(t);
-        continue;
-      }
-      // what stays here is staged row by row: a tensor whose rows exceed a work item cannot stay
-      if (t.phase != PH_ADA_FINAL && t.phase != PH_ADA_FLAT && pl->h_tensors[t.tensor].cols > CAP) pl->long_rows_ok = false;
-      keep.push_back(t);
-    }
-    KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_na[variant], sizeof(Task) * std::max<size_t>(keep.size(), 1)));
-    KAON_CUDA(cudaMemcpy(pl->d_tasks_na[variant], keep.data(), sizeof(Task) * keep.size(), cudaMemcpyHostToDevice));
-    pl->n_tasks_na[variant] = (int)keep.size();
-    flat_only[variant] = std::all_of(keep.begin(), keep.end(), [](const Task& t) { return t.phase == PH_ADA_FLAT; });
-    pl->device_bytes += (int64_t)(sizeof(Task) * keep.size());
-  }
-  // The persistent kernel's short lists run beside STATS: a few 1-D tensors, or any list where both launches find room.  (Its
-  // blocks fill a multiprocessor each: beside a STATS that needs the whole machine, a list with stages that wait for one
-  // another cost 40 us more than the two in turn, and the 540 1-D tensors of the 2.6 B list gained nothing.)
+  auto fetch = [](const Task* src, int n, std::vector<Task>& out) -> cudaError_t {
+    out.resize((size_t)n);
+    return n ? cudaMemcpy(out.data(), src, sizeof(Task) * out.size(), cudaMemcpyDeviceToHost) : cudaSuccess;
+  };
+  std::vector<Task> small, src[2], items, strips;
+  KAON_CUDA(fetch(pl->d_tasks_small, pl->n_tasks_small, small));
+  KAON_CUDA(fetch(pl->d_tasks_main, pl->n_tasks_main, src[0]));
+  KAON_CUDA(fetch(pl->d_tasks_full, pl->n_tasks_full, src[1]));
+  const AdaLists a = ada_lists(pl, small, src);
+  if (!a.any) return KAON_OK;
+  auto put = [&](const std::vector<Task>& list, Task** dev, int* n) -> cudaError_t {
+    *n = (int)list.size();
+    if (list.empty()) return cudaSuccess;
+    pl->device_bytes += (int64_t)(sizeof(Task) * list.size());
+    if (cudaError_t e = cudaMalloc((void**)dev, sizeof(Task) * list.size())) return e;
+    return cudaMemcpy(*dev, list.data(), sizeof(Task) * list.size(), cudaMemcpyHostToDevice);
+  };
+  pl->long_rows_ok = a.long_rows_ok;
+  pl->stats_first = a.stats_first;
   for (int variant = 0; variant < 2; ++variant) {
-    const int n = pl->n_tasks_na[variant];
-    pl->na_beside[variant] = n > 0 && n <= pl->sm_count / 2 && (flat_only[variant] || n + (int)stats.size() / 4 <= pl->sm_count);
+    KAON_CUDA(put(a.keep[variant], &pl->d_tasks_na[variant], &pl->n_tasks_na[variant]));
+    pl->na_beside[variant] = a.beside[variant];
   }
-  if (!stats.empty()) {
-    KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_stats, sizeof(Task) * stats.size()));
-    KAON_CUDA(cudaMemcpy(pl->d_tasks_stats, stats.data(), sizeof(Task) * stats.size(), cudaMemcpyHostToDevice));
-    pl->n_tasks_stats = (int)stats.size();
-    final_items(pl, leaves, strips, pl->n_tasks_strips);
-    if (!strips.empty()) {
-      KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_final, sizeof(Task) * strips.size()));
-      KAON_CUDA(cudaMemcpy(pl->d_tasks_final, strips.data(), sizeof(Task) * strips.size(), cudaMemcpyHostToDevice));
-      pl->n_tasks_final = (int)strips.size();
-      pl->device_bytes += (int64_t)(sizeof(Task) * strips.size());
-    }
-    pl->device_bytes += (int64_t)(sizeof(Task) * stats.size());
-  }
-  KAON_CUDA(cudaMalloc((void**)&pl->d_tasks_apply2, sizeof(Task) * items.size()));
-  KAON_CUDA(cudaMemcpy(pl->d_tasks_apply2, items.data(), sizeof(Task) * items.size(), cudaMemcpyHostToDevice));
-  pl->n_tasks_apply2 = (int)items.size();
-  pl->device_bytes += (int64_t)(sizeof(Task) * items.size());
+  KAON_CUDA(put(a.stats, &pl->d_tasks_stats, &pl->n_tasks_stats));
+  final_items(pl, a.leaves, strips, pl->n_tasks_strips);
+  KAON_CUDA(put(strips, &pl->d_tasks_final, &pl->n_tasks_final));
+  sweep_units(pl, a.elig, items);
+  KAON_CUDA(put(items, &pl->d_tasks_apply2, &pl->n_tasks_apply2));
   pl->apply2 = 1;
   return KAON_OK;
 }
@@ -1856,11 +1800,6 @@ int launch_persistent(kaon_plan* pl, const PlanView& v, const AdaDev& hp, cudaSt
   KAON_CUDA(cudaGetLastError());
   pl->launches += 1;
   return KAON_OK;
-}
-
-bool stats_item_ok(const kaon_plan* pl, const Task& t) {
-  const DevTensor& dt = pl->h_tensors[t.tensor];
-  return dt.cols >= 256 && (dt.cols & 7) == 0 && t.n / dt.cols <= ST_MAXROWS && (dt.aux_off & 3) == 0;
 }
 
 int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* tasks, int n, bool beside, cudaStream_t s) {
@@ -1880,6 +1819,21 @@ int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Ta
   KAON_CUDA(cudaGetLastError());
   pl->launches += 1;
   return KAON_OK;
+}
+
+// The persistent kernel, STATS and FINAL of a plan whose COUNT and APPLY are launches of their own (`base`: its pointers).
+// STATS comes second, so that a short list runs beside it, unless the persistent kernel's FINAL items wait for it.
+int launch_statistics(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s) {
+  const int variant = hp.cautious ? 1 : 0;
+  PlanView v = base;
+  v.tasks = pl->d_tasks_na[variant];
+  v.n_tasks = pl->n_tasks_na[variant];
+  if (pl->stats_first)
+    if (int rc = launch_stats(pl, base, hp, pl->d_tasks_stats, pl->n_tasks_stats, false, s)) return rc;
+  if (int rc = launch_persistent(pl, v, hp, s)) return rc;
+  if (!pl->stats_first)
+    if (int rc = launch_stats(pl, base, hp, pl->d_tasks_stats, pl->n_tasks_stats, pl->na_beside[variant], s)) return rc;
+  return launch_final(pl, base, hp, pl->d_tasks_final, pl->n_tasks_strips, pl->n_tasks_final, s);
 }
 
 }  // namespace kaon
@@ -1925,16 +1879,15 @@ extern "C" int kaon_adakaon_step(kaon_plan* pl, const kaon_adakaon_hparams* h, u
                 "a tensor's rows exceed a work item of %d elements: such rows are stepped by the streaming launches "
                 "only (bf16 weights, a row length that is a multiple of 8 (16 with int8 momentum), 4-bit block 128, "
                 "int8 momentum with the cautious mask on)", CAP);
-  // the persistent kernel: the 1-D tensors and the stages of tensors that do not stream; STATS, FINAL, COUNT and APPLY of the
-  // others as launches after it
-  if (two) { v.tasks = pl->d_tasks_na[hp.cautious ? 1 : 0]; v.n_tasks = pl->n_tasks_na[hp.cautious ? 1 : 0]; }
-  else if (hp.cautious) { v.tasks = pl->d_tasks_full; v.n_tasks = pl->n_tasks_full; }
-  else { v.tasks = pl->d_tasks_main; v.n_tasks = pl->n_tasks_main; }
   KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-  if (int rc = launch_persistent(pl, v, hp, s)) return rc;
+  // the persistent kernel: the 1-D tensors and the stages of tensors that do not stream; STATS, FINAL, COUNT and APPLY of the
+  // others as launches of their own
   if (two) {
-    if (int rc = launch_stats(pl, pl->view, hp, pl->d_tasks_stats, pl->n_tasks_stats, pl->na_beside[hp.cautious ? 1 : 0], s)) return rc;
-    if (int rc = launch_final(pl, pl->view, hp, pl->d_tasks_final, pl->n_tasks_strips, pl->n_tasks_final, s)) return rc;
+    if (int rc = launch_statistics(pl, v, hp, s)) return rc;
+  } else {
+    v.tasks = hp.cautious ? pl->d_tasks_full : pl->d_tasks_main;
+    v.n_tasks = hp.cautious ? pl->n_tasks_full : pl->n_tasks_main;
+    if (int rc = launch_persistent(pl, v, hp, s)) return rc;
   }
   if (int rc = launch_small(pl, pl->view, hp, s)) return rc;
   if (two) {

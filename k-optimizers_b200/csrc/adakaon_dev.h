@@ -47,12 +47,14 @@ void sweep_units(const kaon_plan* pl, const std::vector<char>& elig, std::vector
 int ensure_apply2(kaon_plan* pl);
 int launch_small(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
 int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
-// the STATS launch over a caller's list of STATS items (all of which pass stats_item_ok); `beside`: the launch before it on the
-// stream is the persistent kernel's, and the two may run at the same time
-bool stats_item_ok(const kaon_plan* pl, const Task& t);
+// the STATS launch over a caller's list of STATS items (all of which pass stats_item_ok, ada_lists.h); `beside`: the launch
+// before it on the stream is the persistent kernel's, and the two may run at the same time
 int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* tasks, int n, bool beside, cudaStream_t s);
 // FINAL as launches of its own (ada_final.cu)
 void final_items(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out, int& n_strips);
 int launch_final(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* items, int n_strips, int n, cudaStream_t s);
+
+// all of that for a plan with apply2 == 1
+int launch_statistics(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s);
 
 }  // namespace kaon

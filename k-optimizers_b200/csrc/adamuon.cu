@@ -598,13 +598,13 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
   ada_finish(hp);
   if (int rc = ensure_apply2(pl)) return rc;
   const bool three = pl->apply2 == 1;  // STATS/FINAL/FLAT here, COUNT and APPLY as launches of their own
-  if (three) { v.tasks = pl->d_tasks_na[hp.cautious ? 1 : 0]; v.n_tasks = pl->n_tasks_na[hp.cautious ? 1 : 0]; }
-  else if (hp.cautious) { v.tasks = pl->d_tasks_full; v.n_tasks = pl->n_tasks_full; }
-  else { v.tasks = pl->d_tasks_main; v.n_tasks = pl->n_tasks_main; }
-  if (int rc = launch_persistent(pl, v, hp, s)) return rc;
   if (three) {
-    if (int rc = launch_stats(pl, v, hp, pl->d_tasks_stats, pl->n_tasks_stats, pl->na_beside[hp.cautious ? 1 : 0], s)) return rc;
-    if (int rc = launch_final(pl, v, hp, pl->d_tasks_final, pl->n_tasks_strips, pl->n_tasks_final, s)) return rc;
+    if (int rc = launch_statistics(pl, v, hp, s)) return rc;
+  } else {
+    PlanView w = v;
+    w.tasks = hp.cautious ? pl->d_tasks_full : pl->d_tasks_main;
+    w.n_tasks = hp.cautious ? pl->n_tasks_full : pl->n_tasks_main;
+    if (int rc = launch_persistent(pl, w, hp, s)) return rc;
   }
   if (int rc = launch_small(pl, v, hp, s)) return rc;
   if (three) {

@@ -24,6 +24,7 @@
 
 #include <type_traits>
 
+#include "ada_lists.h"
 #include "adakaon_dev.h"
 #include "kaon_device.cuh"
 #include "kaon_host.h"

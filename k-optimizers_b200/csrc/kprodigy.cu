@@ -20,6 +20,7 @@
 #include <cmath>
 #include <vector>
 
+#include "ada_lists.h"
 #include "adakaon_dev.h"
 #include "kaon_device.cuh"
 #include "kaon_elem.cuh"
