@@ -16,12 +16,9 @@ namespace kaon {
 // in the order of the runs (the rule at warp_sum_d in adakaon.cu).
 constexpr int FS_COLS = 128, FS_THREADS = 256, FS_WARPS = FS_THREADS / 32;
 
-__global__ void __launch_bounds__(FS_THREADS) ada_final_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+__device__ __forceinline__ void final_strip(const PlanView& pv, const AdaDev& hp, const Task& t) {
   __shared__ double sum_s[FS_WARPS][2][FS_COLS];
   __shared__ double red[FS_WARPS];
-  const Task t = pv.tasks[blockIdx.x];
-  early_launch();
-  after_launch_before();
   if (pv.grads[t.tensor] == nullptr) return;
   const DevTensor& d = pv.tensors[t.tensor];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -111,10 +108,7 @@ __global__ void __launch_bounds__(FS_THREADS) ada_final_kernel(const __grid_cons
 
 // The row table of FINAL's tensors, FS_THREADS rows a CTA.  (By the tensor's last strip alone it was the step's longest chain
 // of loads: 68 us of FINAL on the 269 M list, whose tallest tensors have 10 240 rows.)
-__global__ void __launch_bounds__(FS_THREADS) ada_rowtab_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
-  const Task t = pv.tasks[blockIdx.x];
-  early_launch();
-  after_launch_before();
+__device__ __forceinline__ void rowtab_run(const PlanView& pv, const AdaDev& hp, const Task& t) {
   if (pv.grads[t.tensor] == nullptr) return;
   const DevTensor& d = pv.tensors[t.tensor];
   const int r = t.row0 + threadIdx.x;
@@ -129,6 +123,34 @@ __global__ void __launch_bounds__(FS_THREADS) ada_rowtab_kernel(const __grid_con
     reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d))[r] = 0u;
     pv.aux[aux_oldsc(d) + r] = sc;
   }
+}
+
+// A block an item; with reserved multiprocessors, whose blocks leave, the others claim the items.
+template <typename Item>
+__device__ __forceinline__ void each_item(const PlanView& pv, const Item& item) {
+  __shared__ int next_s;
+  if (on_reserved_sm(pv.sm_reserve)) return;
+  if (pv.sm_reserve == 0u) {
+    const Task t = pv.tasks[blockIdx.x];
+    early_launch();
+    after_launch_before();
+    item(t);
+    return;
+  }
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) next_s = (int)atomicAdd(pv.task_counter, 1u);
+    __syncthreads();
+    if (next_s >= pv.n_tasks) return;
+    item(pv.tasks[next_s]);
+  }
+}
+
+__global__ void __launch_bounds__(FS_THREADS) ada_final_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+  each_item(pv, [&](const Task& t) { final_strip(pv, hp, t); });
+}
+__global__ void __launch_bounds__(FS_THREADS) ada_rowtab_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+  each_item(pv, [&](const Task& t) { rowtab_run(pv, hp, t); });
 }
 
 // ----------------------------------------------------------------------------- host
@@ -149,11 +171,12 @@ void final_items(const kaon_plan* pl, const std::vector<char>& elig, std::vector
 
 int launch_final(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* items, int n_strips, int n, cudaStream_t s) {
   if (n == 0) return KAON_OK;
+  const int most = pl->sm_count * 4;
   PlanView v = base;
-  v.tasks = items;
-  KAON_CUDA(launch_early(ada_final_kernel, n_strips, FS_THREADS, s, v, hp));
-  v.tasks = items + n_strips;
-  KAON_CUDA(launch_early(ada_rowtab_kernel, n - n_strips, FS_THREADS, s, v, hp));
+  v.tasks = items; v.n_tasks = n_strips; v.task_counter = base.counters2 + 3;
+  KAON_CUDA(launch_early(!v.sm_reserve, ada_final_kernel, v.sm_reserve ? most : v.n_tasks, FS_THREADS, s, v, hp));
+  v.tasks = items + n_strips; v.n_tasks = n - n_strips; v.task_counter = base.counters2 + 4;
+  KAON_CUDA(launch_early(!v.sm_reserve, ada_rowtab_kernel, v.sm_reserve ? most : v.n_tasks, FS_THREADS, s, v, hp));
   pl->launches += 2;
   return KAON_OK;
 }

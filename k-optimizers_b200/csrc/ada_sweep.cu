@@ -263,9 +263,9 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
 
 template <typename PT, int MKP, bool MUON, bool MS, bool APPLY, bool CP>
 __global__ void __launch_bounds__(SWT, 4) ada_sweep_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+  if (on_reserved_sm(pv.sm_reserve)) return;
   early_launch();
   after_launch_before();
-  if (on_reserved_sm(pv.sm_reserve)) return;
   const int lane = threadIdx.x & 31;
   // The first unit is the warp's own number (with reserved multiprocessors, whose warps leave, a claimed one), the
   // others are claimed, one ahead.
@@ -554,11 +554,11 @@ int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cu
     va.task_counter = base.counters2 + 1;
     SweepKernel k = hp.has_wd && hp.cautious ? pick_sweep<false, true>(pl->param_dtype, pl->momentum_kind, muon, ms)
                                              : pick_sweep<false, false>(pl->param_dtype, pl->momentum_kind, muon, false);
-    KAON_CUDA(launch_early(k, grid, SWT, s, va, hp));
+    KAON_CUDA(launch_early(!base.sm_reserve, k, grid, SWT, s, va, hp));
     pl->launches += 1;
   }
   va.task_counter = base.counters2 + 2;
-  KAON_CUDA(launch_early(pick_sweep<true, false>(pl->param_dtype, pl->momentum_kind, muon, ms), grid, SWT, s, va, hp));
+  KAON_CUDA(launch_early(!base.sm_reserve, pick_sweep<true, false>(pl->param_dtype, pl->momentum_kind, muon, ms), grid, SWT, s, va, hp));
   pl->launches += 1;
   return KAON_OK;
 }

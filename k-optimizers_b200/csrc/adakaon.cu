@@ -1814,9 +1814,7 @@ int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Ta
   v.n_tasks = n;
   v.task_counter = base.counters2;
   const int grid = v.sm_reserve ? pl->stats_grid : std::min(pl->stats_grid, n);
-  if (beside) KAON_CUDA(launch_early(ada_stats_kernel, grid, STT, s, v, hp));
-  else ada_stats_kernel<<<grid, STT, 0, s>>>(v, hp);
-  KAON_CUDA(cudaGetLastError());
+  KAON_CUDA(launch_early(beside && !v.sm_reserve, ada_stats_kernel, grid, STT, s, v, hp));
   pl->launches += 1;
   return KAON_OK;
 }

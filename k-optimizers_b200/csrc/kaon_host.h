@@ -26,16 +26,17 @@ int check_device(const kaon_plan* pl);
 
 // A launch that may begin while the launch before it on the stream drains (programmatic stream serialization): the kernel calls
 // after_launch_before() ahead of the first access to what that launch writes, or, where the two have nothing to do with
-// each other, at its end.
+// each other, at its end.  Not with reserved multiprocessors (`early` false): its blocks would find room on those first, while
+// the others are full, and either sit there or, as they should, leave, all of them, with the work undone.
 template <typename... P, typename... A>
-cudaError_t launch_early(void (*kernel)(P...), int grid, int block, cudaStream_t s, const A&... args) {
+cudaError_t launch_early(bool early, void (*kernel)(P...), int grid, int block, cudaStream_t s, const A&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
   cfg.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);

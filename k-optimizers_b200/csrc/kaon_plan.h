@@ -116,7 +116,7 @@ struct PlanView {
   unsigned* done;          // Lion: [n_tensors] MAIN items finished.  Adakaon: [4][n_tensors] =
                            //   STATS items done | FINAL strips arrived | FINAL complete | COUNT items done
   unsigned* kept;          // [n_tensors] cautious kept count
-  unsigned* counters2;     // [4] claim counters of the Adakaon launches beside the persistent kernel: STATS, COUNT, APPLY, -
+  unsigned* counters2;     // [5] claim counters of the Adakaon launches beside the persistent kernel: STATS, COUNT, APPLY, FINAL, row table
   float* aux;              // Adakaon scratch (see DevTensor::aux_off)
   const void* const* signal;  // AdaMuon: per-tensor orthogonalised momentum (bf16); null otherwise
   unsigned* status;        // 0 = ok; else the code of the first bounded wait that ran out

@@ -335,7 +335,7 @@ int kaon_plan_create(kaon_plan** out, int optimizer, int param_dtype, int moment
   size_t o_m = o_f + up(sizeof(Task) * full_list.size()), o_a = o_m + up(sizeof(Task) * main_list.size());
   size_t o_s = o_a + up(sizeof(Task) * axpy_list.size()), o_w = o_s + up(sizeof(Task) * small_list.size());
   size_t o_c = o_w + up(sizeof(Task) * warp_list.size());
-  pl->counters_bytes = sizeof(unsigned) * (size_t)(2 + 5 * n + 4);
+  pl->counters_bytes = sizeof(unsigned) * (size_t)(2 + 5 * n + 5);
   size_t tot = o_c + up(pl->counters_bytes);
   ce = cudaMalloc(&pl->d_block, tot);
   if (ce != cudaSuccess) { delete pl; return cuda_fail(ce, "cudaMalloc(plan tables)"); }
