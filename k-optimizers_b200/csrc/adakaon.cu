@@ -28,7 +28,6 @@
 
 #include "ada_lists.h"
 #include "adakaon_dev.h"
-#include "kaon_elem.cuh"
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
 #include "kaon_packed.cuh"
@@ -685,7 +684,6 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
     double rowsum = 0.0;
     float *stat = d.stat_a + t.row0, *mean = pv.aux + aux_mean(d) + t.row0;
     const bool plain = d.shift != nullptr;
-    const float fC = (float)C, rC = __frcp_rn(fC);
     const uint4* gitem = reinterpret_cast<const uint4*>(g + (ok ? t.e0 * 2 : 0));
     // a run of rows on its way to L2 while the one before it is worked on
     auto ahead = [&](int ra, int rb) {
@@ -714,7 +712,7 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
             a0 = add2(a0, add2(pairs(q0.x), pairs(q0.y)));
             a1 = add2(a1, add2(pairs(q0.z), pairs(q0.w)));
           }
-          mu = round_bf16(div_by(warp_sum_d((a0.x + a0.y) + (a1.x + a1.y), plain), fC, rC));
+          mu = round_bf16(__fdiv_rn(warp_sum_d((a0.x + a0.y) + (a1.x + a1.y), plain), (float)C));
         }
         const uint32_t mu2 = pack_bf16_rn(mu, mu);
         auto sq2 = [&](uint32_t w) {
@@ -737,7 +735,8 @@ __global__ void __launch_bounds__(STT, 4) ada_stats_kernel(PlanView pv, AdaDev h
         }
         const float s2 = warp_sum_d((b0.x + b0.y) + (b1.x + b1.y), plain);
         if (lane == 0) {
-          const float rn = lerp_torch(old, div_by(s2, fC, rC), hp.w2, hp.w2m1, hp.small_w2 != 0);
+          // (the division, not div_by: a sum that has overflowed stays infinite, as in the reference)
+          const float rn = lerp_torch(old, __fdiv_rn(s2, (float)C), hp.w2, hp.w2m1, hp.small_w2 != 0);
           stat[r] = rn;
           mean2_s[r] = mu2;
           if (gc) mean[r] = mu;

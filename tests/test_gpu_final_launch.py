@@ -70,3 +70,32 @@ def test_final_edges_vs_oracle(name, kw):
             total += diff.size
         assert bad <= 1e-3 * total, (step, bad, total)
         assert bad_codes <= 2 + 1e-4 * codes, (step, bad_codes, codes)
+
+
+@pytest.mark.parametrize("name", ["Adakaon", "AdaPNM"])
+def test_a_row_whose_squares_overflow_has_an_infinite_statistic(name):
+    """Gradients of 1e20 in one row, of either sign in turn (so that the row's mean is zero whatever the order of its sum): its
+    statistic, and those of the columns, are infinite, as the oracle's are, and not NaN; other rows keep theirs."""
+    import kaon_b200
+    from _gpu import state_np, to_bits
+    shape = (65, 512)
+    gen = torch.Generator().manual_seed(3)
+    host = (torch.randn(shape, generator=gen) * 0.02).bfloat16()
+    grad = (torch.randn(shape, generator=gen) * 1e-3).bfloat16()
+    grad[7] = 1e20
+    grad[7, 1::2] = -1e20
+    p = torch.nn.Parameter(host.clone().cuda())
+    opt = getattr(kaon_b200, name)([p], lr=1e-3)
+    orc = getattr(ko, "Oracle" + name)([to_bits(host)], [shape], lr=1e-3)
+    p.grad = grad.cuda()
+    opt.step()
+    torch.cuda.synchronize()
+    opt.check_device_status()
+    orc.step([to_bits(grad)])
+    want = orc.tensors[0].state
+    assert np.isinf(want["row"]).sum() == 1 and np.isinf(want["col"]).all()
+    for key in ("row", "col"):
+        got = state_np(opt.state[p], key)
+        assert np.array_equal(np.isinf(got), np.isinf(want[key])) and not np.isnan(got).any(), key
+        fine = np.isfinite(want[key])
+        assert np.abs(got[fine] - want[key][fine]).max(initial=0.0) <= 2e-6 * np.abs(want[key][fine]).max(initial=1e-30), key
