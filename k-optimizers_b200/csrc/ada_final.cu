@@ -114,11 +114,10 @@ __device__ __forceinline__ void rowtab_run(const PlanView& pv, const AdaDev& hp,
   const int r = t.row0 + threadIdx.x;
   if ((int)threadIdx.x >= t.n) return;
   const float rn = __ldcg(d.stat_a + r), mu = hp.gc ? __ldcg(pv.aux + aux_mean(d) + r) : 0.0f, sc = hp.int8 ? __ldcg(d.m_scale + r) : 1.0f;
-  const float4 scal = __ldcg(reinterpret_cast<const float4*>(pv.aux + aux_scal(d)));
-  const float rf = rsqrt_torch(__fdiv_rn(rn, scal.x));
+  const float rf = rsqrt_torch(__fdiv_rn(rn, __ldcg(pv.aux + aux_scal(d))));
   pv.aux[aux_rfac(d) + r] = rf;
   reinterpret_cast<float4*>(pv.aux + aux_rowtab(d))[r] =
-      make_float4(pv.param_bf16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, rf, sc, __fmul_rn(rf, update_factor(hp, scal.y)));
+      make_float4(pv.param_bf16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, rf, sc, 0.0f);
   if (hp.int8) {   // COUNT starts from zeroed row maxima; APPLY decodes with the old scales
     reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d))[r] = 0u;
     pv.aux[aux_oldsc(d) + r] = sc;

@@ -106,7 +106,7 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
   // the vector whose words are in gq, mq; `act`: this lane has one; `more`: and one in the next trip
   auto trip = [&](const bool act, const bool more) {
     if (!AHEAD && act) load(std::integral_constant<int, 0>{});
-    const float4 f = rowtab[row];   // {mean, r_i, int8: scale of the stored codes, r_i / div * scale}
+    const float4 f = rowtab[row];   // {mean, r_i, int8: scale of the stored codes, -}
     if (need_p) P.load(act ? pp : reinterpret_cast<unsigned char*>(d.p));
     f32x2 CF[4], G[4], MO[4];
     {
@@ -130,27 +130,22 @@ __device__ __forceinline__ void sweep_unit(const PlanView& pv, const AdaDev& hp,
       if (!APPLY && act) P.store(pp, nullptr);
     }
     // ---- u = ((g r) c) / div * scale (reference src/kaon/adakaon.py:885-888), m' = lerp(m, u) ----
-    // A COUNT that only counts takes r / div * scale as one factor (three roundings fewer); where codes, row maxima or a
-    // compensation come of u, the reference's order of roundings stays (an ulp moves codes, and with them the next scales)
+    // (the same roundings in COUNT and APPLY: what is counted is what APPLY keeps, also where an ulp turns a sign)
     f32x2 MN[4], F[4];
-    const bool folded = !APPLY && MK != KAON_M_INT8 && !hp.kahan;
-    const f32x2 RF = folded ? pack2(f.w, f.w) : pack2(f.y, f.y);
+    const f32x2 RF = pack2(f.y, f.y);
 #pragma unroll
     for (int j = 0; j < 4; ++j) MN[j] = mul2(mul2(G[j], RF), CF[j]);
-    if (!folded) {
-      if (clipped) {
-        const f32x2 DIVN = pack2(-div, -div), RCPD = pack2(rcp_div, rcp_div);
+    if (clipped) {
+      const f32x2 DIVN = pack2(-div, -div), RCPD = pack2(rcp_div, rcp_div);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const f32x2 qq = mul2(MN[j], RCPD);
-          MN[j] = fma2(fma2(qq, DIVN, MN[j]), RCPD, qq);
-        }
+      for (int j = 0; j < 4; ++j) {
+        const f32x2 qq = mul2(MN[j], RCPD);
+        MN[j] = fma2(fma2(qq, DIVN, MN[j]), RCPD, qq);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) MN[j] = mul2(MN[j], pack2(hp.upd_scale, hp.upd_scale));
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
+      MN[j] = mul2(MN[j], pack2(hp.upd_scale, hp.upd_scale));
       if constexpr (MK == KAON_M_BF16) {
         const uint32_t ub = pack_bf16_rn(MN[j].x, MN[j].y);
         MN[j] = pack2(bf16lo(ub), bf16hi(ub));
@@ -447,7 +442,6 @@ __global__ void __launch_bounds__(SWT, 5) ada_small_kernel(const __grid_constant
   for (int r = tid; r < R; r += SWT) {
     const float rf = rsqrt_torch(__fdiv_rn(d.stat_a[r], rowmean));
     rowtab[r].y = rf;
-    rowtab[r].w = __fmul_rn(rf, update_factor(hp, div));
     pv.aux[aux_rfac(d) + r] = rf;
   }
   if (hp.stats_only) return;

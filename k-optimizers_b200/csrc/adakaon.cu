@@ -923,19 +923,18 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
       scal[2] = rms;
       scal[3] = __fdiv_rn(1.0f, scal[1]);
       sm.part_s[0] = rowmean;
-      sm.part_s[1] = update_factor(hp, scal[1]);
     }
   }
   last = __syncthreads_or(last);
   if (last) {  // the whole CTA: r_i of every row, then release COUNT / APPLY
-    const float rowmean = sm.part_s[0], uf = sm.part_s[1];
+    const float rowmean = sm.part_s[0];
     float* rfac = pv.aux + aux_rfac(d);
     float4* rowtab = reinterpret_cast<float4*>(pv.aux + aux_rowtab(d));
     for (int r = tid; r < d.rows; r += AT) {
       const float rf = rsqrt_torch(__fdiv_rn(__ldcg(d.stat_a + r), rowmean));
       rfac[r] = rf;
       const float mu = hp.gc ? __ldcg(pv.aux + aux_mean(d) + r) : 0.0f;
-      rowtab[r] = make_float4(pv.param_bf16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, rf, hp.int8 ? d.m_scale[r] : 1.0f, __fmul_rn(rf, uf));
+      rowtab[r] = make_float4(pv.param_bf16 ? __uint_as_float(pack_bf16_rn(mu, mu)) : mu, rf, hp.int8 ? d.m_scale[r] : 1.0f, 0.0f);
     }
     if (hp.int8) {  // int8 momentum: COUNT starts from zeroed row maxima; APPLY decodes with the old scales
       unsigned* rowmax = reinterpret_cast<unsigned*>(pv.aux + aux_rowmax(d));

@@ -36,11 +36,6 @@ inline void ada_finish(AdaDev& hp) {
   hp.mask_off = !hp.cautious;
 }
 
-#ifdef __CUDACC__
-// what r_i is multiplied by for a COUNT that takes the clip divisor and the step's scale with it
-__device__ __forceinline__ float update_factor(const AdaDev& hp, float div) { return (float)((double)hp.upd_scale / (double)div); }
-#endif
-
 int launch_persistent(kaon_plan* pl, const PlanView& v, const AdaDev& hp, cudaStream_t s);
 // COUNT and APPLY as launches of their own (ada_sweep.cu), for the factored tensors whose rows stream
 void sweep_units(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out);

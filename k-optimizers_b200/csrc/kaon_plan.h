@@ -82,7 +82,7 @@ __host__ __device__ inline long long aux_rfac(const DevTensor& d) { return aux_o
 // scratch of a 1-D tensor stepped from global memory: 8 floats | n floats (padded) | one word per 4-bit block (>= 32 elements)
 __host__ __device__ inline long long flat_long_pad(long long n) { return (n + 63) / 64 * 64; }
 __host__ __device__ inline long long flat_long_size(long long n) { return 8 + flat_long_pad(n) + ((n + 31) / 32 + 1 + 63) / 64 * 64; }
-// {mean (bf16 weights: two bf16 copies), r_i, int8: old scale, r_i / clip divisor * update scale} of every row, for COUNT / APPLY (16-byte aligned)
+// {mean (bf16 weights: two bf16 copies), r_i, int8: old scale, -} of every row, for COUNT / APPLY (16-byte aligned)
 __host__ __device__ inline long long aux_rowtab(const DevTensor& d) { return (aux_rfac(d) + d.rows + 3) / 4 * 4; }
 __host__ __device__ inline long long aux_size(const DevTensor& d) { return aux_rowtab(d) + 4ll * d.rows - d.aux_off; }
 

@@ -46,3 +46,34 @@ def test_subnormal_products_are_masked_by_their_sign(name, size, kw):
             # fp32 chains that differ by an ulp of a statistic, a rare code one step off
             bad = np.abs(got - want) > 2e-4 * np.abs(want) + 1e-6 * np.abs(want).max()
             assert bad.mean() < (1e-2 if kw["momentum_dtype"] == "int8" and step else 1e-3), (step, SHAPES[i], bad.mean())
+
+
+@pytest.mark.parametrize("shape", [(96, 512), (64, 256), (60, 333)])
+def test_the_kept_count_is_that_of_the_mask(shape):
+    """Weights chosen so that the decay cancels the new momentum to within a rounding, m' + (lr wd) p: the sign of what is left turns
+    on the last bit of m', and the count has to be taken of the very m' that is stored.  (m' does not depend on the weights, so a
+    first run with weights of zero tells it; fp32 gradients, no centralization.  m' + (lr wd) p is exact in fp64: 24 + 24 bits
+    beside 24 at the same magnitude.)"""
+    import kaon_b200
+    gen = torch.Generator().manual_seed(29)
+    grad = (torch.randn(shape, generator=gen) * 1e-3).cuda()
+    lr, wd = 0.05, 0.1
+    lrwd = np.float64(np.float32(lr * wd))
+
+    def run(weights):
+        p = torch.nn.Parameter(weights.clone())
+        p.grad = grad.clone()
+        opt = kaon_b200.Adakaon([p], lr=lr, weight_decay=wd, momentum_dtype="float32", gradient_centralization=False)
+        opt.step()
+        torch.cuda.synchronize()
+        opt.check_device_status()
+        (plan,) = opt._plans.values()
+        return opt.state[p]["m"].double().cpu().numpy().reshape(-1), plan.kept_counts(torch.cuda.current_stream().cuda_stream)[0]
+
+    m, _ = run(torch.zeros(shape, device="cuda"))
+    w = (-m / lrwd).astype(np.float32)
+    again, kept = run(torch.from_numpy(w).reshape(shape).cuda())
+    assert np.array_equal(m, again)
+    delta = m + lrwd * w.astype(np.float64)
+    assert np.abs(delta).max() <= 2.0 ** -23 * np.abs(m).max()
+    assert kept == int((np.sign(delta) * np.sign(grad.double().cpu().numpy().reshape(-1)) > 0).sum())
