@@ -124,7 +124,8 @@ __device__ __forceinline__ void rowtab_run(const PlanView& pv, const AdaDev& hp,
   }
 }
 
-// A block an item; with reserved multiprocessors, whose blocks leave, the others claim the items.
+// A block an item; with reserved multiprocessors, whose blocks leave, the others claim the items.  Nothing where a wait of this
+// plan has run out: STATS then left no sums to go by (the status stays; no kernel that could set it runs beside this one).
 template <typename Item>
 __device__ __forceinline__ void each_item(const PlanView& pv, const Item& item) {
   __shared__ int next_s;
@@ -133,9 +134,10 @@ __device__ __forceinline__ void each_item(const PlanView& pv, const Item& item) 
     const Task t = pv.tasks[blockIdx.x];
     early_launch();
     after_launch_before();
-    item(t);
+    if (*reinterpret_cast<volatile unsigned*>(pv.status) == 0u) item(t);
     return;
   }
+  if (*reinterpret_cast<volatile unsigned*>(pv.status) != 0u) return;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) next_s = (int)atomicAdd(pv.task_counter, 1u);
