@@ -17,6 +17,13 @@ inline bool stats_item_ok(const kaon_plan* pl, const Task& t) {
   return dt.cols >= 256 && (dt.cols & 7) == 0 && t.n / dt.cols <= ST_MAXROWS && (dt.aux_off & 3) == 0;
 }
 
+// Whether a list of n small tensors runs the build of ada_small_kernel for five blocks an SM (48 registers, which spill) or the one
+// for four: `four`, `five`: the blocks that registers and shared memory let in of either.  Only where that saves a round of blocks.
+inline bool small_takes_five(int n, int four, int five, int sms) {
+  auto rounds = [&](int blocks) { return (n - 1) / (blocks * sms) + 1; };
+  return five > four && four > 0 && rounds(five) < rounds(four);
+}
+
 struct AdaLists {
   bool any = false;               // some tensor's COUNT and APPLY are launches of their own; nothing below where none's are
   std::vector<char> elig;         // those tensors

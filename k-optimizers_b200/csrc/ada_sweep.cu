@@ -16,6 +16,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "ada_lists.h"
 #include "adakaon_dev.h"
 #include "kaon_host.h"
 #include "kaon_ops.cuh"
@@ -290,8 +291,7 @@ __global__ void __launch_bounds__(SWT, 4) ada_sweep_kernel(const __grid_constant
 // COUNT and APPLY with barriers in between.  A list of adapter matrices has hundreds of them, each far too small to
 // share out; as items of the stages above they spent the step waiting for one another (720 matrices of 10 240
 // elements: 700 us).  The gradient is kept in shared memory for the statistics.  Sums in a fixed order.
-// Bound by the latency of a matrix's phases, so five blocks an SM, in 48 registers: those 720 matrices are then one round
-// of blocks instead of one and a fifth (a step 70 -> 65 us with what the registers spill).
+// Bound by the latency of a matrix's phases, so by the rounds of blocks a list takes: BLOCKS of them an SM (small_takes_five).
 __device__ __forceinline__ double small_sum(double v, double* red, int tid) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -304,8 +304,8 @@ __device__ __forceinline__ double small_sum(double v, double* red, int tid) {
   return t;
 }
 
-template <typename PT, int MKP, bool MUON, bool MS>
-__global__ void __launch_bounds__(SWT, 5) ada_small_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
+template <typename PT, int MKP, bool MUON, bool MS, int BLOCKS>
+__global__ void __launch_bounds__(SWT, BLOCKS) ada_small_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ AdaDev hp) {
   using ST = typename std::conditional<MUON, __nv_bfloat16, PT>::type;
   using S = Elems<ST>;
   extern __shared__ __align__(128) unsigned char g_s[];
@@ -480,32 +480,43 @@ static SweepKernel pick_sweep(int pdt, int mk, bool muon, bool ms) {
 }
 
 typedef void (*SmallKernel)(PlanView, AdaDev);
-template <typename PT, bool MS>
+template <typename PT, bool MS, int BLOCKS>
 static SmallKernel pick_small_pt(int mk) {
   switch (mk) {
-    case KAON_M_F32: return ada_small_kernel<PT, KAON_M_F32, false, MS>;
-    case KAON_M_BF16: return ada_small_kernel<PT, KAON_M_BF16, false, MS>;
-    case KAON_M_INT8: return ada_small_kernel<PT, KAON_M_INT8, false, MS>;
-    case KAON_M_4BIT: return ada_small_kernel<PT, KAON_M_4BIT, false, MS>;
-    case KAON_M_NONE: return ada_small_kernel<PT, KAON_M_NONE, false, false>;
+    case KAON_M_F32: return ada_small_kernel<PT, KAON_M_F32, false, MS, BLOCKS>;
+    case KAON_M_BF16: return ada_small_kernel<PT, KAON_M_BF16, false, MS, BLOCKS>;
+    case KAON_M_INT8: return ada_small_kernel<PT, KAON_M_INT8, false, MS, BLOCKS>;
+    case KAON_M_4BIT: return ada_small_kernel<PT, KAON_M_4BIT, false, MS, BLOCKS>;
+    case KAON_M_NONE: return ada_small_kernel<PT, KAON_M_NONE, false, false, BLOCKS>;
     default: return nullptr;
   }
 }
+template <int BLOCKS>
 static SmallKernel pick_small(int pdt, int mk, bool muon, bool ms) {
   const bool bf = pdt == KAON_DT_BF16;
-  if (muon) return bf ? ada_small_kernel<__nv_bfloat16, KAON_M_NONE, true, false> : ada_small_kernel<float, KAON_M_NONE, true, false>;
-  if (ms) return bf ? pick_small_pt<__nv_bfloat16, true>(mk) : pick_small_pt<float, true>(mk);
-  return bf ? pick_small_pt<__nv_bfloat16, false>(mk) : pick_small_pt<float, false>(mk);
+  if (muon) return bf ? ada_small_kernel<__nv_bfloat16, KAON_M_NONE, true, false, BLOCKS> : ada_small_kernel<float, KAON_M_NONE, true, false, BLOCKS>;
+  if (ms) return bf ? pick_small_pt<__nv_bfloat16, true, BLOCKS>(mk) : pick_small_pt<float, true, BLOCKS>(mk);
+  return bf ? pick_small_pt<__nv_bfloat16, false, BLOCKS>(mk) : pick_small_pt<float, false, BLOCKS>(mk);
 }
 
 // The plan's small tensors (their statistics only, for AdaPNM and KProdigy).
 int launch_small(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStream_t s) {
   if (pl->n_tasks_small == 0) return KAON_OK;
   const bool muon = pl->optimizer == KAON_OPT_ADAMUON;
-  SmallKernel k = pick_small(pl->param_dtype, hp.stats_only ? KAON_M_NONE : pl->momentum_kind, muon, hp.remove || hp.climb);
+  const bool ms = hp.remove || hp.climb;
+  const int mk = hp.stats_only ? KAON_M_NONE : pl->momentum_kind;
+  SmallKernel k = pick_small<4>(pl->param_dtype, mk, muon, ms);
   if (!k) return fail(KAON_E_INVALID, "no Adakaon kernel for this dtype combination");
   const size_t smem = (size_t)pl->small_max * (muon || pl->param_dtype == KAON_DT_BF16 ? 2 : 4);
-  KAON_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, ADA_SMALL_MAX * 4));
+  const SmallKernel five = pick_small<5>(pl->param_dtype, mk, muon, ms);
+  int* blocks = pl->small_blocks[ms];
+  if (blocks[0] == 0) {
+    KAON_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, ADA_SMALL_MAX * 4));
+    KAON_CUDA(cudaFuncSetAttribute((const void*)five, cudaFuncAttributeMaxDynamicSharedMemorySize, ADA_SMALL_MAX * 4));
+    KAON_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[1], (const void*)five, SWT, smem));
+    KAON_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[0], (const void*)k, SWT, smem));
+  }
+  if (small_takes_five(pl->n_tasks_small, blocks[0], blocks[1], pl->sm_count)) k = five;
   PlanView v = base;
   v.tasks = pl->d_tasks_small;
   v.n_tasks = pl->n_tasks_small;

@@ -174,6 +174,7 @@ struct kaon_plan {
   bool long_rows_ok = false;                 // every tensor whose rows exceed a work item left the persistent kernel
   kaon::Task* d_tasks_small = nullptr;       // factored tensors one CTA steps on its own
   int n_tasks_small = 0, small_max = 0;      // and the elements of the largest
+  int small_blocks[2][2] = {{0, 0}, {0, 0}}; // blocks an SM of that kernel's builds for four and five (second row: with the climb)
   // STATS as a launch of its own: the STATS items that qualify
   kaon::Task* d_tasks_stats = nullptr;
   int n_tasks_stats = 0, stats_grid = 0;

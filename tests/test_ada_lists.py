@@ -1,6 +1,6 @@
 """The share-out of the Adakaon family's work items (csrc/ada_lists.h, host code): every item has one place, and no item waits
 for a launch that comes after its own.  On the GPU, a list whose tensors part ways: 4-bit blocks of 256 beside a matrix of 128
-elements, which is one block of 128."""
+elements, which is one block of 128; and lists long enough to run five blocks an SM."""
 import os
 import subprocess
 
@@ -140,3 +140,44 @@ def test_blocks_of_256_beside_a_block_of_128_vs_oracle(name, kw):
                     assert (got != want).sum() <= 2 + 2e-4 * got.size, (step, shapes[i], key)
             diff = np.abs(to_bits(p).astype(np.int32) - orc.tensors[i].p.reshape(-1).astype(np.int32))
             assert diff.max() <= (2 if name == "Nekaon" else 1) and (diff != 0).sum() <= 1 + 1e-3 * diff.size, (step, shapes[i])
+
+
+RULE = r"""
+#include <cstdlib>
+#include "ada_lists.h"
+int main(int argc, char** argv) { return kaon::small_takes_five(atoi(argv[1]), atoi(argv[2]), atoi(argv[3]), 148); }
+"""
+
+
+def test_five_blocks_only_where_they_save_a_round(tmp_path):
+    (tmp_path / "main.cpp").write_text(RULE)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", f"-I{CSRC}", f"-I{CUDA}", str(tmp_path / "main.cpp"), "-o", str(tmp_path / "main")])
+    takes = lambda n, four=4, five=5: subprocess.run([str(tmp_path / "main"), str(n), str(four), str(five)]).returncode == 1  # noqa: E731
+    assert [n for n in (1, 16, 592, 593, 740, 741, 1184, 1185, 1480, 1481, 1776, 1777, 2220, 2221) if takes(n)] == [593, 740, 1185, 1480, 1777, 2220]
+    assert not takes(700, 3, 3) and not takes(700, 4, 4)   # (shared memory lets no fifth in)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,kw", [("Adakaon", dict()), ("Adakaon", dict(momentum_dtype="int8", weight_decay=0.1)), ("Nekaon", dict())])
+def test_a_long_list_steps_as_two_short_ones(name, kw):
+    """700 matrices in one list (five blocks an SM) and in two of 350 (four): the same arithmetic, the same bits."""
+    import kaon_b200
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    shapes = [(8, 128), (64, 8), (16, 264), (128, 32), (5, 1600)] * 140
+    values = [(torch.randn(s, device="cuda", generator=gen) * 0.02, torch.randn(s, device="cuda", generator=gen) * 1e-3) for s in shapes]
+    runs = []
+    for parts in (1, 2):
+        params = [torch.nn.Parameter(v.clone()) for v, _ in values]
+        for p, (_, g) in zip(params, values):
+            p.grad = g.clone()
+        n = len(params) // parts
+        opts = [getattr(kaon_b200, name)(params[i * n:(i + 1) * n], lr=1e-3, **kw) for i in range(parts)]
+        for _ in range(2):
+            for o in opts:
+                o.step()
+        torch.cuda.synchronize()
+        for o in opts:
+            o.check_device_status()
+        runs.append([p.detach() for p in params])
+    for a, b in zip(*runs):
+        assert torch.equal(a, b), a.shape
