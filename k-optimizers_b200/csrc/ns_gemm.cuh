@@ -165,14 +165,17 @@ struct NsWork {
 __device__ __forceinline__ void store_tile(const GemmParams& p, const uint32_t tmem, const unsigned row0, const int n0, const int half, const float alpha,
                                            const float beta, unsigned char* stage, const int lane) {
   const unsigned row = row0 + lane, M = p.M, N = p.N;
-  const bool vec = ((reinterpret_cast<uintptr_t>(p.out) | (uintptr_t)(p.ld_out * 2) | reinterpret_cast<uintptr_t>(p.aux) | (uintptr_t)(p.aux ? p.ld_aux * 2 : 0)) & 15) == 0;
+  // (rows of `out` off the 16-byte grid, those of the last product where the length is no multiple of eight, go out as
+  // 32 consecutive elements an instruction)
+  const bool vec_out = ((reinterpret_cast<uintptr_t>(p.out) | (uintptr_t)(p.ld_out * 2)) & 15) == 0;
+  const bool vec_aux = ((reinterpret_cast<uintptr_t>(p.aux) | (uintptr_t)(p.aux ? p.ld_aux * 2 : 0)) & 15) == 0;
   const int pr = lane >> 2, ps = lane & 3;   // the row (of eight) and the piece of it that this lane moves to and from memory
   auto piece = [&](int r, int s) { return reinterpret_cast<uint4*>(stage + r * 64 + ((s ^ ((r >> 1) & 3)) << 4)); };
   for (int c0 = half * (p.BN / 2); c0 < (half + 1) * (p.BN / 2); c0 += 32) {
     const unsigned col = (unsigned)n0 + c0;
     uint32_t v[32];
     tmem_ld32(tmem + (uint32_t)c0, v);
-    const bool full = vec && col + 32 <= N && (!p.sym || row0 + 32 <= M);   // (the warp's)
+    const bool full = vec_aux && col + 32 <= N && (!p.sym || (vec_out && row0 + 32 <= M));   // (the warp's)
     uint4 x[4];
     if (full && p.aux) {
 #pragma unroll
@@ -203,11 +206,18 @@ __device__ __forceinline__ void store_tile(const GemmParams& p, const uint32_t t
 #pragma unroll
       for (int q = 0; q < 4; ++q) *piece(lane, q) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
       __syncwarp();
+      if (vec_out) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const unsigned r = row0 + i * 8 + pr;
-        const uint4 o = *piece(i * 8 + pr, ps);
-        if (r < M) *reinterpret_cast<uint4*>(p.out + (long long)r * p.ld_out + col + ps * 8) = o;
+        for (int i = 0; i < 4; ++i) {
+          const unsigned r = row0 + i * 8 + pr;
+          const uint4 o = *piece(i * 8 + pr, ps);
+          if (r < M) *reinterpret_cast<uint4*>(p.out + (long long)r * p.ld_out + col + ps * 8) = o;
+        }
+      } else {
+        unsigned short* orow = reinterpret_cast<unsigned short*>(p.out + (long long)row0 * p.ld_out + col) + lane;
+        const int rows = (int)min(32u, M > row0 ? M - row0 : 0u);
+#pragma unroll 4
+        for (int i = 0; i < rows; ++i, orow += p.ld_out) *orow = reinterpret_cast<const unsigned short*>(piece(i, lane >> 3))[lane & 7];
       }
       __syncwarp();
       if (p.sym) {   // the mirror image: out[col + j, row0 ..], a column of the block a row of it
