@@ -24,6 +24,13 @@ inline bool small_takes_five(int n, int four, int five, int sms) {
   return five > four && four > 0 && rounds(five) < rounds(four);
 }
 
+// Whether the persistent kernel's list of n items runs beside a STATS launch of n_stats: a few 1-D tensors, or any list where both
+// launches find room.  (Its blocks fill a multiprocessor each: beside a STATS that needs the whole machine, a list with
+// stages that wait for one another cost 40 us more than the two in turn, and the 540 1-D tensors of the 2.6 B list gained nothing.)
+inline bool runs_beside(int n, bool flat_only, int n_stats, int sms) {
+  return n > 0 && ((flat_only && n <= sms / 2) || n + n_stats / 4 <= sms);
+}
+
 struct AdaLists {
   bool any = false;               // some tensor's COUNT and APPLY are launches of their own; nothing below where none's are
   std::vector<char> elig;         // those tensors
@@ -74,11 +81,7 @@ inline AdaLists ada_lists(const kaon_plan* pl, const std::vector<Task>& small, c
       flat_only = flat_only && t.phase == PH_ADA_FLAT;
       a.keep[variant].push_back(t);
     }
-    // The persistent kernel's short lists run beside STATS: a few 1-D tensors, or any list where both launches find room.  (Its
-    // blocks fill a multiprocessor each: beside a STATS that needs the whole machine, a list with stages that wait for one
-    // another cost 40 us more than the two in turn, and the 540 1-D tensors of the 2.6 B list gained nothing.)
-    const int n = (int)a.keep[variant].size();
-    a.beside[variant] = n > 0 && n <= pl->sm_count / 2 && (flat_only || n + (int)a.stats.size() / 4 <= pl->sm_count);
+    a.beside[variant] = runs_beside((int)a.keep[variant].size(), flat_only, (int)a.stats.size(), pl->sm_count);
   }
   if (a.stats_first) a.beside[0] = a.beside[1] = false;
   return a;

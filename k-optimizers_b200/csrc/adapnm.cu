@@ -831,7 +831,7 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
     v.tasks = ph->d_final; v.n_tasks = ph->n_final;
     if (int rc = launch_persistent(pl, v, ad, s)) return rc;
-    if (int rc = launch_stats(pl, pl->view, ad, ph->d_stats, ph->n_stats, false, s)) return rc;
+    if (int rc = launch_stats(pl, pl->view, ad, ph->d_stats, ph->n_stats, runs_beside(ph->n_final, false, ph->n_stats, pl->sm_count), s)) return rc;
     if (int rc = launch_final(pl, pl->view, ad, ph->d_strips, ph->n_strips, ph->n_final_items, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
     // 2-4. the two sweeps over the flat items

@@ -849,7 +849,7 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
     v.tasks = kh->d_final; v.n_tasks = kh->n_final;
     if (int rc = launch_persistent(pl, v, ad, s)) return rc;
-    if (int rc = launch_stats(pl, pl->view, ad, kh->d_stats, kh->n_stats, false, s)) return rc;
+    if (int rc = launch_stats(pl, pl->view, ad, kh->d_stats, kh->n_stats, runs_beside(kh->n_final, false, kh->n_stats, pl->sm_count), s)) return rc;
     if (int rc = launch_final(pl, pl->view, ad, kh->d_strips, kh->n_strips, kh->n_final_items, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
   } else if (hp.gc && x.n_row_units > 0) {
