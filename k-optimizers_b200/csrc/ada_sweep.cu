@@ -319,13 +319,6 @@ __global__ void __launch_bounds__(SWT, BLOCKS) ada_small_kernel(const __grid_con
   const unsigned char* sig = MUON ? reinterpret_cast<const unsigned char*>(pv.signal[ti]) : g;
   const int n = (int)d.numel, R = d.rows, C = d.cols;
   const bool gc = hp.gc != 0 && !MUON;   // AdaMuon's statistics are of a matrix that is not centralised
-  if (tid == 0 && !hp.stats_only) {   // what the sweeps will read, on its way to L2 meanwhile
-    auto ahead = [](const void* p, long long bytes) {
-      if (p != nullptr && bytes >= 16) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"((unsigned)bytes & ~15u) : "memory");
-    };
-    ahead(d.p, (long long)n * Elems<PT>::BYTES);
-    if constexpr (!MUON && MKP != KAON_M_NONE) ahead(d.m, (long long)(n >> 3) * MBytes<MKP>::V);
-  }
 #pragma unroll 4
   for (int k = tid; k < n * S::BYTES / 16; k += SWT)
     reinterpret_cast<uint4*>(g_s)[k] = reinterpret_cast<const uint4*>(sig)[k];
