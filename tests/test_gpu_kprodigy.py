@@ -5,6 +5,8 @@ Every step starts from the reference's state after the step before (weights, per
 d / d_max / d_numerator / k): the estimate feeds on p0 - p, so one stochastic-rounding draw or one
 cautious-mask bit that differs moves every later step by a per cent or so, in the reference's own trajectory
 as much as here.  The gates are those of the oracle's test (tests/test_oracle_golden.py)."""
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -196,3 +198,20 @@ def test_kprodigy_constructor_errors_and_resume():
     assert oc.get_d() == oa.get_d()
     for a, c in zip(pa, pc):
         assert torch.equal(a.view(torch.int16), c.view(torch.int16))
+
+
+# rows of 1024 elements and more of tensors of 2^19 and more: units of several whole rows, which take their means themselves
+# (three rows, the last unit fewer; a row's last trip in part; one row a unit; 4-bit: rows of whole blocks only)
+ROWS = [(641, 1032), (514, 1280), (260, 2056), (515, 1024), (1280,)]
+
+
+@pytest.mark.parametrize("kw", [
+    dict(cautious=True),
+    dict(momentum_dtype="int8", cautious=True, weight_decay=0.01),
+    dict(momentum_dtype="4bit", cautious=True, bf16_method="none"),
+    dict(momentum_dtype="float32", cautious=True, bf16_method="kahan"),
+])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_units_of_whole_rows_vs_oracle(kw, dtype, monkeypatch):
+    monkeypatch.setattr(sys.modules[__name__], "BIG", ROWS)
+    test_kprodigy_vs_oracle_bigger_shapes(kw, dtype)

@@ -1,6 +1,6 @@
 """Products by pairs of CTAs (csrc/ns_share.h, csrc/ns_gemm.cuh): their tiles are handed out once each with the coordinates they
-have; on the GPU, the iteration over batches that take them, at extents that end inside a tile, inside one CTA's half of it and
-inside a k-block, against fp64."""
+have; on the GPU, the iteration against fp64 over batches small and large, and over batches all of whose products are pairs'
+(the share-out says so), at extents that end inside a tile, inside either CTA's half of it and inside a k-block."""
 import os
 import subprocess
 
@@ -82,3 +82,40 @@ def test_iteration_vs_fp64(shapes):
             x = 3.4445 * x + (-4.7750 * a + 2.0315 * a @ a) @ x
         # a chain of bf16 products: a few 2^-8 of an entry's size
         assert ((got.double() - x).norm() / x.norm()).item() < 2e-2, p.shape
+
+
+PAIRS = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "ns_share.h"
+using namespace kaon;
+// arguments: multiprocessors, then R C of each matrix of a batch; exit code 0 where every product of an iteration takes pairs
+int main(int argc, char** argv) {
+  NsShares::Key key;
+  for (int i = 2; i + 1 < argc; i += 2) key.push_back({atoll(argv[i]), atoll(argv[i + 1])});
+  NsShares shares;
+  for (const NsShare& s : shares.get(key, atoi(argv[1]))) if (!s.pair) return 1;
+  return 0;
+}
+"""
+
+# 3080 = 12 x 256 + 8: the last tile's second CTA has no row; 2952 = 11 x 256 + 136: it has eight; 100, 104: tiles of 128 columns;
+# 264 and 3336 end inside a k-block of 64; 2001: rows of the last product off the 16-byte grid
+RAGGED = [
+    [(2952, 4104), (4104, 2952), (3096, 3096), (100, 3000), (3000, 104)],
+    [(3080, 3400), (3400, 3080), (264, 3336), (3001, 264), (264, 2001)],
+]
+
+
+@pytest.mark.parametrize("shapes", RAGGED)
+def test_ragged_batches_take_pairs(shapes, tmp_path):
+    (tmp_path / "main.cpp").write_text(PAIRS)
+    subprocess.check_call(["g++", "-std=c++17", "-O2", f"-I{CSRC}", str(tmp_path / "main.cpp"), "-o", str(tmp_path / "main")])
+    subprocess.check_call([str(tmp_path / "main"), "148", *[str(x) for s in shapes for x in s]])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shapes", RAGGED)
+def test_ragged_pairs_vs_fp64(shapes):
+    assert torch.cuda.get_device_properties(0).multi_processor_count == 148   # (of the share-out above)
+    test_iteration_vs_fp64(shapes)
