@@ -125,19 +125,21 @@ __device__ __forceinline__ void rowtab_run(const PlanView& pv, const AdaDev& hp,
 }
 
 // A block an item; with reserved multiprocessors, whose blocks leave, the others claim the items.  Nothing where a wait of this
-// plan has run out: STATS then left no sums to go by (the status stays; no kernel that could set it runs beside this one).
+// plan has run out: STATS then left no sums to go by (the status stays).
 template <typename Item>
 __device__ __forceinline__ void each_item(const PlanView& pv, const Item& item) {
   __shared__ int next_s;
   if (on_reserved_sm(pv.sm_reserve)) return;
+  auto failed = [&]() { return __syncthreads_or(*reinterpret_cast<volatile unsigned*>(pv.status) != 0u) != 0; };   // (the block's)
   if (pv.sm_reserve == 0u) {
     const Task t = pv.tasks[blockIdx.x];
     early_launch();
     after_launch_before();
-    if (*reinterpret_cast<volatile unsigned*>(pv.status) == 0u) item(t);
+    if (failed()) return;
+    item(t);
     return;
   }
-  if (*reinterpret_cast<volatile unsigned*>(pv.status) != 0u) return;
+  if (failed()) return;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) next_s = (int)atomicAdd(pv.task_counter, 1u);
@@ -175,9 +177,9 @@ int launch_final(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Ta
   const int most = pl->sm_count * 4;
   PlanView v = base;
   v.tasks = items; v.n_tasks = n_strips; v.task_counter = base.counters2 + 3;
-  KAON_CUDA(launch_early(!v.sm_reserve, ada_final_kernel, v.sm_reserve ? most : v.n_tasks, FS_THREADS, s, v, hp));
+  KAON_CUDA(launch_early(!v.sm_reserve, ada_final_kernel, v.sm_reserve ? most : v.n_tasks, FS_THREADS, 0, s, v, hp));
   v.tasks = items + n_strips; v.n_tasks = n - n_strips; v.task_counter = base.counters2 + 4;
-  KAON_CUDA(launch_early(!v.sm_reserve, ada_rowtab_kernel, v.sm_reserve ? most : v.n_tasks, FS_THREADS, s, v, hp));
+  KAON_CUDA(launch_early(!v.sm_reserve, ada_rowtab_kernel, v.sm_reserve ? most : v.n_tasks, FS_THREADS, 0, s, v, hp));
   pl->launches += 2;
   return KAON_OK;
 }

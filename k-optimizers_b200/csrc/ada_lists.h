@@ -24,6 +24,14 @@ inline bool small_takes_five(int n, int four, int five, int sms) {
   return five > four && four > 0 && rounds(five) < rounds(four);
 }
 
+// The tensors (of bf16 rows) whose STATS items in `list` the STATS launch can take, all of them
+inline std::vector<char> stats_tensors(const kaon_plan* pl, const std::vector<Task>& list) {
+  std::vector<char> ok((size_t)pl->n_tensors, 0);
+  for (const Task& t : list) if (t.phase == PH_ADA_STATS) ok[t.tensor] = 1;
+  for (const Task& t : list) if (t.phase == PH_ADA_STATS && !stats_item_ok(pl, t)) ok[t.tensor] = 0;
+  return ok;
+}
+
 // Whether the persistent kernel's list of n items runs beside a STATS launch of n_stats: a few 1-D tensors, or any list where both
 // launches find room.  (Its blocks fill a multiprocessor each: beside a STATS that needs the whole machine, a list with
 // stages that wait for one another cost 40 us more than the two in turn, and the 540 1-D tensors of the 2.6 B list gained nothing.)
@@ -62,19 +70,17 @@ inline AdaLists ada_lists(const kaon_plan* pl, const std::vector<Task>& small, c
   for (const Task& t : small) a.elig[t.tensor] = 0;
   a.any = std::find(a.elig.begin(), a.elig.end(), 1) != a.elig.end();
   if (!a.any) return a;
-  std::vector<char> gone((size_t)pl->n_tensors, 0);   // tensors with items in the STATS launch
+  // the tensors whose STATS leave
+  const std::vector<char> gone = stats_dtype ? stats_tensors(pl, src[0]) : std::vector<char>((size_t)pl->n_tensors, 0);
   for (const Task& t : src[0])
-    if (t.phase == PH_ADA_STATS && stats_dtype && stats_item_ok(pl, t)) {
-      a.stats.push_back(t);
-      gone[t.tensor] = 1;
-    }
+    if (t.phase == PH_ADA_STATS && gone[t.tensor]) a.stats.push_back(t);
   for (int i = 0; i < pl->n_tensors; ++i) a.leaves[i] = gone[i] && a.elig[i];
   for (int variant = 0; variant < 2; ++variant) {
     bool flat_only = true;
     for (const Task& t : src[variant]) {
       if (t.phase == PH_ADA_FINAL && a.leaves[t.tensor]) continue;
       if ((t.phase == PH_ADA_APPLY || t.phase == PH_ADA_COUNT) && a.elig[t.tensor]) continue;
-      if (t.phase == PH_ADA_STATS && stats_dtype && stats_item_ok(pl, t)) continue;
+      if (t.phase == PH_ADA_STATS && gone[t.tensor]) continue;
       // what stays here is staged row by row: a tensor whose rows exceed a work item cannot stay
       if (t.phase != PH_ADA_FINAL && t.phase != PH_ADA_FLAT && pl->h_tensors[t.tensor].cols > CAP) a.long_rows_ok = false;
       if (t.phase == PH_ADA_FINAL && gone[t.tensor]) a.stats_first = true;

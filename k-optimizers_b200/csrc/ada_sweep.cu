@@ -552,11 +552,11 @@ int launch_count_apply(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cu
     va.task_counter = base.counters2 + 1;
     SweepKernel k = hp.has_wd && hp.cautious ? pick_sweep<false, true>(pl->param_dtype, pl->momentum_kind, muon, ms)
                                              : pick_sweep<false, false>(pl->param_dtype, pl->momentum_kind, muon, false);
-    KAON_CUDA(launch_early(!base.sm_reserve, k, grid, SWT, s, va, hp));
+    KAON_CUDA(launch_early(!base.sm_reserve, k, grid, SWT, 0, s, va, hp));
     pl->launches += 1;
   }
   va.task_counter = base.counters2 + 2;
-  KAON_CUDA(launch_early(!base.sm_reserve, pick_sweep<true, false>(pl->param_dtype, pl->momentum_kind, muon, ms), grid, SWT, s, va, hp));
+  KAON_CUDA(launch_early(!base.sm_reserve, pick_sweep<true, false>(pl->param_dtype, pl->momentum_kind, muon, ms), grid, SWT, 0, s, va, hp));
   pl->launches += 1;
   return KAON_OK;
 }

@@ -599,12 +599,12 @@ extern "C" int kaon_adamuon_step(kaon_plan* pl, const kaon_adamuon_hparams* h, v
   if (int rc = ensure_apply2(pl)) return rc;
   const bool three = pl->apply2 == 1;  // STATS/FINAL/FLAT here, COUNT and APPLY as launches of their own
   if (three) {
-    if (int rc = launch_statistics(pl, v, hp, s)) return rc;
+    if (int rc = launch_statistics(pl, v, hp, ada_stages(pl, hp.cautious), s)) return rc;
   } else {
     PlanView w = v;
     w.tasks = hp.cautious ? pl->d_tasks_full : pl->d_tasks_main;
     w.n_tasks = hp.cautious ? pl->n_tasks_full : pl->n_tasks_main;
-    if (int rc = launch_persistent(pl, w, hp, s)) return rc;
+    if (int rc = launch_persistent(pl, w, hp, false, s)) return rc;
   }
   if (int rc = launch_small(pl, v, hp, s)) return rc;
   if (three) {

@@ -710,14 +710,14 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
   begin[n] = slots;
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
-    std::vector<char> leaves(n, 0);   // tensors whose STATS and FINAL are launches of their own
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
     // STATS items the small-CTA launch can take go there, the others stay with FINAL in the persistent
     // kernel (which stages whole rows, so it cannot take rows longer than a work item)
-    const bool bf16 = pl->param_dtype == KAON_DT_BF16;
+    // (the tensors whose STATS and FINAL are launches of their own)
+    const std::vector<char> leaves = pl->param_dtype == KAON_DT_BF16 ? stats_tensors(pl, hm) : std::vector<char>(n, 0);
     for (const Task& t : hm) {
       if (t.phase == PH_ADA_STATS) {
-        if (bf16 && stats_item_ok(pl, t)) { stats.push_back(t); leaves[t.tensor] = 1; }
+        if (leaves[t.tensor]) stats.push_back(t);
         else if (pl->h_tensors[t.tensor].cols > CAP)
           return fail(KAON_E_UNSUPPORTED, "AdaPNM: tensor %d: rows longer than %d elements need bf16 weights and a row length that is a multiple of 8", t.tensor, CAP);
         else fin.push_back(t);
@@ -829,10 +829,9 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
     ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-    v.tasks = ph->d_final; v.n_tasks = ph->n_final;
-    if (int rc = launch_persistent(pl, v, ad, s)) return rc;
-    if (int rc = launch_stats(pl, pl->view, ad, ph->d_stats, ph->n_stats, runs_beside(ph->n_final, false, ph->n_stats, pl->sm_count), s)) return rc;
-    if (int rc = launch_final(pl, pl->view, ad, ph->d_strips, ph->n_strips, ph->n_final_items, s)) return rc;
+    const AdaStages st{ph->d_final, ph->n_final, runs_beside(ph->n_final, false, ph->n_stats, pl->sm_count), false, ph->d_stats, ph->n_stats,
+                       ph->d_strips, ph->n_strips, ph->n_final_items};
+    if (int rc = launch_statistics(pl, v, ad, st, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
     // 2-4. the two sweeps over the flat items
     const int grid = std::min(x.n_items, pl->sm_count * 8);

@@ -29,10 +29,11 @@ int check_device(const kaon_plan* pl);
 // each other, at its end.  Not with reserved multiprocessors (`early` false): its blocks would find room on those first, while
 // the others are full, and either sit there or, as they should, leave, all of them, with the work undone.
 template <typename... P, typename... A>
-cudaError_t launch_early(bool early, void (*kernel)(P...), int grid, int block, cudaStream_t s, const A&... args) {
+cudaError_t launch_early(bool early, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, const A&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

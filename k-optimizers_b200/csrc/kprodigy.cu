@@ -750,12 +750,12 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   std::stable_sort(units.begin(), units.end(), [](const Task& a, const Task& b) { return a.n > b.n; });
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
-    std::vector<char> leaves(n, 0);   // tensors whose STATS and FINAL are launches of their own
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
-    const bool bf16 = pl->param_dtype == KAON_DT_BF16;
+    // (the tensors whose STATS and FINAL are launches of their own)
+    const std::vector<char> leaves = pl->param_dtype == KAON_DT_BF16 ? stats_tensors(pl, hm) : std::vector<char>(n, 0);
     for (const Task& t : hm) {
       if (t.phase == PH_ADA_STATS) {
-        if (bf16 && stats_item_ok(pl, t)) { stats.push_back(t); leaves[t.tensor] = 1; }
+        if (leaves[t.tensor]) stats.push_back(t);
         else fin.push_back(t);
       } else if (t.phase == PH_ADA_FINAL && !leaves[t.tensor]) {
         fin.push_back(t);
@@ -847,10 +847,9 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
     ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-    v.tasks = kh->d_final; v.n_tasks = kh->n_final;
-    if (int rc = launch_persistent(pl, v, ad, s)) return rc;
-    if (int rc = launch_stats(pl, pl->view, ad, kh->d_stats, kh->n_stats, runs_beside(kh->n_final, false, kh->n_stats, pl->sm_count), s)) return rc;
-    if (int rc = launch_final(pl, pl->view, ad, kh->d_strips, kh->n_strips, kh->n_final_items, s)) return rc;
+    const AdaStages st{kh->d_final, kh->n_final, runs_beside(kh->n_final, false, kh->n_stats, pl->sm_count), false, kh->d_stats, kh->n_stats,
+                       kh->d_strips, kh->n_strips, kh->n_final_items};
+    if (int rc = launch_statistics(pl, v, ad, st, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;
   } else if (hp.gc && x.n_row_units > 0) {
     const int grid = std::min((x.n_row_units + KP_THREADS / 32 - 1) / (KP_THREADS / 32), pl->sm_count * 8);

@@ -58,6 +58,9 @@ int main(int argc, char** argv) {
       const bool sweep = (t.phase == PH_ADA_COUNT || t.phase == PH_ADA_APPLY) && a.elig[t.tensor];
       const bool final_launch = t.phase == PH_ADA_FINAL && a.leaves[t.tensor];
       if ((int)here + there + sweep + final_launch != 1) return 3;
+      if (final_launch)   // (that launch may run ahead of the persistent kernel)
+        for (const Task& k : src[v])
+          if (k.tensor == t.tensor && k.phase == PH_ADA_STATS && !stats.count(id(k))) return 8;
       if (!here) continue;
       flat_only = flat_only && t.phase == PH_ADA_FLAT;
       // a kept COUNT or APPLY waits for its FINAL, which has to be kept; a kept FINAL for its STATS, kept or launched before

@@ -2,6 +2,8 @@
 exactly two wide, a last strip of eight columns, one row beyond a run, fewer runs of rows than warps; int8 momentum over rows
 that are whole trips of a warp (their maxima wait for the row's end) and over rows that are not.  Two steps against the CPU
 oracle: statistics, scales and codes, weights."""
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -99,3 +101,15 @@ def test_a_row_whose_squares_overflow_has_an_infinite_statistic(name):
         assert np.array_equal(np.isinf(got), np.isinf(want[key])) and not np.isnan(got).any(), key
         fine = np.isfinite(want[key])
         assert np.abs(got[fine] - want[key][fine]).max(initial=0.0) <= 2e-6 * np.abs(want[key][fine]).max(initial=1e-30), key
+
+
+@pytest.mark.parametrize("name,kw", [
+    ("Adakaon", dict(momentum_dtype="int8")),
+    ("AdaPNM", dict(momentum_dtype="4bit")),
+    ("KProdigy", dict(second_moment="factored", cautious=True)),
+])
+def test_odd_tensors_beside_the_statistics_of_others(name, kw, monkeypatch):
+    """Rows that are no multiple of eight keep their stages in the persistent kernel, which runs at the same time as the STATS
+    launch of the other tensors."""
+    monkeypatch.setattr(sys.modules[__name__], "EDGES", [(333, 77), (640, 512), (160, 100), (257, 264), (300,)])
+    test_final_edges_vs_oracle(name, kw)
