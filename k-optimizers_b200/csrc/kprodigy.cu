@@ -151,9 +151,10 @@ __global__ void __launch_bounds__(KP_THREADS) kp_prep_kernel(PlanView pv, KpView
 // The sweeps over tensors whose rows (1-D tensors: whose length) are a multiple of eight elements, with 4-bit blocks of
 // 128 and every element on the slice: a warp per unit of up to 4096 elements, vector accesses without guards, nothing
 // shared between warps.  Bound by HBM where the state is wide (MODE 0 reads and writes 28 bytes an element with the
-// full second moment: 1243 us for 269 M elements with bf16 momentum, the row means in it, 6.0 TB/s; MODE 3 524 us).  The guarded form, a
+// full second moment: 1225-1258 us for 269 M elements with bf16 momentum, the means of half of its rows in it, 6.0-6.1 TB/s; MODE 3 521 us).  The guarded form, a
 // CTA per 16 K-element item, took 1976 and 1102 us.
-template <typename PT, int MK, int MODE>
+// ROWS (MODE 0): the build for lists with units of whole rows (the one loop for both cost lists without them 2 % of a step).
+template <typename PT, int MK, int MODE, bool ROWS>
 __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(const __grid_constant__ PlanView pv, const __grid_constant__ KpDev hp,
                                                                               const __grid_constant__ KpView x) {
   using E = Elems<PT>;
@@ -197,8 +198,9 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
     double acc_a = 0.0, acc_b = 0.0;
     f32x2 kept2 = pack2(0.0f, 0.0f);
     // Pass 1 with the full second moment takes the means of a unit of whole rows itself, row by row (the second reading of the
-    // gradient hits a cache: a launch of their own read all of it once more, 133 us on 269 M elements of bf16)
-    const bool own_mean = MODE == 0 && gc && !fac && t.phase == PH_KP_ROWS;
+    // gradient hits a cache: a launch of their own reads all of it once more, 133 us on 269 M elements of bf16, 45 on the rows it is
+    // left there)
+    const bool own_mean = ROWS && gc && !fac && t.phase == PH_KP_ROWS;
     float mu_row = 0.0f;
     auto trip = [&](const unsigned v, const bool act) {
       const unsigned o = act ? v : 0u;
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
         }
       }
     };
-    {
+    if constexpr (ROWS) {
       // (one place for the trip: it is long, and the compiler spills where it has it twice)
       const int seg = own_mean ? nv : nvec;
       for (int v0 = 0; v0 < nvec; v0 += seg) {
@@ -354,6 +356,14 @@ __global__ void __launch_bounds__(KP_THREADS, MODE == 0 ? 3 : 4) kp_warp_kernel(
         }
         if (own_mean) { ++row; cv = lane; }
       }
+    } else {
+      int v0 = 0;
+      for (; v0 + 32 <= nvec; v0 += 32) {
+        trip((unsigned)(v0 + lane), true);
+        row += adv_r; cv += adv_c;
+        if (cv >= nv) { cv -= nv; ++row; }
+      }
+      if (v0 < nvec) trip((unsigned)(v0 + lane), v0 + lane < nvec);
     }
     if constexpr (MODE == 0 || MODE == 2) {
       if (MODE == 2) acc_a = (double)(kept2.x + kept2.y);
@@ -641,20 +651,21 @@ struct KpHost {
   int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0;
   long long slice_p = 1;
   bool any_rows = false;     // a tensor of two dimensions or more
+  bool any_whole = false;    // units of whole rows
   std::vector<float> h_sums;
   int64_t bytes = 0;
 };
 
 typedef void (*KpSweep)(PlanView, KpDev, KpView);
 
-template <typename PT, int MODE>
+template <typename PT, int MODE, bool ROWS>
 static KpSweep pick_warp_pt(int mk) {
   switch (mk) {
-    case KAON_M_F32: return kp_warp_kernel<PT, KAON_M_F32, MODE>;
-    case KAON_M_BF16: return kp_warp_kernel<PT, KAON_M_BF16, MODE>;
-    case KAON_M_INT8: return kp_warp_kernel<PT, KAON_M_INT8, MODE>;
-    case KAON_M_4BIT: return kp_warp_kernel<PT, KAON_M_4BIT, MODE>;
-    case KAON_M_NONE: return kp_warp_kernel<PT, KAON_M_NONE, MODE>;
+    case KAON_M_F32: return kp_warp_kernel<PT, KAON_M_F32, MODE, ROWS>;
+    case KAON_M_BF16: return kp_warp_kernel<PT, KAON_M_BF16, MODE, ROWS>;
+    case KAON_M_INT8: return kp_warp_kernel<PT, KAON_M_INT8, MODE, ROWS>;
+    case KAON_M_4BIT: return kp_warp_kernel<PT, KAON_M_4BIT, MODE, ROWS>;
+    case KAON_M_NONE: return kp_warp_kernel<PT, KAON_M_NONE, MODE, ROWS>;
     default: return nullptr;
   }
 }
@@ -670,11 +681,11 @@ static KpSweep pick_sweep_pt(int mk) {
   }
 }
 // The sweep of a mode over the plan's units and items.
-template <int MODE>
+template <int MODE, bool ROWS = false>
 static int launch_sweep(kaon_plan* pl, const KpDev& hp, const KpView& x, cudaStream_t s) {
   const bool bf = pl->param_dtype == KAON_DT_BF16;
   const int mk = pl->momentum_kind;
-  KpSweep kw = bf ? pick_warp_pt<__nv_bfloat16, MODE>(mk) : pick_warp_pt<float, MODE>(mk);
+  KpSweep kw = bf ? pick_warp_pt<__nv_bfloat16, MODE, ROWS>(mk) : pick_warp_pt<float, MODE, ROWS>(mk);
   KpSweep ki = bf ? pick_sweep_pt<__nv_bfloat16, MODE>(mk) : pick_sweep_pt<float, MODE>(mk);
   if (!kw || !ki) return fail(KAON_E_INVALID, "no KProdigy kernel for this dtype combination");
   if (x.n_units > 0) {
@@ -725,13 +736,16 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
     if (((t.rows > 0 ? t.cols : t.numel) & 7) == 0 && (pl->momentum_kind != KAON_M_4BIT || t.bshift == 7) && slice_p == 1 &&
         (ptrs & 15) == 0) {
       // a warp's unit: small tensors in more pieces (the tensor alone decides, so the order of its sums stays); whole rows
-      // where rows are long beside their mean's latency and the tensor has warps enough of them (with rows from 256 elements on, a
-      // list of width 448 took 256 us a step for 250, and adapters of four rows of 1088 elements 111 for 108; 4-bit: and rows of
-      // whole blocks)
+      // where rows are long beside their mean's latency, the tensor has warps enough of them, and they fill seven eighths of a unit
+      // (with rows from 256 elements on, a list of width 448 took 256 us a step for 250, and adapters of four rows of 1088 elements
+      // 111 for 108; with units half empty by one row of 2304, or stretched by one of 5184, one of width 576 172 for 160, and width 768
+      // 747 for 732; where rows fill units, width 1024 1235 for 1247 and 176 for 191; 4-bit: and rows of whole blocks)
       long long u = 512;
       while (u < 4096 && u * 128 <= t.numel) u *= 2;
-      rowwise = t.numel >= (1ll << 19) && t.rows > 0 && t.cols >= 1024 && (pl->momentum_kind != KAON_M_4BIT || t.cols % 128 == 0);
-      if (rowwise) u = std::max<long long>(1, u / t.cols) * t.cols;
+      rowwise = t.numel >= (1ll << 19) && t.rows > 0 && t.cols >= 1024 && u / t.cols * t.cols * 8 >= u * 7 &&
+                (pl->momentum_kind != KAON_M_4BIT || t.cols % 128 == 0);
+      h->any_whole = h->any_whole || rowwise;
+      if (rowwise) u = u / t.cols * t.cols;
       for (long long e = 0; e < t.numel; e += u)
         units.push_back(Task{i, rowwise ? PH_KP_ROWS : PH_ADA_APPLY, e, (int)std::min<long long>(u, t.numel - e), t.rows > 0 ? (int)(e / t.cols) : 0, slots++,
                              t.rows > 0 ? (int)(e % t.cols) : 0});
@@ -746,8 +760,6 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
     }
   }
   begin[n] = slots;
-  // the long units first (rows of 11 520 elements at a list's end were a last wave of their own)
-  std::stable_sort(units.begin(), units.end(), [](const Task& a, const Task& b) { return a.n > b.n; });
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
@@ -862,7 +874,8 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
       kp_prep_kernel<<<pl->n_tensors, KP_THREADS, 0, s>>>(pl->view, x);
       pl->launches += 1;
     }
-    if (int rc = launch_sweep<0>(pl, hp, x, s)) return rc;
+    const bool rows = kh->any_whole && hp.gc && !hp.factored;   // units that take their means themselves
+    if (int rc = rows ? launch_sweep<0, true>(pl, hp, x, s) : launch_sweep<0>(pl, hp, x, s)) return rc;
     if (mk == KAON_M_INT8)
       if (int rc = launch_sweep<1>(pl, hp, x, s)) return rc;
     if (hp.do_d) {

@@ -200,9 +200,9 @@ def test_kprodigy_constructor_errors_and_resume():
         assert torch.equal(a.view(torch.int16), c.view(torch.int16))
 
 
-# rows of 1024 elements and more of tensors of 2^19 and more: units of several whole rows, which take their means themselves
-# (three rows, the last unit fewer; a row's last trip in part; one row a unit; 4-bit: rows of whole blocks only)
-ROWS = [(641, 1032), (514, 1280), (260, 2056), (515, 1024), (1280,)]
+# rows that fill a unit, of tensors of 2^19 elements and more: units of whole rows, which take their means themselves
+# (three or four rows, the last unit fewer; a row's last trip in part; one row a unit; 4-bit: rows of whole blocks only); and one that does not
+ROWS = [(641, 1200), (514, 1280), (140, 4032), (515, 1024), (260, 2056), (1280,)]
 
 
 @pytest.mark.parametrize("kw", [
