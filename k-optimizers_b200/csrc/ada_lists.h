@@ -32,11 +32,26 @@ inline std::vector<char> stats_tensors(const kaon_plan* pl, const std::vector<Ta
   return ok;
 }
 
-// Whether the persistent kernel's list of n items runs beside a STATS launch of n_stats: a few 1-D tensors, or any list where both
-// launches find room.  (Its blocks fill a multiprocessor each: beside a STATS that needs the whole machine, a list with
-// stages that wait for one another cost 40 us more than the two in turn, and the 540 1-D tensors of the 2.6 B list gained nothing.)
-inline bool runs_beside(int n, bool flat_only, int n_stats, int sms) {
-  return n > 0 && ((flat_only && n <= sms / 2) || n + n_stats / 4 <= sms);
+// The place of the persistent kernel's list among the STATS and FINAL launches of the tensors whose FINAL may leave: first, and beside
+// STATS; first; last, beginning while FINAL and the row table drain; or between STATS and FINAL, because its own FINAL items
+// wait for STATS items that left.
+enum : int { ADA_KEPT_BESIDE = 0, ADA_KEPT_FIRST = 1, ADA_KEPT_LAST = 2, ADA_KEPT_WAITS = 3 };
+
+// The place of a list of n items that waits for nothing of the others', beside n_stats STATS items and n_final FINAL items (strips of
+// FINAL_STRIP columns) of theirs; ADA_KEPT_WAITS: their FINAL had better stay in the list.  A block of the persistent kernel
+// fills a multiprocessor.  Us a step:
+// - beside STATS where both find room, or where 1-D tensors alone leave half the machine (AdaPNM, width-448 UNet: 252, as separate launches
+//   300; beside a STATS that needs the whole machine, 40 more than the two in turn);
+// - 1-D tensors alone, many: first (the 540 of the 2.6 B list gained nothing elsewhere);
+// - stages that wait for one another, with little else in STATS: last (Adakaon int8, ragged list: 76, first 95, FINAL kept 90);
+// - with STATS enough to fill half the machine, but few strips: FINAL kept, which such a list finds blocks for while it waits
+//   (Nekaon, forty pairs of rank 32 and width 1280: 173, last 226); with many strips last (120 pairs of rank 64 and width 1536: 455,
+//   FINAL kept 491).
+inline int kept_place(int n, bool flat_only, int n_stats, int n_final, int sms) {
+  if (n == 0) return ADA_KEPT_FIRST;
+  if ((flat_only && n <= sms / 2) || n + n_stats / 4 <= sms) return ADA_KEPT_BESIDE;
+  if (flat_only) return ADA_KEPT_FIRST;
+  return n_stats <= sms / 2 || n_final > 2 * sms ? ADA_KEPT_LAST : ADA_KEPT_WAITS;
 }
 
 struct AdaLists {
@@ -45,14 +60,13 @@ struct AdaLists {
   std::vector<char> leaves;       // and those of them whose FINAL is a launch, too
   std::vector<Task> stats;        // the STATS launch's items
   std::vector<Task> keep[2];      // the persistent kernel's: from the list without COUNT items, from the full list
-  bool stats_first = false;       // its FINAL items wait for items of the STATS launch, which then has to come before it
-  bool beside[2] = {false, false};  // the list may run beside the STATS launch
+  int order[2] = {ADA_KEPT_FIRST, ADA_KEPT_FIRST};   // and their place
   bool long_rows_ok = true;       // no tensor whose rows exceed a work item is left to it
 };
 
 // Per factored tensor: COUNT and APPLY leave the persistent kernel when its rows stream (a multiple of 8 elements; 4-bit
-// block 128), its STATS items when they qualify (stats_item_ok, bf16 gradients or AdaMuon's bf16 signal), and FINAL with both: a COUNT
-// that stays waits for its FINAL.  Everything else - the 1-D tensors, the stages of tensors that do not qualify - stays.
+// block 128), its STATS items when they qualify (stats_item_ok, bf16 gradients or AdaMuon's bf16 signal), and FINAL with both (a COUNT
+// that stays waits for its FINAL), unless it had better stay (kept_place).  Everything else - the 1-D tensors, the stages of tensors that do not qualify - stays.
 // `src`: the plan's list without COUNT items and its full one; `small`: the tensors one CTA steps on its own.
 inline AdaLists ada_lists(const kaon_plan* pl, const std::vector<Task>& small, const std::vector<Task> src[2]) {
   AdaLists a;
@@ -75,21 +89,32 @@ inline AdaLists ada_lists(const kaon_plan* pl, const std::vector<Task>& small, c
   for (const Task& t : src[0])
     if (t.phase == PH_ADA_STATS && gone[t.tensor]) a.stats.push_back(t);
   for (int i = 0; i < pl->n_tensors; ++i) a.leaves[i] = gone[i] && a.elig[i];
-  for (int variant = 0; variant < 2; ++variant) {
-    bool flat_only = true;
+  // the list a tensor's FINAL may leave, without what leaves in any case
+  auto stays = [&](const Task& t) {
+    return !((t.phase == PH_ADA_APPLY || t.phase == PH_ADA_COUNT) && a.elig[t.tensor]) && !(t.phase == PH_ADA_STATS && gone[t.tensor]);
+  };
+  {
+    int n = 0, n_final = 0;
+    bool flat_only = true, waits = false;
+    for (const Task& t : src[1]) {
+      if (!stays(t)) continue;
+      if (t.phase == PH_ADA_FINAL && a.leaves[t.tensor]) { ++n_final; continue; }
+      ++n;
+      flat_only = flat_only && t.phase == PH_ADA_FLAT;
+      waits = waits || (t.phase == PH_ADA_FINAL && gone[t.tensor]);
+    }
+    int place = kept_place(n, flat_only, (int)a.stats.size(), n_final, pl->sm_count);
+    if (place == ADA_KEPT_WAITS) a.leaves.assign((size_t)pl->n_tensors, 0);
+    if (waits) place = ADA_KEPT_WAITS;
+    a.order[0] = a.order[1] = place;
+  }
+  for (int variant = 0; variant < 2; ++variant)
     for (const Task& t : src[variant]) {
-      if (t.phase == PH_ADA_FINAL && a.leaves[t.tensor]) continue;
-      if ((t.phase == PH_ADA_APPLY || t.phase == PH_ADA_COUNT) && a.elig[t.tensor]) continue;
-      if (t.phase == PH_ADA_STATS && gone[t.tensor]) continue;
+      if (!stays(t) || (t.phase == PH_ADA_FINAL && a.leaves[t.tensor])) continue;
       // what stays here is staged row by row: a tensor whose rows exceed a work item cannot stay
       if (t.phase != PH_ADA_FINAL && t.phase != PH_ADA_FLAT && pl->h_tensors[t.tensor].cols > CAP) a.long_rows_ok = false;
-      if (t.phase == PH_ADA_FINAL && gone[t.tensor]) a.stats_first = true;
-      flat_only = flat_only && t.phase == PH_ADA_FLAT;
       a.keep[variant].push_back(t);
     }
-    a.beside[variant] = runs_beside((int)a.keep[variant].size(), flat_only, (int)a.stats.size(), pl->sm_count);
-  }
-  if (a.stats_first) a.beside[0] = a.beside[1] = false;
   return a;
 }
 

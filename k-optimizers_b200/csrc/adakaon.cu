@@ -872,62 +872,78 @@ __device__ void ada_final(const PlanView& pv, const AdaDev& hp, const Task& t, c
   const int C = d.cols, j0 = t.row0, nc = t.n;
   const float* part = pv.aux + d.aux_off;
   float* cfac = pv.aux + aux_cfac(d);
+  // The sums in the order of the FINAL launch (ada_final.cu: every eighth run, 128 columns, 256 threads), bit for bit: where a
+  // tensor's FINAL runs depends on the list it is in, what comes of it must not.
   double tl = 0.0;
-  for (int j = tid; j < nc; j += AT) {
+  if (tid < nc) {   // (a strip is a column a thread)
+    const int j = j0 + tid;
     double s1 = 0.0, s2 = 0.0;
-    auto add = [&](double a, float x) { return d.shift ? (double)((float)a + x) : a + (double)x; };   // (see warp_sum_d)
-    int s = 0;
-    for (; s + 8 <= d.n_stats; s += 8) {  // eight slots' loads in flight; the sums keep the slot order
-      float x1[8], x2[8];
+    if (d.shift != nullptr) {   // (see warp_sum_d)
+      float f1 = 0.0f, f2 = 0.0f;
+#pragma unroll 8
+      for (int s = 0; s < d.n_stats; ++s) {
+        f1 += __ldcg(part + 2ll * s * C + j);
+        f2 += __ldcg(part + 2ll * s * C + C + j);
+      }
+      s1 = (double)f1; s2 = (double)f2;
+    } else {
+      double a[8], b[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        x1[u] = __ldcg(part + 2ll * (s + u) * C + j0 + j);
-        x2[u] = __ldcg(part + 2ll * (s + u) * C + C + j0 + j);
+      for (int u = 0; u < 8; ++u) a[u] = b[u] = 0.0;
+      for (int s = 0; s < d.n_stats; s += 8) {   // eight slots' loads in flight
+        float x1[8], x2[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool in = s + u < d.n_stats;
+          x1[u] = in ? __ldcg(part + 2ll * (s + u) * C + j) : 0.0f;
+          x2[u] = in ? __ldcg(part + 2ll * (s + u) * C + C + j) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) { a[u] += (double)x1[u]; b[u] += (double)x2[u]; }
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) { s1 = add(s1, x1[u]); s2 = add(s2, x2[u]); }
-    }
-    for (; s < d.n_stats; ++s) {
-      s1 = add(s1, __ldcg(part + 2ll * s * C + j0 + j));
-      s2 = add(s2, __ldcg(part + 2ll * s * C + C + j0 + j));
+      for (int u = 0; u < 8; ++u) { s1 += a[u]; s2 += b[u]; }
     }
     const float mean = __fdiv_rn((float)s1, (float)d.rows);
-    const float cn = lerp_torch(d.stat_b[j0 + j], mean, hp.w2, hp.w2m1, hp.small_w2 != 0);
-    d.stat_b[j0 + j] = cn;
-    cfac[j0 + j] = rsqrt_torch(cn);
-    tl += s2 / (double)cn;
+    const float cn = lerp_torch(d.stat_b[j], mean, hp.w2, hp.w2m1, hp.small_w2 != 0);
+    d.stat_b[j] = cn;
+    cfac[j] = rsqrt_torch(cn);
+    tl = s2 / (double)cn;
   }
-  const double tot = block_sum_d(tl, sm.red, tid);
+  static_assert(FINAL_STRIP <= AT && FINAL_STRIP % 128 == 0, "a strip is a column a thread, and whole strips of the FINAL launch");
+  block_sum_d(tl, sm.red, tid);   // (leaves the warps' sums)
   double* tpart = reinterpret_cast<double*>(pv.aux + aux_tpart(d));
-  if (tid == 0) tpart[t.slot] = tot;
+  if (tid < FINAL_STRIP / 128 && tid * 128 < nc) {
+    double t4 = 0.0;
+    for (int w = 0; w < 4; ++w) t4 += sm.red[tid * 4 + w];
+    tpart[t.slot * (FINAL_STRIP / 128) + tid] = t4;
+  }
   __threadfence();
   __syncthreads();
   int last = 0;
   if (tid == 0) {
     unsigned old;
     asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(pv.done + 1 * pv.n_tensors + t.tensor) : "memory");
-    if (old == (unsigned)d.n_strips - 1u) {  // last strip: combine, in slot order
-      last = 1;
-      __threadfence();
-      const volatile double* rowpart = reinterpret_cast<const volatile double*>(pv.aux + aux_rowpart(d));
-      const volatile double* tp = tpart;
-      double rs = 0.0, T = 0.0;
-      for (int s = 0; s < d.n_stats; ++s) rs += rowpart[s];
-      for (int s = 0; s < d.n_strips; ++s) T += tp[s];
-      const float rowmean = __fdiv_rn((float)rs, (float)d.rows);
-      const double ss = (double)rowmean * T;
-      const float rms = __fdiv_rn((float)sqrt(ss), (float)sqrt((double)d.rows * (double)C));
-      float* scal = pv.aux + aux_scal(d);
-      scal[0] = rowmean;
-      scal[1] = fmaxf(__fdiv_rn(rms, hp.clip), 1.0f);
-      scal[2] = rms;
-      scal[3] = __fdiv_rn(1.0f, scal[1]);
-      sm.part_s[0] = rowmean;
-    }
+    last = old == (unsigned)d.n_strips - 1u;
+    if (last) __threadfence();
   }
   last = __syncthreads_or(last);
-  if (last) {  // the whole CTA: r_i of every row, then release COUNT / APPLY
-    const float rowmean = sm.part_s[0];
+  if (last) {  // the whole CTA: mean row statistic, clip divisor, r_i of every row, then release COUNT / APPLY
+    const double* rowpart = reinterpret_cast<const double*>(pv.aux + aux_rowpart(d));
+    double rs = 0.0, T = 0.0;
+    if (tid < 256) {
+      for (int s = tid; s < d.n_stats; s += 256) rs += __ldcg(rowpart + s);
+      for (int s = tid; s < (C + 127) / 128; s += 256) T += __ldcg(tpart + s);
+    }
+    rs = block_sum_d(rs, sm.red, tid);
+    T = block_sum_d(T, sm.red, tid);
+    const float rowmean = __fdiv_rn((float)rs, (float)d.rows);
+    if (tid == 0) {
+      const double ss = (double)rowmean * T;
+      const float rms = __fdiv_rn((float)sqrt(ss), (float)sqrt((double)d.rows * (double)C));
+      const float div = fmaxf(__fdiv_rn(rms, hp.clip), 1.0f);
+      *reinterpret_cast<float4*>(pv.aux + aux_scal(d)) = make_float4(rowmean, div, rms, __fdiv_rn(1.0f, div));
+    }
     float* rfac = pv.aux + aux_rfac(d);
     float4* rowtab = reinterpret_cast<float4*>(pv.aux + aux_rowtab(d));
     for (int r = tid; r < d.rows; r += AT) {
@@ -1775,10 +1791,9 @@ int ensure_apply2(kaon_plan* pl) {
     return cudaMemcpy(*dev, list.data(), sizeof(Task) * list.size(), cudaMemcpyHostToDevice);
   };
   pl->long_rows_ok = a.long_rows_ok;
-  pl->stats_first = a.stats_first;
   for (int variant = 0; variant < 2; ++variant) {
     KAON_CUDA(put(a.keep[variant], &pl->d_tasks_na[variant], &pl->n_tasks_na[variant]));
-    pl->na_beside[variant] = a.beside[variant];
+    pl->ada_order[variant] = a.order[variant];
   }
   KAON_CUDA(put(a.stats, &pl->d_tasks_stats, &pl->n_tasks_stats));
   final_items(pl, a.leaves, strips, pl->n_tasks_strips);
@@ -1818,28 +1833,29 @@ int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Ta
   return KAON_OK;
 }
 
-// The persistent kernel, STATS and FINAL over the lists of `st` (`base`: the plan's pointers).  A persistent list that may run beside
-// STATS goes first, one that waits for STATS items after it, and any other last, where it fills what FINAL and the row table,
-// which are short, leave of the machine.  (Ahead of STATS it left FINAL's launches a place of their own in the chain: the int8 step of a
-// ragged list took 95 us, 76 in this order, and 89-92 when FINAL was the persistent kernel's own.)
+// The persistent kernel, STATS and FINAL over the lists of `st`, in the order it names (`base`: the plan's pointers)
 int launch_statistics(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const AdaStages& st, cudaStream_t s) {
   PlanView v = base;
   v.tasks = st.keep;
   v.n_tasks = st.n_keep;
+  auto kept = [&](bool early) { return launch_persistent(pl, v, hp, early, s); };
   auto stats = [&](bool beside) { return launch_stats(pl, base, hp, st.stats, st.n_stats, beside, s); };
   auto final = [&]() { return launch_final(pl, base, hp, st.final, st.n_strips, st.n_final, s); };
-  if (st.beside) {
-    if (int rc = launch_persistent(pl, v, hp, false, s)) return rc;
-    if (int rc = stats(true)) return rc;
-    return final();
+  int rc = KAON_OK;
+  switch (st.order) {
+    case ADA_KEPT_BESIDE: case ADA_KEPT_FIRST:
+      if ((rc = kept(false))) return rc;
+      if ((rc = stats(st.order == ADA_KEPT_BESIDE))) return rc;
+      return final();
+    case ADA_KEPT_WAITS:
+      if ((rc = stats(false))) return rc;
+      if ((rc = kept(false))) return rc;
+      return final();
+    default:
+      if ((rc = stats(false))) return rc;
+      if ((rc = final())) return rc;
+      return kept(st.n_final > 0);
   }
-  if (int rc = stats(false)) return rc;
-  if (st.stats_first) {
-    if (int rc = launch_persistent(pl, v, hp, false, s)) return rc;
-    return final();
-  }
-  if (int rc = final()) return rc;
-  return launch_persistent(pl, v, hp, st.n_final > 0, s);
 }
 
 }  // namespace kaon

@@ -49,18 +49,18 @@ int launch_stats(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Ta
 void final_items(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out, int& n_strips);
 int launch_final(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const Task* items, int n_strips, int n, cudaStream_t s);
 
-// All of that over a plan's lists: the persistent kernel's, which may run `beside` STATS or, `stats_first`, waits for items of it; the STATS
-// launch's; the FINAL launch's strips and the row-table launch's runs
+// All of that over a plan's lists: the persistent kernel's and its place (ada_lists.h); the STATS launch's; the FINAL launch's
+// strips and the row-table launch's runs
 struct AdaStages {
   const Task* keep; int n_keep;
-  bool beside, stats_first;
+  int order;
   const Task* stats; int n_stats;
   const Task* final; int n_strips, n_final;
 };
 int launch_statistics(kaon_plan* pl, const PlanView& base, const AdaDev& hp, const AdaStages& st, cudaStream_t s);
 inline AdaStages ada_stages(const kaon_plan* pl, bool cautious) {   // (of a plan with apply2 == 1)
   const int i = cautious ? 1 : 0;
-  return AdaStages{pl->d_tasks_na[i], pl->n_tasks_na[i], pl->na_beside[i], pl->stats_first, pl->d_tasks_stats, pl->n_tasks_stats,
+  return AdaStages{pl->d_tasks_na[i], pl->n_tasks_na[i], pl->ada_order[i], pl->d_tasks_stats, pl->n_tasks_stats,
                    pl->d_tasks_final, pl->n_tasks_strips, pl->n_tasks_final};
 }
 

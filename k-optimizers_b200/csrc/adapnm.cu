@@ -626,7 +626,7 @@ struct PnmHost {
   Task* d_stats = nullptr;   // STATS items the launch of its own takes
   Task* d_final = nullptr;   // the other STATS items and the FINAL items, for the persistent kernel
   Task* d_strips = nullptr;  // and their FINAL strips and row-table runs
-  int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0;
+  int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0, order = ADA_KEPT_FIRST;
   bool attached = false;
   int64_t bytes = 0;
 };
@@ -713,17 +713,24 @@ static int pnm_build(kaon_plan* pl, const void* const* m_neg, float* const* m_ne
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
     // STATS items the small-CTA launch can take go there, the others stay with FINAL in the persistent
     // kernel (which stages whole rows, so it cannot take rows longer than a work item)
-    // (the tensors whose STATS and FINAL are launches of their own)
-    const std::vector<char> leaves = pl->param_dtype == KAON_DT_BF16 ? stats_tensors(pl, hm) : std::vector<char>(n, 0);
+    // the tensors whose STATS are a launch of their own, and their FINAL, unless it had better stay
+    std::vector<char> leaves = pl->param_dtype == KAON_DT_BF16 ? stats_tensors(pl, hm) : std::vector<char>(n, 0);
+    int n_final = 0;
     for (const Task& t : hm) {
       if (t.phase == PH_ADA_STATS) {
         if (leaves[t.tensor]) stats.push_back(t);
         else if (pl->h_tensors[t.tensor].cols > CAP)
           return fail(KAON_E_UNSUPPORTED, "AdaPNM: tensor %d: rows longer than %d elements need bf16 weights and a row length that is a multiple of 8", t.tensor, CAP);
         else fin.push_back(t);
-      } else if (t.phase == PH_ADA_FINAL && !leaves[t.tensor]) {
-        fin.push_back(t);
+      } else if (t.phase == PH_ADA_FINAL) {
+        if (leaves[t.tensor]) ++n_final;
+        else fin.push_back(t);
       }
+    }
+    h->order = kept_place((int)fin.size(), false, (int)stats.size(), n_final, pl->sm_count);
+    if (h->order == ADA_KEPT_WAITS) {
+      for (const Task& t : hm) if (t.phase == PH_ADA_FINAL && leaves[t.tensor]) fin.push_back(t);
+      leaves.assign(n, 0);
     }
     final_items(pl, leaves, strips, h->n_strips);
   }
@@ -829,7 +836,7 @@ extern "C" int kaon_adapnm_step(kaon_plan* pl, const kaon_adapnm_hparams* h, uin
     ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-    const AdaStages st{ph->d_final, ph->n_final, runs_beside(ph->n_final, false, ph->n_stats, pl->sm_count), false, ph->d_stats, ph->n_stats,
+    const AdaStages st{ph->d_final, ph->n_final, ph->order, ph->d_stats, ph->n_stats,
                        ph->d_strips, ph->n_strips, ph->n_final_items};
     if (int rc = launch_statistics(pl, v, ad, st, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;

@@ -169,8 +169,7 @@ struct kaon_plan {
   // the persistent kernel's lists beside those launches: [0] without COUNT items, [1] with them
   kaon::Task* d_tasks_na[2] = {nullptr, nullptr};
   int n_tasks_na[2] = {0, 0};
-  bool na_beside[2] = {false, false};        // the list may run beside the STATS launch
-  bool stats_first = false;                  // the lists wait for the STATS launch, which comes before them
+  int ada_order[2] = {0, 0};                 // and their place among STATS and FINAL (ada_lists.h)
   bool long_rows_ok = false;                 // every tensor whose rows exceed a work item left the persistent kernel
   kaon::Task* d_tasks_small = nullptr;       // factored tensors one CTA steps on its own
   int n_tasks_small = 0, small_max = 0;      // and the elements of the largest

@@ -648,7 +648,7 @@ struct KpHost {
   Task* d_stats = nullptr;   // STATS items the launch of its own takes
   Task* d_final = nullptr;
   Task* d_strips = nullptr;  // and their FINAL strips and row-table runs
-  int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0;
+  int n_stats = 0, n_final = 0, n_strips = 0, n_final_items = 0, order = ADA_KEPT_FIRST;
   long long slice_p = 1;
   bool any_rows = false;     // a tensor of two dimensions or more
   bool any_whole = false;    // units of whole rows
@@ -763,15 +763,22 @@ static int kp_build(kaon_plan* pl, float* const* s, const float* const* p0, long
   {
     std::vector<Task> hm((size_t)pl->n_tasks_main);
     KAON_CUDA(cudaMemcpy(hm.data(), pl->d_tasks_main, sizeof(Task) * hm.size(), cudaMemcpyDeviceToHost));
-    // (the tensors whose STATS and FINAL are launches of their own)
-    const std::vector<char> leaves = pl->param_dtype == KAON_DT_BF16 ? stats_tensors(pl, hm) : std::vector<char>(n, 0);
+    // the tensors whose STATS are a launch of their own, and their FINAL, unless it had better stay
+    std::vector<char> leaves = pl->param_dtype == KAON_DT_BF16 ? stats_tensors(pl, hm) : std::vector<char>(n, 0);
+    int n_final = 0;
     for (const Task& t : hm) {
       if (t.phase == PH_ADA_STATS) {
         if (leaves[t.tensor]) stats.push_back(t);
         else fin.push_back(t);
-      } else if (t.phase == PH_ADA_FINAL && !leaves[t.tensor]) {
-        fin.push_back(t);
+      } else if (t.phase == PH_ADA_FINAL) {
+        if (leaves[t.tensor]) ++n_final;
+        else fin.push_back(t);
       }
+    }
+    h->order = kept_place((int)fin.size(), false, (int)stats.size(), n_final, pl->sm_count);
+    if (h->order == ADA_KEPT_WAITS) {
+      for (const Task& t : hm) if (t.phase == PH_ADA_FINAL && leaves[t.tensor]) fin.push_back(t);
+      leaves.assign(n, 0);
     }
     final_items(pl, leaves, strips, h->n_strips);
   }
@@ -859,7 +866,7 @@ extern "C" int kaon_kprodigy_pass1(kaon_plan* pl, const kaon_kprodigy_pass1_hpar
     ada_finish(ad);
     PlanView v = pl->view;
     KAON_CUDA(cudaMemsetAsync(v.task_counter, 0, pl->counters_bytes - sizeof(unsigned), s));
-    const AdaStages st{kh->d_final, kh->n_final, runs_beside(kh->n_final, false, kh->n_stats, pl->sm_count), false, kh->d_stats, kh->n_stats,
+    const AdaStages st{kh->d_final, kh->n_final, kh->order, kh->d_stats, kh->n_stats,
                        kh->d_strips, kh->n_strips, kh->n_final_items};
     if (int rc = launch_statistics(pl, v, ad, st, s)) return rc;
     if (int rc = launch_small(pl, pl->view, ad, s)) return rc;

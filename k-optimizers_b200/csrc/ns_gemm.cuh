@@ -161,7 +161,7 @@ struct NsWork {
 // lanes at `tmem`.  A lane holds a row; rows go through the warp's 2 KB of shared memory (16-byte pieces, swizzled
 // against bank conflicts), so that global memory sees eight rows of 64 consecutive bytes an instruction: straight from the
 // lanes, 32 rows of 16 bytes, and of a symmetric product's mirror image 64 bytes, it was the epilogue that the tensor cores
-// waited for (DiT list of four blocks, all products: 9.2 -> 7.8 ms without its stores).
+// waited for (DiT list of four blocks, all products: 9.2 ms, and 7.6 without its stores).
 __device__ __forceinline__ void store_tile(const GemmParams& p, const uint32_t tmem, const unsigned row0, const int n0, const int half, const float alpha,
                                            const float beta, unsigned char* stage, const int lane) {
   const unsigned row = row0 + lane, M = p.M, N = p.N;

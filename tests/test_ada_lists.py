@@ -67,9 +67,8 @@ int main(int argc, char** argv) {
       if ((t.phase == PH_ADA_COUNT || t.phase == PH_ADA_APPLY) && !kept.count(Id(t.tensor, PH_ADA_FINAL, 0))) return 4;
       if (t.phase == PH_ADA_FINAL)
         for (const Task& k : src[v])
-          if (k.tensor == t.tensor && k.phase == PH_ADA_STATS && !kept.count(id(k)) && !a.stats_first) return 5;
+          if (k.tensor == t.tensor && k.phase == PH_ADA_STATS && !kept.count(id(k)) && a.order[v] != ADA_KEPT_WAITS) return 5;
     }
-    if (a.beside[v] && a.stats_first) return 6;
     if ((int)kept.size() != (int)a.keep[v].size()) return 7;
   }
   int stay = 0, out = 0, part = 0;
@@ -78,7 +77,7 @@ int main(int argc, char** argv) {
     else if (a.elig[i]) ++part;
     else ++stay;
   }
-  std::printf("%d %d %d %d\n", stay, out, part, (int)a.stats_first);
+  std::printf("%d %d %d %d\n", stay, out, part, (int)(a.order[1] == ADA_KEPT_WAITS));
   return 0;
 }
 """

@@ -113,3 +113,32 @@ def test_odd_tensors_beside_the_statistics_of_others(name, kw, monkeypatch):
     launch of the other tensors."""
     monkeypatch.setattr(sys.modules[__name__], "EDGES", [(333, 77), (640, 512), (160, 100), (257, 264), (300,)])
     test_final_edges_vs_oracle(name, kw)
+
+
+@pytest.mark.parametrize("name,kw", [
+    ("Adakaon", dict(momentum_dtype="int8")),
+    ("Adakaon", dict(bf16_method="kahan", weight_decay=0.1)),
+    ("AdaPNM", dict(momentum_dtype="4bit")),
+])
+def test_final_gives_the_same_bits_wherever_it_runs(name, kw):
+    """Three tensors by themselves, whose FINAL is a launch, and at the head of a list that keeps FINAL in the persistent kernel
+    (thirty tall matrices, whose stages stay there, beside STATS of twenty wide ones): statistics and weights of the three are the same."""
+    import kaon_b200
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    shapes = [(40, 1032), (640, 512), (1300, 264)] + [(1280, 32)] * 30 + [(32, 1280)] * 20
+    values = [((torch.randn(s, device="cuda", generator=gen) * 0.02).bfloat16(), (torch.randn(s, device="cuda", generator=gen) * 1e-3).bfloat16())
+              for s in shapes]
+    runs = []
+    for n in (3, len(shapes)):
+        params = [torch.nn.Parameter(v.clone()) for v, _ in values[:n]]
+        for p, (_, g) in zip(params, values):
+            p.grad = g.clone()
+        opt = getattr(kaon_b200, name)(params, lr=1e-3, **kw)
+        opt.sr_seed = 5
+        for _ in range(2):
+            opt.step()
+        torch.cuda.synchronize()
+        opt.check_device_status()
+        runs.append([t for p in params[:3] for t in (p.detach().view(torch.int16), opt.state[p]["row"], opt.state[p]["col"])])
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
