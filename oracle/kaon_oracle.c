@@ -1,7 +1,7 @@
 /*
  * kaon_oracle.c — CPU restatement of the kaon (Koronos/K-Optimizers 0.7.4) fused optimizer step.
  *
- * TEST INFRASTRUCTURE ONLY.  This file is the checker the CUDA kernels are compared against and the
+ * TEST INFRASTRUCTURE ONLY.  This file is what the CUDA kernels are compared against and the
  * timed CPU baseline.  Nothing in the shipped package may import, link or call it; the product path
  * has no CPU fallback and fails loudly when the CUDA library is missing.
  *

@@ -1,6 +1,6 @@
 """ctypes front end of the CPU oracle (oracle/kaon_oracle.c).
 
-TEST INFRASTRUCTURE ONLY: imported by tests/, by ``__graft_entry__.smoke()`` as the checker and by
+TEST INFRASTRUCTURE ONLY: imported by tests/, by ``__graft_entry__.smoke()`` and by
 ``bench.py``'s CPU-baseline legs.  The shipped package never imports this module.
 
 Arrays are numpy.  bf16 tensors travel as ``np.uint16`` bit patterns; fp32 as ``np.float32``.
