@@ -522,7 +522,8 @@ int launch_small(kaon_plan* pl, const PlanView& base, const AdaDev& hp, cudaStre
 // The units of the tensors marked in `elig`: as large as leaves each warp of the machine a dozen (a warp's time per
 // unit is then small beside the launch's), at most 8192 elements, where the fetches at a unit's head cost little.  AdaMuon's
 // chain is short (no momentum), so that a unit's head and its claim cost more beside it: three to a warp, at most 32 768 elements
-// (COUNT of four width-3072 blocks 617 -> 313 us; Nekaon's APPLY, on 269 M elements, 568 -> 625 with such units).
+// (COUNT of four width-3072 blocks 617 -> 313 us, 334 since it rounds as APPLY does; Nekaon's APPLY, on 269 M elements,
+// 568 -> 625 with such units).
 void sweep_units(const kaon_plan* pl, const std::vector<char>& elig, std::vector<Task>& out) {
   const bool muon = pl->optimizer == KAON_OPT_ADAMUON;
   long long total = 0;
